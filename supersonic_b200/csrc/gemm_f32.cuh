@@ -1,0 +1,417 @@
+// Float32 products C[m, n] (+)= sum_k A[m, k] W[n, k] whose operands can be fetched in 16-byte pieces.
+//
+// The sums are those of gemm_nt_plain_kernel bit for bit: 16 products a chunk, one FMA chain in k order, the chunks'
+// sums added in k order with compensation (Kahan).  Nothing here is re-associated, so a row's result does not depend on
+// which kernel took it, how many rows it came with or which tile it lay in.
+#pragma once
+#include "common.cuh"
+
+constexpr int GF_CHUNK = 16;               // products of one FMA chain
+constexpr int GF_LD = GF_CHUNK + 4;        // a chunk's place in shared memory: 80 bytes, so that eight neighbouring chunks
+                                           // (or rows) start in eight different groups of four banks
+
+__device__ __forceinline__ void gf_cp16(float* dst, const float* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void gf_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void gf_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// One compensated addition, its roundings written out: nothing is re-associated.
+__device__ __forceinline__ void gf_kahan(float& acc, float& lost, float part) {
+    const float y = __fsub_rn(part, lost);
+    const float t = __fadd_rn(acc, y);
+    lost = __fsub_rn(__fsub_rn(t, acc), y);
+    acc = t;
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Few rows (a decode step, a short prompt): the weights are streamed once per group of MB rows.  A block takes 8 R rows
+// of W and 512 columns a turn: a lane of the eight product warps makes the sum of one chunk of R rows of W with all MB rows
+// of A; the chunks' sums go through shared memory, two turns deep, to further warps whose threads add them in order, one
+// result each: 32 additions of four dependent steps a turn, which nobody else waits for.  W and A come by cp.async, STAGES
+// turns deep, in one stream over all the tiles that a block of the grid walks.
+// Bound by the weights' bytes at one row and by the shared-memory reads of the products from 8 on; the general kernel read
+// the weights again for every row and spent a dependent chain of 4 additions per 16 products in every thread.
+// Weights of 16384 x 2048 (134 MB), us: 1 row 270 on the general kernel and 36 here, 8 rows 270 and 54, 16 rows 270 and 91;
+// of 2048 x 8192, 2 rows 805 and 24.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int GF_PRODUCT_THREADS = 256;
+constexpr int GF_SKINNY_CHUNKS = 32;                                  // chunks a turn: one a lane
+__host__ __device__ constexpr int gf_adders(int mb, int r) { return (8 * r * mb + 31) / 32 * 32; }      // threads that add
+
+template <int MB, int R, int STAGES>
+constexpr size_t gf_skinny_smem() {
+    return sizeof(float) * ((size_t)STAGES * (8 * R + MB) * GF_SKINNY_CHUNKS * GF_LD + 2 * 8 * R * MB * (GF_SKINNY_CHUNKS + 1));
+}
+__device__ __forceinline__ void gf_bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+__device__ __forceinline__ void gf_bar_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+
+template <int MB, int R, int STAGES>
+__global__ void __launch_bounds__(GF_PRODUCT_THREADS + gf_adders(MB, R))
+gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C,
+                       int ldc, int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int m_groups,
+                       int accumulate) {
+    constexpr int NB = 8 * R, CH = GF_SKINNY_CHUNKS, TURN = CH * GF_CHUNK, PIECES = TURN / 4;
+    constexpr int ALL = GF_PRODUCT_THREADS + gf_adders(MB, R), SUMS = NB * MB * (CH + 1);
+    // named barriers: the product warps among themselves; a turn's sums are written; a turn's sums have been added (two each)
+    constexpr int BAR_PRODUCTS = 1, BAR_WRITTEN = 2, BAR_ADDED = 4;
+    extern __shared__ __align__(16) float gf_smem[];
+    float* w_s = gf_smem;                                             // [stage][row of W][chunk]
+    float* a_s = w_s + STAGES * NB * CH * GF_LD;                      // [stage][row of A][chunk]
+    float* sums = a_s + STAGES * MB * CH * GF_LD;                     // [2][row of W][row of A][chunk]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    A += (size_t)blockIdx.z * a_batch;
+    W += (size_t)blockIdx.z * w_batch;
+    C += (size_t)blockIdx.z * c_batch;
+    const int turns = (K + TURN - 1) / TURN, tiles = m_groups * ((N + NB - 1) / NB);
+    // this block's tiles, every gridDim.x-th (the groups of rows of A that share rows of W lie side by side), and their turns
+    const int total = ((tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * turns;
+    auto m_of = [&](int tile) { return tile % m_groups * MB; };
+    auto n_of = [&](int tile) { return tile / m_groups * NB; };
+
+    if (tid >= GF_PRODUCT_THREADS) {
+        const int o = tid - GF_PRODUCT_THREADS, n = o / MB, m = o % MB;
+        const bool mine = o < NB * MB;
+        float acc = 0.f, lost = 0.f;
+        int turn = 0, tile = blockIdx.x;
+        for (int g = 0; g < total; ++g) {
+            const int buf = g & 1;
+            gf_bar_sync(BAR_WRITTEN + buf, ALL);
+            if (mine) {
+                const int n_chunks = min(CH, (K - turn * TURN + GF_CHUNK - 1) / GF_CHUNK);
+                const float* sp = sums + buf * SUMS + o * (CH + 1);
+                if (n_chunks == CH) {
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) gf_kahan(acc, lost, sp[c]);
+                } else {
+                    for (int c = 0; c < n_chunks; ++c) gf_kahan(acc, lost, sp[c]);
+                }
+            }
+            __syncwarp();
+            if (g + 2 < total) gf_bar_arrive(BAR_ADDED + buf, ALL);
+            if (++turn == turns) {                                    // the tile's last turn
+                const int row = m_of(tile) + m, col = n_of(tile) + n;
+                if (mine && row < M && col < N) {
+                    float* dst = C + (size_t)row * ldc + col;
+                    *dst = accumulate ? *dst + acc : acc;
+                }
+                acc = lost = 0.f;
+                turn = 0;
+                tile += gridDim.x;
+            }
+        }
+        return;
+    }
+    // what lies outside the operands arrives as zeros (a copy of no bytes)
+    int ahead_turn = 0, ahead_tile = blockIdx.x;                      // of the next load
+    auto load = [&](int s) {
+        const int k0 = ahead_turn * TURN, m0 = m_of(ahead_tile), n0 = n_of(ahead_tile);
+        const int m_here = M - m0, n_here = N - n0;
+        const float* At = A + (size_t)m0 * lda;
+        const float* Wt = W + (size_t)n0 * ldw;
+#pragma unroll
+        for (int e = 0; e < NB * PIECES / GF_PRODUCT_THREADS; ++e) {
+            const int p = tid + e * GF_PRODUCT_THREADS, r = p / PIECES, c = p % PIECES, k = k0 + c * 4;
+            const bool in = r < n_here && k < K;
+            gf_cp16(w_s + ((s * NB + r) * CH + c / 4) * GF_LD + (c % 4) * 4, in ? Wt + (size_t)r * ldw + k : W, in ? 16 : 0);
+        }
+#pragma unroll
+        for (int e = 0; e < (MB * PIECES + GF_PRODUCT_THREADS - 1) / GF_PRODUCT_THREADS; ++e) {
+            const int p = tid + e * GF_PRODUCT_THREADS, r = p / PIECES, c = p % PIECES, k = k0 + c * 4;
+            const bool in = r < m_here && k < K;
+            if (MB * PIECES % GF_PRODUCT_THREADS == 0 || p < MB * PIECES)
+                gf_cp16(a_s + ((s * MB + r) * CH + c / 4) * GF_LD + (c % 4) * 4, in ? At + (size_t)r * lda + k : A, in ? 16 : 0);
+        }
+        if (++ahead_turn == turns) { ahead_turn = 0; ahead_tile += gridDim.x; }
+    };
+#pragma unroll
+    for (int t = 0; t < STAGES - 1; ++t) {
+        if (t < total) load(t);
+        gf_commit();
+    }
+    for (int g = 0; g < total; ++g) {
+        const int buf = g & 1;
+        gf_wait<STAGES - 2>();
+        gf_bar_sync(BAR_PRODUCTS, GF_PRODUCT_THREADS);                // the turn has landed; everyone is done with the one before
+        if (g + STAGES - 1 < total) load((g + STAGES - 1) % STAGES);
+        gf_commit();
+        const int s = g % STAGES;
+        const float* wp = w_s + ((s * NB + warp * R) * CH + lane) * GF_LD;
+        const float* ap = a_s + (s * MB * CH + lane) * GF_LD;
+        float part[R][MB];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int m = 0; m < MB; ++m) part[r][m] = 0.f;
+#pragma unroll
+        for (int q = 0; q < GF_CHUNK / 4; ++q) {
+            float4 w[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) w[r] = *reinterpret_cast<const float4*>(wp + r * CH * GF_LD + q * 4);
+#pragma unroll
+            for (int m = 0; m < MB; ++m) {
+                const float4 a = *reinterpret_cast<const float4*>(ap + m * CH * GF_LD + q * 4);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    part[r][m] = fmaf(a.x, w[r].x, part[r][m]);
+                    part[r][m] = fmaf(a.y, w[r].y, part[r][m]);
+                    part[r][m] = fmaf(a.z, w[r].z, part[r][m]);
+                    part[r][m] = fmaf(a.w, w[r].w, part[r][m]);
+                }
+            }
+        }
+        if (g >= 2) gf_bar_sync(BAR_ADDED + buf, ALL);                // the sums of two turns ago have been added
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int m = 0; m < MB; ++m) sums[buf * SUMS + ((warp * R + r) * MB + m) * (CH + 1) + lane] = part[r][m];
+        gf_bar_arrive(BAR_WRITTEN + buf, ALL);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Many rows (a prompt): tiles of 64 x 64 to 128 x 128, 4 x 4 to 8 x 8 results a thread, one chunk of k a turn.  A chunk comes
+// by cp.async as it lies in memory, GF_RAW deep, and is turned k-major in shared memory on the way to its two buffers, so that
+// a thread reads four neighbouring columns at a time and the multiply-adds go two columns an instruction (fma.rn.f32x2: each
+// half rounds as the scalar one does).  Bound by the FP32 pipes: a chunk's 16 multiply-adds of a result are followed by the
+// four steps of its compensated addition, so 4/5 of the peak is what this sum leaves.
+// 1000 rows, us on the general kernel and here: 2048 x 2048 504 and 291, 3072 x 2048 746 and 483, 16384 x 2048 3563 and 2003
+// (33.5 TFLOP/s), 2048 x 8192 2033 and 1145.
+// ---------------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long gf_twice(float x) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ unsigned long long gf_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long gf_add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Two compensated additions; `kept` is what the last ones rounded away, with the sign it is added back with.
+__device__ __forceinline__ void gf_kahan2(unsigned long long& acc, unsigned long long& kept, unsigned long long part,
+                                          unsigned long long minus_one) {
+    const unsigned long long y = gf_add2(part, kept);
+    const unsigned long long t = gf_add2(acc, y);
+    kept = gf_add2(y, gf_fma2(t, minus_one, acc));
+    acc = t;
+}
+
+constexpr int GF_TILE_THREADS = 256, GF_RAW = 3;                     // GF_RAW: chunks on their way from memory, and at work
+
+template <int RM, int RN>
+constexpr size_t gf_tile_smem() { return sizeof(float) * (size_t)(2 + GF_RAW) * GF_CHUNK * 16 * (RM + RN); }
+
+template <int RM, int RN, int MIN_BLOCKS>                             // results a thread; tiles of 16 RM x 16 RN
+__global__ void __launch_bounds__(GF_TILE_THREADS, MIN_BLOCKS)
+gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C,
+                     int ldc, int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int accumulate) {
+    constexpr int TM = 16 * RM, TN = 16 * RN, PA = TM / 64, PW = TN / 64;     // PA, PW: 16-byte pieces of A and W a thread fetches
+    extern __shared__ __align__(16) float gf_smem[];
+    float (*a_s)[GF_CHUNK][TM] = reinterpret_cast<float (*)[GF_CHUNK][TM]>(gf_smem);                       // [2]: a chunk, k-major
+    float (*w_s)[GF_CHUNK][TN] = reinterpret_cast<float (*)[GF_CHUNK][TN]>(gf_smem + 2 * GF_CHUNK * TM);   // [2]
+    float4* raw = reinterpret_cast<float4*>(gf_smem + 2 * GF_CHUNK * (TM + TN));       // [GF_RAW][piece][thread]: as it lay
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = lane % 8 + 8 * (warp % 2), ty = lane / 8 + 4 * (warp / 2);    // columns 4 tx .. + 3 (and + 64); rows likewise
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+    A += (size_t)blockIdx.z * a_batch + (size_t)m0 * lda;
+    W += (size_t)blockIdx.z * w_batch + (size_t)n0 * ldw;
+    C += (size_t)blockIdx.z * c_batch;
+    const int m_here = min(TM, M - m0), n_here = min(TN, N - n0);
+    const int turns = (K + GF_CHUNK - 1) / GF_CHUNK;
+    // a thread's pieces: neighbouring k of one row of A and of one of W
+    const int a_row = tid % TM, a_k = tid / TM * 4 * PA, w_row = tid % TN, w_k = tid / TN * 4 * PW;
+    const bool a_in = a_row < m_here, w_in = w_row < n_here;
+    const float* a_src = A + (size_t)(a_in ? a_row : 0) * lda + a_k;
+    const float* w_src = W + (size_t)(w_in ? w_row : 0) * ldw + w_k;
+    auto fetch = [&](int turn) {
+        float4* dst = raw + (turn % GF_RAW) * (PA + PW) * GF_TILE_THREADS + tid;
+        const int k = turn * GF_CHUNK;
+#pragma unroll
+        for (int e = 0; e < PA; ++e) {
+            const bool in = a_in && k + a_k + 4 * e < K;
+            gf_cp16(reinterpret_cast<float*>(dst + e * GF_TILE_THREADS), in ? a_src + k + 4 * e : A, in ? 16 : 0);
+        }
+#pragma unroll
+        for (int e = 0; e < PW; ++e) {
+            const bool in = w_in && k + w_k + 4 * e < K;
+            gf_cp16(reinterpret_cast<float*>(dst + (PA + e) * GF_TILE_THREADS), in ? w_src + k + 4 * e : W, in ? 16 : 0);
+        }
+    };
+    // k-major: a thread turns over what it fetched itself, so its own wait is all that comes between
+    auto stage = [&](int turn) {
+        const float4* src = raw + (turn % GF_RAW) * (PA + PW) * GF_TILE_THREADS + tid;
+#pragma unroll
+        for (int e = 0; e < PA; ++e) {
+            const float4 x = src[e * GF_TILE_THREADS];
+            float* dst = &a_s[turn & 1][a_k + 4 * e][a_row];
+            dst[0] = x.x; dst[TM] = x.y; dst[2 * TM] = x.z; dst[3 * TM] = x.w;
+        }
+#pragma unroll
+        for (int e = 0; e < PW; ++e) {
+            const float4 x = src[(PA + e) * GF_TILE_THREADS];
+            float* dst = &w_s[turn & 1][w_k + 4 * e][w_row];
+            dst[0] = x.x; dst[TN] = x.y; dst[2 * TN] = x.z; dst[3 * TN] = x.w;
+        }
+    };
+    unsigned long long acc[RM][RN / 2], kept[RM][RN / 2];             // two columns each
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN / 2; ++j) { acc[i][j] = 0ull; kept[i][j] = 0ull; }
+    const unsigned long long minus_one = gf_twice(-1.0f);
+#pragma unroll
+    for (int t = 0; t < GF_RAW - 1; ++t) {
+        if (t < turns) fetch(t);
+        gf_commit();
+    }
+    gf_wait<GF_RAW - 2>();
+    stage(0);
+    __syncthreads();
+    for (int turn = 0; turn < turns; ++turn) {
+        if (turn + GF_RAW - 1 < turns) fetch(turn + GF_RAW - 1);
+        gf_commit();
+        const float (*ab)[TM] = a_s[turn & 1];
+        const float (*wb)[TN] = w_s[turn & 1];
+        unsigned long long part[RM][RN / 2];
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN / 2; ++j) part[i][j] = 0ull;
+#pragma unroll
+        for (int k = 0; k < GF_CHUNK; ++k) {
+            float a[RM];
+            unsigned long long w[RN / 2];
+#pragma unroll
+            for (int g = 0; g < RM / 4; ++g) {
+                const float4 x = *reinterpret_cast<const float4*>(&ab[k][64 * g + 4 * ty]);
+                a[4 * g] = x.x; a[4 * g + 1] = x.y; a[4 * g + 2] = x.z; a[4 * g + 3] = x.w;
+            }
+#pragma unroll
+            for (int g = 0; g < RN / 4; ++g) {
+                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&wb[k][64 * g + 4 * tx]);
+                w[2 * g] = x.x; w[2 * g + 1] = x.y;
+            }
+#pragma unroll
+            for (int i = 0; i < RM; ++i) {
+                const unsigned long long aa = gf_twice(a[i]);
+#pragma unroll
+                for (int j = 0; j < RN / 2; ++j) part[i][j] = gf_fma2(aa, w[j], part[i][j]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN / 2; ++j) gf_kahan2(acc[i][j], kept[i][j], part[i][j], minus_one);
+        gf_wait<GF_RAW - 2>();
+        if (turn + 1 < turns) stage(turn + 1);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+        const int m = 64 * (i / 4) + 4 * ty + i % 4;
+        if (m >= m_here) continue;
+#pragma unroll
+        for (int j = 0; j < RN / 2; ++j) {
+            const int n = 64 * (j / 2) + 4 * tx + 2 * (j % 2);
+            float* dst = C + (size_t)(m0 + m) * ldc + n0 + n;
+            const float lo = __uint_as_float((unsigned)acc[i][j]), hi = __uint_as_float((unsigned)(acc[i][j] >> 32));
+            if (n < n_here) dst[0] = accumulate ? dst[0] + lo : lo;
+            if (n + 1 < n_here) dst[1] = accumulate ? dst[1] + hi : hi;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Whether the operands can be fetched in 16-byte pieces (rows of W and A start on 16-byte boundaries, K in whole pieces).
+static inline bool gemm_f32_ok(const void* A, int lda, long long a_batch, const void* W, int ldw, long long w_batch, int K) {
+    return !(((uintptr_t)A | (uintptr_t)W) & 15) && !((lda | ldw | K) & 3) && !((a_batch | w_batch) & 3);
+}
+
+static inline int gf_sms() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
+        sms = n;
+    }
+    return sms;
+}
+
+// Which kernel takes a product: up to 16 rows, the one that streams the weights once for all of them.  Above, whichever is
+// done first by the time a chunk of 16 k takes it: the blocks run in waves over the SMs, and tiles that are too large leave
+// SMs idle where tiles that are too small fetch more often than they multiply.  Microseconds a chunk, measured for 1 and
+// for each further wave: 16 rows x 16 columns a block 0.13 + 0.10; tiles of 64 x 64 0.90 + 0.60, of 128 x 64 1.45 + 1.15,
+// of 128 x 128 2.24 + 2.24.  Sides of the lines it draws (us): 128 x 2048 x 2048 (rows, columns, k) 89 with 16 rows and
+// 116 with tiles of 64; 100 x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072 186 with 128 x 64, 192 with 64 x 64;
+// 1000 x 2048 291 with 128 x 128, 321 with 128 x 64.
+static inline int gemm_f32_form(int n_batch, int M, int N) {
+    if (M <= 16) return M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
+    const long long sms = gf_sms();
+    const auto waves = [&](int rows, int cols) {
+        return ((long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * n_batch + sms - 1) / sms;
+    };
+    const int forms[4] = {16, 100, 101, 102};
+    const long long cost[4] = {3 + 10 * waves(16, 16), 30 + 60 * waves(64, 64), 30 + 115 * waves(128, 64), 224 * waves(128, 128)};
+    int best = 0;
+    for (int f = 1; f < 4; ++f)
+        if (cost[f] < cost[best]) best = f;
+    return forms[best];
+}
+
+// form 0: chosen by the sizes; else one of the kernels: 1, 2, 4, 8, 16 (few rows, that many a group), 100, 101, 102 (tiles of
+// 64 x 64, 128 x 64 and 128 x 128)
+static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, const float* W, int ldw, long long w_batch,
+                                  float* C, int ldc, long long c_batch, int n_batch, int M, int N, int K, int accumulate,
+                                  int form, cudaStream_t stream) {
+    if (form == 0) form = gemm_f32_form(n_batch, M, N);
+#define GF_CONFIGURE(kernel, smem) do { \
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)); \
+        if (e != cudaSuccess) return (int)e; \
+    } while (0)
+#define GF_SKINNY(MB, R, STAGES) do { \
+        constexpr size_t smem = gf_skinny_smem<MB, R, STAGES>(); \
+        auto kernel = gemm_f32_skinny_kernel<MB, R, STAGES>; \
+        GF_CONFIGURE(kernel, smem); \
+        const int groups = (M + MB - 1) / MB; \
+        const long long tiles = (long long)groups * ((N + 8 * R - 1) / (8 * R)); \
+        if (tiles > 0x7fffffffLL) return SSB_ERR_BAD_SIZE; \
+        /* as many blocks as are resident at once (by shared memory), each walking its share of the tiles; a block a tile */ \
+        /* for one or two rows, whose turns are so short that a block's last additions are better hidden by the next block */ \
+        /* (2048 x 16384, us: one row 36.4 with a block a tile and 40.6 walking, 8 rows 60.5 and 53.9) */ \
+        const long long held = MB <= 2 ? tiles : gf_sms() * (228 * 1024 / (long long)(smem + 1024)); \
+        const long long blocks = tiles < held ? tiles : held; \
+        kernel<<<dim3((unsigned)blocks, 1, n_batch), GF_PRODUCT_THREADS + gf_adders(MB, R), smem, stream>>>( \
+            A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, groups, accumulate); \
+    } while (0)
+#define GF_TILES(RM, RN, MINB) do { \
+        constexpr size_t smem = gf_tile_smem<RM, RN>(); \
+        auto kernel = gemm_f32_tile_kernel<RM, RN, MINB>; \
+        GF_CONFIGURE(kernel, smem); \
+        const int rows = 16 * RM, cols = 16 * RN; \
+        if ((M + rows - 1) / rows > 65535) return SSB_ERR_BAD_SIZE; \
+        kernel<<<dim3((N + cols - 1) / cols, (M + rows - 1) / rows, n_batch), GF_TILE_THREADS, smem, stream>>>( \
+            A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
+    } while (0)
+    switch (form) {
+        case 1: GF_SKINNY(1, 1, 4); break;
+        case 2: GF_SKINNY(2, 1, 4); break;
+        case 4: GF_SKINNY(4, 1, 3); break;
+        case 8: GF_SKINNY(8, 2, 3); break;
+        case 16: GF_SKINNY(16, 2, 2); break;
+        case 100: GF_TILES(4, 4, 3); break;
+        case 101: GF_TILES(8, 4, 2); break;
+        case 102: GF_TILES(8, 8, 1); break;
+        default: return SSB_ERR_BAD_SIZE;
+    }
+#undef GF_SKINNY
+#undef GF_TILES
+#undef GF_CONFIGURE
+    return ssb_launch_status();
+}

@@ -14,6 +14,7 @@
 //   swiglu      kernels/full_attention_cuda.cuh:1995-2010
 //   argmax      kernels/prefill_helpers_bridge_cuda.cu:247-287 (lowest index wins ties)
 #include "common.cuh"
+#include "gemm_f32.cuh"
 #include <math.h>
 
 typedef __nv_bfloat16 bf16;
@@ -241,6 +242,10 @@ static int gemm_nt_plain_launch(const void* A, int lda, long long a_batch, const
     if (M <= 0 || N <= 0 || n_batch <= 0) return 0;
     if (K <= 0 || n_batch > 65535) return SSB_ERR_BAD_SIZE;
     if (accumulate && out_dtype != SSB_F32) return SSB_ERR_BAD_DTYPE;
+    // float32 operands in whole 16-byte pieces: the same sums, bit for bit, from kernels made for their number of rows
+    if (in_dtype == SSB_F32 && out_dtype == SSB_F32 && gemm_f32_ok(A, lda, a_batch, W, ldw, w_batch, K))
+        return gemm_f32_launch((const float*)A, lda, a_batch, (const float*)W, ldw, w_batch, (float*)C, ldc, c_batch, n_batch,
+                               M, N, K, accumulate, 0, stream);
     dim3 grid((N + 63) / 64, (M + 63) / 64, n_batch);
 #define SSB_GEMM(TA, TC, ACC) \
     gemm_nt_plain_kernel<TA, TC, ACC><<<grid, 256, 0, stream>>>( \
