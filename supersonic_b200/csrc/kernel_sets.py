@@ -59,6 +59,8 @@ class PlainKernels:
                             # dependent kernel become resident while a long kernel before it still runs, and a prompt of
                             # 2,048 tokens whose recurrences take a millisecond each ran 8.1 ms chained and 5.1 ms unchained
 
+    F32_PROMPT_MIN_NEW = 8  # new tokens of a float32 prompt from which 64 (token, head) rows of a kv head share a block
+
     def _chain(self, rows) -> bool:
         return bool(self.pdl) and int(rows) <= self.PDL_MAX_ROWS
 
@@ -145,6 +147,12 @@ class PlainKernels:
 
     def attention(self, q, k_cache, v_cache, batch, page_table, out, n_q, n_kv, head_dim, page_shift,
                   window: Optional[int], scale: float):
+        # a float32 prompt: 64 (token, head) rows share the fetch of a key, the same sums in the same order
+        if not window and not batch.is_decode and batch.max_new >= self.F32_PROMPT_MIN_NEW \
+                and ops.attention_f32_prompt_ok(q, k_cache, v_cache, out, head_dim):
+            ops.attention_f32_prompt(q, k_cache, v_cache, batch.cu_new, batch.seq_start, batch.seq_slot, page_table, out,
+                                     batch.max_new, n_q, n_kv, head_dim, page_shift, scale)
+            return
         ops.attention_plain(q, k_cache, v_cache, batch.pos, batch.slot_of_token, page_table, out,
                             n_q, n_kv, head_dim, page_shift, window, scale)
 

@@ -218,6 +218,33 @@ def attention_plain(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
         _stream()), "attention_plain")
 
 
+def attention_f32_prompt_ok(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,
+                            head_dim: int) -> bool:
+    """Whether ``attention_f32_prompt`` takes these: float32 rows and caches in whole 16-byte pieces."""
+    return (q.dtype == torch.float32 and head_dim in (64, 128) and k_cache.is_contiguous() and v_cache.is_contiguous()
+            and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, out)))
+
+
+def attention_f32_prompt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, cu_new: torch.Tensor,
+                         seq_start: torch.Tensor, seq_slot: torch.Tensor, page_table: torch.Tensor, out: torch.Tensor,
+                         max_new: int, n_q: int, n_kv: int, head_dim: int, page_shift: int, scale: float) -> None:
+    """``attention_plain`` (no window, no sinks, values as wide as keys) for a step's float32 prompts: the same bits."""
+    _need(q, "q", torch.float32, 2); _need(out, "out", torch.float32, 2)
+    _need(k_cache, "k_cache", torch.float32); _need(v_cache, "v_cache", torch.float32)
+    for t, name in ((cu_new, "cu_new"), (seq_start, "seq_start"), (seq_slot, "seq_slot")):
+        _need(t, name, torch.int32, 1)
+    _need(page_table, "page_table", torch.int32, 2)
+    n_seqs = seq_slot.shape[0]
+    if cu_new.shape[0] != n_seqs + 1 or seq_start.shape[0] != n_seqs or out.shape[0] != q.shape[0] \
+            or out.shape[1] < n_q * head_dim or q.shape[1] < n_q * head_dim or n_q % n_kv:
+        raise KernelError("attention_f32_prompt: shapes")
+    _check(_fn("plain_ops", "ssb_attention_f32_prompt")(
+        _ptr(q), c_int(q.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(cu_new), _ptr(seq_start), _ptr(seq_slot),
+        _ptr(page_table), c_int(page_table.shape[1]), _ptr(out), c_int(out.stride(0)), c_int(n_seqs), c_int(max_new),
+        c_int(n_q), c_int(n_kv), c_int(head_dim), c_int(page_shift), c_float(scale), _stream()), "attention_f32_prompt")
+
+
 def swiglu(gate_up: torch.Tensor, out: torch.Tensor, interleaved: bool = False) -> None:
     """out[t, c] = silu(gate[t, c]) * up[t, c]; gate and up are the halves of a row of
     ``gate_up``, or (interleaved) alternate as [8 gate | 8 up] per 16 columns."""

@@ -15,6 +15,7 @@
 //   argmax      kernels/prefill_helpers_bridge_cuda.cu:247-287 (lowest index wins ties)
 #include "common.cuh"
 #include "gemm_f32.cuh"
+#include "attention_f32.cuh"
 #include <math.h>
 
 typedef __nv_bfloat16 bf16;
@@ -380,10 +381,11 @@ attention_plain_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ k
                        const int* __restrict__ slot, const int* __restrict__ page_table, int max_pages,
                        T* __restrict__ out, int ldo, int n_q, int n_kv, int head_dim, int page_shift,
                        int window, float scale, int v_dim, int v_row, const float* __restrict__ sinks) {
-    __shared__ float q_s[ATT_MAX_HEAD_DIM];
+    __shared__ __align__(16) float q_s[ATT_MAX_HEAD_DIM];
     __shared__ float p_s[ATT_THREADS];
     __shared__ float red[ATT_THREADS];
     const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+    const bool pieces = sizeof(T) == 4 && head_dim % 4 == 0 && ((uintptr_t)k_cache & 15) == 0;
     T* o = out + (size_t)t * ldo + (size_t)h * v_dim;
     const int s = slot[t];
     if (s < 0) {
@@ -408,7 +410,19 @@ attention_plain_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ k
         if (j <= p) {
             const T* kr = k_cache + ssb_cache_row(page_table, max_pages, s, j, page_shift, n_kv, kvh, head_dim);
             float dot = 0.f;
-            for (int d = 0; d < head_dim; ++d) dot = fmaf(q_s[d], ssb_to_float(kr[d]), dot);
+            if (pieces) {                                // the same chain, four elements a load
+#pragma unroll 4
+                for (int d = 0; d < head_dim; d += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(kr) + d);
+                    const float4 q4 = *reinterpret_cast<const float4*>(q_s + d);
+                    dot = fmaf(q4.x, k4.x, dot);
+                    dot = fmaf(q4.y, k4.y, dot);
+                    dot = fmaf(q4.z, k4.z, dot);
+                    dot = fmaf(q4.w, k4.w, dot);
+                }
+            } else {
+                for (int d = 0; d < head_dim; ++d) dot = fmaf(q_s[d], ssb_to_float(kr[d]), dot);
+            }
             sc = dot * scale;
         }
         const float cm = block_reduce_max(sc, red);
@@ -424,6 +438,7 @@ attention_plain_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ k
             const int d = tid + i * ATT_THREADS;
             if (d < v_dim) {
                 float a = acc[i] * alpha;
+#pragma unroll 8
                 for (int jj = 0; jj < n_in; ++jj) {
                     const T* vr = v_cache + ssb_cache_row(page_table, max_pages, s, base + jj, page_shift,
                                                           n_kv, kvh, v_row);
@@ -472,6 +487,30 @@ SSB_API int ssb_attention_plain(const void* q, int ldq, int dtype, const void* k
             max_pages, (bf16*)out, ldo, n_q, n_kv, head_dim, page_shift, window, scale, v_dim, v_row, sinks);
     else
         return SSB_ERR_BAD_DTYPE;
+    return ssb_launch_status();
+}
+
+// The same attention for a step of float32 prompts: the new tokens of each sequence seq_start .. of slot seq_slot, at packed
+// rows cu_new[b] .. cu_new[b + 1] - 1 (attention_f32.cuh).  head_dim 64 or 128, values as wide as keys.
+SSB_API int ssb_attention_f32_prompt(const float* q, int ldq, const float* k_cache, const float* v_cache, const int* cu_new,
+                                     const int* seq_start, const int* seq_slot, const int* page_table, int max_pages,
+                                     float* out, int ldo, int n_seqs, int max_new, int n_q, int n_kv, int head_dim,
+                                     int page_shift, float scale, cudaStream_t stream) {
+    if (n_seqs <= 0 || max_new <= 0) return 0;
+    if ((head_dim != 64 && head_dim != 128) || n_kv <= 0 || n_kv > 65535 || n_seqs > 65535 || n_q % n_kv) return SSB_ERR_BAD_SIZE;
+    if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) || ((ldq | ldo) & 3)) return SSB_ERR_BAD_SIZE;
+    const long long tiles = ((long long)max_new * (n_q / n_kv) + AF_ROWS - 1) / AF_ROWS;
+    if (tiles > 0x7fffffffLL) return SSB_ERR_BAD_SIZE;
+    const dim3 grid((unsigned)tiles, n_kv, n_seqs);
+#define SSB_AF(HD) do { \
+        const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                                   (int)attention_f32_smem<HD>()); \
+        if (e != cudaSuccess) return (int)e; \
+        attention_f32_kernel<HD><<<grid, AF_THREADS, attention_f32_smem<HD>(), stream>>>( \
+            q, ldq, k_cache, v_cache, cu_new, seq_start, seq_slot, page_table, max_pages, out, ldo, n_q, n_kv, page_shift, scale); \
+    } while (0)
+    if (head_dim == 64) SSB_AF(64); else SSB_AF(128);
+#undef SSB_AF
     return ssb_launch_status();
 }
 

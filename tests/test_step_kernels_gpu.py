@@ -52,3 +52,32 @@ def test_float32_head_products_are_the_general_kernels_bit_for_bit(T, H, K, N):
     ops().head_linear_plain(off_by_one(x.contiguous()), w, want)
     ops().head_linear_plain(x, w, got)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("hd,n_q,n_kv", [(64, 8, 2), (128, 6, 2), (128, 3, 3), (64, 12, 1)])
+def test_float32_prompt_attention_is_the_plain_kernels_bit_for_bit(hd, n_q, n_kv):
+    """Prompts that continue a cache, of one token, of exactly a chunk of keys and a page; pages that belong to nobody are
+    not numbers, and the last value of a sequence is infinite: only the rows that see it may be."""
+    lens, starts, slots = [100, 300, 1, 128, 9, 64], [0, 64, 200, 0, 119, 128], [4, 0, 2, 5, 1, 3]
+    T, pages = sum(lens), sum((n + s + 63) // 64 for n, s in zip(lens, starts))
+    perm = torch.randperm(pages + 3, generator=torch.Generator().manual_seed(hd)).to(torch.int32)
+    table, at = torch.zeros(6, 16, dtype=torch.int32), 0
+    k, v = rnd(pages + 3, n_kv, 64, hd, seed=1), rnd(pages + 3, n_kv, 64, hd, seed=2)
+    for slot, n, s in zip(slots, lens, starts):
+        need = (n + s + 63) // 64
+        table[slot, :need] = perm[at:at + need]
+        at += need
+        v[int(table[slot, need - 1]), 0, (n + s - 1) % 64, 3] = math.inf
+    k[perm[at:].long()] = math.nan
+    v[perm[at:].long()] = math.nan
+    q = rnd(T, n_q * hd + 64, seed=3, scale=2.0)[:, : n_q * hd]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos = torch.cat([torch.arange(s, s + n) for n, s in zip(lens, starts)]).to(torch.int32).to(DEV)
+    slot_of = torch.cat([torch.full((n,), s) for n, s in zip(lens, slots)]).to(torch.int32).to(DEV)
+    cu = i32([sum(lens[:i]) for i in range(len(lens) + 1)])
+    want, got = torch.empty(T, n_q * hd, device=DEV), torch.full((T, n_q * hd), 7.0, device=DEV)
+    assert ops().attention_f32_prompt_ok(q, k, v, got, hd)
+    ops().attention_plain(q, k, v, pos, slot_of, table.to(DEV), want, n_q, n_kv, hd, 6, None, hd ** -0.5)
+    ops().attention_f32_prompt(q, k, v, cu, i32(starts), i32(slots), table.to(DEV), got, max(lens), n_q, n_kv, hd, 6, hd ** -0.5)
+    assert bool(torch.isinf(want).any())
+    assert torch.equal(torch.nan_to_num(got, nan=7.0), torch.nan_to_num(want, nan=7.0))
