@@ -81,3 +81,26 @@ def test_float32_prompt_attention_is_the_plain_kernels_bit_for_bit(hd, n_q, n_kv
     ops().attention_f32_prompt(q, k, v, cu, i32(starts), i32(slots), table.to(DEV), got, max(lens), n_q, n_kv, hd, 6, hd ** -0.5)
     assert bool(torch.isinf(want).any())
     assert torch.equal(torch.nan_to_num(got, nan=7.0), torch.nan_to_num(want, nan=7.0))
+
+
+@pytest.mark.parametrize("top_k", [1, 5, 40, 64])
+def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top_k):
+    """A top-k cut of a large step is searched over candidates, of a small one over the row in shared memory: the same
+    tokens.  Rows with ties at the cut, everything tied, one huge token, few finite ones, not-a-numbers."""
+    n, vocab = 18, 70001
+    lg = rnd(n, vocab, seed=top_k, scale=2.5)
+    lg[0] = (lg[0] * 2).round() / 2
+    lg[1, :] = 1.25
+    lg[2, vocab // 2] = 90.0
+    lg[3, 30:] = -math.inf
+    lg[4, 17] = math.nan
+    lg[5] = lg[5].sort(descending=True).values
+    lg[6, :] = -math.inf
+    lg[7, 9] = math.inf
+    seeds = torch.arange(1, n + 1, dtype=torch.int64, device=DEV) * 0x1E3779B97F4A7C15
+    state, out = seeds.clone(), torch.empty(n, dtype=torch.int32, device=DEV)
+    ops().sample(lg, 0.7, top_k, 1.0, None, state, out)
+    for lo in range(0, n, 9):
+        alone, got = seeds[lo:lo + 9].clone(), torch.empty(9, dtype=torch.int32, device=DEV)
+        ops().sample(lg[lo:lo + 9].contiguous(), 0.7, top_k, 1.0, None, alone, got)
+        assert torch.equal(got, out[lo:lo + 9])
