@@ -43,6 +43,7 @@ LIBRARIES: Dict[str, Dict[str, List[str]]] = {
     "gemm_tc": {"sources": ["gemm_tc.cu"], "flags": [], "link": []},
     "attention_decode_static": {"sources": ["attention_decode_static.cu"], "flags": [], "link": []},
     "latent_attention": {"sources": ["latent_attention.cu"], "flags": [], "link": []},
+    "latent_attention_tc": {"sources": ["latent_attention_tc.cu"], "flags": [], "link": []},
     "batched_gemm": {"sources": ["batched_gemm.cu"], "flags": [], "link": []},
     "grouped_gemm_tc": {"sources": ["grouped_gemm_tc.cu"], "flags": [], "link": []},
     "latent_ops": {"sources": ["latent_ops.cu"], "flags": [], "link": []},

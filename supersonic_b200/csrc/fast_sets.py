@@ -22,6 +22,7 @@ STREAM_ROWS = ops.GEMV_TC_MAX_ROWS   # steps of up to this many rows take the pr
 CLUSTER_CHUNK_PAGES = 8       # the most pages a chunk holds when a sequence's chunks run as a cluster
 EXPERT_NARROW_ROWS = 24       # mean rows an expert up to which its products take tiles of 64 rows ...
 EXPERT_MIDDLE_ROWS = 64       # ... and of 128
+LATENT_TC_MIN_ROWS = 128      # (token, head) rows of the longest prompt from which latent attention runs on tcgen05
 TC_ATTENTION_MIN_NEW = 96     # prompts at least this long take the tcgen05 attention (tiles of 128 rows)
 
 
@@ -381,6 +382,11 @@ class FastKernels(PlainKernels):
         if not ops.latent_attention_mma_ok(q_abs, cache, out, n_heads, dk, kv_rank, page_shift):
             super().latent_attention(q_abs, cache, batch, page_table, out, n_heads, kv_rank, rot_dim, page_shift,
                                      window, scale, sinks)
+            return
+        if not batch.is_decode and not self.deterministic and batch.max_new * n_heads >= LATENT_TC_MIN_ROWS \
+                and ops.latent_attention_tc_ok(q_abs, cache, out, n_heads, dk, kv_rank, page_shift):
+            ops.latent_attention_tc(q_abs, cache, batch.cu_new, batch.seq_start, batch.seq_slot, page_table, out, sinks,
+                                    batch.max_new, n_heads, dk, kv_rank, page_shift, window, scale)
             return
         splits, partial = 1, None
         if batch.is_decode and not self.deterministic:

@@ -484,6 +484,47 @@ def latent_attention_mma(q: torch.Tensor, cache: torch.Tensor, cu_new: torch.Ten
         c_int(n_splits), c_int(form), c_int(1 if pdl else 0), _stream()), "latent_attention_mma")
 
 
+_latent_tc_fits = {}
+
+
+def latent_attention_tc_ok(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, n_heads: int, dk: int, dv: int,
+                           page_shift: int) -> bool:
+    """Whether the tcgen05 latent attention takes these operands: those of ``latent_attention_mma`` whose query rows fit
+    shared memory."""
+    if not latent_attention_mma_ok(q, cache, out, n_heads, dk, dv, page_shift):
+        return False
+    fits = _latent_tc_fits.get((dk, dv))
+    if fits is None:
+        fits = _latent_tc_fits[(dk, dv)] = bool(_fn("latent_attention_tc", "ssb_latent_attention_tc_fits")(c_int(dk), c_int(dv)))
+    return fits and q.shape[0] * n_heads < 2 ** 31 and cache.shape[0] * 64 < 2 ** 31
+
+
+def latent_attention_tc(q: torch.Tensor, cache: torch.Tensor, cu_new: torch.Tensor, seq_start: torch.Tensor,
+                        seq_slot: torch.Tensor, page_table: torch.Tensor, out: torch.Tensor, sinks: Optional[torch.Tensor],
+                        max_new: int, n_heads: int, dk: int, dv: int, page_shift: int, window: Optional[int],
+                        scale: float) -> None:
+    """``latent_attention_mma`` of a prompt step on tcgen05.  A wait that runs out sets the device's error word
+    (``check_device_errors``)."""
+    if not latent_attention_tc_ok(q, cache, out, n_heads, dk, dv, page_shift):
+        raise KernelError("latent_attention_tc: operands it does not take")
+    _need(cu_new, "cu_new", torch.int32, 1); _need(seq_start, "seq_start", torch.int32, 1)
+    _need(seq_slot, "seq_slot", torch.int32, 1); _need(page_table, "page_table", torch.int32, 2)
+    T, B = q.shape[0], seq_slot.shape[0]
+    if out.shape[0] != T or cu_new.shape[0] != B + 1 or seq_start.shape[0] != B:
+        raise KernelError("latent_attention_tc: sizes")
+    if sinks is not None:
+        _need(sinks, "sinks", torch.float32, 1)
+        if sinks.shape[0] != n_heads:
+            raise KernelError("latent_attention_tc: one sink per head")
+    global _tc_unchecked
+    _tc_unchecked += 1
+    _check(_fn("latent_attention_tc", "ssb_latent_attention_tc")(
+        _ptr(q), _ptr(cache), c_int(cache.shape[0]), _ptr(cu_new), _ptr(seq_start), _ptr(seq_slot), _ptr(page_table),
+        c_int(page_table.shape[1]), _ptr(out), _ptr(sinks), c_int(B), c_int(max_new), c_int(T), c_int(n_heads), c_int(dk),
+        c_int(dv), c_int(page_shift), c_int(int(window) if window else 0), c_float(scale), _ptr(tc_error_word(q.device)),
+        _stream()), "latent_attention_tc")
+
+
 # ---- many small matrix products on the tensor cores -------------------------------------------
 def head_gemm_mma_ok(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
     return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32)

@@ -83,6 +83,27 @@ def test_float32_prompt_attention_is_the_plain_kernels_bit_for_bit(hd, n_q, n_kv
     assert torch.equal(torch.nan_to_num(got, nan=7.0), torch.nan_to_num(want, nan=7.0))
 
 
+@pytest.mark.parametrize("H,dk,dv,window", [(16, 576, 512, None), (16, 576, 512, 100), (8, 288, 256, None), (6, 224, 192, 96),
+                                            (3, 400, 384, 7), (5, 48, 32, None), (1, 64, 16, 64)])
+def test_latent_attention_of_prompts_on_tcgen05(H, dk, dv, window):
+    """Against float64 attention over the same bfloat16 rows: as close as the mma.sync kernel (both round their result to
+    bfloat16 and keep 16 bits of a weight, so the error is the result's rounding: 2^-9 relative, root mean square)."""
+    from test_sotavik_kernels_gpu import latent_case, latent_reference
+    o, scale = ops(), dk ** -0.5
+    for lengths, new, sinks in (([200, 65, 1, 130], [70, 65, 1, 3], None), ([300, 64, 129], [300, 1, 129], torch.linspace(-1.0, 2.0, H, device=DEV))):
+        cache, batch, store, table, q, rows = latent_case(lengths, new, H, dk, dv, seed=H + dk)
+        T = sum(new)
+        ref = latent_reference(q, rows, lengths, new, H, dk, dv, scale, sinks, window).double()
+        out = torch.full((T, H * dv), 7.0, dtype=torch.bfloat16, device=DEV)
+        assert o.latent_attention_tc_ok(q, store, out, H, dk, dv, 6)
+        o.latent_attention_tc(q, store, batch.cu_new, batch.seq_start, batch.seq_slot, table, out, sinks, batch.max_new, H, dk, dv,
+                              6, window, scale)
+        torch.cuda.synchronize()
+        o.check_device_errors(torch.device(DEV))
+        err = float((out.double() - ref).norm() / ref.norm())
+        assert err < 2.0 ** -9, (lengths, new, err)
+
+
 @pytest.mark.parametrize("top_k", [1, 5, 40, 64])
 def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top_k):
     """A top-k cut of a large step is searched over candidates, of a small one over the row in shared memory: the same
