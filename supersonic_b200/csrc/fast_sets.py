@@ -453,7 +453,10 @@ class FastKernels(PlainKernels):
 
     def gated_linear_scan(self, proj, q_off, k_off, v_off, z, z_bias, tau, q_scale, state, batch, out, n_heads,
                           dim, vdim):
-        chunk, n_sums, n_decays = ops.scan_chunking(batch.n_seqs, batch.max_new, n_heads, dim, vdim)
+        if self.deterministic:                 # chunks of one length whatever else is in the step
+            chunk, n_sums, n_decays = ops.scan_chunking(batch.n_seqs, batch.max_new, n_heads, dim, vdim)
+        else:
+            chunk, n_sums, n_decays = ops.gated_scan_chunking(batch.n_seqs, batch.max_new, n_heads, dim, vdim, ops.sm_count())
         sums = decays = None
         if chunk:
             sums = self._buffer("scan_sums", n_sums, torch.float32, out.device)

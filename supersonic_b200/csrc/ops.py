@@ -691,6 +691,19 @@ def tied_scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim: 
     return chunk, n_seqs * n * per, n_seqs * n * n_heads * dim
 
 
+def gated_scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim: int, sms: int):
+    """(chunk, floats of sums, floats of decays) for ``gated_linear_scan``: as many chunks as give the SMs two blocks each
+    (blocks own 64 value columns of a head); one walk a sequence where that is no more than two chunks."""
+    blocks = n_seqs * n_heads * (-(-vdim // 64))
+    per = n_heads * dim * vdim
+    n = min(2 * sms // max(blocks, 1), max_new // 64, SCAN_SCRATCH_BYTES // (4 * per * n_seqs))
+    if n < 3:
+        return 0, 0, 0
+    chunk = -(-(-(-max_new // n)) // 8) * 8           # whole turns of eight tokens
+    n = -(-max_new // chunk)
+    return chunk, n_seqs * n * per, n_seqs * n * n_heads * dim
+
+
 def tied_scan(proj: torch.Tensor, q_off: int, f_off: int, v_off: int, z_bias: torch.Tensor, lower: torch.Tensor,
               state: torch.Tensor, cu_new: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, n_heads: int, dim: int,
               vdim: int, norm_w: Optional[torch.Tensor] = None, eps: float = 0.0, pdl: bool = False, chunk: int = 0,

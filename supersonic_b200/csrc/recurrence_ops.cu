@@ -14,27 +14,13 @@
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int SCAN_COLS = 32;        // value columns a block owns
-constexpr int SCAN_GROUPS = 16;      // row groups: thread (g, j) owns a run of rows of column j
-constexpr int SCAN_MAX_ROWS = 16;    // rows per thread: dim up to 256
-constexpr int SCAN_TOKENS = 4;       // tokens staged in shared memory a turn (one pair of barriers for all of them)
-constexpr int SCAN_ITEMS = SCAN_TOKENS * SCAN_MAX_ROWS * SCAN_GROUPS / (SCAN_COLS * SCAN_GROUPS);   // staged items a thread
+constexpr int SCAN_MAX_DIM = 256;    // key channels of a head
 
 __device__ __forceinline__ float log_sigmoid(float z) {
     // log(1 / (1 + exp(-z))) without overflow on either side
     return fminf(z, 0.f) - log1pf(expf(-fabsf(z)));
 }
 
-// One kernel serves three uses.  A block walks tokens [t_lo, t_hi) of one sequence for one head and one
-// tile of value columns:
-//   whole run   (chunk = 0): from the slot's state, writing outputs, leaving the state in the slot;
-//   chunk sums  (chunk > 0, sums != null, out == null): from zero over chunk blockIdx.x % max_chunks of the
-//               sequence, leaving the chunk's own sum in ``sums`` and the product of its decays in ``decays``;
-//   chunk outputs (chunk > 0, out != null): from the state at the chunk's start, which the carry kernel below
-//               left in ``sums``, writing outputs.
-// A long prompt is run as chunk sums, carry, chunk outputs: the chunks of a sequence in parallel, the same
-// float32 recurrence within each.  Tokens are staged four at a time, and the next four are fetched while
-// these are worked on.
 // z <- sigmoid(z + bias)^(1 / tau), in place: the decays of every token and channel, once for all the blocks
 // that walk them
 __global__ void decay_kernel(float* __restrict__ z, int ldz, const float* __restrict__ z_bias, float inv_tau,
@@ -47,128 +33,6 @@ __global__ void decay_kernel(float* __restrict__ z, int ldz, const float* __rest
     const int c = (int)(idx % width);
     float* p = z + t * ldz + c;
     *p = expf(log_sigmoid(*p + z_bias[c]) * inv_tau);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(SCAN_COLS * SCAN_GROUPS)
-gated_linear_scan_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off,
-                         const float* __restrict__ z, int ldz, float q_scale, float* __restrict__ state,
-                         const int* __restrict__ cu_new, const int* __restrict__ seq_slot,
-                         float* __restrict__ out, int ldo, int n_heads, int dim, int vdim,
-                         int chunk, int max_chunks, float* __restrict__ sums, float* __restrict__ decays) {
-    constexpr int NT = SCAN_COLS * SCAN_GROUPS;
-    extern __shared__ __align__(16) float sm[];
-    // rows per thread, a multiple of four: thread (g, j) owns rows g * rpt .. + rpt - 1 of column j, and reads
-    // their decays, keys and queries four at a time; the arrays are padded with zeros up to 8 * rpt rows
-    const int rpt = ((dim + SCAN_GROUPS - 1) / SCAN_GROUPS + 3) & ~3, dimp = rpt * SCAN_GROUPS;
-    float* a_s = sm;                          // [SCAN_TOKENS][dimp] decays
-    float* k_s = a_s + SCAN_TOKENS * dimp;    // [SCAN_TOKENS][dimp]
-    float* q_s = k_s + SCAN_TOKENS * dimp;    // [SCAN_TOKENS][dimp]
-    float* v_s = q_s + SCAN_TOKENS * dimp;    // [SCAN_TOKENS][SCAN_COLS]
-    float* o_s = v_s + SCAN_TOKENS * SCAN_COLS;   // [SCAN_TOKENS][SCAN_GROUPS][SCAN_COLS]
-    const int b = chunk > 0 ? blockIdx.x / max_chunks : blockIdx.x, c = chunk > 0 ? blockIdx.x % max_chunks : 0;
-    const int h = blockIdx.y, j0 = blockIdx.z * SCAN_COLS;
-    const int tid = threadIdx.x, j = tid % SCAN_COLS, g = tid / SCAN_COLS;
-    ssb_pdl_launch_dependents();
-    ssb_pdl_wait();
-    const int slot = seq_slot[b];
-    if (slot < 0) return;                                // padding row
-    int t0 = cu_new[b], t1 = cu_new[b + 1];
-    if (chunk > 0) {
-        t0 += c * chunk;
-        t1 = min(t1, t0 + chunk);
-        if (t0 >= t1) return;
-    }
-    const bool col = j0 + j < vdim;
-    const bool emit = out != nullptr;
-    float* S = chunk > 0 ? sums + (((size_t)blockIdx.x * n_heads + h) * dim) * vdim
-                         : state + ((size_t)slot * n_heads + h) * dim * vdim;
-    float s_reg[SCAN_MAX_ROWS];
-#pragma unroll
-    for (int r = 0; r < SCAN_MAX_ROWS; ++r) {
-        const int i = g * rpt + r;
-        s_reg[r] = (col && r < rpt && i < dim && (chunk == 0 || emit)) ? S[(size_t)i * vdim + j0 + j] : 0.f;
-    }
-    for (int e = tid; e < 3 * SCAN_TOKENS * dimp; e += NT) sm[e] = 0.f;      // the padding stays zero
-    // a turn stages SCAN_TOKENS tokens: item (token, channel) n * NT + tid of the turn is this thread's
-    float zz[SCAN_ITEMS], kk[SCAN_ITEMS], qq[SCAN_ITEMS], vv = 0.f, a_prod = 1.f;
-    int item_tt[SCAN_ITEMS], item_i[SCAN_ITEMS];         // the same in every turn: divided once
-#pragma unroll
-    for (int n = 0; n < SCAN_ITEMS; ++n) {
-        const int item = n * NT + tid;
-        item_tt[n] = item < SCAN_TOKENS * dim ? item / dim : SCAN_TOKENS;
-        item_i[n] = item % dim;
-    }
-    auto fetch = [&](int t) {
-        const int n_tok = min(SCAN_TOKENS, t1 - t);
-#pragma unroll
-        for (int n = 0; n < SCAN_ITEMS; ++n) {
-            const int tt = item_tt[n], i = item_i[n];
-            if (tt < n_tok) {
-                const T* row = proj + (size_t)(t + tt) * ld;
-                zz[n] = z[(size_t)(t + tt) * ldz + h * dim + i];
-                kk[n] = ssb_to_float(row[k_off + h * dim + i]);
-                qq[n] = ssb_to_float(row[q_off + h * dim + i]);
-            }
-        }
-        if (tid < SCAN_TOKENS * SCAN_COLS) {
-            const int tt = tid / SCAN_COLS, jj = tid % SCAN_COLS;
-            vv = (tt < n_tok && j0 + jj < vdim) ? ssb_to_float(proj[(size_t)(t + tt) * ld + v_off + h * vdim + j0 + jj]) : 0.f;
-        }
-    };
-    fetch(t0);
-    __syncthreads();
-    for (int t = t0; t < t1; t += SCAN_TOKENS) {
-        const int n_tok = min(SCAN_TOKENS, t1 - t);
-#pragma unroll
-        for (int n = 0; n < SCAN_ITEMS; ++n) {
-            const int tt = item_tt[n], i = item_i[n];
-            if (tt < n_tok) {
-                a_s[tt * dimp + i] = zz[n];
-                k_s[tt * dimp + i] = kk[n];
-                q_s[tt * dimp + i] = qq[n] * q_scale;
-            }
-        }
-        if (tid < SCAN_TOKENS * SCAN_COLS) v_s[tid] = vv;
-        __syncthreads();
-        if (t + SCAN_TOKENS < t1) fetch(t + SCAN_TOKENS);
-        if (decays != nullptr && tid < dim)
-            for (int tt = 0; tt < n_tok; ++tt) a_prod *= a_s[tt * dimp + tid];
-        for (int tt = 0; tt < n_tok; ++tt) {
-            const float v = v_s[tt * SCAN_COLS + j];
-            const float4* a4 = reinterpret_cast<const float4*>(a_s + tt * dimp + g * rpt);
-            const float4* k4 = reinterpret_cast<const float4*>(k_s + tt * dimp + g * rpt);
-            const float4* q4 = reinterpret_cast<const float4*>(q_s + tt * dimp + g * rpt);
-            float o = 0.f;
-#pragma unroll
-            for (int r = 0; r < SCAN_MAX_ROWS; r += 4)
-                if (r < rpt) {
-                    const float4 a = a4[r >> 2], k = k4[r >> 2], q = q4[r >> 2];
-                    s_reg[r] = fmaf(a.x, s_reg[r], k.x * v);          o = fmaf(s_reg[r], q.x, o);
-                    s_reg[r + 1] = fmaf(a.y, s_reg[r + 1], k.y * v);  o = fmaf(s_reg[r + 1], q.y, o);
-                    s_reg[r + 2] = fmaf(a.z, s_reg[r + 2], k.z * v);  o = fmaf(s_reg[r + 2], q.z, o);
-                    s_reg[r + 3] = fmaf(a.w, s_reg[r + 3], k.w * v);  o = fmaf(s_reg[r + 3], q.w, o);
-                }
-            if (emit) o_s[(tt * SCAN_GROUPS + g) * SCAN_COLS + j] = o;
-        }
-        __syncthreads();
-        if (emit && tid < n_tok * SCAN_COLS) {
-            const int tt = tid / SCAN_COLS, jj = tid % SCAN_COLS;
-            if (j0 + jj < vdim) {
-                float sum = 0.f;
-#pragma unroll
-                for (int gg = 0; gg < SCAN_GROUPS; ++gg) sum += o_s[(tt * SCAN_GROUPS + gg) * SCAN_COLS + jj];
-                out[(size_t)(t + tt) * ldo + h * vdim + j0 + jj] = sum;
-            }
-        }
-    }
-    if (chunk > 0 && emit) return;                       // the state was carried by the carry kernel
-#pragma unroll
-    for (int r = 0; r < SCAN_MAX_ROWS; ++r) {
-        const int i = g * rpt + r;
-        if (col && r < rpt && i < dim) S[(size_t)i * vdim + j0 + j] = s_reg[r];
-    }
-    if (chunk > 0 && blockIdx.z == 0 && tid < dim) decays[((size_t)blockIdx.x * n_heads + h) * dim + tid] = a_prod;
 }
 
 // Carries the state across a sequence's chunks: with S the state before chunk c, chunk c's place in
@@ -205,6 +69,11 @@ gated_linear_carry_kernel(float* __restrict__ state, float* __restrict__ sums, c
     state[(size_t)slot * per + e] = cur;
 }
 
+static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
+                      float q_scale, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo, int n_seqs,
+                      int n_heads, int dim, int vdim, int chunk, int max_chunks, float* sums, float* decays, bool pdl,
+                      cudaStream_t stream);
+
 // proj [T, ld] holds q, k (n_heads x dim each) and v (n_heads x vdim) from the given columns;
 // z [T, ldz] float32 is the decay's pre-activation without its bias z_bias [n_heads x dim], and is overwritten
 // with the decays;
@@ -218,47 +87,19 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
                                   int n_seqs, int n_tokens, int n_heads, int dim, int vdim, int chunk, int max_chunks,
                                   float* sums, float* decays, int pdl, cudaStream_t stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
-    if (dim <= 0 || dim > SCAN_MAX_ROWS * SCAN_GROUPS || vdim <= 0 || !(tau > 0.f)) return SSB_ERR_BAD_SIZE;
+    if (dim <= 0 || dim > SCAN_MAX_DIM || vdim <= 0 || !(tau > 0.f)) return SSB_ERR_BAD_SIZE;
     if (chunk < 0 || (chunk > 0 && (max_chunks <= 0 || sums == nullptr || decays == nullptr))) return SSB_ERR_BAD_SIZE;
     const long long items = chunk > 0 ? (long long)n_seqs * max_chunks : n_seqs;
     if (items > 0x7fffffffll) return SSB_ERR_BAD_SIZE;
-    const dim3 grid((unsigned)items, n_heads, (vdim + SCAN_COLS - 1) / SCAN_COLS);
-    if (grid.y > 65535 || grid.z > 65535 || n_seqs > 65535) return SSB_ERR_BAD_SIZE;
-    const int rpt = ((dim + SCAN_GROUPS - 1) / SCAN_GROUPS + 3) & ~3;
-    const size_t smem = (size_t)SCAN_TOKENS * (3 * rpt * SCAN_GROUPS + SCAN_COLS + SCAN_COLS * SCAN_GROUPS) * sizeof(float);
-    int rc = 0;
-    {
-        const size_t total = (size_t)n_tokens * n_heads * dim;
-        rc = ssb_launch(decay_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, pdl != 0, z, ldz, z_bias,
+    if (n_heads > 65535 || (vdim + 31) / 32 > 65535 || n_seqs > 65535) return SSB_ERR_BAD_SIZE;
+    if (dtype != SSB_F32 && dtype != SSB_BF16) return SSB_ERR_BAD_DTYPE;
+    const size_t total = (size_t)n_tokens * n_heads * dim;
+    int rc = ssb_launch(decay_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, pdl != 0, z, ldz, z_bias,
                         1.0f / tau, n_heads * dim, total);
-        if (!rc) rc = ssb_launch_status();
-        if (rc) return rc;
-    }
-#define SSB_SCAN(T, OUT) \
-    rc = ssb_launch(gated_linear_scan_kernel<T>, grid, dim3(SCAN_COLS * SCAN_GROUPS), smem, stream, pdl != 0, \
-                    (const T*)proj, ld, q_off, k_off, v_off, (const float*)z, ldz, q_scale, state, cu_new, seq_slot, \
-                    OUT, ldo, n_heads, dim, vdim, chunk, max_chunks, sums, decays)
-#define SSB_SCAN_BOTH(OUT) do { \
-        if (dtype == SSB_F32) SSB_SCAN(float, OUT); \
-        else if (dtype == SSB_BF16) SSB_SCAN(bf16, OUT); \
-        else return SSB_ERR_BAD_DTYPE; \
-        if (!rc) rc = ssb_launch_status(); \
-        if (rc) return rc; \
-    } while (0)
-    if (chunk == 0) {
-        SSB_SCAN_BOTH(out);
-        return 0;
-    }
-    SSB_SCAN_BOTH((float*)nullptr);
-    const size_t per = (size_t)n_heads * dim * vdim;
-    rc = ssb_launch(gated_linear_carry_kernel, dim3((unsigned)((per + 255) / 256), n_seqs), dim3(256), 0, stream, pdl != 0,
-                    state, sums, (const float*)decays, cu_new, seq_slot, n_heads, dim, vdim, chunk, max_chunks);
     if (!rc) rc = ssb_launch_status();
     if (rc) return rc;
-    SSB_SCAN_BOTH(out);
-#undef SSB_SCAN_BOTH
-#undef SSB_SCAN
-    return 0;
+    return gated_walk(proj, ld, dtype, q_off, k_off, v_off, z, ldz, q_scale, state, cu_new, seq_slot, out, ldo, n_seqs,
+                      n_heads, dim, vdim, chunk, max_chunks, sums, decays, pdl != 0, stream);
 }
 
 // =======================================================================================
@@ -274,6 +115,10 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
 // their way from memory.
 //   OUT = false: chunk sums, from zero, with the product of the chunk's decays;
 //   OUT = true: outputs from the state at the start (the slot's, or what the carry kernel left for the chunk).
+// GATED: the gated linear attention at the top of this file on the same tiles, S <- a S + k v with decays that a kernel before
+// this one made, o = S^T (q_scale q).  (A kernel of its own, a
+// column a thread with the sums through shared memory, took 1,011 us for 4 heads of 256 x 512 and 2,048 tokens where this
+// takes 518, 412 us for 128 x 256 where this takes 133, and 128 us for one token of 64 sequences where this takes 112.)
 // norm_w given (one block holds all of the head's columns): the head norm is taken where the outputs meet in shared
 // memory, y = o / rms(o) * norm_w, a warp a token; else o itself goes out in float32.
 // =======================================================================================
@@ -283,8 +128,9 @@ constexpr int TW_TOKENS = 8;
 __device__ __forceinline__ float tied_share(float z, float lower) { return (1.0f - lower) / (1.0f + expf(z)); }
 
 struct TiedArgs {
-    const void* proj; int ld, q_off, f_off, v_off;
+    const void* proj; int ld, q_off, f_off, v_off;        // gated form: f_off is where the keys start
     const float* z_bias; const float* lower;
+    const float* decay; int ldz; float q_scale;            // gated form: every token's and channel's decay
     float* state; const int* cu_new; const int* seq_slot;
     float* out; int ldo;
     const float* norm_w; float eps; void* y; int ldy;
@@ -292,7 +138,7 @@ struct TiedArgs {
     float* sums; float* decays;
 };
 
-template <typename T, int R4, int NT, bool OUT>
+template <typename T, int R4, int NT, bool OUT, bool GATED>
 __global__ void __launch_bounds__(NT)
 tied_walk_kernel(const TiedArgs a) {
     constexpr int DIMP = 64 * R4, COLS = NT / 4;          // padded rows; columns a block owns
@@ -302,6 +148,7 @@ tied_walk_kernel(const TiedArgs a) {
     float* q_s = k_s + 2 * TW_TOKENS * DIMP;               // [2][TW_TOKENS][DIMP]
     float* v_s = q_s + 2 * TW_TOKENS * DIMP;               // [2][TW_TOKENS][COLS]
     float* o_s = v_s + 2 * TW_TOKENS * COLS;               // [2][TW_TOKENS][COLS]
+    float* d_s = o_s + 2 * TW_TOKENS * COLS;               // GATED: [2][TW_TOKENS][DIMP]
     const int dim = a.dim, vdim = a.vdim, h = blockIdx.y, j0 = blockIdx.z * COLS;
     const int b = a.chunk > 0 ? blockIdx.x / a.max_chunks : blockIdx.x, ch = a.chunk > 0 ? blockIdx.x % a.max_chunks : 0;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane & 15, cg = lane >> 4;
@@ -319,16 +166,21 @@ tied_walk_kernel(const TiedArgs a) {
     float* S = a.chunk > 0 ? a.sums + (((size_t)blockIdx.x * a.n_heads + h) * dim) * vdim
                            : a.state + ((size_t)slot * a.n_heads + h) * dim * vdim;
     const int col0 = warp * 8 + cg * 4;                    // this lane's four columns, within the block's
+    const bool pieces = vdim % 4 == 0 && ((uintptr_t)S & 15) == 0;       // a lane's four columns in one access
     float s[R4][4][4];
 #pragma unroll
     for (int g = 0; g < R4; ++g)
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int i = (g * 16 + rg) * 4 + r, j = j0 + col0 + c;
-                s[g][r][c] = (OUT && i < dim && j < vdim) ? S[(size_t)i * vdim + j] : 0.f;
+        for (int r = 0; r < 4; ++r) {
+            const int i = (g * 16 + rg) * 4 + r, j = j0 + col0;
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (OUT && i < dim && j < vdim) {
+                const float* src = S + (size_t)i * vdim + j;
+                if (pieces) x = *reinterpret_cast<const float4*>(src);
+                else x = make_float4(src[0], j + 1 < vdim ? src[1] : 0.f, j + 2 < vdim ? src[2] : 0.f, j + 3 < vdim ? src[3] : 0.f);
             }
+            s[g][r][0] = x.x; s[g][r][1] = x.y; s[g][r][2] = x.z; s[g][r][3] = x.w;
+        }
     float prod[R4][4];
 #pragma unroll
     for (int g = 0; g < R4; ++g)
@@ -339,10 +191,10 @@ tied_walk_kernel(const TiedArgs a) {
 #pragma unroll
     for (int n = 0; n < KI; ++n) {
         const int i = (n * NT + tid) % DIMP;
-        bias[n] = i < dim ? a.z_bias[h * dim + i] : 0.f;
-        low[n] = i < dim ? a.lower[h * dim + i] : 0.f;
+        bias[n] = !GATED && i < dim ? a.z_bias[h * dim + i] : 0.f;
+        low[n] = !GATED && i < dim ? a.lower[h * dim + i] : 0.f;
     }
-    float zz[KI], qq[KI], vv[VI];
+    float zz[KI], qq[KI], dd[KI], vv[VI];
     auto fetch = [&](int t) {
 #pragma unroll
         for (int n = 0; n < KI; ++n) {
@@ -351,6 +203,7 @@ tied_walk_kernel(const TiedArgs a) {
             const T* row = proj + (size_t)(t + tt) * a.ld + h * dim + i;
             zz[n] = ok ? ssb_to_float(row[a.f_off]) : 0.f;
             qq[n] = OUT && ok ? ssb_to_float(row[a.q_off]) : 0.f;
+            dd[n] = GATED && ok ? a.decay[(size_t)(t + tt) * a.ldz + h * dim + i] : 1.f;
         }
 #pragma unroll
         for (int n = 0; n < VI; ++n) {
@@ -389,8 +242,14 @@ tied_walk_kernel(const TiedArgs a) {
         for (int n = 0; n < KI; ++n) {
             const int item = n * NT + tid, tt = item / DIMP, i = item % DIMP;
             const bool ok = t + tt < t1 && i < dim;        // padding rows and tokens leave the state as it is: k = 0
-            kb[item] = ok ? tied_share(zz[n] + bias[n], low[n]) : 0.f;
-            if (OUT) qb[item] = qq[n] / (1.0f + expf(-qq[n]));
+            if (GATED) {
+                kb[item] = zz[n];
+                d_s[buf * TW_TOKENS * DIMP + item] = dd[n];
+                if (OUT) qb[item] = qq[n] * a.q_scale;
+            } else {
+                kb[item] = ok ? tied_share(zz[n] + bias[n], low[n]) : 0.f;
+                if (OUT) qb[item] = qq[n] / (1.0f + expf(-qq[n]));
+            }
         }
 #pragma unroll
         for (int n = 0; n < VI; ++n) vb[n * NT + tid] = vv[n];
@@ -398,8 +257,9 @@ tied_walk_kernel(const TiedArgs a) {
         if (t + TW_TOKENS < t1) fetch(t + TW_TOKENS);
         if (OUT && t > t0) finish(t - TW_TOKENS, buf ^ 1);
         if (j0 + warp * 8 < vdim) {
+            const int n_tok = min(TW_TOKENS, t1 - t);
 #pragma unroll 2
-            for (int tt = 0; tt < TW_TOKENS; ++tt) {
+            for (int tt = 0; tt < n_tok; ++tt) {
                 const float4 v4 = *reinterpret_cast<const float4*>(vb + tt * COLS + col0);
                 const float v[4] = {v4.x, v4.y, v4.z, v4.w};
                 float o[4] = {0.f, 0.f, 0.f, 0.f};
@@ -407,7 +267,11 @@ tied_walk_kernel(const TiedArgs a) {
                 for (int g = 0; g < R4; ++g) {
                     const float4 k4 = *reinterpret_cast<const float4*>(kb + tt * DIMP + (g * 16 + rg) * 4);
                     const float k[4] = {k4.x, k4.y, k4.z, k4.w};
-                    float q[4] = {0.f, 0.f, 0.f, 0.f};
+                    float q[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {1.f, 1.f, 1.f, 1.f};
+                    if (GATED) {
+                        const float4 d4 = *reinterpret_cast<const float4*>(d_s + (buf * TW_TOKENS + tt) * DIMP + (g * 16 + rg) * 4);
+                        d[0] = d4.x; d[1] = d4.y; d[2] = d4.z; d[3] = d4.w;
+                    }
                     if (OUT) {
                         const float4 q4 = *reinterpret_cast<const float4*>(qb + tt * DIMP + (g * 16 + rg) * 4);
                         q[0] = q4.x; q[1] = q4.y; q[2] = q4.z; q[3] = q4.w;
@@ -416,10 +280,10 @@ tied_walk_kernel(const TiedArgs a) {
                     for (int r = 0; r < 4; ++r) {
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
-                            s[g][r][c] = fmaf(k[r], v[c] - s[g][r][c], s[g][r][c]);
+                            s[g][r][c] = GATED ? fmaf(d[r], s[g][r][c], k[r] * v[c]) : fmaf(k[r], v[c] - s[g][r][c], s[g][r][c]);
                             if (OUT) o[c] = fmaf(s[g][r][c], q[r], o[c]);
                         }
-                        if (!OUT && warp == 0) prod[g][r] *= 1.0f - k[r];
+                        if (!OUT && warp == 0) prod[g][r] *= GATED ? d[r] : 1.0f - k[r];
                     }
                 }
                 if (OUT) {
@@ -445,27 +309,32 @@ tied_walk_kernel(const TiedArgs a) {
     for (int g = 0; g < R4; ++g)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const int i = (g * 16 + rg) * 4 + r;
+            const int i = (g * 16 + rg) * 4 + r, j = j0 + col0;
+            if (i < dim && j < vdim) {
+                float* dst = S + (size_t)i * vdim + j;
+                if (pieces) {
+                    *reinterpret_cast<float4*>(dst) = make_float4(s[g][r][0], s[g][r][1], s[g][r][2], s[g][r][3]);
+                } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int j = j0 + col0 + c;
-                if (i < dim && j < vdim) S[(size_t)i * vdim + j] = s[g][r][c];
+                    for (int c = 0; c < 4; ++c)
+                        if (j + c < vdim) dst[c] = s[g][r][c];
+                }
             }
             if (!OUT && blockIdx.z == 0 && warp == 0 && cg == 0 && i < dim)
                 a.decays[((size_t)blockIdx.x * a.n_heads + h) * dim + i] = prod[g][r];
         }
 }
 
-template <typename T, int R4, int NT>
+template <typename T, int R4, int NT, bool GATED = false>
 static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_t stream) {
     constexpr int DIMP = 64 * R4, COLS = NT / 4;
-    constexpr size_t smem = (size_t)TW_TOKENS * (4 * DIMP + 4 * COLS) * sizeof(float);
+    constexpr size_t smem = (size_t)TW_TOKENS * ((GATED ? 6 : 4) * DIMP + 4 * COLS) * sizeof(float);
     const long long items = a.chunk > 0 ? (long long)n_seqs * a.max_chunks : n_seqs;
     const dim3 grid((unsigned)items, a.n_heads, (a.vdim + COLS - 1) / COLS);
     if (items > 0x7fffffffll || grid.y > 65535 || grid.z > 65535 || n_seqs > 65535) return SSB_ERR_BAD_SIZE;
     static_assert(smem <= 200 * 1024, "");
-    auto sums = tied_walk_kernel<T, R4, NT, false>;
-    auto outs = tied_walk_kernel<T, R4, NT, true>;
+    auto sums = tied_walk_kernel<T, R4, NT, false, GATED>;
+    auto outs = tied_walk_kernel<T, R4, NT, true, GATED>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(outs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -484,6 +353,23 @@ static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
     }
     rc = ssb_launch(outs, grid, dim3(NT), smem, stream, pdl, a);
     return rc ? rc : ssb_launch_status();
+}
+
+static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
+                           float q_scale, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo, int n_seqs,
+                           int n_heads, int dim, int vdim, int chunk, int max_chunks, float* sums, float* decays, bool pdl,
+                           cudaStream_t stream) {
+    TiedArgs a = {};
+    a.proj = proj; a.ld = ld; a.q_off = q_off; a.f_off = k_off; a.v_off = v_off; a.decay = decay; a.ldz = ldz; a.q_scale = q_scale;
+    a.state = state; a.cu_new = cu_new; a.seq_slot = seq_slot; a.out = out; a.ldo = ldo; a.n_heads = n_heads; a.dim = dim;
+    a.vdim = vdim; a.chunk = chunk; a.max_chunks = max_chunks; a.sums = sums; a.decays = decays;
+#define SSB_GW(T) \
+    return dim <= 64 ? launch_tied_walk<T, 1, 256, true>(a, n_seqs, pdl, stream) \
+         : dim <= 128 ? launch_tied_walk<T, 2, 256, true>(a, n_seqs, pdl, stream) \
+                      : launch_tied_walk<T, 4, 256, true>(a, n_seqs, pdl, stream)
+    if (dtype == SSB_F32) SSB_GW(float);
+    SSB_GW(bf16);
+#undef SSB_GW
 }
 
 // proj [T, ld] holds q and the gate's pre-activation (n_heads x dim each) and v (n_heads x vdim) from the given columns;
@@ -535,7 +421,7 @@ tied_step_kernel(const T* __restrict__ proj, int ld, int q_off, int f_off, int v
                  const float* __restrict__ lower, float* __restrict__ state, const int* __restrict__ cu_new,
                  const int* __restrict__ seq_slot, const float* __restrict__ w, float eps, T* __restrict__ y, int ldy,
                  int n_heads, int dim, int vdim) {
-    __shared__ float k_s[SCAN_MAX_ROWS * SCAN_GROUPS], q_s[SCAN_MAX_ROWS * SCAN_GROUPS];
+    __shared__ float k_s[SCAN_MAX_DIM], q_s[SCAN_MAX_DIM];
     __shared__ float o_s[TS_WARPS][NC * 32];
     __shared__ float red[TS_WARPS];
     const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -605,7 +491,7 @@ SSB_API int ssb_tied_step(const void* proj, int ld, int dtype, int q_off, int f_
                           const float* lower, float* state, const int* cu_new, const int* seq_slot, const float* w, float eps,
                           void* y, int ldy, int n_seqs, int n_heads, int dim, int vdim, int pdl, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
-    if (dim <= 0 || dim > SCAN_MAX_ROWS * SCAN_GROUPS || vdim <= 0 || n_heads <= 0 || n_heads > 65535 || z_bias == nullptr ||
+    if (dim <= 0 || dim > SCAN_MAX_DIM || vdim <= 0 || n_heads <= 0 || n_heads > 65535 || z_bias == nullptr ||
         lower == nullptr)
         return SSB_ERR_BAD_SIZE;
     if (vdim > TS_MAX_VDIM) return SSB_ERR_UNSUPPORTED;

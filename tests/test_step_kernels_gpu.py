@@ -125,3 +125,33 @@ def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top
         alone, got = seeds[lo:lo + 9].clone(), torch.empty(9, dtype=torch.int32, device=DEV)
         ops().sample(lg[lo:lo + 9].contiguous(), 0.7, top_k, 1.0, None, alone, got)
         assert torch.equal(got, out[lo:lo + 9])
+
+
+@pytest.mark.parametrize("H,d,dv", [(4, 256, 512), (3, 40, 24), (2, 128, 72)])
+def test_gated_scan_in_register_tiles(H, d, dv):
+    """Runs long and short of whole turns of eight tokens, whole and in chunks, against the recurrence in float64; float32
+    sums of d terms after hundreds of float32 state updates: 2e-6 relative."""
+    lens = [70, 9, 133]
+    T, B = sum(lens), len(lens)
+    proj, z0, bias = rnd(T, 2 * H * d + H * dv, seed=d), rnd(T, H * d, seed=1), rnd(H * d, seed=2) + 1.0
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    cu, slots, state0 = i32([0, 70, 79, 212]), i32([2, 0, 3]), rnd(4, H * d * dv, seed=3)
+    decay = (torch.sigmoid((z0 + bias).double()) ** (1 / 16)).view(T, H, d)
+    q, k, v = proj[:, :H * d].double().view(T, H, d), proj[:, H * d:2 * H * d].double().view(T, H, d), proj[:, 2 * H * d:].double().view(T, H, dv)
+    want, end, at = torch.empty(T, H, dv, dtype=torch.float64, device=DEV), state0.double().view(4, H, d, dv).clone(), 0
+    for slot, n in zip((2, 0, 3), lens):
+        S = end[slot]
+        for t in range(at, at + n):
+            S = decay[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+            want[t] = torch.einsum("hdv,hd->hv", S, q[t]) * 0.25
+        end[slot] = S
+        at += n
+    for chunk in (0, 24, 64):
+        n = -(-max(lens) // chunk) if chunk else 0
+        sums = torch.empty(max(B * n * H * d * dv, 1), device=DEV)
+        decays = torch.empty(max(B * n * H * d, 1), device=DEV)
+        state, z, out = state0.clone(), z0.clone(), torch.empty(T, H * dv, device=DEV)
+        ops().gated_linear_scan(proj, 0, H * d, 2 * H * d, z, bias, 16.0, 0.25, state, cu, slots, out, H, d, dv, chunk=chunk,
+                                max_new=max(lens), sums=sums if chunk else None, decays=decays if chunk else None)
+        assert float((out.double() - want.view(T, -1)).norm() / want.norm()) < 2e-6, chunk
+        assert float((state.double().view(-1) - end.view(-1)).norm() / end.norm()) < 2e-6, chunk
