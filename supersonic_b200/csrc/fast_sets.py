@@ -421,12 +421,31 @@ class FastKernels(PlainKernels):
                               pdl=self._chain(batch.n_tokens))
         return True
 
+    @staticmethod
+    def _most_pages(batch) -> int:
+        """The most pages a sequence of this batch can span: the upper end of its bucket."""
+        return 2 * batch.kv_pages - 1 if batch.kv_pages > 1 else 1
+
+    def _shares(self, batch, n_kv: int, pages: int) -> int:
+        """Blocks of a cluster that share the pages of a (sequence, kv head) in a decode step: as many as leave a block an SM
+        and a page or more a block; a sequence of fewer than four pages stays in one, the exchange costs more than it
+        saves there (a step of 8 Ronelorn sequences of two pages: 2.7 % slower shared).  Deterministic sets keep one order."""
+        if not batch.is_decode or self.deterministic:
+            return 1
+        for c in (8, 4, 2):
+            if batch.n_seqs * n_kv * c <= ops.sm_count() and max(c, 4) <= pages:
+                return c
+        return 1
+
     def sigmoid_attention(self, q, k_cache, v_cache, batch, page_table, bias, out, n_q, n_kv, dim, vdim, page_shift,
                           chunk, window, scale):
         if ops.sigmoid_attention_mma_ok(q, k_cache, v_cache, out, dim, vdim, page_shift):
+            pages = self._most_pages(batch)
+            if chunk or window:
+                pages = min(pages, -(-min(c for c in (chunk, window) if c) >> page_shift) + 1)
             ops.sigmoid_attention_mma(q, k_cache, v_cache, batch.cu_new, batch.seq_start, batch.seq_slot, page_table, bias,
                                       out, batch.max_new, n_q, n_kv, dim, vdim, page_shift, chunk, window, scale,
-                                      pdl=self._chain(batch.n_tokens))
+                                      pdl=self._chain(batch.n_tokens), cluster=self._shares(batch, n_kv, pages))
         else:
             super().sigmoid_attention(q, k_cache, v_cache, batch, page_table, bias, out, n_q, n_kv, dim, vdim, page_shift,
                                       chunk, window, scale)
@@ -446,10 +465,14 @@ class FastKernels(PlainKernels):
         if value_position is not None:
             vcos, vsin, _ = value_position.rotary_tables()
             v_inter = bool(getattr(value_position, "interleaved", False))
+        pages = self._most_pages(batch)
+        if window:
+            pages = min(pages, (window >> page_shift) + 2) + (-(-pages // pool) if pool else 0)     # and those of pooled runs
         ops.window_attention_mma(q, k_cache, v_cache, table, pooled, batch.cu_new, batch.seq_start, batch.seq_slot, out,
                                  batch.max_new, n_q, n_kv, dim, vdim, page_shift, window, keep_first, pool, scale, softcap,
                                  sinks, vcos, vsin, v_inter, out_scale, pdl=self._chain(batch.n_tokens), v_share=v_share,
-                                 gate=gate, gate_elems=gate_elems, slopes=slopes, head_mul=head_mul)
+                                 gate=gate, gate_elems=gate_elems, slopes=slopes, head_mul=head_mul,
+                                 cluster=self._shares(batch, n_kv, pages))
 
     def gated_linear_scan(self, proj, q_off, k_off, v_off, z, z_bias, tau, q_scale, state, batch, out, n_heads,
                           dim, vdim):

@@ -1206,10 +1206,11 @@ def sigmoid_attention_mma(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
                           seq_start: torch.Tensor, seq_slot: torch.Tensor, page_table: torch.Tensor,
                           bias: Optional[torch.Tensor], out: torch.Tensor, max_new: int, n_q: int, n_kv: int, dim: int,
                           vdim: int, page_shift: int, chunk: Optional[int], window: Optional[int], scale: float,
-                          split: Optional[bool] = None, pdl: bool = False) -> None:
+                          split: Optional[bool] = None, pdl: bool = False, cluster: int = 1) -> None:
     """``sigmoid_attention_plain`` on mma.sync for bfloat16: a block streams a sequence's pages once for a tile of
     (token, head of one kv group) rows; weights float32, entering the second product as hi + lo bfloat16.
-    ``split`` (default: steps of one token a sequence): 16 rows a block, the warps share a page's keys."""
+    ``split`` (default: steps of one token a sequence): 16 rows a block, the warps share a page's keys; ``cluster``
+    (1 to 8) blocks share the pages."""
     if not sigmoid_attention_mma_ok(q, k_cache, v_cache, out, dim, vdim, page_shift) or n_q % n_kv:
         raise KernelError(f"sigmoid_attention_mma: dim {dim}, vdim {vdim}, heads {n_q}/{n_kv} or operands not supported")
     _need(cu_new, "cu_new", torch.int32, 1); _need(seq_start, "seq_start", torch.int32, 1); _need(seq_slot, "seq_slot", torch.int32, 1)
@@ -1229,7 +1230,7 @@ def sigmoid_attention_mma(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
         _ptr(page_table), c_int(page_table.shape[1]), _ptr(bias), _ptr(out), c_int(out.stride(0)), c_int(B),
         c_int(max_new), c_int(n_q), c_int(n_kv), c_int(dim), c_int(vdim), c_int(page_shift),
         c_int(int(chunk) if chunk else 0), c_int(int(window) if window else 0), c_float(scale), c_int(1 if split else 0),
-        c_int(1 if pdl else 0), _stream()), "sigmoid_attention_mma")
+        c_int(cluster if split else 1), c_int(1 if pdl else 0), _stream()), "sigmoid_attention_mma")
 
 
 def sigmoid_attention_plain(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos: torch.Tensor,
@@ -1472,11 +1473,12 @@ def window_attention_mma(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
                          v_cos: Optional[torch.Tensor], v_sin: Optional[torch.Tensor], v_interleaved: bool,
                          out_scale: float = 1.0, split: Optional[bool] = None, pdl: bool = False, v_share: int = 1,
                          gate: Optional[torch.Tensor] = None, gate_elems: bool = False,
-                         slopes: Optional[torch.Tensor] = None, head_mul: Optional[torch.Tensor] = None) -> None:
+                         slopes: Optional[torch.Tensor] = None, head_mul: Optional[torch.Tensor] = None,
+                         cluster: int = 1) -> None:
     """``window_attention_plain`` on mma.sync for bfloat16: a block streams what a tile of (token, head of one kv
     group) rows can see once (pooled rows, kept first tokens, the window's pages); scores, weights and sums
     float32, the weights entering the second product as hi + lo bfloat16.  ``split`` (default: steps of one
-    token a sequence): 16 rows a block, the warps share a page's keys."""
+    token a sequence): 16 rows a block, the warps share a page's keys; ``cluster`` (1 to 8) blocks share the pages."""
     if not window_attention_mma_ok(q, k_cache, v_cache, pooled if pool else None, out, dim, vdim, page_shift):
         raise KernelError(f"window_attention_mma: dim {dim}, vdim {vdim} or operands not supported")
     pk, pv, ptable, positions = _window_attention_args(q, k_cache, v_cache, page_table, pooled, out, n_q, n_kv, dim, vdim,
@@ -1497,7 +1499,7 @@ def window_attention_mma(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
         _ptr(None if (sinks is None or isinstance(sinks, bool)) else sinks), c_int(1 if sinks is True else 0), _ptr(v_cos),
         _ptr(v_sin), c_int(1 if v_interleaved else 0), c_int(positions), c_float(out_scale), c_int(v_share), _ptr(gate),
         c_int(gate.stride(0) if gate is not None else 0), c_int(1 if gate_elems else 0), _ptr(slopes), _ptr(head_mul),
-        c_int(1 if split else 0), c_int(1 if pdl else 0), _stream()), "window_attention_mma")
+        c_int(1 if split else 0), c_int(cluster if split else 1), c_int(1 if pdl else 0), _stream()), "window_attention_mma")
 
 
 def map_difference(maps: torch.Tensor, out: torch.Tensor, n_heads: int, n_kv: int, vdim: int, lam: float, eps: float,

@@ -13,6 +13,10 @@
 //   SPLIT = false: 64 rows a block, 16 a warp, every warp over all 64 keys of a page (prompts);
 //   SPLIT = true:  16 rows a block, the four warps take 16 keys each of a page and merge their maxima, sums
 //                  and outputs through shared memory at the end (decode steps: few rows, many keys).
+// A decode step of few sequences has fewer blocks than SMs, and each would stream its pages one after another: the blocks of
+// a cluster then share a (sequence, kv head)'s pages in runs, and merge maxima, sums and outputs through the cluster's
+// shared memory, every block finishing the rows whose number is its rank modulo the cluster's size.  A decode step of 8
+// Ronelorn sequences of 100 to 1,500 tokens: 215.7 us with one block each, 200.9 with up to 8.
 // DIM and VDIM are the padded head sizes (64 or 128); the real ones may be any multiple of 8 up to them: the
 // padding columns of the keys are zero in shared memory, those of the values are never written out.
 #include "common.cuh"
@@ -46,6 +50,7 @@ struct WmArgs {
     int gate_elems;               // ... or one per element of a head's result
     const float* slopes;          // per query head, or none: slope * (p - j) is taken off the score (after the cap)
     const float* head_mul;        // per query head, or none: a factor on the scale
+    int cluster;                  // blocks of a cluster that share a row tile's pages (SPLIT only; 1: none)
 };
 
 template <int DIM, int VDIM, bool SPLIT, int ST>          // ST: pages in the ring
@@ -57,8 +62,9 @@ window_attention_mma_kernel(const WmArgs a) {
     extern __shared__ __align__(16) unsigned char wm_smem[];
     bf16* Ks = reinterpret_cast<bf16*>(wm_smem);          // [ST][64][KP]
     bf16* Vs = Ks + ST * WM_PAGE * KP;                    // [ST][64][VP]
-    __shared__ float m_s[4][16], l_s[4][16], f_s[4][16];
-    const int b = blockIdx.z, kvh = blockIdx.y, tile = blockIdx.x;
+    __shared__ float m_s[4][16], l_s[4][16], f_s[4][16], blk_m[16], blk_l[16];
+    const int shares = SPLIT ? a.cluster : 1, share = SPLIT ? (int)blockIdx.x % shares : 0;
+    const int b = blockIdx.z, kvh = blockIdx.y, tile = blockIdx.x / shares;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int dim = a.dim, vdim = a.vdim, window = a.window, pool = a.pool, n_kv = a.n_kv;
     ssb_pdl_launch_dependents();
@@ -77,7 +83,10 @@ window_attention_mma_kernel(const WmArgs a) {
     const int t_pool = pool > 0 ? (lo_last / pool + WM_PAGE - 1) / WM_PAGE : 0;
     const int t_keep = (min(a.keep_first, lo_last) + WM_PAGE - 1) / WM_PAGE;
     const int page_lo = lo_first / WM_PAGE, page_hi = p_last / WM_PAGE;
-    const int n_tiles = t_pool + t_keep + (page_hi - page_lo + 1);
+    const int all_tiles = t_pool + t_keep + (page_hi - page_lo + 1);
+    // this block's run of them: the tiles are counted from all of the sequence's first
+    const int per_share = (all_tiles + shares - 1) / shares;
+    const int tile0 = min(share * per_share, all_tiles), n_tiles = min(tile0 + per_share, all_tiles);
     const int* pages = a.page_table + (size_t)slot * a.max_pages;
     const int* pool_pages = pool > 0 ? a.pool_table + (size_t)slot * a.pool_max_pages : nullptr;
 
@@ -117,10 +126,10 @@ window_attention_mma_kernel(const WmArgs a) {
     // every turn commits one group, an empty one where no page is left: the wait below counts groups
 #pragma unroll
     for (int i = 0; i < ST - 1; ++i) {
-        if (i < n_tiles) load_tile(i, i, tile_page(i));
+        if (tile0 + i < n_tiles) load_tile(tile0 + i, i, tile_page(tile0 + i));
         else cp_async_commit();
     }
-    int page_ahead = tile_page(ST - 1);
+    int page_ahead = tile_page(tile0 + ST - 1);
 
     // this warp's rows: g and g + 8 of its 16
     const int wrow0 = row0 + (SPLIT ? 0 : warp * 16);
@@ -160,11 +169,11 @@ window_attention_mma_kernel(const WmArgs a) {
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};     // l_run: this thread's share of the row's sum
     const float inv_cap = a.softcap > 0.f ? 1.0f / a.softcap : 0.f;
 
-    for (int t = 0; t < n_tiles; ++t) {
-        const int stage = t % ST;
+    for (int t = tile0; t < n_tiles; ++t) {
+        const int stage = (t - tile0) % ST;
         const int page_now = page_ahead;
         page_ahead = tile_page(t + ST);
-        if (t + ST - 1 < n_tiles) load_tile(t + ST - 1, (t + ST - 1) % ST, page_now);   // the stage the turn before this one left
+        if (t + ST - 1 < n_tiles) load_tile(t + ST - 1, (t - tile0 + ST - 1) % ST, page_now);   // the stage the turn before this one left
         else cp_async_commit();
         cp_async_wait<ST - 1>();
         __syncthreads();
@@ -276,6 +285,7 @@ window_attention_mma_kernel(const WmArgs a) {
         __syncthreads();                                  // the stage is free for the tile after next
     }
 
+    if (SPLIT && tile0 >= n_tiles) __syncthreads();       // a share without pages: the padding's zeros come before the sums
     // the rows' sums, divided, as float32 [ROWS][VDIM] where the pages were staged
     float* fin = reinterpret_cast<float*>(wm_smem);
     const bool has_sink = a.sinks != nullptr || a.zero_sink;
@@ -323,7 +333,7 @@ window_attention_mma_kernel(const WmArgs a) {
             const int R = row0 + tid;
             float m = fmaxf(fmaxf(m_s[0][tid], m_s[1][tid]), fmaxf(m_s[2][tid], m_s[3][tid]));
             float sink_term = 0.f;
-            if (has_sink && R < n_rows) {
+            if (has_sink && R < n_rows && shares == 1) {
                 const float sk = a.sinks != nullptr ? a.sinks[kvh * G + R % G] : 0.f;
                 m = fmaxf(m, sk);
                 sink_term = __expf(sk - m);
@@ -334,9 +344,11 @@ window_attention_mma_kernel(const WmArgs a) {
                 f[w] = (m_s[w][tid] == -INFINITY) ? 0.f : __expf(m_s[w][tid] - m);
                 l += l_s[w][tid] * f[w];
             }
-            const float inv = l > 0.f ? 1.0f / l : 0.f;
+            const float inv = shares > 1 ? 1.0f : l > 0.f ? 1.0f / l : 0.f;
 #pragma unroll
             for (int w = 0; w < 4; ++w) f_s[w][tid] = f[w] * inv;
+            blk_m[tid] = m;
+            blk_l[tid] = l;
         }
         __syncthreads();
         for (int e = tid; e < 16 * VDIM; e += WM_THREADS) {
@@ -345,12 +357,36 @@ window_attention_mma_kernel(const WmArgs a) {
                      red[3 * 16 * VDIM + e] * f_s[3][r];
         }
         __syncthreads();
+        if (shares > 1) {
+            ssb_cluster_sync();                           // every block's maxima, sums and outputs are in place
+            for (int r = share; r < 16 && row0 + r < n_rows; r += shares) {
+                float m = -INFINITY, l = 0.f;
+                for (int q = 0; q < shares; ++q) m = fmaxf(m, ssb_cluster_f32(&blk_m[r], q));
+                const float sk = a.sinks != nullptr ? a.sinks[kvh * G + (row0 + r) % G] : 0.f;
+                if (has_sink) m = fmaxf(m, sk);
+                for (int q = 0; q < shares; ++q) {
+                    const float mq = ssb_cluster_f32(&blk_m[r], q);
+                    if (mq != -INFINITY) l += ssb_cluster_f32(&blk_l[r], q) * __expf(mq - m);
+                }
+                if (has_sink) l += __expf(sk - m);
+                const float inv = l > 0.f ? 1.0f / l : 0.f;
+                for (int c = tid; c < VDIM; c += WM_THREADS) {
+                    float x = 0.f;
+                    for (int q = 0; q < shares; ++q) {
+                        const float mq = ssb_cluster_f32(&blk_m[r], q);
+                        if (mq != -INFINITY) x += ssb_cluster_f32(&red[r * VDIM + c], q) * (__expf(mq - m) * inv);
+                    }
+                    red[r * VDIM + c] = x;                // only this block reads its own copy of its rows
+                }
+            }
+            __syncthreads();
+        }
     }
     // turned back by the row's position where values are stored turned, times out_scale, as bfloat16 pairs
     const int half = vdim >> 1;
     for (int e = tid; e < ROWS * half; e += WM_THREADS) {
         const int r = e / half, c2 = e - r * half, R = row0 + r;
-        if (R >= n_rows) continue;
+        if (R >= n_rows || (SPLIT && r % shares != share)) continue;
         const int tok = R / G, head = kvh * G + R % G, p = start + tok;
         const int c = 2 * c2;
         float x0 = fin[(size_t)r * VDIM + c], x1 = fin[(size_t)r * VDIM + c + 1];
@@ -383,6 +419,7 @@ window_attention_mma_kernel(const WmArgs a) {
         bf16* o = a.out + (size_t)(t0 + tok) * a.ldo + (size_t)head * vdim + c;
         *reinterpret_cast<uint32_t*>(o) = pack2(x0 * mul, x1 * mul1);
     }
+    if (SPLIT && shares > 1) ssb_cluster_sync();          // no block leaves while its outputs may be read
 }
 
 template <int DIM, int VDIM, bool SPLIT, int ST>
@@ -397,14 +434,15 @@ static int launch_window_mma(const WmArgs& a, int n_seqs, int max_new, int pdl, 
         if (e != cudaSuccess) return (int)e;
     }
     const int rows = max_new * (a.n_q / a.n_kv);
-    const dim3 grid((rows + ROWS - 1) / ROWS, a.n_kv, n_seqs);
+    const dim3 grid((rows + ROWS - 1) / ROWS * (SPLIT ? a.cluster : 1), a.n_kv, n_seqs);
     if (grid.y > 65535 || grid.z > 65535) return SSB_ERR_BAD_SIZE;
-    const int rc = ssb_launch(kern, grid, dim3(WM_THREADS), smem, stream, pdl != 0, a);
+    const int rc = ssb_launch_cluster(kern, grid, dim3(WM_THREADS), smem, stream, pdl != 0, SPLIT ? a.cluster : 1, a);
     return rc ? rc : ssb_launch_status();
 }
 
 // q [T, ldq] bfloat16 (n_q x dim, normed and rotated); the caches' pages hold 64 rows (page_shift 6); dim and vdim
-// multiples of 8 up to 128; ldq and ldo multiples of 2 elements.  split: the decode form (16 rows a block).
+// multiples of 8 up to 128; ldq and ldo multiples of 2 elements.  split: the decode form (16 rows a block), whose pages
+// `cluster` blocks share (1 to 8).
 SSB_API int ssb_window_attention_mma(const void* q, int ldq, const void* k_cache, const void* v_cache, const int* page_table,
                                      int max_pages, const void* pk_cache, const void* pv_cache, const int* pool_table,
                                      int pool_max_pages, const int* cu_new, const int* seq_start, const int* seq_slot,
@@ -413,7 +451,7 @@ SSB_API int ssb_window_attention_mma(const void* q, int ldq, const void* k_cache
                                      const float* sinks, int zero_sink, const float* vcos_t, const float* vsin_t,
                                      int v_interleaved, int table_positions, float out_scale, int v_share, const void* gate,
                                      int ldg, int gate_elems, const float* slopes, const float* head_mul, int split,
-                                     int pdl, cudaStream_t stream) {
+                                     int cluster, int pdl, cudaStream_t stream) {
     if (n_seqs <= 0 || max_new <= 0) return 0;
     if (v_share < 1 || n_kv <= 0 || n_kv % v_share || (pool > 0 && (v_share > 1 || slopes != nullptr))) return SSB_ERR_BAD_SIZE;
     if (page_shift != 6 || n_kv <= 0 || n_q % n_kv || (ldq & 1) || (ldo & 1) || window < 0 || keep_first < 0 || pool < 0 ||
@@ -436,8 +474,10 @@ SSB_API int ssb_window_attention_mma(const void* q, int ldq, const void* k_cache
     a.out_scale = out_scale;
     a.v_share = v_share; a.gate = (const bf16*)gate; a.ldg = ldg;
     a.gate_elems = gate_elems; a.slopes = slopes; a.head_mul = head_mul;
+    if (cluster < 1 || cluster > 8 || (cluster > 1 && !split)) return SSB_ERR_BAD_SIZE;
+    a.cluster = cluster;
     const int D = dim <= 64 ? 64 : 128, V = vdim <= 64 ? 64 : 128;
-    const long long blocks = (long long)((max_new * (n_q / n_kv) + 15) / 16) * n_kv * n_seqs;     // of the decode form
+    const long long blocks = (long long)((max_new * (n_q / n_kv) + 15) / 16) * n_kv * n_seqs * cluster;     // of the decode form
     const bool deep = split && blocks <= WM_DEEP_MAX_BLOCKS;
 #define SSB_WM(D_, V_) \
     if (D == D_ && V == V_) \

@@ -155,3 +155,42 @@ def test_gated_scan_in_register_tiles(H, d, dv):
                                 max_new=max(lens), sums=sums if chunk else None, decays=decays if chunk else None)
         assert float((out.double() - want.view(T, -1)).norm() / want.norm()) < 2e-6, chunk
         assert float((state.double().view(-1) - end.view(-1)).norm() / end.norm()) < 2e-6, chunk
+
+
+@pytest.mark.parametrize("kind", ["window", "pooled", "all", "sigmoid"])
+@pytest.mark.parametrize("dim", [128, 64])
+def test_a_cluster_of_blocks_shares_a_decode_steps_pages(kind, dim):
+    """Every size of cluster against one block a (sequence, kv head), on sequences of one token, of fewer pages than blocks,
+    of a window's edge and of many pages: float32 sums of a row merged in another order, then one rounding to bfloat16."""
+    lens, n_q, n_kv = [1, 63, 64, 65, 130, 517, 700], 6, 2
+    B, pages = len(lens), sum((n + 63) // 64 for n in lens)
+    perm = torch.randperm(pages + 2, generator=torch.Generator().manual_seed(dim)).to(torch.int32)
+    table, ptable, at = torch.zeros(B, 16, dtype=torch.int32), torch.arange(B, dtype=torch.int32)[:, None].repeat(1, 2), 0
+    for b, n in enumerate(lens):
+        table[b, :(n + 63) // 64] = perm[at:at + (n + 63) // 64]
+        at += (n + 63) // 64
+    k, v = (rnd(pages + 2, n_kv, 64, dim, seed=s, dtype=torch.bfloat16) for s in (1, 2))
+    pk, pv = (rnd(B, n_kv, 64, dim, seed=s, dtype=torch.bfloat16) for s in (3, 4))
+    q = rnd(B, n_q * dim, seed=5, dtype=torch.bfloat16)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    cu, start, slots, table, ptable = i32(list(range(B + 1))), i32([n - 1 for n in lens]), i32(list(range(B))), table.to(DEV), ptable.to(DEV)
+    gate, sinks = rnd(B, n_q, seed=6, dtype=torch.bfloat16), rnd(n_q, seed=7)
+    cos, sin = torch.cos(rnd(800, dim // 2, seed=8)), torch.sin(rnd(800, dim // 2, seed=8))
+
+    def run(cluster):
+        out = torch.full((B, n_q * dim), 9.0, device=DEV, dtype=torch.bfloat16)
+        if kind == "sigmoid":
+            ops().sigmoid_attention_mma(q, k, v, cu, start, slots, table, sinks, out, 1, n_q, n_kv, dim, dim, 6, 256, None,
+                                        dim ** -0.5, split=True, cluster=cluster)
+            return out.float()
+        pooled = (pk, pv, ptable) if kind == "pooled" else None
+        ops().window_attention_mma(q, k, v, table, pooled, cu, start, slots, out, 1, n_q, n_kv, dim, dim, 6,
+                                   None if kind == "all" else 128, 3 if kind == "window" else 0, 16 if pooled else 0, dim ** -0.5,
+                                   30.0, sinks if kind != "pooled" else None, cos if pooled else None, sin if pooled else None,
+                                   False, split=True, gate=gate, cluster=cluster)
+        return out.float()
+    one = run(1)
+    for cluster in (2, 3, 4, 8):
+        got = run(cluster)
+        # a value next to a rounding boundary may go either way: one step of bfloat16, 2^-8 of its size
+        assert bool(((got - one).abs() <= 2.0 ** -7 * one.abs() + 1e-6).all()), cluster
