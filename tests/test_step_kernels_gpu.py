@@ -194,3 +194,34 @@ def test_a_cluster_of_blocks_shares_a_decode_steps_pages(kind, dim):
         got = run(cluster)
         # a value next to a rounding boundary may go either way: one step of bfloat16, 2^-8 of its size
         assert bool(((got - one).abs() <= 2.0 ** -7 * one.abs() + 1e-6).all()), cluster
+
+
+@pytest.mark.parametrize("dim,vdim,n_q,n_kv,n_v", [(128, 128, 16, 4, 4), (64, 64, 32, 8, 8), (64, 128, 40, 20, 10), (128, 64, 3, 1, 1)])
+@pytest.mark.parametrize("norm,rot,interleaved", [("head", 64, False), ("row", 32, True), (None, 0, False), ("head", 16, False)])
+def test_rows_prepared_a_warp_a_head(dim, vdim, n_q, n_kv, n_v, norm, rot, interleaved):
+    """Against the kernel that takes any width (which rows at an odd address still get): queries, cached keys and values, and
+    the pooled rows of tokens that end a run; float32 in between, so one step of bfloat16 apart at the most."""
+    T, pool = 7, (16 if n_v == n_kv else 0)
+    width, positions = (n_q + n_kv) * dim + n_v * vdim, [0, 15, 63, 64, 127, 200, 31]
+    rows = rnd(T, width + 8, seed=dim + n_q, dtype=torch.bfloat16)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos, slots = i32(positions), i32([0, 1, 2, 3, 4, 5, -1])
+    table = torch.arange(6 * 4, dtype=torch.int32, device=DEV).view(6, 4)
+    ptable = torch.arange(6, dtype=torch.int32, device=DEV).view(6, 1)
+    qw, kw = (rnd(dim if norm == "head" else n * dim, seed=n) + 1.0 for n in (n_q, n_kv))
+    cos, sin = (f(rnd(256, rot // 2, seed=5)) for f in (torch.cos, torch.sin)) if rot else (None, None)
+    vcos, vsin = (f(rnd(256, vdim // 2, seed=6)) for f in (torch.cos, torch.sin))
+    mix = (rnd(T, n_v * vdim, seed=9, dtype=torch.bfloat16), 0.3)
+    got = []
+    for odd in (True, False):
+        qkv = rows.clone()[:, 2:2 + width] if odd else rows[:, 2:2 + width].contiguous()
+        k, v = (rnd(24, n, 64, d, seed=n, dtype=torch.bfloat16) for n, d in ((n_kv, dim), (n_v, vdim)))
+        pk, pv = (torch.zeros(6, n_kv, 64, d, device=DEV, dtype=torch.bfloat16) for d in (dim, vdim))
+        ops().qkv_prepare(qkv, qw if norm else None, kw if norm else None, norm, 1e-5, cos, sin, rot, interleaved, vcos, vsin,
+                          interleaved, pos, slots, table, k, v, n_q, n_kv, dim, vdim, 6, pooled=(pk, pv, ptable) if pool else None,
+                          pool=pool, n_v=n_v, v_mix=mix, q_temp=(0.2, 8))
+        got.append([x.float() for x in (qkv[:, : n_q * dim], k, v, pk, pv)])
+    for a, b in zip(*got):
+        assert bool(((a - b).abs() <= 2.0 ** -7 * a.abs() + 1e-5).all())
+    if pool:                                                        # the tokens at 15, 63 and 127 end a run
+        assert (got[1][3].abs().sum((1, 2, 3)) > 0).tolist() == [False, True, True, False, True, False]
