@@ -28,10 +28,14 @@ constexpr int GV_BM = 128;                // rows of W per block
 __host__ __device__ constexpr int gv_stages(int bnb) { return bnb <= 16 ? 6 : (bnb <= 32 ? 5 : (bnb <= 64 ? 4 : 3)); }
 constexpr int GV_MAX_ROWS = 128;
 constexpr unsigned GV_ROT = 5;            // k-blocks by which neighbouring row tiles start apart (see the producer)
-constexpr int GV_THREADS = 192;           // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5: epilogue
+// warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5: epilogue; from 64 batch rows on warps 6-9 too, which take the second
+// half of the rows: a block's last step is serial to its products (a decode step of 64 sequences, 1B: 1,111 us with one group
+// of warps, 1,040 with two)
+__host__ __device__ constexpr int gv_groups(int bnb) { return bnb >= 64 ? 2 : 1; }
+__host__ __device__ constexpr int gv_threads(int bnb) { return 64 + 128 * gv_groups(bnb); }
 
 template <int BNB>                        // batch rows per tile: 16, 32, 64 or 128
-__global__ void __launch_bounds__(GV_THREADS, 2)
+__global__ void __launch_bounds__(gv_threads(BNB), 2)
 gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                void* __restrict__ out, int ldo, int out_is_f32, int n_rows, int N, int K, int mode, int splits,
                float* __restrict__ partials, int* __restrict__ counters, int* __restrict__ error_word, int gate_kind, float gate_limit, const float* __restrict__ row_scale) {
@@ -133,7 +137,9 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     } else {
         // epilogue: thread = one row of W (tensor-memory lane); the BNB batch columns are taken CW at a
         // time so that a pass's sums fit the registers
-        constexpr int CW = BNB < 64 ? BNB : 64;
+        constexpr int COLS = BNB / gv_groups(BNB), CW = COLS < 64 ? COLS : 64, EPI = 128 * gv_groups(BNB);
+        // this group's batch rows: g0 .. g0 + COLS - 1
+        const int g0 = gv_groups(BNB) > 1 ? (warp - 2) / 4 * COLS : 0;
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;                   // row within the tile
         const int n = n0 + r;
@@ -144,7 +150,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             ok = mbar_wait(acc_full, 0, abort_flag);
             if (!ok) { *abort_flag = 1; atomicCAS(error_word, 0, TC_ERR_EPILOGUE); }
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");       // the four epilogue warps agree on the outcome
+        asm volatile("bar.sync 1, %0;" ::"n"(EPI) : "memory");       // the epilogue warps agree on the outcome
         ok = abort_flag[0] == 0;
         if (ok && my_blocks > 0) tc_fence_after();
         // this block's sums of columns c0 .. c0 + CW - 1 (zeros for a block without k-blocks)
@@ -172,25 +178,26 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         if (ok && through_scratch) {
             // partial tile to scratch; the block that arrives last adds all of them in split order
             float* mine = partials + (((size_t)tile * splits + split) * GV_BM + r) * BNB;
-            for (int c0 = 0; c0 < BNB; c0 += CW) {
+            for (int c0 = g0; c0 < g0 + COLS; c0 += CW) {
                 own_sums(c0);
 #pragma unroll
                 for (int j = 0; j < CW; j += 4)
                     *reinterpret_cast<float4*>(mine + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             }
             __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");   // the four epilogue warps
+            asm volatile("bar.sync 1, %0;" ::"n"(EPI) : "memory");
             if (warp == 2 && lane == 0) {
                 const int arrived = atomicAdd(counters + tile, 1);
                 *is_last = (arrived == splits - 1);
                 if (*is_last) counters[tile] = 0;            // ready for the next launch
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            asm volatile("bar.sync 1, %0;" ::"n"(EPI) : "memory");
             ok = *is_last != 0;
             if (ok) __threadfence();
         }
         if (ok) {
-            for (int c0 = 0; c0 < BNB; c0 += CW) {
+            for (int c0 = g0; c0 < g0 + COLS; c0 += CW) {
+                if (gv_groups(BNB) > 1 && c0 >= n_rows) break;
                 if (through_scratch) {
 #pragma unroll
                     for (int j = 0; j < CW; ++j) v[j] = 0.f;
@@ -264,7 +271,7 @@ static int launch_gv(const CUtensorMap& mw, const CUtensorMap& mx, void* out, in
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    const int rc = ssb_launch(kern, dim3((N + GV_BM - 1) / GV_BM, splits), dim3(GV_THREADS), smem, stream, pdl, mw, mx,
+    const int rc = ssb_launch(kern, dim3((N + GV_BM - 1) / GV_BM, splits), dim3(gv_threads(BNB)), smem, stream, pdl, mw, mx,
                               out, ldo, out_is_f32, n_rows, N, K, mode, splits, partials, counters, error_word, gate_kind, gate_limit,
                               row_scale);
     return rc ? rc : ssb_launch_status();
