@@ -48,23 +48,68 @@ struct TcRope {
     const float* row_scale;    // ... and one factor per row of the result, or none
 };
 
-__device__ __forceinline__ void tc_store32_bf16(__nv_bfloat16* dst, const float (&v)[32]) {
+// A warp's 32 rows of WORDS 32-bit words each, a row a lane, to memory as whole runs: the rows meet in shared memory and go
+// out several lanes a row, whole runs of memory an instruction instead of 16 bytes of each of 32 rows.  ``dst``: the warp's first
+// row; ADD: float32 added in memory (red.global.add.v4.f32), which nobody waits for.
+constexpr int TC_STAGE_LD = 36;                               // words a row (of 32 or less): eight rows start in eight groups of four banks
+constexpr int TC_STAGE_BYTES = 4 * 32 * TC_STAGE_LD * 4;      // of the four epilogue warps
+
+template <int WORDS, bool ADD>
+__device__ __forceinline__ void tc_put_rows(float* stage, const uint32_t (&v)[WORDS], char* dst, size_t row_bytes, int rows) {
+    constexpr int LD = WORDS + 4, PER = WORDS / 4, ROWS = 32 / PER;
+    static_assert(LD <= TC_STAGE_LD, "");
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < WORDS; j += 4)
+        *reinterpret_cast<uint4*>(stage + lane * LD + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int r0 = 0; r0 < 32; r0 += ROWS) {
+        const int r = r0 + lane / PER, c = lane % PER * 4;
+        const float4 x = *reinterpret_cast<const float4*>(stage + r * LD + c);
+        if (r < rows) {
+            float4* at = reinterpret_cast<float4*>(dst + (size_t)r * row_bytes) + lane % PER;
+            if (ADD) atomicAdd(at, x);
+            else *at = x;
+        }
+    }
+    __syncwarp();
+}
+
+// The same for 32 bfloat16 values a lane whose rows lie anywhere: lane r's go to dst + at (dst null: nowhere).
+__device__ __forceinline__ void tc_put32_bf16(float* stage, const float (&v)[32], bf16* dst, int at) {
+    constexpr int LD = 20;
+    const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int j = 0; j < 32; j += 8) {
-        uint4 u;
-        __nv_bfloat162 p0 = __floats2bfloat162_rn(v[j], v[j + 1]), p1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
-        __nv_bfloat162 p2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]), p3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-        u.x = *reinterpret_cast<uint32_t*>(&p0); u.y = *reinterpret_cast<uint32_t*>(&p1);
-        u.z = *reinterpret_cast<uint32_t*>(&p2); u.w = *reinterpret_cast<uint32_t*>(&p3);
-        *reinterpret_cast<uint4*>(dst + j) = u;
+        uint32_t p[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[j + 2 * e], v[j + 2 * e + 1]);
+            p[e] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+        *reinterpret_cast<uint4*>(stage + lane * LD + j / 2) = make_uint4(p[0], p[1], p[2], p[3]);
     }
+    __syncwarp();
+#pragma unroll
+    for (int r0 = 0; r0 < 32; r0 += 8) {
+        const int r = r0 + lane / 4;
+        bf16* row = reinterpret_cast<bf16*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst), r));
+        const uint4 x = *reinterpret_cast<const uint4*>(stage + r * LD + lane % 4 * 4);
+        if (row != nullptr) reinterpret_cast<uint4*>(row + at)[lane % 4] = x;
+    }
+    __syncwarp();
 }
 
 // One warp's share of a finished tile: tensor-memory lanes 32 * quarter .. + 31 (rows of the
-// tile; ``row`` is this thread's row of C) and BN accumulator columns from column address ``acc``.
+// tile; ``row`` is this thread's row of C) and BN accumulator columns from column address ``acc``; ``stage``: its shared memory.
+// Sums that are added to a float32 result are added in memory, whether K is cut into parts or not: a load of what was there,
+// waited for before every store, was most of the epilogue (2,048 x 2,048 x 2,048, pairs: 35.6 us with loads and stores, 29.5 added
+// in memory row by row, 25.6 with the rows staged as above; results stored in bfloat16, 2,048 x 16,384 x 2,048: 128 and 113).
+// One addition an element either way, so a result without parts has the same bits.
 template <int BN>
 __device__ __forceinline__ void tc_epilogue(uint32_t acc, int quarter, int row, int n0, int M, int N, void* __restrict__ C,
-                                            int ldc, int out_is_f32, int mode, bool part, const TcRope& rope) {
+                                            int ldc, int out_is_f32, int mode, float* stage, const TcRope& rope) {
     if (mode == TC_ROPE_APPEND) {
         // a head at a time: its low and high halves meet in this thread (the row's token)
         const int hd = rope.head_dim, half = hd / 2, halves32 = half / 32;
@@ -79,16 +124,16 @@ __device__ __forceinline__ void tc_epilogue(uint32_t acc, int quarter, int row, 
             const int head = (n0 + hh * hd) / hd;
             const bool is_q = head < rope.n_q, is_v = head >= rope.n_q + rope.n_kv;
             const int kvh = is_q ? 0 : (is_v ? head - rope.n_q - rope.n_kv : head - rope.n_q);
-            bf16* dst = is_q ? (bf16*)C + (size_t)row * ldc + (size_t)head * hd
-                             : (is_v ? rope.v_cache : rope.k_cache) +
-                                   (tok + ((size_t)kvh << rope.page_shift)) * hd;
+            bf16* dst = !live || sl < 0 ? nullptr
+                        : is_q ? (bf16*)C + (size_t)row * ldc + (size_t)head * hd
+                               : (is_v ? rope.v_cache : rope.k_cache) +
+                                     (tok + ((size_t)kvh << rope.page_shift)) * hd;
 #pragma unroll 1
             for (int pc = 0; pc < halves32; ++pc) {
                 uint32_t lo_r[32], hi_r[32];
                 const uint32_t at = acc + ((uint32_t)(quarter * 32) << 16) + hh * hd + pc * 32;
                 tc_ld32(at, lo_r);                       // every lane takes part in the loads
                 tc_ld32(at + half, hi_r);
-                if (!live || sl < 0) continue;
                 float lo[32], hi[32];
                 if (is_v) {
 #pragma unroll
@@ -109,24 +154,25 @@ hi[4 * i4 + e] = a_ * sv + b_ * cv;                                             
 #undef TC_ROTATE
                     }
                 }
-                tc_store32_bf16(dst + pc * 32, lo);
-                tc_store32_bf16(dst + half + pc * 32, hi);
+                tc_put32_bf16(stage, lo, dst, pc * 32);
+                tc_put32_bf16(stage, hi, dst, half + pc * 32);
             }
         }
-    } else
+    } else {
+        const int lane = threadIdx.x & 31, row0 = row - lane, rows = M - row0;      // the warp's rows
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
             uint32_t r[32];
             tc_ld32(acc + ((uint32_t)(quarter * 32) << 16) + c * 32, r);
             const int n = n0 + c * 32;
-            if (row >= M || n >= N) continue;
+            if (rows <= 0 || n >= N) continue;
+            const bool whole = n + 32 <= N;
             if (mode == TC_SWIGLU) {
-                bf16* dst = (bf16*)C + (size_t)row * ldc + n / 2;
-                const float rs = rope.row_scale ? rope.row_scale[row] : 1.0f;
+                const float rs = rope.row_scale && row < M ? rope.row_scale[row] : 1.0f;
                 uint32_t packed[8];
-    #pragma unroll
+#pragma unroll
                 for (int g = 0; g < 2; ++g)
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 8; j += 2) {
                         const float g0 = __uint_as_float(r[g * 16 + j]), u0 = __uint_as_float(r[g * 16 + 8 + j]);
                         const float g1 = __uint_as_float(r[g * 16 + j + 1]), u1 = __uint_as_float(r[g * 16 + 9 + j]);
@@ -134,57 +180,48 @@ hi[4 * i4 + e] = a_ * sv + b_ * cv;                                             
                                                                   ssb_gate_fast(g1, u1, rope.gate_kind, rope.gate_limit) * rs);
                         packed[g * 4 + j / 2] = *reinterpret_cast<uint32_t*>(&v);
                     }
-                if (n + 32 <= N) {
-                    reinterpret_cast<uint4*>(dst)[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    reinterpret_cast<uint4*>(dst)[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                } else {
-                    for (int j = 0; j < 16; ++j)            // N is a multiple of 16: whole groups only
-                        if (n + (j / 8) * 16 + 16 <= N) dst[j] = reinterpret_cast<bf16*>(packed)[j];
+                if (whole) {
+                    tc_put_rows<8, false>(stage, packed, (char*)((bf16*)C + (size_t)row0 * ldc + n / 2), (size_t)ldc * 2, rows);
+                } else if (row < M) {                       // N is a multiple of 16: the first group of 8 results only
+                    *reinterpret_cast<uint4*>((bf16*)C + (size_t)row * ldc + n / 2) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
                 }
             } else if (out_is_f32) {
-                float* dst = (float*)C + (size_t)row * ldc + n;
-                if (n + 32 <= N) {
-    #pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        float4 v = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                               __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-                        if (part) { atomicAdd(reinterpret_cast<float4*>(dst + j), v); continue; }
-                        if (mode == TC_ACCUMULATE) {
-                            const float4 o = *reinterpret_cast<const float4*>(dst + j);
-                            v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+                if (whole) {
+                    char* dst = (char*)((float*)C + (size_t)row0 * ldc + n);
+                    if (mode == TC_ACCUMULATE) tc_put_rows<32, true>(stage, r, dst, (size_t)ldc * 4, rows);
+                    else tc_put_rows<32, false>(stage, r, dst, (size_t)ldc * 4, rows);
+                } else if (row < M) {
+                    float* dst = (float*)C + (size_t)row * ldc + n;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (n + j < N) {
+                            if (mode == TC_ACCUMULATE) atomicAdd(dst + j, __uint_as_float(r[j]));
+                            else dst[j] = __uint_as_float(r[j]);
                         }
-                        *reinterpret_cast<float4*>(dst + j) = v;
-                    }
-                } else {
-                    for (int j = 0; j < 32 && n + j < N; ++j) {
-                        if (part) atomicAdd(dst + j, __uint_as_float(r[j]));
-                        else dst[j] = __uint_as_float(r[j]) + (mode == TC_ACCUMULATE ? dst[j] : 0.f);
-                    }
                 }
             } else {
-                bf16* dst = (bf16*)C + (size_t)row * ldc + n;
                 if (mode >= TC_ACT) {                     // on the float32 sums, before their one rounding
-    #pragma unroll
+#pragma unroll
                     for (int j = 0; j < 32; ++j)
                         r[j] = __float_as_uint(ssb_activate(__uint_as_float(r[j]), mode - TC_ACT) * rope.act_scale);
                 }
-                if (n + 32 <= N) {
-    #pragma unroll
-                    for (int j = 0; j < 32; j += 8) {
-                        uint4 v;
-                        __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-                        __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-                        __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(r[j + 4]), __uint_as_float(r[j + 5]));
-                        __nv_bfloat162 p3 = __floats2bfloat162_rn(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7]));
-                        v.x = *reinterpret_cast<uint32_t*>(&p0); v.y = *reinterpret_cast<uint32_t*>(&p1);
-                        v.z = *reinterpret_cast<uint32_t*>(&p2); v.w = *reinterpret_cast<uint32_t*>(&p3);
-                        *reinterpret_cast<uint4*>(dst + j) = v;
-                    }
-                } else {
-                    for (int j = 0; j < 32 && n + j < N; ++j) dst[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
+                uint32_t packed[16];
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                    const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+                    packed[j / 2] = *reinterpret_cast<const uint32_t*>(&p);
+                }
+                if (whole) {
+                    tc_put_rows<16, false>(stage, packed, (char*)((bf16*)C + (size_t)row0 * ldc + n), (size_t)ldc * 2, rows);
+                } else if (row < M) {
+                    bf16* dst = (bf16*)C + (size_t)row * ldc + n;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (n + j < N) dst[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
                 }
             }
         }
+    }
 }
 
 // Order of the tiles: bands of ``group_m`` row tiles; inside a band the row tile runs fastest, then
@@ -228,7 +265,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     // full[STAGES], empty[STAGES], acc_full[2], acc_empty[2]
-    uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE_BYTES);
+    float* put = (float*)(smem + STAGES * STAGE_BYTES);             // the epilogue warps' rows on their way out
+    uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE_BYTES + TC_STAGE_BYTES);
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 2 * N_ACC);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);     // [0]: a role gave up; [1]: stays zero
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -313,7 +351,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // epilogue: warp w may read tensor-memory lanes 32 * (w % 4) .. + 31 = rows of the tile
         const int quarter = warp & 3;
         int i = 0;
-        const bool part = splits > 1;                            // parts of a tile add with atomics
         for (int item = blockIdx.x; item < n_tiles_total * splits; item += gridDim.x, ++i) {
             const TcItem it(item, n_tiles_total, k_blocks, splits);
             const int m0 = (it.tile % m_tiles) * TC_BM, n0 = (it.tile / m_tiles) * BN;
@@ -328,7 +365,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
             tc_fence_after();
             const uint32_t acc = tmem + buf * BN;
-            tc_epilogue<BN>(acc, quarter, row, n0, M, N, C, ldc, out_is_f32, mode, part, rope);
+            tc_epilogue<BN>(acc, quarter, row, n0, M, N, C, ldc, out_is_f32, mode, put + quarter * 32 * TC_STAGE_LD, rope);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty0 + 8 * buf);   // this warp has read its quarter of the region
@@ -360,7 +397,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     constexpr int N_ACC = 2;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE_BYTES);
+    float* put = (float*)(smem + STAGES * STAGE_BYTES);             // the epilogue warps' rows on their way out
+    uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE_BYTES + TC_STAGE_BYTES);
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 2 * N_ACC);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);     // [0]: a role gave up; [1]: stays zero
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -465,7 +503,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 break;
             }
             tc_fence_after();
-            tc_epilogue<BN>(tmem + buf * BN, quarter, row, n0, M, N, C, ldc, out_is_f32, mode, false, rope);
+            tc_epilogue<BN>(tmem + buf * BN, quarter, row, n0, M, N, C, ldc, out_is_f32, mode, put + quarter * 32 * TC_STAGE_LD, rope);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(leader_acc_empty0 + 8 * buf);
@@ -483,7 +521,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 template <int STAGES>
 static int launch_tc_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int ldc, int out_is_f32, int M, int N,
                           int K, int mode, int* error_word, const TcRope& rope, cudaStream_t stream) {
-    constexpr size_t smem = STAGES * 2 * 128 * TC_BK * 2 + (2 * STAGES + 4) * 8 + 16 + 1024;
+    constexpr size_t smem = STAGES * 2 * 128 * TC_BK * 2 + TC_STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024;
     auto kern = gemm_tc_pair_kernel<STAGES>;
     static int max_pairs = 0;
     if (!max_pairs) {
@@ -523,7 +561,7 @@ static int launch_tc_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* C,
 template <int BN, int STAGES>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int ldc, int out_is_f32, int M, int N,
                      int K, int mode, int splits, int* error_word, const TcRope& rope, cudaStream_t stream) {
-    constexpr size_t smem = STAGES * (TC_BM + BN) * TC_BK * 2 + (2 * STAGES + 4) * 8 + 16 + 1024;
+    constexpr size_t smem = STAGES * (TC_BM + BN) * TC_BK * 2 + TC_STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024;
     auto kern = gemm_tc_kernel<BN, STAGES>;
     static bool configured = false;
     if (!configured) {

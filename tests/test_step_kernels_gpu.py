@@ -225,3 +225,24 @@ def test_rows_prepared_a_warp_a_head(dim, vdim, n_q, n_kv, n_v, norm, rot, inter
         assert bool(((a - b).abs() <= 2.0 ** -7 * a.abs() + 1e-5).all())
     if pool:                                                        # the tokens at 15, 63 and 127 end a run
         assert (got[1][3].abs().sum((1, 2, 3)) > 0).tolist() == [False, True, True, False, True, False]
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 64), (31, 40, 128), (33, 72, 64), (129, 264, 192), (257, 1000, 128), (300, 256, 512)])
+@pytest.mark.parametrize("tile", [64, 128, 256, "pair"])
+def test_products_leave_in_whole_rows(m, n, k, tile):
+    """Every way out of the tcgen05 product at ragged edges: the float32 sums stored, the same added to what is there (one
+    rounding, whoever adds), the same rounded to bfloat16; nothing beside the result is touched."""
+    o = ops()
+    tile = o.TC_TILE_PAIR if tile == "pair" else tile
+    a, w, c = rnd(m, k, seed=m, dtype=torch.bfloat16), rnd(n, k, seed=n, dtype=torch.bfloat16), rnd(m, n, seed=k)
+    wide = [torch.full((m + 1, n + 8), 5.0, device=DEV, dtype=t) for t in (torch.float32, torch.float32, torch.bfloat16)]
+    sums, added, rounded = (x[:m, :n] for x in wide)
+    added.copy_(c)
+    for out, mode in ((sums, o.TC_STORE), (added, o.TC_ACCUMULATE), (rounded, o.TC_STORE)):
+        o.gemm_tc(a, w, out, mode, tile_n=tile)
+    o.check_device_errors(torch.device(DEV))
+    want = a.double() @ w.double().t()
+    # k products of float32 sums: k 2^-24 of the sum of their sizes
+    assert bool(((sums.double() - want).abs() <= k * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()) + 1e-30).all())
+    assert torch.equal(added, c + sums) and torch.equal(rounded, sums.to(torch.bfloat16))
+    assert all(bool((x[m] == 5.0).all() and (x[:, n:] == 5.0).all()) for x in wide)
