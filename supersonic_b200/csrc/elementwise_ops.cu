@@ -130,6 +130,8 @@ rope_append_vec_kernel(bf16* __restrict__ qkv, int ld, const float* __restrict__
                        const int* __restrict__ pos, const int* __restrict__ slot, const int* __restrict__ page_table,
                        int max_pages, bf16* __restrict__ k_cache, bf16* __restrict__ v_cache, int n_q, int n_kv,
                        int head_dim, int page_shift) {
+    ssb_pdl_launch_dependents();
+    ssb_pdl_wait();
     const int t = blockIdx.x;
     const int s = slot[t];
     if (s < 0) return;
@@ -172,12 +174,11 @@ rope_append_vec_kernel(bf16* __restrict__ qkv, int ld, const float* __restrict__
 SSB_API int ssb_rope_append_vec(void* qkv, int ld, const float* cos_t, const float* sin_t, int table_positions,
                                 const int* pos, const int* slot, const int* page_table, int max_pages,
                                 void* k_cache, void* v_cache, int n_tokens, int n_q, int n_kv, int head_dim,
-                                int page_shift, cudaStream_t stream) {
+                                int page_shift, int pdl, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (head_dim % 8 || ld % 8 || !cos_t || !sin_t || table_positions <= 0) return SSB_ERR_BAD_SIZE;
     if (((uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15)
         return SSB_ERR_BAD_SIZE;
-    rope_append_vec_kernel<0><<<n_tokens, 256, 0, stream>>>((bf16*)qkv, ld, cos_t, sin_t, pos, slot, page_table, max_pages,
-                                                            (bf16*)k_cache, (bf16*)v_cache, n_q, n_kv, head_dim, page_shift);
-    return ssb_launch_status();
+    const int rc = ssb_launch(rope_append_vec_kernel<0>, dim3(n_tokens), dim3(256), 0, stream, pdl != 0, (bf16*)qkv, ld, cos_t, sin_t, pos, slot, page_table, max_pages, (bf16*)k_cache, (bf16*)v_cache, n_q, n_kv, head_dim, page_shift);
+    return rc ? rc : ssb_launch_status();
 }

@@ -55,8 +55,18 @@ class FastKernels(PlainKernels):
             if t is not None:
                 t.zero_()
 
+    PROMPT_CHAIN_ROWS = 4096
+
+    def _prompt_chain(self, rows) -> bool:
+        """Whether a step of this many rows launches its norms, products and attention as programmatic dependents: a product
+        then has its first weights in shared memory when the kernel before it ends.  us without and with: Llama 1B, 131 rows
+        1,429 and 1,398, 2,000 rows 4,139 and 4,059; 8B, 131 rows 4,983 and 4,786; Vufadra, 200 rows 781 and 745, 2 x 1,000
+        2,444 and 2,407.  Beyond 4,096 rows a kernel's end is too small a part of it: 8,000 rows of the 1B model 14,692 and
+        14,908."""
+        return bool(self.pdl) and int(rows) <= self.PROMPT_CHAIN_ROWS
+
     def rmsnorm(self, x, weight, eps, out, rows=None):
-        pdl = self.pdl and out.shape[0] <= 64
+        pdl = self._prompt_chain(out.shape[0])
         if ops.rmsnorm_vec_ok(x, weight, out):
             ops.rmsnorm_vec(x, weight, eps, out, rows, pdl=pdl)
         else:
@@ -69,7 +79,7 @@ class FastKernels(PlainKernels):
                                 rotary_dim, page_shift, write_cache, interleaved)
         elif ops.rope_append_vec_ok(qkv, cos, head_dim, rotary_dim, write_cache):
             ops.rope_append_vec(qkv, cos, sin, batch.pos, batch.slot_of_token, page_table, k_cache, v_cache,
-                                n_q, n_kv, head_dim, page_shift)
+                                n_q, n_kv, head_dim, page_shift, pdl=self._prompt_chain(qkv.shape[0]))
         else:
             super().rope_append(qkv, cos, sin, batch, page_table, k_cache, v_cache, n_q, n_kv, head_dim,
                                 rotary_dim, page_shift, write_cache)
@@ -92,7 +102,7 @@ class FastKernels(PlainKernels):
                 # one kernel for every row count, K never split: a row's sums are taken in the same order
                 # whatever else is in the step (decode steps pay for it: few blocks stream the weights)
                 ops.gemm_tc(x, weight, out, ops.TC_ACCUMULATE if accumulate else ops.TC_STORE,
-                            tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else self._tile_n(rows, n))
+                            tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else self._tile_n(rows, n), pdl=self._prompt_chain(rows))
             elif rows <= STREAM_ROWS and accumulate:
                 # weights on the M side, K split over blocks that add with float atomics
                 ops.gemv_tc(x, weight, out, ops.TC_ACCUMULATE, splits=ops.gemv_tc_splits(n, k), pdl=self.pdl)
@@ -111,18 +121,19 @@ class FastKernels(PlainKernels):
                 # a prompt of a few hundred tokens: fewer output tiles than SMs.  K is cut into parts
                 # that add with float atomics, into the residual or, for a stored result, into the
                 # zeroed scratch that round_and_clear turns into bfloat16 (as for decode above)
+                chain = self._prompt_chain(rows)
                 tile_n = self._tile_n(rows, n)
                 splits = self._gemm_splits(rows, n, k, tile_n)
                 if splits == 1 and self._pair_tiles(rows, n):
                     tile_n = ops.TC_TILE_PAIR
                 if splits > 1 and accumulate:
-                    ops.gemm_tc(x, weight, out, ops.TC_ACCUMULATE, tile_n=tile_n, splits=splits)
+                    ops.gemm_tc(x, weight, out, ops.TC_ACCUMULATE, tile_n=tile_n, splits=splits, pdl=chain)
                 elif splits > 1 and out.dtype == torch.bfloat16 and n % 8 == 0 and out.stride(0) % 8 == 0:
                     sums = self._buffer("split_sums", rows * n, torch.float32, out.device, zero=True)[: rows * n].view(rows, n)
-                    ops.gemm_tc(x, weight, sums, ops.TC_ACCUMULATE, tile_n=tile_n, splits=splits)
+                    ops.gemm_tc(x, weight, sums, ops.TC_ACCUMULATE, tile_n=tile_n, splits=splits, pdl=chain)
                     ops.round_and_clear(sums, out, pdl=self.pdl)
                 else:
-                    ops.gemm_tc(x, weight, out, ops.TC_ACCUMULATE if accumulate else ops.TC_STORE, tile_n=tile_n)
+                    ops.gemm_tc(x, weight, out, ops.TC_ACCUMULATE if accumulate else ops.TC_STORE, tile_n=tile_n, pdl=chain)
             return
         if rows <= 64 and weight.dtype == torch.bfloat16 and (out.dtype == torch.float32 or not accumulate):
             if self._skinny(x, weight, out, ops.SG_ACCUMULATE if accumulate else ops.SG_STORE):
@@ -149,15 +160,16 @@ class FastKernels(PlainKernels):
             ops.gemv_tc(xt, weight, out, ops.TC_STORE, pdl=self.pdl)
             self.activation(out, out, kind, scale)
         else:
+            chain = self._prompt_chain(rows)
             tile_n = self._tile_n(rows, n)
             splits = self._gemm_splits(rows, n, k, tile_n)
             if splits > 1:
                 sums = self._buffer("split_sums", rows * n, torch.float32, out.device, zero=True)[: rows * n].view(rows, n)
-                ops.gemm_tc(xt, weight, sums, ops.TC_ACCUMULATE, tile_n=tile_n, splits=splits)
+                ops.gemm_tc(xt, weight, sums, ops.TC_ACCUMULATE, tile_n=tile_n, splits=splits, pdl=chain)
                 ops.round_and_clear(sums, out, pdl=self.pdl, act=kind, scale=scale)
             else:
                 ops.gemm_tc_act(xt, weight, out, kind, scale,
-                                tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else tile_n)
+                                tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else tile_n, pdl=chain)
 
     @staticmethod
     def _gemm_splits(rows: int, n: int, k: int, tile_n: int, sms: Optional[int] = None) -> int:
@@ -205,9 +217,9 @@ class FastKernels(PlainKernels):
                     n2 = w_gate_up.shape[0]
                     tile_n = ops.TC_TILE_PAIR if self._pair_tiles(rows, n2) else self._tile_n(rows, n2)
                     if plain_gate:
-                        ops.gemm_tc(xt, w_gate_up, out, ops.TC_SWIGLU, tile_n=tile_n)
+                        ops.gemm_tc(xt, w_gate_up, out, ops.TC_SWIGLU, tile_n=tile_n, pdl=self._prompt_chain(rows))
                     else:
-                        ops.gemm_tc_gate(xt, w_gate_up, out, act, row_scale, tile_n=tile_n)
+                        ops.gemm_tc_gate(xt, w_gate_up, out, act, row_scale, tile_n=tile_n, pdl=self._prompt_chain(rows))
                 return
         if plain_gate and layout == "interleaved" and rows <= 64 and self._skinny(x, w_gate_up, out, ops.SG_SWIGLU):
             return
@@ -317,7 +329,7 @@ class FastKernels(PlainKernels):
         position.check_range(batch)
         ops.gemm_tc_rope_append(x, w_qkv, qkv, cos, sin, batch.pos, batch.slot_of_token, page_table, k_cache,
                                 v_cache, n_q, n_kv, head_dim, page_shift,
-                                tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else 256)
+                                tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else 256, pdl=self._prompt_chain(rows))
         return True
 
     def rope_attention(self, qkv, position, kv, batch, out, n_q, n_kv, head_dim, page_shift, window,
@@ -347,7 +359,8 @@ class FastKernels(PlainKernels):
         if not batch.is_decode and (batch.max_new >= TC_ATTENTION_MIN_NEW or self.deterministic) and k_cache.is_contiguous() \
                 and v_cache.is_contiguous() and ops.attention_prefill_tc_ok(q, out, head_dim, page_shift):
             ops.attention_prefill_tc(q, k_cache, v_cache, batch.cu_new, batch.seq_start, batch.seq_slot,
-                                     page_table, out, batch.max_new, n_q, n_kv, head_dim, page_shift, window, scale)
+                                     page_table, out, batch.max_new, n_q, n_kv, head_dim, page_shift, window, scale,
+                                     pdl=self._prompt_chain(q.shape[0]))
             return
         if not batch.is_decode and ops.attention_prefill_ok(q, head_dim) and out.stride(0) % 2 == 0:
             ops.attention_prefill(q, k_cache, v_cache, batch.cu_new, batch.seq_start, batch.seq_slot,
@@ -507,7 +520,7 @@ class FastKernels(PlainKernels):
         if rows <= STREAM_ROWS:
             ops.gemv_tc(x, weight, logits, ops.TC_ACCUMULATE, splits=splits, pdl=self.pdl)
         else:
-            ops.gemm_tc(x, weight, logits, ops.TC_ACCUMULATE, tile_n=tile_n, splits=splits)
+            ops.gemm_tc(x, weight, logits, ops.TC_ACCUMULATE, tile_n=tile_n, splits=splits, pdl=self._prompt_chain(rows))
         ops.route_softmax(logits, n_experts, renormalize, scale, expert_of, pair_weight, clear=True, pdl=self._chain(rows),
                           bias=bias)
 

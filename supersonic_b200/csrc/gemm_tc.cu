@@ -289,24 +289,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    ssb_pdl_launch_dependents();          // this block has its tensor memory: a dependent's cannot take it first
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
         if (lane == 0) {
-            int c = 0, issued_from = 0;                        // k-blocks issued so far (ring position)
+            int c = 0, issued_from = 0, ahead = 0;             // k-blocks issued so far (ring position); weights fetched ahead
             for (int item = blockIdx.x; item < n_tiles_total * splits && !*abort_flag; item += gridDim.x) {
                 const TcItem it(item, n_tiles_total, k_blocks, splits);
                 const int m0 = (it.tile % m_tiles) * TC_BM, n0 = (it.tile / m_tiles) * BN;
+                if (item == (int)blockIdx.x) {
+                    // the first stages' weights are nobody's output: they come while the predecessor still runs
+                    ahead = min(STAGES, it.kb_hi - it.kb_lo);
+                    for (int s = 0; s < ahead; ++s) {
+                        mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+                        tma_load_2d(smem_u32(smem + s * STAGE_BYTES) + A_BYTES, &map_w, full0 + 8 * s, (it.kb_lo + s) * TC_BK, n0);
+                    }
+                    ssb_pdl_wait();                            // A is the predecessor's output
+                }
                 for (int kb = it.kb_lo; kb < it.kb_hi; ++kb, ++c) {
                     const int s = c % STAGES;
                     const uint32_t phase = (c / STAGES) & 1;
-                    if (!mbar_wait(empty0 + 8 * s, phase ^ 1, abort_flag)) {
-                        *abort_flag = 1; atomicCAS(error_word, 0, TC_ERR_PRODUCER); break;
-                    }
                     const uint32_t a_dst = smem_u32(smem + s * STAGE_BYTES), w_dst = a_dst + A_BYTES;
-                    mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+                    if (c >= ahead) {
+                        if (!mbar_wait(empty0 + 8 * s, phase ^ 1, abort_flag)) {
+                            *abort_flag = 1; atomicCAS(error_word, 0, TC_ERR_PRODUCER); break;
+                        }
+                        mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+                        tma_load_2d(w_dst, &map_w, full0 + 8 * s, kb * TC_BK, n0);
+                    }
                     tma_load_2d(a_dst, &map_a, full0 + 8 * s, kb * TC_BK, m0);
-                    tma_load_2d(w_dst, &map_w, full0 + 8 * s, kb * TC_BK, n0);
                 }
             }
             if (*abort_flag) {
@@ -317,6 +329,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else if (warp == 1) {
+        ssb_pdl_wait();                                        // what follows spins on barriers: not while the predecessor runs
         if (lane == 0) {
             // instruction descriptor: D float32, A and B bfloat16, both K-major, N = BN, M = 128
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
@@ -349,6 +362,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     } else {
         // epilogue: warp w may read tensor-memory lanes 32 * (w % 4) .. + 31 = rows of the tile
+        ssb_pdl_wait();                                          // C may still be the predecessor's
         const int quarter = warp & 3;
         int i = 0;
         for (int item = blockIdx.x; item < n_tiles_total * splits; item += gridDim.x, ++i) {
@@ -423,26 +437,37 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tc_fence_before();
     cluster_sync_all();   // both blocks' barriers are initialised before either signals the other
     tc_fence_after();
+    ssb_pdl_launch_dependents();
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
         if (lane == 0) {
             const uint32_t leader_full0 = cluster_map(full0, 0);
-            int c = 0;
+            int c = 0, ahead = 0;
             for (int tile = pair; tile < n_tiles_total && !*abort_flag; tile += n_pairs) {
                 const TcTileAt at(tile, m_tiles, n_tiles_total / m_tiles, group_m);
                 const int m0 = at.m * 2 * HALF + (int)rank * HALF;
                 const int n0 = at.n * BN + (int)rank * HALF;
+                if (tile == pair) {                            // as above: weights first, then what the predecessor makes
+                    ahead = min(STAGES, k_blocks);
+                    for (int s = 0; s < ahead; ++s) {
+                        if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);
+                        tma_load_2d_pair(smem_u32(smem + s * STAGE_BYTES) + A_BYTES, &map_w, leader_full0 + 8 * s, s * TC_BK, n0);
+                    }
+                    ssb_pdl_wait();
+                }
                 for (int kb = 0; kb < k_blocks; ++kb, ++c) {
                     const int s = c % STAGES;
                     const uint32_t phase = (c / STAGES) & 1;
-                    if (!mbar_wait(empty0 + 8 * s, phase ^ 1, abort_flag)) {
-                        *abort_flag = 1; atomicCAS(error_word, 0, TC_ERR_PRODUCER); break;
-                    }
                     const uint32_t a_dst = smem_u32(smem + s * STAGE_BYTES), w_dst = a_dst + A_BYTES;
-                    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);
+                    if (c >= ahead) {
+                        if (!mbar_wait(empty0 + 8 * s, phase ^ 1, abort_flag)) {
+                            *abort_flag = 1; atomicCAS(error_word, 0, TC_ERR_PRODUCER); break;
+                        }
+                        if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);
+                        tma_load_2d_pair(w_dst, &map_w, leader_full0 + 8 * s, kb * TC_BK, n0);
+                    }
                     tma_load_2d_pair(a_dst, &map_a, leader_full0 + 8 * s, kb * TC_BK, m0);
-                    tma_load_2d_pair(w_dst, &map_w, leader_full0 + 8 * s, kb * TC_BK, n0);
                 }
             }
             if (*abort_flag) {
@@ -458,6 +483,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     } else if (warp == 1) {
+        ssb_pdl_wait();
         if (lane == 0 && rank == 0) {
             // instruction descriptor: D float32, A and B bfloat16, both K-major, N 256, M 256 over the pair
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -487,6 +513,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     } else {
+        ssb_pdl_wait();
         const int quarter = warp & 3;
         const uint32_t leader_acc_empty0 = cluster_map(acc_empty0, 0);
         int i = 0;
@@ -520,7 +547,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
 template <int STAGES>
 static int launch_tc_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int ldc, int out_is_f32, int M, int N,
-                          int K, int mode, int* error_word, const TcRope& rope, cudaStream_t stream) {
+                          int K, int mode, int* error_word, const TcRope& rope, bool pdl, cudaStream_t stream) {
     constexpr size_t smem = STAGES * 2 * 128 * TC_BK * 2 + TC_STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024;
     auto kern = gemm_tc_pair_kernel<STAGES>;
     static int max_pairs = 0;
@@ -553,14 +580,14 @@ static int launch_tc_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* C,
     // bands of 16 row tiles (4,096 rows): at 8,192 rows the gate/up projection took 1,412 us with all row
     // tiles in one band, 1,368 / 1,341 / 1,305 us with bands of 4 / 8 / 16; at 2,048 rows bands of 4 lose 4 %
     const int group_m = 16;
-    kern<<<2 * pairs, TC_THREADS, smem, stream>>>(ma, mw, C, ldc, out_is_f32, M, N, K, mode, m_tiles, total,
-                                                  group_m < m_tiles ? group_m : m_tiles, error_word, rope);
-    return ssb_launch_status();
+    const int rc = ssb_launch(kern, dim3(2 * pairs), dim3(TC_THREADS), smem, stream, pdl, ma, mw, C, ldc, out_is_f32, M, N, K, mode,
+                              m_tiles, total, group_m < m_tiles ? group_m : m_tiles, error_word, rope);
+    return rc ? rc : ssb_launch_status();
 }
 
 template <int BN, int STAGES>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int ldc, int out_is_f32, int M, int N,
-                     int K, int mode, int splits, int* error_word, const TcRope& rope, cudaStream_t stream) {
+                     int K, int mode, int splits, int* error_word, const TcRope& rope, bool pdl, cudaStream_t stream) {
     constexpr size_t smem = STAGES * (TC_BM + BN) * TC_BK * 2 + TC_STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024;
     auto kern = gemm_tc_kernel<BN, STAGES>;
     static bool configured = false;
@@ -584,9 +611,9 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int 
         splits = (k_blocks + per - 1) / per;
     }
     const long long items = (long long)total * splits;
-    kern<<<items < n_sms ? (int)items : n_sms, TC_THREADS, smem, stream>>>(ma, mw, C, ldc, out_is_f32, M, N, K, mode,
-                                                                           m_tiles, total, splits, error_word, rope);
-    return ssb_launch_status();
+    const int rc = ssb_launch(kern, dim3(items < n_sms ? (int)items : n_sms), dim3(TC_THREADS), smem, stream, pdl, ma, mw, C, ldc,
+                              out_is_f32, M, N, K, mode, m_tiles, total, splits, error_word, rope);
+    return rc ? rc : ssb_launch_status();
 }
 
 // A block that waits on a barrier at which nothing ever arrives: the bounded wait gives up after
@@ -617,7 +644,7 @@ SSB_API int ssb_tc_wait_probe(int* error_word, cudaStream_t stream) {
 // 256 x 256 tiles on SM pairs (no K parts).  error_word: device int, zero while all is well.
 static int gemm_tc_any(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int out_dtype, int M,
                        int N, int K, int mode, int tile_n, int splits, int* error_word, const TcRope& rope,
-                       cudaStream_t stream) {
+                       bool pdl, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 8 || lda % 8 || ldw % 8 || N % 8 || !error_word) return SSB_ERR_BAD_SIZE;
     if (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15) return SSB_ERR_BAD_SIZE;
@@ -635,36 +662,36 @@ static int gemm_tc_any(const void* A, int lda, const void* W, int ldw, void* C, 
     if (rc) return rc;
     const int f32o = out_dtype == SSB_F32;
     // six stages of 32 KB: four to seven measured the same, the ring is not what bounds the kernel
-    if (pair) return launch_tc_pair<6>(ma, mw, C, ldc, f32o, M, N, K, mode, error_word, rope, stream);
-    if (bn == 64) return launch_tc<64, 8>(ma, mw, C, ldc, f32o, M, N, K, mode, splits, error_word, rope, stream);
-    if (bn == 128) return launch_tc<128, 6>(ma, mw, C, ldc, f32o, M, N, K, mode, splits, error_word, rope, stream);
-    return launch_tc<256, 4>(ma, mw, C, ldc, f32o, M, N, K, mode, splits, error_word, rope, stream);
+    if (pair) return launch_tc_pair<6>(ma, mw, C, ldc, f32o, M, N, K, mode, error_word, rope, pdl, stream);
+    if (bn == 64) return launch_tc<64, 8>(ma, mw, C, ldc, f32o, M, N, K, mode, splits, error_word, rope, pdl, stream);
+    if (bn == 128) return launch_tc<128, 6>(ma, mw, C, ldc, f32o, M, N, K, mode, splits, error_word, rope, pdl, stream);
+    return launch_tc<256, 4>(ma, mw, C, ldc, f32o, M, N, K, mode, splits, error_word, rope, pdl, stream);
 }
 
 // C (bfloat16) = activation(A W^T) * scale; act: a kind of ssb_activate.
 SSB_API int ssb_gemm_tc_act(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N, int K, int act,
-                            float scale, int tile_n, int* error_word, cudaStream_t stream) {
+                            float scale, int tile_n, int* error_word, int pdl, cudaStream_t stream) {
     if (act < 0 || act > SSB_ACT_SILU) return SSB_ERR_BAD_SIZE;
     TcRope extra{};
     extra.act_scale = scale;
-    return gemm_tc_any(A, lda, W, ldw, C, ldc, SSB_BF16, M, N, K, TC_ACT + act, tile_n, 1, error_word, extra, stream);
+    return gemm_tc_any(A, lda, W, ldw, C, ldc, SSB_BF16, M, N, K, TC_ACT + act, tile_n, 1, error_word, extra, pdl != 0, stream);
 }
 
 // C (bfloat16, [M, N/2]) = gate_fn(A gate^T, A up^T) * row_scale with W's rows as [8 gate | 8 up] per 16: mode 2 with
 // another inner step of the gated unit (a kind of ssb_gate) and one float32 factor per row (or none).
 SSB_API int ssb_gemm_tc_gate(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N, int K,
-                             int gate_kind, float gate_limit, const float* row_scale, int tile_n, int* error_word,
+                             int gate_kind, float gate_limit, const float* row_scale, int tile_n, int* error_word, int pdl,
                              cudaStream_t stream) {
     if (gate_kind < 0 || gate_kind > SSB_GATE_LAST) return SSB_ERR_BAD_SIZE;
     TcRope extra{};
     extra.gate_kind = gate_kind; extra.gate_limit = gate_limit; extra.row_scale = row_scale;
-    return gemm_tc_any(A, lda, W, ldw, C, ldc, SSB_BF16, M, N, K, TC_SWIGLU, tile_n, 1, error_word, extra, stream);
+    return gemm_tc_any(A, lda, W, ldw, C, ldc, SSB_BF16, M, N, K, TC_SWIGLU, tile_n, 1, error_word, extra, pdl != 0, stream);
 }
 
 SSB_API int ssb_gemm_tc(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int out_dtype, int M,
-                        int N, int K, int mode, int tile_n, int splits, int* error_word, cudaStream_t stream) {
+                        int N, int K, int mode, int tile_n, int splits, int* error_word, int pdl, cudaStream_t stream) {
     if (mode < TC_STORE || mode > TC_SWIGLU) return SSB_ERR_BAD_SIZE;
-    return gemm_tc_any(A, lda, W, ldw, C, ldc, out_dtype, M, N, K, mode, tile_n, splits, error_word, TcRope{}, stream);
+    return gemm_tc_any(A, lda, W, ldw, C, ldc, out_dtype, M, N, K, mode, tile_n, splits, error_word, TcRope{}, pdl != 0, stream);
 }
 
 // The fused query/key/value projection of packed tokens with rotation and cache append in the
@@ -673,7 +700,7 @@ SSB_API int ssb_gemm_tc(const void* A, int lda, const void* W, int ldw, void* C,
 SSB_API int ssb_gemm_tc_rope_append(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int K,
                                     const int* pos, const int* slot, const int* page_table, int max_pages,
                                     void* k_cache, void* v_cache, const float* cos_t, const float* sin_t,
-                                    int n_q, int n_kv, int head_dim, int page_shift, int tile_n, int* error_word,
+                                    int n_q, int n_kv, int head_dim, int page_shift, int tile_n, int* error_word, int pdl,
                                     cudaStream_t stream) {
     if ((head_dim != 64 && head_dim != 128) || n_q <= 0 || n_kv <= 0 || !pos || !slot || !page_table || !cos_t ||
         !sin_t || !k_cache || !v_cache || page_shift < 0 || page_shift > 20)
@@ -682,5 +709,5 @@ SSB_API int ssb_gemm_tc_rope_append(const void* A, int lda, const void* W, int l
     TcRope rope{pos, slot, page_table, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, cos_t, sin_t,
                 max_pages, n_q, n_kv, head_dim, page_shift};
     return gemm_tc_any(A, lda, W, ldw, C, ldc, SSB_BF16, M, (n_q + 2 * n_kv) * head_dim, K, TC_ROPE_APPEND,
-                       tile_n == TC_TILE_PAIR ? TC_TILE_PAIR : 256, 1, error_word, rope, stream);
+                       tile_n == TC_TILE_PAIR ? TC_TILE_PAIR : 256, 1, error_word, rope, pdl != 0, stream);
 }

@@ -2105,7 +2105,7 @@ def gemm_tc_ok(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
 
 
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = TC_STORE,
-            tile_n: Optional[int] = None, splits: int = 1) -> None:
+            tile_n: Optional[int] = None, splits: int = 1, pdl: bool = False) -> None:
     """out = a @ w^T on the tensor cores (tcgen05, TMA-fed).  mode: store, add into float32
     ``out``, or SwiGLU over rows of ``w`` that come as [8 gate | 8 up] per 16.  ``splits`` > 1
     (mode accumulate): every tile's K range is cut into that many parts, which add with float atomics."""
@@ -2124,7 +2124,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = TC_
     _check(_fn("gemm_tc", "ssb_gemm_tc")(
         _ptr(a), c_int(a.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(out), c_int(out.stride(0)),
         c_int(dtype_code(out.dtype)), c_int(M), c_int(N), c_int(K), c_int(mode), c_int(tile_n), c_int(splits),
-        _ptr(tc_error_word(a.device)), _stream()), "gemm_tc")
+        _ptr(tc_error_word(a.device)), c_int(1 if pdl else 0), _stream()), "gemm_tc")
 
 
 def _gate_args(act, row_scale, rows: int, what: str):
@@ -2139,7 +2139,7 @@ def _gate_args(act, row_scale, rows: int, what: str):
 
 
 def gemm_tc_gate(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act=None, row_scale: Optional[torch.Tensor] = None,
-                 tile_n: Optional[int] = None) -> None:
+                 tile_n: Optional[int] = None, pdl: bool = False) -> None:
     """out = f(a @ gate^T, a @ up^T) * row_scale on the tensor cores, the inner step on the float32 sums; ``w``'s rows
     come as [8 gate | 8 up] per 16; ``act`` = (kind, limit) as in :func:`gated_activation`, None for silu(g) u."""
     _need(a, "a", torch.bfloat16, 2); _need(w, "w", torch.bfloat16, 2); _need(out, "out", torch.bfloat16, 2)
@@ -2154,12 +2154,12 @@ def gemm_tc_gate(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act=None, 
     _tc_unchecked += 1
     _check(_fn("gemm_tc", "ssb_gemm_tc_gate")(
         _ptr(a), c_int(a.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(out), c_int(out.stride(0)), c_int(M), c_int(N),
-        c_int(K), c_int(kind), c_float(limit), _ptr(row_scale), c_int(tile_n), _ptr(tc_error_word(a.device)), _stream()),
-        "gemm_tc_gate")
+        c_int(K), c_int(kind), c_float(limit), _ptr(row_scale), c_int(tile_n), _ptr(tc_error_word(a.device)), c_int(1 if pdl else 0),
+        _stream()), "gemm_tc_gate")
 
 
 def gemm_tc_act(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: str, scale: float = 1.0,
-                tile_n: Optional[int] = None) -> None:
+                tile_n: Optional[int] = None, pdl: bool = False) -> None:
     """out (bfloat16) = act(a @ w^T) * scale on the tensor cores: the activation (a kind of ``ACTIVATIONS``) is taken
     on the float32 sums where the product finishes them, before their one rounding."""
     _need(a, "a", torch.bfloat16, 2); _need(w, "w", torch.bfloat16, 2); _need(out, "out", torch.bfloat16, 2)
@@ -2175,14 +2175,14 @@ def gemm_tc_act(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: str, 
     _tc_unchecked += 1
     _check(_fn("gemm_tc", "ssb_gemm_tc_act")(
         _ptr(a), c_int(a.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(out), c_int(out.stride(0)), c_int(M), c_int(N),
-        c_int(K), c_int(ACTIVATIONS[kind]), c_float(scale), c_int(tile_n), _ptr(tc_error_word(a.device)), _stream()),
-        "gemm_tc_act")
+        c_int(K), c_int(ACTIVATIONS[kind]), c_float(scale), c_int(tile_n), _ptr(tc_error_word(a.device)), c_int(1 if pdl else 0),
+        _stream()), "gemm_tc_act")
 
 
 def gemm_tc_rope_append(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cos: torch.Tensor,
                         sin: torch.Tensor, pos: torch.Tensor, slot: torch.Tensor, page_table: torch.Tensor,
                         k_cache: torch.Tensor, v_cache: torch.Tensor, n_q: int, n_kv: int, head_dim: int,
-                        page_shift: int, tile_n: int = 256) -> None:
+                        page_shift: int, tile_n: int = 256, pdl: bool = False) -> None:
     """The fused query/key/value projection of packed tokens (``w`` = [q; k; v] rows) on tcgen05
     whose epilogue rotates q and k from the float32 sums, writes q (bfloat16) into ``q_out`` and
     k and v into the paged cache entry; nothing else is written.  head_dim 64 or 128, full-width
@@ -2211,7 +2211,7 @@ def gemm_tc_rope_append(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, c
         _ptr(a), c_int(a.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(q_out), c_int(q_out.stride(0)), c_int(M),
         c_int(K), _ptr(pos), _ptr(slot), _ptr(page_table), c_int(page_table.shape[1]), _ptr(k_cache), _ptr(v_cache),
         _ptr(cos), _ptr(sin), c_int(n_q), c_int(n_kv), c_int(head_dim), c_int(page_shift), c_int(tile_n),
-        _ptr(tc_error_word(a.device)), _stream()), "gemm_tc_rope_append")
+        _ptr(tc_error_word(a.device)), c_int(1 if pdl else 0), _stream()), "gemm_tc_rope_append")
 
 
 # ---- prefill attention -------------------------------------------------------------------------
@@ -2250,7 +2250,7 @@ def attention_prefill_tc_ok(q: torch.Tensor, out: torch.Tensor, head_dim: int, p
 def attention_prefill_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, cu_new: torch.Tensor,
                          seq_start: torch.Tensor, seq_slot: torch.Tensor, page_table: torch.Tensor,
                          out: torch.Tensor, max_new: int, n_q: int, n_kv: int, head_dim: int, page_shift: int,
-                         window: Optional[int], scale: float) -> None:
+                         window: Optional[int], scale: float, pdl: bool = False) -> None:
     """``attention_prefill`` on tcgen05: scores and probabilities in tensor memory, pages by TMA.
     head_dim 64 or 128 and 64-token pages only.  A wait that runs out sets the device's error word
     (``check_device_errors``)."""
@@ -2274,7 +2274,7 @@ def attention_prefill_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
         _ptr(cu_new), _ptr(seq_start), _ptr(seq_slot), _ptr(page_table), c_int(page_table.shape[1]),
         _ptr(out), c_int(out.stride(0)), c_int(n_seqs), c_int(max_new), c_int(n_q), c_int(n_kv),
         c_int(head_dim), c_int(page_shift), c_int(int(window) if window else 0), c_float(scale),
-        _ptr(tc_error_word(q.device)), _stream()), "attention_prefill_tc")
+        _ptr(tc_error_word(q.device)), c_int(1 if pdl else 0), _stream()), "attention_prefill_tc")
 
 
 # ---- decode projections on tcgen05, weights on the M side ------------------------------------------
@@ -2399,7 +2399,7 @@ def rope_append_vec_ok(qkv: torch.Tensor, cos, head_dim: int, rotary_dim: int, w
 
 def rope_append_vec(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: torch.Tensor,
                     slot: torch.Tensor, page_table: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
-                    n_q: int, n_kv: int, head_dim: int, page_shift: int) -> None:
+                    n_q: int, n_kv: int, head_dim: int, page_shift: int, pdl: bool = False) -> None:
     """As :func:`rope_append` for bfloat16, full-width rotation, with vector loads and stores."""
     _need(qkv, "qkv", torch.bfloat16, 2); _need(pos, "pos", torch.int32, 1); _need(slot, "slot", torch.int32, 1)
     _need(page_table, "page_table", torch.int32, 2); _need(cos, "cos", torch.float32, 2); _need(sin, "sin", torch.float32, 2)
@@ -2412,4 +2412,4 @@ def rope_append_vec(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos
     _check(_fn("elementwise_ops", "ssb_rope_append_vec")(
         _ptr(qkv), c_int(qkv.stride(0)), _ptr(cos), _ptr(sin), c_int(cos.shape[0]), _ptr(pos), _ptr(slot),
         _ptr(page_table), c_int(page_table.shape[1]), _ptr(k_cache), _ptr(v_cache), c_int(T), c_int(n_q),
-        c_int(n_kv), c_int(head_dim), c_int(page_shift), _stream()), "rope_append_vec")
+        c_int(n_kv), c_int(head_dim), c_int(page_shift), c_int(1 if pdl else 0), _stream()), "rope_append_vec")

@@ -119,6 +119,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     uint32_t* tmem_slot = (uint32_t*)(bars + FT_NBARS);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);   // [0]: a role gave up; [1]: stays zero
 
+    ssb_pdl_launch_dependents();
+    ssb_pdl_wait();
     // blocks start in the order of blockIdx.x, then y: every head's longest tiles come first
     const int kvh = blockIdx.x % n_kv, b = blockIdx.x / n_kv;
     const int row0 = cu_new[b], n_new = cu_new[b + 1] - row0;
@@ -402,7 +404,7 @@ SSB_API int ssb_attention_prefill_tc(const void* q, int ldq, int n_rows_q, const
                                      int n_pages, const int* cu_new, const int* seq_start, const int* seq_slot,
                                      const int* page_table, int max_pages, void* out, int ldo, int n_seqs, int max_new,
                                      int n_q, int n_kv, int head_dim, int page_shift, int window, float scale,
-                                     int* error_word, cudaStream_t stream) {
+                                     int* error_word, int pdl, cudaStream_t stream) {
     if (n_seqs <= 0 || max_new <= 0) return 0;
     if ((head_dim != 64 && head_dim != 128) || page_shift != 6) return SSB_ERR_UNSUPPORTED;
     if (n_kv <= 0 || n_q % n_kv || ldq % 8 || ldo % 8 || !error_word ) return SSB_ERR_BAD_SIZE;
@@ -428,9 +430,9 @@ SSB_API int ssb_attention_prefill_tc(const void* q, int ldq, int n_rows_q, const
             if (e != cudaSuccess) return (int)e; \
             configured = true; \
         } \
-        prefill_attention_tc_kernel<HD_><<<grid, FT_THREADS, smem, stream>>>( \
-            mq, mk, mv, cu_new, seq_start, seq_slot, page_table, max_pages, (bf16*)out, ldo, n_q, n_kv, window, \
-            scale * 1.4426950408889634f, error_word); \
+        const int rc_ = ssb_launch(prefill_attention_tc_kernel<HD_>, grid, dim3(FT_THREADS), smem, stream, pdl != 0, \
+            mq, mk, mv, cu_new, seq_start, seq_slot, page_table, max_pages, (bf16*)out, ldo, n_q, n_kv, window, scale * 1.4426950408889634f, error_word); \
+        if (rc_) return rc_; \
     } while (0)
     if (head_dim == 64) SSB_FT(64); else SSB_FT(128);
 #undef SSB_FT

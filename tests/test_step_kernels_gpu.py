@@ -246,3 +246,29 @@ def test_products_leave_in_whole_rows(m, n, k, tile):
     assert bool(((sums.double() - want).abs() <= k * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()) + 1e-30).all())
     assert torch.equal(added, c + sums) and torch.equal(rounded, sums.to(torch.bfloat16))
     assert all(bool((x[m] == 5.0).all() and (x[:, n:] == 5.0).all()) for x in wide)
+
+
+@pytest.mark.parametrize("rows", [129, 300, 1024])
+def test_a_chain_of_dependent_launches_reads_what_was_written(rows):
+    """Norm, product, product into the stream, attention's preparation: launched as programmatic dependents of one another or
+    one after the other, many times over the same buffers, the same bits."""
+    o, n = ops(), 512
+    w1, w2 = (rnd(n, n, seed=s, scale=n ** -0.5, dtype=torch.bfloat16) for s in (1, 2))
+    gain, pos = torch.ones(n, device=DEV), torch.arange(rows, dtype=torch.int32, device=DEV)
+    slot, table = torch.zeros(rows, dtype=torch.int32, device=DEV), torch.arange(16, dtype=torch.int32, device=DEV).view(1, 16)
+    angle = rnd(1024, 32, seed=3)
+    cos, sin = torch.cos(angle), torch.sin(angle)
+    got = []
+    for pdl in (False, True):
+        x, h, y = rnd(rows, n, seed=rows), torch.empty(rows, n, dtype=torch.bfloat16, device=DEV), torch.empty(rows, n, dtype=torch.bfloat16, device=DEV)
+        k, v = (torch.zeros(16, 2, 64, 64, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        torch.cuda.synchronize()
+        for turn in range(30):
+            tile = (64, 128, 256, o.TC_TILE_PAIR)[turn % 4]
+            o.rmsnorm_vec(x, gain, 1e-5, h, pdl=pdl)
+            o.gemm_tc(h, w1, y, tile_n=tile, pdl=pdl)
+            o.rope_append_vec(y, cos, sin, pos, slot, table, k, v, 4, 2, 64, 6, pdl=pdl)
+            o.gemm_tc(y, w2, x, o.TC_ACCUMULATE, tile_n=tile, pdl=pdl)
+        o.check_device_errors(torch.device(DEV))
+        got.append((x.clone(), y.clone(), k.clone(), v.clone()))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
