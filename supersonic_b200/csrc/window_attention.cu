@@ -217,6 +217,7 @@ struct WpArgs {
     const bf16* v_first; int ld_first; float v_lambda;
 };
 constexpr int WV_MAX_WARPS = 16, WV_MAX_PER_WARP = 4;     // warps a block; heads a warp
+constexpr int WV_MANY_TOKENS = 296;                       // two a streaming multiprocessor
 
 template <int E>
 __device__ __forceinline__ void wv_load(const bf16* src, float (&x)[E]) {
@@ -274,7 +275,7 @@ template <int E, int EV>
 __global__ void __launch_bounds__(WV_MAX_WARPS * 32)
 qkv_prepare_vec_kernel(const WpArgs a) {
     constexpr int DIM = 32 * E, VDIM = 32 * EV;
-    __shared__ float red[WV_MAX_WARPS];
+    __shared__ float red[WV_MAX_WARPS * WV_MAX_PER_WARP];
     ssb_pdl_launch_dependents();
     ssb_pdl_wait();
     const int t = blockIdx.x, part = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -333,17 +334,18 @@ qkv_prepare_vec_kernel(const WpArgs a) {
     }
     if (turn) wv_angles<E>(a.cos_t, a.sin_t, p, a.rot_dims, a.interleaved, lane, cs, sn);
     const float temp = (part == 0 && a.q_temp_every > 0) ? 1.0f + a.q_temp_coef * logf((float)((p + 1) / a.q_temp_every + 1)) : 1.0f;
-    if (a.norm_mode == 2) {                               // one root mean square for the row: warps in order
+    if (a.norm_mode == 2) {                               // one root mean square for the row: heads in order, whoever held them
 #pragma unroll
         for (int i = 0; i < WV_MAX_PER_WARP; ++i)
-            if (warp + i * warps < heads)
+            if (warp + i * warps < heads) {
+                float sq = 0.f;
 #pragma unroll
-                for (int e = 0; e < E; ++e) total = fmaf(x[i][e], x[i][e], total);
-        total = wa_warp_sum(total);
-        if (lane == 0) red[warp] = total;
+                for (int e = 0; e < E; ++e) sq = fmaf(x[i][e], x[i][e], sq);
+                sq = wa_warp_sum(sq);
+                if (lane == 0) red[warp + i * warps] = sq;
+            }
         __syncthreads();
-        total = 0.f;
-        for (int i = 0; i < warps; ++i) total += red[i];
+        for (int h = 0; h < heads; ++h) total += red[h];
     }
 #pragma unroll
     for (int i = 0; i < WV_MAX_PER_WARP; ++i) {
@@ -410,7 +412,11 @@ SSB_API int ssb_qkv_prepare(void* qkv, int ld, int dtype, const float* q_w, cons
         a.v_off = v_off; a.n_v = n_v; a.q_temp_coef = q_temp_coef; a.q_temp_every = q_temp_every;
         a.v_first = (const bf16*)v_first; a.ld_first = v_first ? ld_first : 0; a.v_lambda = v_lambda;
         if (wv_ok(a, dim, vdim)) {
-            const int threads = 32 * min(WV_MAX_WARPS, max(n_q, max(n_kv, n_v)));
+            // few tokens: a warp a head, the shortest chain; many: four heads a warp, whose loads share the latency of a block's
+            // chain slot - position - page, and several times the tokens resident (6,400 tokens, 16 heads of 128: 122 us a warp a head, 42 so, 79 in the kernel above;
+            // 32 heads of 64: 118, 69 and 79).
+            const int most = max(n_q, max(n_kv, n_v)), each = n_tokens >= WV_MANY_TOKENS ? WV_MAX_PER_WARP : 1;
+            const int threads = 32 * min(WV_MAX_WARPS, (most + each - 1) / each);
             auto kern = dim == 64 ? (vdim == 64 ? qkv_prepare_vec_kernel<2, 2> : qkv_prepare_vec_kernel<2, 4>)
                                   : (vdim == 64 ? qkv_prepare_vec_kernel<4, 2> : qkv_prepare_vec_kernel<4, 4>);
             const int st = ssb_launch(kern, dim3(n_tokens, 3), dim3(threads), 0, stream, pdl != 0, a);

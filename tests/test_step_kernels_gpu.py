@@ -198,14 +198,15 @@ def test_a_cluster_of_blocks_shares_a_decode_steps_pages(kind, dim):
 
 @pytest.mark.parametrize("dim,vdim,n_q,n_kv,n_v", [(128, 128, 16, 4, 4), (64, 64, 32, 8, 8), (64, 128, 40, 20, 10), (128, 64, 3, 1, 1)])
 @pytest.mark.parametrize("norm,rot,interleaved", [("head", 64, False), ("row", 32, True), (None, 0, False), ("head", 16, False)])
-def test_rows_prepared_a_warp_a_head(dim, vdim, n_q, n_kv, n_v, norm, rot, interleaved):
+@pytest.mark.parametrize("T", [7, 300])
+def test_rows_prepared_a_warp_a_head(dim, vdim, n_q, n_kv, n_v, norm, rot, interleaved, T):
     """Against the kernel that takes any width (which rows at an odd address still get): queries, cached keys and values, and
     the pooled rows of tokens that end a run; float32 in between, so one step of bfloat16 apart at the most."""
-    T, pool = 7, (16 if n_v == n_kv else 0)
-    width, positions = (n_q + n_kv) * dim + n_v * vdim, [0, 15, 63, 64, 127, 200, 31]
+    pool = 16 if n_v == n_kv and T == 7 else 0
+    width, positions = (n_q + n_kv) * dim + n_v * vdim, [0, 15, 63, 64, 127, 200, 31] if T == 7 else [t % 250 for t in range(T)]
     rows = rnd(T, width + 8, seed=dim + n_q, dtype=torch.bfloat16)
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
-    pos, slots = i32(positions), i32([0, 1, 2, 3, 4, 5, -1])
+    pos, slots = i32(positions), i32([0, 1, 2, 3, 4, 5, -1] if T == 7 else [t // 250 for t in range(T)])
     table = torch.arange(6 * 4, dtype=torch.int32, device=DEV).view(6, 4)
     ptable = torch.arange(6, dtype=torch.int32, device=DEV).view(6, 1)
     qw, kw = (rnd(dim if norm == "head" else n * dim, seed=n) + 1.0 for n in (n_q, n_kv))
