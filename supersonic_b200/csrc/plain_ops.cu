@@ -785,10 +785,44 @@ __global__ void stream_mix_kernel(const float* __restrict__ streams, size_t stri
     out[i] = acc;
 }
 
+// The same sums, four elements a thread and the terms' loads in groups of four (2,048 x 2,048,
+// two to five terms: 35 us a launch with one element a thread, 25 so).
+__global__ void __launch_bounds__(256)
+stream_mix_vec_kernel(const float4* __restrict__ streams, size_t stride, const float* __restrict__ w, int n_terms,
+                      float4* __restrict__ out, size_t n) {
+    constexpr int AHEAD = 4;
+    ssb_pdl_launch_dependents();
+    ssb_pdl_wait();
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j0 = 0; j0 < n_terms; j0 += AHEAD) {
+        float4 v[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j)
+            if (j0 + j < n_terms) v[j] = streams[(size_t)(j0 + j) * stride + i];
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j)
+            if (j0 + j < n_terms) {
+                const float s = w[j0 + j];
+                acc.x = fmaf(s, v[j].x, acc.x);
+                acc.y = fmaf(s, v[j].y, acc.y);
+                acc.z = fmaf(s, v[j].z, acc.z);
+                acc.w = fmaf(s, v[j].w, acc.w);
+            }
+    }
+    out[i] = acc;
+}
+
 SSB_API int ssb_stream_mix(const float* streams, long long stride, const float* w, int n_terms, float* out,
                            long long n, int pdl, cudaStream_t stream) {
     if (n <= 0) return 0;
     if (n_terms <= 0) return SSB_ERR_BAD_SIZE;
+    if (n % 4 == 0 && stride % 4 == 0 && (((uintptr_t)streams | (uintptr_t)out) & 15) == 0) {
+        const int st = ssb_launch(stream_mix_vec_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, pdl != 0,
+                                  (const float4*)streams, (size_t)stride / 4, w, n_terms, (float4*)out, (size_t)n / 4);
+        return st ? st : ssb_launch_status();
+    }
     const int rc = ssb_launch(stream_mix_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, pdl != 0,
                               streams, (size_t)stride, w, n_terms, out, (size_t)n);
     return rc ? rc : ssb_launch_status();

@@ -273,3 +273,22 @@ def test_a_chain_of_dependent_launches_reads_what_was_written(rows):
         o.check_device_errors(torch.device(DEV))
         got.append((x.clone(), y.clone(), k.clone(), v.clone()))
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("width", [8, 2048, 516, 1030])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sums_of_a_few_rows_in_their_order(width, dtype):
+    """Experts' rows and streams added up four columns a thread (or, in rows that are not whole pieces, one): the same chain
+    of multiply-adds, against the rows at an odd address."""
+    for tokens, top in ((1, 1), (5, 6), (300, 4), (3, 9)):
+        y, w, res = rnd(tokens * top, width, seed=top, dtype=dtype), rnd(tokens, top, seed=tokens), rnd(tokens, width, seed=3)
+        want, got = res.clone(), res.clone()
+        ops().expert_combine(want, off_by_one(y), w, top)
+        ops().expert_combine(got, y, w, top)
+        assert torch.equal(got, want)
+        if dtype == torch.float32:
+            streams = rnd(top, tokens, width, seed=5)
+            one, other = torch.empty(tokens, width, device=DEV), torch.empty(tokens, width, device=DEV)
+            ops().stream_mix(off_by_one(streams), w[0].contiguous(), top, one)
+            ops().stream_mix(streams, w[0].contiguous(), top, other)
+            assert torch.equal(one, other)
