@@ -31,10 +31,11 @@ __device__ __forceinline__ void gf_kahan(float& acc, float& lost, float part) {
 // of A; the chunks' sums go through shared memory, two turns deep, to further warps whose threads add them in order, one
 // result each: 32 additions of four dependent steps a turn, which nobody else waits for.  W and A come by cp.async, STAGES
 // turns deep, in one stream over all the tiles that a block of the grid walks.
-// Bound by the weights' bytes at one row and by the shared-memory reads of the products from 8 on; the general kernel read
-// the weights again for every row and spent a dependent chain of 4 additions per 16 products in every thread.
-// Weights of 16384 x 2048 (134 MB), us: 1 row 270 on the general kernel and 36 here, 8 rows 270 and 54, 16 rows 270 and 91;
-// of 2048 x 8192, 2 rows 805 and 24.
+// Bound by the latency of a turn at one row (48 % of the issue slots, 42 % of the memory's time) and by the shared-memory reads
+// of the products from 8 on; the general kernel read the weights again for every row and spent a dependent chain of 4 additions
+// per 16 products in every thread.  Weights of 16384 x 2048 (134 MB), us: 1 row 270 on the general kernel and 33 here, 8 rows
+// 270 and 54, 16 rows 270 and 91; of 2048 x 8192, 2 rows 805 and 23.  16 rows of W a block (R = 2): with 8, and a block a tile,
+// 1 row of 16384 x 2048 took 40 and of 128256 x 2048 246 where this takes 205.
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int GF_PRODUCT_THREADS = 256;
 constexpr int GF_SKINNY_CHUNKS = 32;                                  // chunks a turn: one a lane
@@ -382,10 +383,8 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         const int groups = (M + MB - 1) / MB; \
         const long long tiles = (long long)groups * ((N + 8 * R - 1) / (8 * R)); \
         if (tiles > 0x7fffffffLL) return SSB_ERR_BAD_SIZE; \
-        /* as many blocks as are resident at once (by shared memory), each walking its share of the tiles; a block a tile */ \
-        /* for one or two rows, whose turns are so short that a block's last additions are better hidden by the next block */ \
-        /* (2048 x 16384, us: one row 36.4 with a block a tile and 40.6 walking, 8 rows 60.5 and 53.9) */ \
-        const long long held = MB <= 2 ? tiles : gf_sms() * (228 * 1024 / (long long)(smem + 1024)); \
+        /* as many blocks as are resident at once (by shared memory), each walking its share of the tiles */ \
+        const long long held = gf_sms() * (228 * 1024 / (long long)(smem + 1024)); \
         const long long blocks = tiles < held ? tiles : held; \
         kernel<<<dim3((unsigned)blocks, 1, n_batch), GF_PRODUCT_THREADS + gf_adders(MB, R), smem, stream>>>( \
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, groups, accumulate); \
@@ -400,9 +399,9 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
     } while (0)
     switch (form) {
-        case 1: GF_SKINNY(1, 1, 4); break;
-        case 2: GF_SKINNY(2, 1, 4); break;
-        case 4: GF_SKINNY(4, 1, 3); break;
+        case 1: GF_SKINNY(1, 2, 3); break;
+        case 2: GF_SKINNY(2, 2, 3); break;
+        case 4: GF_SKINNY(4, 2, 3); break;
         case 8: GF_SKINNY(8, 2, 3); break;
         case 16: GF_SKINNY(16, 2, 2); break;
         case 100: GF_TILES(4, 4, 3); break;
