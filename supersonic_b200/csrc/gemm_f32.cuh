@@ -177,8 +177,8 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __rest
 // a thread reads four neighbouring columns at a time and the multiply-adds go two columns an instruction (fma.rn.f32x2: each
 // half rounds as the scalar one does).  Bound by the FP32 pipes: a chunk's 16 multiply-adds of a result are followed by the
 // four steps of its compensated addition, so 4/5 of the peak is what this sum leaves.
-// 1000 rows, us on the general kernel and here: 2048 x 2048 504 and 291, 3072 x 2048 746 and 483, 16384 x 2048 3563 and 2003
-// (33.5 TFLOP/s), 2048 x 8192 2033 and 1145.
+// 1000 rows, us on the general kernel and here: 2048 x 2048 504 and 291, 3072 x 2048 746 and 483, 16384 x 2048 3563 and 1794
+// (37.4 TFLOP/s), 2048 x 8192 2033 and 1145.
 // ---------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long gf_twice(float x) {
     unsigned long long r;
@@ -204,12 +204,35 @@ __device__ __forceinline__ void gf_kahan2(unsigned long long& acc, unsigned long
     acc = t;
 }
 
+// Sixteen words a lane of tensor memory, which a warp may also use as storage of its own lanes.
+__device__ __forceinline__ unsigned long long gf_pair(uint32_t lo, uint32_t hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ void gf_tld16(uint32_t at, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(at) : "memory");
+}
+// Every load issued so far has arrived; the registers of one of them are not read before.
+__device__ __forceinline__ void gf_tld_wait(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[i]));
+}
+__device__ __forceinline__ void gf_tst16(uint32_t at, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                   "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(at) : "memory");
+}
+
 constexpr int GF_TILE_THREADS = 256, GF_RAW = 3;                     // GF_RAW: chunks on their way from memory, and at work
 
 template <int RM, int RN>
 constexpr size_t gf_tile_smem() { return sizeof(float) * (size_t)(2 + GF_RAW) * GF_CHUNK * 16 * (RM + RN); }
 
-template <int RM, int RN, int MIN_BLOCKS>                             // results a thread; tiles of 16 RM x 16 RN
+template <int RM, int RN, int MIN_BLOCKS, bool TMEM = false>          // results a thread; tiles of 16 RM x 16 RN
 __global__ void __launch_bounds__(GF_TILE_THREADS, MIN_BLOCKS)
 gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C,
                      int ldc, int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int accumulate) {
@@ -261,11 +284,35 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
             dst[0] = x.x; dst[TN] = x.y; dst[2 * TN] = x.z; dst[3 * TN] = x.w;
         }
     };
+    constexpr int RES = RM * RN;
     unsigned long long acc[RM][RN / 2], kept[RM][RN / 2];             // two columns each
+    // TMEM: the running sums and what their additions rounded away, RES columns each of this warp's lanes of tensor memory; a
+    // thread then fits in 128 registers, and two blocks an SM
+    __shared__ uint32_t tmem_slot;
+    uint32_t t_acc = 0, t_kept = 0;
+    if constexpr (TMEM) {
+        if (warp == 0) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"((uint32_t)__cvta_generic_to_shared(&tmem_slot)), "r"(4 * RES) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        t_acc = tmem_slot + ((uint32_t)(warp % 4 * 32) << 16) + warp / 4 * 2 * RES;
+        t_kept = t_acc + RES;
+        uint32_t zero[16];
 #pragma unroll
-    for (int i = 0; i < RM; ++i)
+        for (int i = 0; i < 16; ++i) zero[i] = 0u;
 #pragma unroll
-        for (int j = 0; j < RN / 2; ++j) { acc[i][j] = 0ull; kept[i][j] = 0ull; }
+        for (int c = 0; c < 2 * RES; c += 16) gf_tst16(t_acc + c, zero);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN / 2; ++j) { acc[i][j] = 0ull; kept[i][j] = 0ull; }
+    }
     const unsigned long long minus_one = gf_twice(-1.0f);
 #pragma unroll
     for (int t = 0; t < GF_RAW - 1; ++t) {
@@ -306,13 +353,51 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
                 for (int j = 0; j < RN / 2; ++j) part[i][j] = gf_fma2(aa, w[j], part[i][j]);
             }
         }
+        if constexpr (TMEM) {
 #pragma unroll
-        for (int i = 0; i < RM; ++i)
+            for (int c = 0; c < RES; c += 16) {
+                uint32_t x[16], y[16];
+                gf_tld16(t_acc + c, x);
+                gf_tld16(t_kept + c, y);
+                gf_tld_wait(x);
+                gf_tld_wait(y);
 #pragma unroll
-            for (int j = 0; j < RN / 2; ++j) gf_kahan2(acc[i][j], kept[i][j], part[i][j], minus_one);
+                for (int e = 0; e < 16; e += 2) {
+                    const int at = (c + e) / 2;
+                    unsigned long long sum = gf_pair(x[e], x[e + 1]), lost = gf_pair(y[e], y[e + 1]);
+                    gf_kahan2(sum, lost, part[at / (RN / 2)][at % (RN / 2)], minus_one);
+                    x[e] = (uint32_t)sum; x[e + 1] = (uint32_t)(sum >> 32);
+                    y[e] = (uint32_t)lost; y[e + 1] = (uint32_t)(lost >> 32);
+                }
+                gf_tst16(t_acc + c, x);
+                gf_tst16(t_kept + c, y);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        } else {
+#pragma unroll
+            for (int i = 0; i < RM; ++i)
+#pragma unroll
+                for (int j = 0; j < RN / 2; ++j) gf_kahan2(acc[i][j], kept[i][j], part[i][j], minus_one);
+        }
         gf_wait<GF_RAW - 2>();
         if (turn + 1 < turns) stage(turn + 1);
         __syncthreads();
+    }
+    if constexpr (TMEM) {
+#pragma unroll
+        for (int c = 0; c < RES; c += 16) {
+            uint32_t x[16];
+            gf_tld16(t_acc + c, x);
+            gf_tld_wait(x);
+#pragma unroll
+            for (int e = 0; e < 16; e += 2) acc[(c + e) / 2 / (RN / 2)][(c + e) / 2 % (RN / 2)] = gf_pair(x[e], x[e + 1]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        if (warp == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(4 * RES) : "memory");
+        }
     }
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
@@ -349,25 +434,27 @@ static inline int gf_sms() {
 // done first by the time a chunk of 16 k takes it: the blocks run in waves over the SMs, and tiles that are too large leave
 // SMs idle where tiles that are too small fetch more often than they multiply.  Microseconds a chunk, measured for 1 and
 // for each further wave: 16 rows x 16 columns a block 0.13 + 0.10; tiles of 64 x 64 0.90 + 0.60, of 128 x 64 1.45 + 1.15,
-// of 128 x 128 2.24 + 2.24.  Sides of the lines it draws (us): 128 x 2048 x 2048 (rows, columns, k) 89 with 16 rows and
-// 116 with tiles of 64; 100 x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072 186 with 128 x 64, 192 with 64 x 64;
-// 1000 x 2048 291 with 128 x 128, 321 with 128 x 64.
+// of 128 x 128 2.24 + 2.24, with the sums in tensor memory 2.33 + 2.00.  Sides of the lines it draws (us; rows x columns, k
+// 2048): 128 x 2048 89 with 16 rows and 116 with tiles of 64; 100 x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072
+// 186 with 128 x 64, 192 with 64 x 64; 1000 x 2048 291 with 128 x 128, 299 with the sums in tensor memory, 321 with 128 x 64;
+// 1000 x 16384 2003, 1794 and 2148.
 static inline int gemm_f32_form(int n_batch, int M, int N) {
     if (M <= 16) return M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
     const long long sms = gf_sms();
     const auto waves = [&](int rows, int cols) {
         return ((long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * n_batch + sms - 1) / sms;
     };
-    const int forms[4] = {16, 100, 101, 102};
-    const long long cost[4] = {3 + 10 * waves(16, 16), 30 + 60 * waves(64, 64), 30 + 115 * waves(128, 64), 224 * waves(128, 128)};
+    const int forms[5] = {16, 100, 101, 102, 103};
+    const long long cost[5] = {3 + 10 * waves(16, 16), 30 + 60 * waves(64, 64), 30 + 115 * waves(128, 64), 224 * waves(128, 128),
+                               33 + 200 * waves(128, 128)};
     int best = 0;
-    for (int f = 1; f < 4; ++f)
+    for (int f = 1; f < 5; ++f)
         if (cost[f] < cost[best]) best = f;
     return forms[best];
 }
 
-// form 0: chosen by the sizes; else one of the kernels: 1, 2, 4, 8, 16 (few rows, that many a group), 100, 101, 102 (tiles of
-// 64 x 64, 128 x 64 and 128 x 128)
+// form 0: chosen by the sizes; else one of the kernels: 1, 2, 4, 8, 16 (few rows, that many a group), 100, 101, 102, 103 (tiles
+// of 64 x 64, 128 x 64 and twice 128 x 128, the last with its sums in tensor memory)
 static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, const float* W, int ldw, long long w_batch,
                                   float* C, int ldc, long long c_batch, int n_batch, int M, int N, int K, int accumulate,
                                   int form, cudaStream_t stream) {
@@ -389,9 +476,9 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         kernel<<<dim3((unsigned)blocks, 1, n_batch), GF_PRODUCT_THREADS + gf_adders(MB, R), smem, stream>>>( \
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, groups, accumulate); \
     } while (0)
-#define GF_TILES(RM, RN, MINB) do { \
+#define GF_TILES(RM, RN, ...) do { \
         constexpr size_t smem = gf_tile_smem<RM, RN>(); \
-        auto kernel = gemm_f32_tile_kernel<RM, RN, MINB>; \
+        auto kernel = gemm_f32_tile_kernel<RM, RN, __VA_ARGS__>; \
         GF_CONFIGURE(kernel, smem); \
         const int rows = 16 * RM, cols = 16 * RN; \
         if ((M + rows - 1) / rows > 65535) return SSB_ERR_BAD_SIZE; \
@@ -407,6 +494,7 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         case 100: GF_TILES(4, 4, 3); break;
         case 101: GF_TILES(8, 4, 2); break;
         case 102: GF_TILES(8, 8, 1); break;
+        case 103: GF_TILES(8, 8, 2, true); break;
         default: return SSB_ERR_BAD_SIZE;
     }
 #undef GF_SKINNY
