@@ -32,7 +32,7 @@ class FastKernels(PlainKernels):
 
     def __init__(self, pdl: bool = True, deterministic: bool = False):
         self.pdl = pdl           # decode kernels launch as programmatic dependents of their predecessors
-        # True: no float atomics and one choice of kernel whatever the batch, so that a sequence's
+        # True: no two float atomics on one element and one choice of kernel whatever the batch, so that a sequence's
         # logits are the same bits in every run and in every batch (and a sampled sequence is
         # reproducible from its seed): projections never split K, prompts always take the tcgen05
         # attention, the decode attention cuts a sequence's keys in fixed chunks
@@ -58,15 +58,16 @@ class FastKernels(PlainKernels):
     PROMPT_CHAIN_ROWS = 4096
 
     def _prompt_chain(self, rows) -> bool:
-        """Whether a step of this many rows launches its norms, products and attention as programmatic dependents: a product
+        """Whether a prompt step of this many rows launches its norms, products and attention as programmatic dependents: a product
         then has its first weights in shared memory when the kernel before it ends.  us without and with: Llama 1B, 131 rows
         1,429 and 1,398, 2,000 rows 4,139 and 4,059; 8B, 131 rows 4,983 and 4,786; Vufadra, 200 rows 781 and 745, 2 x 1,000
         2,444 and 2,407.  Beyond 4,096 rows a kernel's end is too small a part of it: 8,000 rows of the 1B model 14,692 and
-        14,908."""
-        return bool(self.pdl) and int(rows) <= self.PROMPT_CHAIN_ROWS
+        14,908.  Smaller steps chain their own kernels: the few products of a decode step that come here would only take the
+        shared memory their neighbours start early in (one Vufadra sequence, width 1,024: a step 190 us, 196 with them)."""
+        return bool(self.pdl) and STREAM_ROWS < int(rows) <= self.PROMPT_CHAIN_ROWS
 
     def rmsnorm(self, x, weight, eps, out, rows=None):
-        pdl = self._prompt_chain(out.shape[0])
+        pdl = (self.pdl and out.shape[0] <= 64) or self._prompt_chain(out.shape[0])
         if ops.rmsnorm_vec_ok(x, weight, out):
             ops.rmsnorm_vec(x, weight, eps, out, rows, pdl=pdl)
         else:

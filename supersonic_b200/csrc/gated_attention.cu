@@ -213,7 +213,7 @@ __device__ __forceinline__ void ldmatrix_x4_plain(uint32_t addr, uint32_t& r0, u
     ldmatrix_x4(addr, r0, r1, r2, r3);
 }
 
-template <int DIM, int VDIM, bool SPLIT>
+template <int DIM, int VDIM, bool SPLIT, bool SHARED>          // SHARED: pages, by the blocks of a cluster
 __global__ void __launch_bounds__(GM_THREADS)
 sigmoid_attention_mma_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k_cache,
                              const bf16* __restrict__ v_cache, const int* __restrict__ cu_new,
@@ -227,8 +227,8 @@ sigmoid_attention_mma_kernel(const bf16* __restrict__ q, int ldq, const bf16* __
     extern __shared__ __align__(16) unsigned char gm_smem[];
     bf16* Ks = reinterpret_cast<bf16*>(gm_smem);          // [2][64][KP]
     bf16* Vs = Ks + 2 * GM_PAGE * KP;                     // [2][64][VP]
-    const int shares = SPLIT ? cluster : 1, share = SPLIT ? (int)blockIdx.x % shares : 0;
-    const int b = blockIdx.z, kvh = blockIdx.y, tile = blockIdx.x / shares;
+    const int shares = SHARED ? cluster : 1, share = SHARED ? (int)blockIdx.x % shares : 0;
+    const int b = blockIdx.z, kvh = blockIdx.y, tile = SHARED ? (int)blockIdx.x / shares : (int)blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     ssb_pdl_launch_dependents();
     ssb_pdl_wait();
@@ -244,7 +244,7 @@ sigmoid_attention_mma_kernel(const bf16* __restrict__ q, int ldq, const bf16* __
     int key_lo = chunk > 0 ? (p_first / chunk) * chunk : 0;
     if (window > 0) key_lo = max(key_lo, p_first - window + 1);
     // this block's run of the pages that hold them
-    const int first = key_lo / GM_PAGE, all_pages = p_last / GM_PAGE - first + 1, per_share = (all_pages + shares - 1) / shares;
+    const int first = key_lo / GM_PAGE, all_pages = p_last / GM_PAGE - first + 1, per_share = SHARED ? (all_pages + shares - 1) / shares : all_pages;
     const int page_lo = first + min(share * per_share, all_pages), page_hi = first + min((share + 1) * per_share, all_pages) - 1;
     const int* pages = page_table + (size_t)slot * max_pages;
 
@@ -378,7 +378,7 @@ sigmoid_attention_mma_kernel(const bf16* __restrict__ q, int ldq, const bf16* __
             r[(g + 8) * VDIM + 1] = acc[n][3];
         }
         __syncthreads();
-        if (shares > 1) {
+        if constexpr (SHARED) {
             for (int e = tid; e < 16 * VDIM; e += GM_THREADS)
                 red[e] = red[e] + red[16 * VDIM + e] + red[2 * 16 * VDIM + e] + red[3 * 16 * VDIM + e];
             ssb_cluster_sync();                           // every block's sums are in place
@@ -419,7 +419,7 @@ static int launch_sigmoid_mma(const bf16* q, int ldq, const bf16* k_cache, const
     constexpr int ROWS = SPLIT ? 16 : 64;
     size_t smem = (size_t)2 * GM_PAGE * (DIM + 8 + VDIM + 8) * sizeof(bf16);
     if (SPLIT && smem < (size_t)4 * 16 * VDIM * sizeof(float)) smem = (size_t)4 * 16 * VDIM * sizeof(float);
-    auto kern = sigmoid_attention_mma_kernel<DIM, VDIM, SPLIT>;
+    auto kern = SPLIT && cluster > 1 ? sigmoid_attention_mma_kernel<DIM, VDIM, SPLIT, SPLIT> : sigmoid_attention_mma_kernel<DIM, VDIM, SPLIT, false>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;

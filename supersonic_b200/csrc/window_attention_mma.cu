@@ -53,7 +53,7 @@ struct WmArgs {
     int cluster;                  // blocks of a cluster that share a row tile's pages (SPLIT only; 1: none)
 };
 
-template <int DIM, int VDIM, bool SPLIT, int ST>          // ST: pages in the ring
+template <int DIM, int VDIM, bool SPLIT, int ST, bool SHARED>          // ST: pages in the ring; SHARED: by the blocks of a cluster
 __global__ void __launch_bounds__(WM_THREADS)
 window_attention_mma_kernel(const WmArgs a) {
     constexpr int ROWS = SPLIT ? 16 : 64;
@@ -63,8 +63,8 @@ window_attention_mma_kernel(const WmArgs a) {
     bf16* Ks = reinterpret_cast<bf16*>(wm_smem);          // [ST][64][KP]
     bf16* Vs = Ks + ST * WM_PAGE * KP;                    // [ST][64][VP]
     __shared__ float m_s[4][16], l_s[4][16], f_s[4][16], blk_m[16], blk_l[16];
-    const int shares = SPLIT ? a.cluster : 1, share = SPLIT ? (int)blockIdx.x % shares : 0;
-    const int b = blockIdx.z, kvh = blockIdx.y, tile = blockIdx.x / shares;
+    const int shares = SHARED ? a.cluster : 1, share = SHARED ? (int)blockIdx.x % shares : 0;
+    const int b = blockIdx.z, kvh = blockIdx.y, tile = SHARED ? (int)blockIdx.x / shares : (int)blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int dim = a.dim, vdim = a.vdim, window = a.window, pool = a.pool, n_kv = a.n_kv;
     ssb_pdl_launch_dependents();
@@ -85,7 +85,7 @@ window_attention_mma_kernel(const WmArgs a) {
     const int page_lo = lo_first / WM_PAGE, page_hi = p_last / WM_PAGE;
     const int all_tiles = t_pool + t_keep + (page_hi - page_lo + 1);
     // this block's run of them: the tiles are counted from all of the sequence's first
-    const int per_share = (all_tiles + shares - 1) / shares;
+    const int per_share = SHARED ? (all_tiles + shares - 1) / shares : all_tiles;
     const int tile0 = min(share * per_share, all_tiles), n_tiles = min(tile0 + per_share, all_tiles);
     const int* pages = a.page_table + (size_t)slot * a.max_pages;
     const int* pool_pages = pool > 0 ? a.pool_table + (size_t)slot * a.pool_max_pages : nullptr;
@@ -285,7 +285,7 @@ window_attention_mma_kernel(const WmArgs a) {
         __syncthreads();                                  // the stage is free for the tile after next
     }
 
-    if (SPLIT && tile0 >= n_tiles) __syncthreads();       // a share without pages: the padding's zeros come before the sums
+    if (SHARED && tile0 >= n_tiles) __syncthreads();       // a share without pages: the padding's zeros come before the sums
     // the rows' sums, divided, as float32 [ROWS][VDIM] where the pages were staged
     float* fin = reinterpret_cast<float*>(wm_smem);
     const bool has_sink = a.sinks != nullptr || a.zero_sink;
@@ -333,7 +333,7 @@ window_attention_mma_kernel(const WmArgs a) {
             const int R = row0 + tid;
             float m = fmaxf(fmaxf(m_s[0][tid], m_s[1][tid]), fmaxf(m_s[2][tid], m_s[3][tid]));
             float sink_term = 0.f;
-            if (has_sink && R < n_rows && shares == 1) {
+            if (has_sink && R < n_rows && !SHARED) {
                 const float sk = a.sinks != nullptr ? a.sinks[kvh * G + R % G] : 0.f;
                 m = fmaxf(m, sk);
                 sink_term = __expf(sk - m);
@@ -344,11 +344,10 @@ window_attention_mma_kernel(const WmArgs a) {
                 f[w] = (m_s[w][tid] == -INFINITY) ? 0.f : __expf(m_s[w][tid] - m);
                 l += l_s[w][tid] * f[w];
             }
-            const float inv = shares > 1 ? 1.0f : l > 0.f ? 1.0f / l : 0.f;
+            const float inv = SHARED ? 1.0f : l > 0.f ? 1.0f / l : 0.f;
 #pragma unroll
             for (int w = 0; w < 4; ++w) f_s[w][tid] = f[w] * inv;
-            blk_m[tid] = m;
-            blk_l[tid] = l;
+            if (SHARED) { blk_m[tid] = m; blk_l[tid] = l; }
         }
         __syncthreads();
         for (int e = tid; e < 16 * VDIM; e += WM_THREADS) {
@@ -357,7 +356,7 @@ window_attention_mma_kernel(const WmArgs a) {
                      red[3 * 16 * VDIM + e] * f_s[3][r];
         }
         __syncthreads();
-        if (shares > 1) {
+        if constexpr (SHARED) {
             ssb_cluster_sync();                           // every block's maxima, sums and outputs are in place
             for (int r = share; r < 16 && row0 + r < n_rows; r += shares) {
                 float m = -INFINITY, l = 0.f;
@@ -386,7 +385,7 @@ window_attention_mma_kernel(const WmArgs a) {
     const int half = vdim >> 1;
     for (int e = tid; e < ROWS * half; e += WM_THREADS) {
         const int r = e / half, c2 = e - r * half, R = row0 + r;
-        if (R >= n_rows || (SPLIT && r % shares != share)) continue;
+        if (R >= n_rows || (SHARED && r % shares != share)) continue;
         const int tok = R / G, head = kvh * G + R % G, p = start + tok;
         const int c = 2 * c2;
         float x0 = fin[(size_t)r * VDIM + c], x1 = fin[(size_t)r * VDIM + c + 1];
@@ -419,7 +418,7 @@ window_attention_mma_kernel(const WmArgs a) {
         bf16* o = a.out + (size_t)(t0 + tok) * a.ldo + (size_t)head * vdim + c;
         *reinterpret_cast<uint32_t*>(o) = pack2(x0 * mul, x1 * mul1);
     }
-    if (SPLIT && shares > 1) ssb_cluster_sync();          // no block leaves while its outputs may be read
+    if (SHARED) ssb_cluster_sync();          // no block leaves while its outputs may be read
 }
 
 template <int DIM, int VDIM, bool SPLIT, int ST>
@@ -428,7 +427,8 @@ static int launch_window_mma(const WmArgs& a, int n_seqs, int max_new, int pdl, 
     const size_t smem = (size_t)ST * WM_PAGE * (DIM + 8 + VDIM + 8) * sizeof(bf16);
     static_assert((size_t)2 * WM_PAGE * (DIM + 8 + VDIM + 8) * sizeof(bf16) >= (size_t)64 * VDIM * sizeof(float),
                   "the staged pages make room for the rows' sums");
-    auto kern = window_attention_mma_kernel<DIM, VDIM, SPLIT, ST>;
+    // a kernel of its own for a block that has the pages to itself: the exchange's code and divisions cost such a step 1 %
+    auto kern = SPLIT && a.cluster > 1 ? window_attention_mma_kernel<DIM, VDIM, SPLIT, ST, SPLIT> : window_attention_mma_kernel<DIM, VDIM, SPLIT, ST, false>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
