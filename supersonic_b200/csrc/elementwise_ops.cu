@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(256)
 rope_append_vec_kernel(bf16* __restrict__ qkv, int ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                        const int* __restrict__ pos, const int* __restrict__ slot, const int* __restrict__ page_table,
                        int max_pages, bf16* __restrict__ k_cache, bf16* __restrict__ v_cache, int n_q, int n_kv,
-                       int head_dim, int page_shift) {
-    ssb_pdl_launch_dependents();
+                       int head_dim, int page_shift, int chain) {
+    if (chain) ssb_pdl_launch_dependents();
     ssb_pdl_wait();
     const int t = blockIdx.x;
     const int s = slot[t];
@@ -179,6 +179,6 @@ SSB_API int ssb_rope_append_vec(void* qkv, int ld, const float* cos_t, const flo
     if (head_dim % 8 || ld % 8 || !cos_t || !sin_t || table_positions <= 0) return SSB_ERR_BAD_SIZE;
     if (((uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15)
         return SSB_ERR_BAD_SIZE;
-    const int rc = ssb_launch(rope_append_vec_kernel<0>, dim3(n_tokens), dim3(256), 0, stream, pdl != 0, (bf16*)qkv, ld, cos_t, sin_t, pos, slot, page_table, max_pages, (bf16*)k_cache, (bf16*)v_cache, n_q, n_kv, head_dim, page_shift);
+    const int rc = ssb_launch(rope_append_vec_kernel<0>, dim3(n_tokens), dim3(256), 0, stream, pdl != 0, (bf16*)qkv, ld, cos_t, sin_t, pos, slot, page_table, max_pages, (bf16*)k_cache, (bf16*)v_cache, n_q, n_kv, head_dim, page_shift, pdl);
     return rc ? rc : ssb_launch_status();
 }

@@ -259,7 +259,7 @@ template <int BN, int STAGES>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                void* __restrict__ C, int ldc, int out_is_f32, int M, int N, int K, int mode, int m_tiles,
-               int n_tiles_total, int splits, int* __restrict__ error_word, const TcRope rope) {
+               int n_tiles_total, int splits, int* __restrict__ error_word, const TcRope rope, int chain) {
     constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2, W_BYTES = BN * TC_BK * 2, STAGE_BYTES = A_BYTES + W_BYTES;
     constexpr int N_ACC = 2;                                        // accumulator regions (2 x BN <= 512 columns)
     extern __shared__ unsigned char smem_raw[];
@@ -289,7 +289,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    ssb_pdl_launch_dependents();          // this block has its tensor memory: a dependent's cannot take it first
+    // this block has its tensor memory: a dependent's cannot take it first.  Only in chained steps: among the small kernels of a
+    // decode step, dependents that start early take the room their neighbours need (one Vufadra sequence: 190 us, 194 with it)
+    if (chain) ssb_pdl_launch_dependents();
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
@@ -405,7 +407,7 @@ template <int STAGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     void* __restrict__ C, int ldc, int out_is_f32, int M, int N, int K, int mode, int m_tiles,
-                    int n_tiles_total, int group_m, int* __restrict__ error_word, const TcRope rope) {
+                    int n_tiles_total, int group_m, int* __restrict__ error_word, const TcRope rope, int chain) {
     constexpr int BN = 256, HALF = 128;
     constexpr uint32_t A_BYTES = HALF * TC_BK * 2, W_BYTES = HALF * TC_BK * 2, STAGE_BYTES = A_BYTES + W_BYTES;
     constexpr int N_ACC = 2;
@@ -437,7 +439,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tc_fence_before();
     cluster_sync_all();   // both blocks' barriers are initialised before either signals the other
     tc_fence_after();
-    ssb_pdl_launch_dependents();
+    if (chain) ssb_pdl_launch_dependents();
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
@@ -581,7 +583,7 @@ static int launch_tc_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* C,
     // tiles in one band, 1,368 / 1,341 / 1,305 us with bands of 4 / 8 / 16; at 2,048 rows bands of 4 lose 4 %
     const int group_m = 16;
     const int rc = ssb_launch(kern, dim3(2 * pairs), dim3(TC_THREADS), smem, stream, pdl, ma, mw, C, ldc, out_is_f32, M, N, K, mode,
-                              m_tiles, total, group_m < m_tiles ? group_m : m_tiles, error_word, rope);
+                              m_tiles, total, group_m < m_tiles ? group_m : m_tiles, error_word, rope, pdl ? 1 : 0);
     return rc ? rc : ssb_launch_status();
 }
 
@@ -612,7 +614,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int 
     }
     const long long items = (long long)total * splits;
     const int rc = ssb_launch(kern, dim3(items < n_sms ? (int)items : n_sms), dim3(TC_THREADS), smem, stream, pdl, ma, mw, C, ldc,
-                              out_is_f32, M, N, K, mode, m_tiles, total, splits, error_word, rope);
+                              out_is_f32, M, N, K, mode, m_tiles, total, splits, error_word, rope, pdl ? 1 : 0);
     return rc ? rc : ssb_launch_status();
 }
 

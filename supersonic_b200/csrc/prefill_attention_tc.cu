@@ -100,7 +100,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const __grid_constant__ CUtensorMap map_v, const int* __restrict__ cu_new,
                             const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
                             const int* __restrict__ page_table, int max_pages, bf16* __restrict__ out, int ldo,
-                            int n_q, int n_kv, int window, float scale_log2, int* __restrict__ error_word) {
+                            int n_q, int n_kv, int window, float scale_log2, int* __restrict__ error_word, int chain) {
     constexpr int HALVES = FT_HD / 64;                           // 64-column boxes a row
     constexpr uint32_t FT_Q_BYTES = FT_BM * FT_HD * 2;           // a query tile
     constexpr uint32_t FT_PAGE_BYTES = 64 * FT_HD * 2;           // a page of keys (or values) of one kv head
@@ -119,7 +119,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     uint32_t* tmem_slot = (uint32_t*)(bars + FT_NBARS);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);   // [0]: a role gave up; [1]: stays zero
 
-    ssb_pdl_launch_dependents();
+    if (chain) ssb_pdl_launch_dependents();
     ssb_pdl_wait();
     // blocks start in the order of blockIdx.x, then y: every head's longest tiles come first
     const int kvh = blockIdx.x % n_kv, b = blockIdx.x / n_kv;
@@ -431,7 +431,7 @@ SSB_API int ssb_attention_prefill_tc(const void* q, int ldq, int n_rows_q, const
             configured = true; \
         } \
         const int rc_ = ssb_launch(prefill_attention_tc_kernel<HD_>, grid, dim3(FT_THREADS), smem, stream, pdl != 0, \
-            mq, mk, mv, cu_new, seq_start, seq_slot, page_table, max_pages, (bf16*)out, ldo, n_q, n_kv, window, scale * 1.4426950408889634f, error_word); \
+            mq, mk, mv, cu_new, seq_start, seq_slot, page_table, max_pages, (bf16*)out, ldo, n_q, n_kv, window, scale * 1.4426950408889634f, error_word, pdl); \
         if (rc_) return rc_; \
     } while (0)
     if (head_dim == 64) SSB_FT(64); else SSB_FT(128);
