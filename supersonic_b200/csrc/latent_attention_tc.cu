@@ -34,7 +34,7 @@ constexpr uint32_t LT_BOX_Q = LT_BM * 128, LT_BOX_K = LT_BN * 128;     // 64 dim
 // tensor-memory columns: the output, the scores of two turns, 64 dims of the query rows per 32 columns
 constexpr uint32_t LT_S0 = 256, LT_Q0 = 384;
 constexpr int LT_TMEM_BOXES = 4;           // query boxes that fit behind them
-constexpr int LT_NBARS = 2 + 2 * LT_MAX_STAGES + 5;
+constexpr int LT_NBARS = 2 + 2 * LT_MAX_STAGES + 6;
 constexpr float LT_LOG2E = 1.4426950408889634f;
 
 __device__ __forceinline__ bool lt_ready(uint32_t bar, uint32_t parity) {
@@ -116,10 +116,13 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const uint32_t stage_bytes = boxes * LT_BOX_K, ring_bytes = max(stages * stage_bytes, tm_boxes * LT_BOX_Q);
     const uint32_t q_s = smem_u32(smem), k_s = q_s + ss_boxes * LT_BOX_Q;
     uint64_t* bars = (uint64_t*)(smem + ss_boxes * LT_BOX_Q + ring_bytes);
-    // q_full, q_moved, k_full[stage], k_empty[stage], s_full[2], p_full[2], o_full: the scores of a turn are issued only
-    // after the weighted sum of the turn two before, so no role meets a barrier two phases on (the end waits for both)
+    // q_full, q_moved, k_full[stage], k_empty[stage], then one each for even and odd turns: s_full[2], p_full[2], o_full[2].  A
+    // wait by parity tells a phase from the next one only.  The scores of a turn are issued after the weighted sum of the turn
+    // two before, and that sum after the row's weights of its turn: whoever waits for a turn's barrier waits for the phase that
+    // is open or for the last one that closed.  One o_full for all turns would not do: after the last weights two sums may
+    // both end before a warp first looks.
     const uint32_t q_full = smem_u32(bars), q_moved = q_full + 8, k_full0 = q_moved + 8, k_empty0 = k_full0 + 8 * LT_MAX_STAGES,
-                   s_full0 = k_empty0 + 8 * LT_MAX_STAGES, p_full0 = s_full0 + 16, o_full = p_full0 + 16;
+                   s_full0 = k_empty0 + 8 * LT_MAX_STAGES, p_full0 = s_full0 + 16, o_full0 = p_full0 + 16;
     uint32_t* tmem_slot = (uint32_t*)(bars + LT_NBARS);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);   // [0]: a role gave up; [1]: stays zero
 
@@ -139,8 +142,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         mbar_init(q_full, 1);
         mbar_init(q_moved, 4);
         for (int s = 0; s < stages; ++s) { mbar_init(k_full0 + 8 * s, 1); mbar_init(k_empty0 + 8 * s, 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(s_full0 + 8 * i, 1); mbar_init(p_full0 + 8 * i, 4); }
-        mbar_init(o_full, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(s_full0 + 8 * i, 1); mbar_init(p_full0 + 8 * i, 4); mbar_init(o_full0 + 8 * i, 1); }
         abort_flag[0] = 0;
         abort_flag[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -209,7 +211,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     lt_mma_values(tmem, p, dv, idesc_o, next_o ? 1u : 0u);
                     lt_mma_values(tmem, p + LT_BN / 2, dv, idesc_o, 1u);
                     tc_commit(k_empty0 + 8 * (next_o % stages));
-                    tc_commit(o_full);
+                    tc_commit(o_full0 + 8 * (next_o & 1));
                     ++next_o;
                     since = clock64();
                 } else if (*abort_flag || clock64() - since > 2000000000LL) {
@@ -293,7 +295,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 const float m_new = fmaxf(m_ref, mx * scale_log2);
                 if (j > 0 && __any_sync(0xffffffffu, m_new > m_ref)) {
                     // rescale what this warp's rows have summed so far to their new maxima
-                    bool wo = mbar_wait(o_full, (j - 1) & 1, abort_flag);
+                    bool wo = mbar_wait(o_full0 + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, abort_flag);
                     wo = __all_sync(0xffffffffu, wo);
                     if (!wo) { ok = false; break; }
                     tc_fence_after();
@@ -320,9 +322,8 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             l_run += sum;
         }
         if (ok) {
-            // the last two weighted sums may both be under way: a wait by parity knows one phase from the next, no more
-            bool w = turns < 2 || mbar_wait(o_full, turns & 1, abort_flag);
-            w = w && mbar_wait(o_full, (turns - 1) & 1, abort_flag);
+            // the last weighted sum: its commit counts every product issued before it
+            const bool w = mbar_wait(o_full0 + 8 * ((turns - 1) & 1), ((turns - 1) >> 1) & 1, abort_flag);
             ok = __all_sync(0xffffffffu, w);
         }
         if (!ok) {

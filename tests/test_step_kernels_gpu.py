@@ -104,6 +104,24 @@ def test_latent_attention_of_prompts_on_tcgen05(H, dk, dv, window):
         assert err < 2.0 ** -9, (lengths, new, err)
 
 
+def test_latent_attention_of_prompts_ends_with_its_last_sums():
+    """Prompts of one to six turns with the shortest products, where the last two weighted sums end close together: run many
+    times, every row is written each time, with the same bits, and no wait runs out."""
+    from test_sotavik_kernels_gpu import latent_case
+    o, H, dk, dv = ops(), 16, 48, 32
+    for lengths in ([8, 64, 65, 128, 129, 190], [192, 193, 256, 257, 320, 384]):
+        cache, batch, store, table, q, rows = latent_case(lengths, lengths, H, dk, dv, seed=sum(lengths))
+        first = None
+        for turn in range(200):
+            out = torch.full((sum(lengths), H * dv), math.nan, dtype=torch.bfloat16, device=DEV)
+            o.latent_attention_tc(q, store, batch.cu_new, batch.seq_start, batch.seq_slot, table, out, None, batch.max_new, H, dk, dv,
+                                  6, None, dk ** -0.5)
+            first = out if first is None else first
+            assert torch.equal(out, first), (lengths, turn)
+        o.check_device_errors(torch.device(DEV))
+        assert bool(torch.isfinite(first).all())
+
+
 @pytest.mark.parametrize("top_k", [1, 5, 40, 64])
 def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top_k):
     """A top-k cut of a large step is searched over candidates, of a small one over the row in shared memory: the same
