@@ -398,7 +398,7 @@ class FastKernels(PlainKernels):
                                      window, scale, sinks)
             return
         if not batch.is_decode and not self.deterministic and batch.max_new * n_heads >= LATENT_TC_MIN_ROWS \
-                and ops.latent_attention_tc_ok(q_abs, cache, out, n_heads, dk, kv_rank, page_shift):
+                and ops.latent_attention_tc_ok(q_abs, cache, out, n_heads, dk, kv_rank, page_shift, batch.max_new):
             ops.latent_attention_tc(q_abs, cache, batch.cu_new, batch.seq_start, batch.seq_slot, page_table, out, sinks,
                                     batch.max_new, n_heads, dk, kv_rank, page_shift, window, scale)
             return

@@ -484,14 +484,16 @@ def latent_attention_mma(q: torch.Tensor, cache: torch.Tensor, cu_new: torch.Ten
         c_int(n_splits), c_int(form), c_int(1 if pdl else 0), _stream()), "latent_attention_mma")
 
 
+LATENT_TC_TILE_ROWS = 128        # (token, head) rows a block of latent_attention_tc.cu takes
 _latent_tc_fits = {}
 
 
 def latent_attention_tc_ok(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, n_heads: int, dk: int, dv: int,
-                           page_shift: int) -> bool:
+                           page_shift: int, max_new: int = 1) -> bool:
     """Whether the tcgen05 latent attention takes these operands: those of ``latent_attention_mma`` whose query rows fit
-    shared memory."""
-    if not latent_attention_mma_ok(q, cache, out, n_heads, dk, dv, page_shift):
+    shared memory, and whose longest prompt has no more row tiles than the y side of a grid counts."""
+    if not latent_attention_mma_ok(q, cache, out, n_heads, dk, dv, page_shift) \
+            or -(-max_new * n_heads // LATENT_TC_TILE_ROWS) > 65535:
         return False
     fits = _latent_tc_fits.get((dk, dv))
     if fits is None:
@@ -505,7 +507,7 @@ def latent_attention_tc(q: torch.Tensor, cache: torch.Tensor, cu_new: torch.Tens
                         scale: float) -> None:
     """``latent_attention_mma`` of a prompt step on tcgen05.  A wait that runs out sets the device's error word
     (``check_device_errors``)."""
-    if not latent_attention_tc_ok(q, cache, out, n_heads, dk, dv, page_shift):
+    if not latent_attention_tc_ok(q, cache, out, n_heads, dk, dv, page_shift, max_new):
         raise KernelError("latent_attention_tc: operands it does not take")
     _need(cu_new, "cu_new", torch.int32, 1); _need(seq_start, "seq_start", torch.int32, 1)
     _need(seq_slot, "seq_slot", torch.int32, 1); _need(page_table, "page_table", torch.int32, 2)

@@ -1,0 +1,36 @@
+"""Which kernel a call goes to, on the CPU with the kernels replaced by recorders: a kernel that does not take a size says so
+before it is launched, and the one that takes every size gets the call."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from supersonic_b200.csrc import ops
+from supersonic_b200.csrc.fast_sets import FastKernels
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    seen = []
+    for name in ("latent_attention_mma", "latent_attention_tc"):
+        monkeypatch.setattr(ops, name, lambda *a, _n=name, **k: seen.append(_n))
+    return seen
+
+
+def batch_of(n_seqs, max_new, is_decode=False):
+    none = torch.empty(0, dtype=torch.int32)
+    return SimpleNamespace(n_seqs=n_seqs, max_new=max_new, is_decode=is_decode, n_tokens=max_new, kv_pages=1, cu_new=none,
+                           seq_start=none, seq_slot=none, slot_of_token=none, pos=none)
+
+
+def test_latent_attention_of_more_row_tiles_than_a_grid_counts(calls):
+    """tcgen05 tiles are 128 (token, head) rows, and a grid's y side counts to 65,535 of them: 128 heads over 65,536 tokens
+    are one too many and go to the kernel that counts them along x."""
+    heads, rank, rot = 128, 32, 16
+    bf16 = lambda *shape: torch.empty(shape, dtype=torch.bfloat16)  # noqa: E731
+    q, cache, out = bf16(1, heads * (rank + rot)), bf16(1, 1, 64, rank + rot), bf16(1, heads * rank)
+    for max_new in (64, 65535, 65536):
+        FastKernels().latent_attention(q, cache, batch_of(1, max_new), None, out, heads, rank, rot, 6, None, 1.0, None)
+    assert calls == ["latent_attention_tc", "latent_attention_tc", "latent_attention_mma"]
+    assert ops.latent_attention_tc_ok(q, cache, out, heads, rank + rot, rank, 6, 65535)
+    assert not ops.latent_attention_tc_ok(q, cache, out, heads, rank + rot, rank, 6, 65536)
