@@ -149,7 +149,7 @@ class PlainKernels:
                   window: Optional[int], scale: float):
         # a float32 prompt: 64 (token, head) rows share the fetch of a key, the same sums in the same order
         if not window and not batch.is_decode and batch.max_new >= self.F32_PROMPT_MIN_NEW \
-                and ops.attention_f32_prompt_ok(q, k_cache, v_cache, out, head_dim):
+                and ops.attention_f32_prompt_ok(q, k_cache, v_cache, out, head_dim, batch.n_seqs):
             ops.attention_f32_prompt(q, k_cache, v_cache, batch.cu_new, batch.seq_start, batch.seq_slot, page_table, out,
                                      batch.max_new, n_q, n_kv, head_dim, page_shift, scale)
             return

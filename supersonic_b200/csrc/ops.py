@@ -219,9 +219,10 @@ def attention_plain(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
 
 
 def attention_f32_prompt_ok(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,
-                            head_dim: int) -> bool:
-    """Whether ``attention_f32_prompt`` takes these: float32 rows and caches in whole 16-byte pieces."""
-    return (q.dtype == torch.float32 and head_dim in (64, 128) and k_cache.is_contiguous() and v_cache.is_contiguous()
+                            head_dim: int, n_seqs: int = 1) -> bool:
+    """Whether ``attention_f32_prompt`` takes these: float32 rows and caches in whole 16-byte pieces, no more sequences than
+    the z side of a grid counts."""
+    return (q.dtype == torch.float32 and n_seqs <= 65535 and head_dim in (64, 128) and k_cache.is_contiguous() and v_cache.is_contiguous()
             and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0
             and all(t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, out)))
 

@@ -7,12 +7,13 @@ import torch
 
 from supersonic_b200.csrc import ops
 from supersonic_b200.csrc.fast_sets import FastKernels
+from supersonic_b200.csrc.kernel_sets import PlainKernels
 
 
 @pytest.fixture
 def calls(monkeypatch):
     seen = []
-    for name in ("latent_attention_mma", "latent_attention_tc"):
+    for name in ("latent_attention_mma", "latent_attention_tc", "attention_plain", "attention_f32_prompt"):
         monkeypatch.setattr(ops, name, lambda *a, _n=name, **k: seen.append(_n))
     return seen
 
@@ -34,3 +35,12 @@ def test_latent_attention_of_more_row_tiles_than_a_grid_counts(calls):
     assert calls == ["latent_attention_tc", "latent_attention_tc", "latent_attention_mma"]
     assert ops.latent_attention_tc_ok(q, cache, out, heads, rank + rot, rank, 6, 65535)
     assert not ops.latent_attention_tc_ok(q, cache, out, heads, rank + rot, rank, 6, 65536)
+
+
+def test_float32_prompts_of_more_sequences_than_a_grid_counts(calls):
+    """Tiles of 64 (token, head) rows have a sequence each along the grid's z side, which counts to 65,535."""
+    q, out = torch.empty(8, 128), torch.empty(8, 128)
+    cache = torch.empty(1, 1, 64, 64)
+    for n_seqs in (2, 65535, 65536):
+        PlainKernels().attention(q, cache, cache, batch_of(n_seqs, 8), None, out, 2, 1, 64, 6, None, 1.0)
+    assert calls == ["attention_f32_prompt", "attention_f32_prompt", "attention_plain"]
