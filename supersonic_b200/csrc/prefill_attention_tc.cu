@@ -119,7 +119,6 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     uint32_t* tmem_slot = (uint32_t*)(bars + FT_NBARS);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);   // [0]: a role gave up; [1]: stays zero
 
-    if (chain) ssb_pdl_launch_dependents();
     ssb_pdl_wait();
     // blocks start in the order of blockIdx.x, then y: every head's longest tiles come first
     const int kvh = blockIdx.x % n_kv, b = blockIdx.x / n_kv;
@@ -172,6 +171,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // this block has its tensor memory: a dependent that allocates some and waits for this kernel cannot take it first
+    if (chain) ssb_pdl_launch_dependents();
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {

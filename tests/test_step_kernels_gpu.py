@@ -293,6 +293,74 @@ def test_a_chain_of_dependent_launches_reads_what_was_written(rows):
     assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("lens,starts,hd", [([129], [0], 64), ([1, 200, 64, 5], [70, 0, 64, 300], 128), ([700, 324], [0, 9], 128)])
+def test_a_chain_of_a_prompts_layer_reads_what_was_written(lens, starts, hd):
+    """A prompt's layer as a step launches it: the projection that rotates and appends, attention, the products of the gated
+    unit, of an activation and into the stream, as programmatic dependents of one another or one after the other: the same bits."""
+    o, rows, n_q, n_kv = ops(), sum(lens), 4, 2
+    n, width = n_q * hd, (n_q + 2 * n_kv) * hd
+    w_qkv, w_o, w_gate, w_down, w_act = (rnd(a, b, seed=s, scale=b ** -0.5, dtype=torch.bfloat16) for s, (a, b) in
+                                         enumerate([(width, n), (n, n), (2 * n, n), (n, n), (n, n)]))
+    gain, angle = torch.ones(n, device=DEV), rnd(2048, hd // 2, seed=7)
+    cos, sin = torch.cos(angle), torch.sin(angle)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    cu, start, seq_slot = i32([sum(lens[:i]) for i in range(len(lens) + 1)]), i32(starts), i32(list(range(len(lens))))
+    pos = torch.cat([torch.arange(s, s + k) for s, k in zip(starts, lens)]).to(torch.int32).to(DEV)
+    slot = torch.repeat_interleave(seq_slot, i32(lens).long())
+    table = torch.arange(16 * len(lens), dtype=torch.int32, device=DEV).view(-1, 16)
+    got = []
+    for pdl in (False, True):
+        x, (k, v) = rnd(rows, n, seed=rows), (rnd(16 * len(lens), n_kv, 64, hd, seed=s, dtype=torch.bfloat16) for s in (8, 9))
+        h, q, att, z, y = (torch.zeros(rows, n, dtype=torch.bfloat16, device=DEV) for _ in range(5))
+        torch.cuda.synchronize()
+        for turn in range(20):
+            wide = (256, o.TC_TILE_PAIR)[turn % 2]
+            tile = (64, 128, 256, o.TC_TILE_PAIR)[turn % 4]
+            o.rmsnorm_vec(x, gain, 1e-5, h, pdl=pdl)
+            o.gemm_tc_rope_append(h, w_qkv, q, cos, sin, pos, slot, table, k, v, n_q, n_kv, hd, 6, tile_n=wide, pdl=pdl)
+            o.attention_prefill_tc(q, k, v, cu, start, seq_slot, table, att, max(lens), n_q, n_kv, hd, 6, None, hd ** -0.5, pdl=pdl)
+            o.gemm_tc(att, w_o, x, o.TC_ACCUMULATE, tile_n=tile, pdl=pdl)
+            o.rmsnorm_vec(x, gain, 1e-5, h, pdl=pdl)
+            if turn % 3:
+                o.gemm_tc(h, w_gate, z, o.TC_SWIGLU, tile_n=tile, pdl=pdl)
+            else:
+                o.gemm_tc_gate(h, w_gate, z, ("gelu_tanh", 0.0), None, tile_n=tile, pdl=pdl)
+            o.gemm_tc_act(z, w_act, y, "silu", 0.5, tile_n=tile, pdl=pdl)
+            o.gemm_tc(y, w_down, x, o.TC_ACCUMULATE, tile_n=tile, pdl=pdl)
+        o.check_device_errors(torch.device(DEV))
+        got.append((x.clone(), q.clone(), k.clone(), v.clone(), att.clone()))
+    assert all(bool(torch.isfinite(t.float()).all()) for t in got[0])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("rows", [129, 300])
+def test_a_chain_of_products_in_parts_reads_what_was_written(rows):
+    """Products whose K is cut into parts, rounded and cleared, the sums used again by the next: chained or not, each turn's
+    result is that of its own inputs.  Parts add in any order: float32 sums of 1,024 products, then one rounding."""
+    o, n, k = ops(), 256, 1024
+    w, back = rnd(n, k, seed=1, scale=k ** -0.5, dtype=torch.bfloat16), rnd(k, n, seed=2, scale=n ** -0.5, dtype=torch.bfloat16)
+    for pdl in (False, True):
+        sums, a, y = torch.zeros(rows, n, device=DEV), rnd(rows, k, seed=rows, dtype=torch.bfloat16), torch.empty(rows, n, dtype=torch.bfloat16, device=DEV)
+        torch.cuda.synchronize()
+        seen = []
+        for turn in range(12):
+            o.gemm_tc(a, w, sums, o.TC_ACCUMULATE, tile_n=128, splits=4, pdl=pdl)
+            o.round_and_clear(sums, y, pdl=pdl, act="silu" if turn % 2 else None)
+            a, before = torch.empty_like(a), a
+            o.gemm_tc(y, back, a, tile_n=128, pdl=pdl)
+            seen.append((before, y.clone(), a))
+        o.check_device_errors(torch.device(DEV))
+        assert bool((sums == 0).all())
+        for turn, (x, y_, a_) in enumerate(seen):
+            want = x.double() @ w.double().t()
+            want = torch.nn.functional.silu(want) if turn % 2 else want
+            bound = k * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) + 2.0 ** -8 * want.abs() + 1e-30
+            assert bool(((y_.double() - want).abs() <= bound).all()), (pdl, turn)
+            want = y_.double() @ back.double().t()
+            bound = n * 2.0 ** -24 * (y_.double().abs() @ back.double().abs().t()) + 2.0 ** -8 * want.abs() + 1e-30
+            assert bool(((a_.double() - want).abs() <= bound).all()), (pdl, turn)
+
+
 @pytest.mark.parametrize("width", [8, 2048, 516, 1030])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_sums_of_a_few_rows_in_their_order(width, dtype):
