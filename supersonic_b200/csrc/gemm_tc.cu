@@ -114,7 +114,7 @@ __device__ __forceinline__ void tc_epilogue(uint32_t acc, int quarter, int row, 
         // a head at a time: its low and high halves meet in this thread (the row's token)
         const int hd = rope.head_dim, half = hd / 2, halves32 = half / 32;
         const bool live = row < M;
-        const int p = live ? rope.pos[row] : 0, sl = live ? rope.slot[row] : -1;
+        const int sl = live ? rope.slot[row] : -1, p = sl >= 0 ? rope.pos[row] : 0;      // a row of no slot has no position
         size_t tok = 0;
         if (sl >= 0) {
             const int page = rope.page_table[(size_t)sl * rope.max_pages + (p >> rope.page_shift)];

@@ -267,6 +267,31 @@ def test_products_leave_in_whole_rows(m, n, k, tile):
     assert all(bool((x[m] == 5.0).all() and (x[:, n:] == 5.0).all()) for x in wide)
 
 
+@pytest.mark.parametrize("tile", [256, "pair"])
+def test_rows_of_no_slot_have_no_position(tile):
+    """The projection that rotates and appends skips rows with a negative slot, whatever their position says: one far outside the
+    rotation tables is not looked up, and the other rows, in the same warps, are as they are without them."""
+    o, rows, hd, n_q, n_kv = ops(), 140, 64, 2, 1
+    tile = o.TC_TILE_PAIR if tile == "pair" else tile
+    a, w = rnd(rows, 128, seed=1, dtype=torch.bfloat16), rnd((n_q + 2 * n_kv) * hd, 128, seed=2, scale=0.1, dtype=torch.bfloat16)
+    cos, sin = torch.cos(rnd(256, hd // 2, seed=3)), torch.sin(rnd(256, hd // 2, seed=3))
+    table = torch.arange(4, dtype=torch.int32, device=DEV).view(1, 4)
+    dead = torch.arange(rows, device=DEV) % 3 == 1
+    got = []
+    for outside in (False, True):
+        pos = torch.arange(rows, dtype=torch.int32, device=DEV)
+        slot = torch.where(dead, -1, 0).to(torch.int32)
+        if outside:
+            pos[dead] = 1 << 30
+        q = torch.full((rows, n_q * hd), 5.0, dtype=torch.bfloat16, device=DEV)
+        k, v = (torch.full((4, n_kv, 64, hd), 5.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        o.gemm_tc_rope_append(a, w, q, cos, sin, pos, slot, table, k, v, n_q, n_kv, hd, 6, tile_n=tile)
+        o.check_device_errors(torch.device(DEV))
+        assert bool((q[dead] == 5.0).all()) and bool((q[~dead] != 5.0).any(1).all())
+        got.append((q, k, v))
+    assert all(torch.equal(x, y) for x, y in zip(*got))
+
+
 @pytest.mark.parametrize("rows", [129, 300, 1024])
 def test_a_chain_of_dependent_launches_reads_what_was_written(rows):
     """Norm, product, product into the stream, attention's preparation: launched as programmatic dependents of one another or
