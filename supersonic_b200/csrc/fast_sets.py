@@ -421,7 +421,7 @@ class FastKernels(PlainKernels):
         return self._buffer("unit_scan_chunks", n, torch.float32, device)
 
     def _tied_chunking(self, batch, n_heads, dim, vdim):
-        if self.deterministic:                 # chunks of one length whatever else is in the step
+        if self.deterministic:                 # cut by the sequence's own length, whatever else is in the step
             return ops.scan_chunking(batch.n_seqs, batch.max_new, n_heads, dim, vdim)
         return super()._tied_chunking(batch, n_heads, dim, vdim)
 
@@ -490,17 +490,18 @@ class FastKernels(PlainKernels):
 
     def gated_linear_scan(self, proj, q_off, k_off, v_off, z, z_bias, tau, q_scale, state, batch, out, n_heads,
                           dim, vdim):
-        if self.deterministic:                 # chunks of one length whatever else is in the step
-            chunk, n_sums, n_decays = ops.scan_chunking(batch.n_seqs, batch.max_new, n_heads, dim, vdim)
+        if self.deterministic:                 # cut by the sequence's own length, whatever else is in the step
+            cut, n_sums, n_decays = ops.scan_chunking(batch.n_seqs, batch.max_new, n_heads, dim, vdim)
         else:
             chunk, n_sums, n_decays = ops.gated_scan_chunking(batch.n_seqs, batch.max_new, n_heads, dim, vdim, ops.sm_count())
+            cut = {"chunk": chunk} if chunk else {}
         sums = decays = None
-        if chunk:
+        if cut:
             sums = self._buffer("scan_sums", n_sums, torch.float32, out.device)
             decays = self._buffer("scan_decays", n_decays, torch.float32, out.device)
         ops.gated_linear_scan(proj, q_off, k_off, v_off, z, z_bias, tau, q_scale, state, batch.cu_new,
-                              batch.seq_slot, out, n_heads, dim, vdim, pdl=self.pdl, chunk=chunk,
-                              max_new=batch.max_new, sums=sums, decays=decays)
+                              batch.seq_slot, out, n_heads, dim, vdim, pdl=self.pdl, max_new=batch.max_new, sums=sums,
+                              decays=decays, **cut)
 
     def route_table(self, token_ids, table, n_experts, expert_of, pair_weight):
         ops.route_table(token_ids, table, n_experts, expert_of, pair_weight, pdl=self.pdl)

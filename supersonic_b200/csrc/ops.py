@@ -625,11 +625,24 @@ def grouped_gemm_mma(a: torch.Tensor, a_index: Optional[torch.Tensor], a_div: in
 SCAN_MAX_DIM = 256
 
 
+def _scan_places(chunk, max_new, n_seqs, places, sums, decays, n_heads, dim, vdim, what):
+    """(chunks of the longest run, (sequence, chunk) pairs the scratch holds) of a chunked scan, (0, 0) of a walk."""
+    if chunk <= 0:
+        return 0, 0
+    max_chunks = -(-max_new // chunk)
+    places = n_seqs * max_chunks if places is None else min(places, n_seqs * max_chunks)
+    _need(sums, "sums", torch.float32); _need(decays, "decays", torch.float32)
+    if places < 1 or sums.numel() < places * n_heads * dim * vdim or decays.numel() < places * n_heads * dim:
+        raise KernelError(f"{what}: the scratch of the chunked run is too small")
+    return max_chunks, places
+
+
 def gated_linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z: torch.Tensor,
                       z_bias: torch.Tensor, tau: float, q_scale: float, state: torch.Tensor,
                       cu_new: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, n_heads: int, dim: int,
                       vdim: int, pdl: bool = False, chunk: int = 0, max_new: int = 0,
-                      sums: Optional[torch.Tensor] = None, decays: Optional[torch.Tensor] = None) -> None:
+                      sums: Optional[torch.Tensor] = None, decays: Optional[torch.Tensor] = None, min_new: int = 0,
+                      places: Optional[int] = None) -> None:
     """Per sequence and head, over the sequence's new tokens in order:
     S = diag(sigmoid(z + z_bias)^(1/tau)) S + k v^T;  out = S^T (q * q_scale), with S [dim, vdim] float32 read
     from and left in ``state[slot]``.  q, k (heads x dim) and v (heads x vdim) are columns of ``proj``; ``z`` is
@@ -637,7 +650,9 @@ def gated_linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z:
     ``chunk`` > 0: every sequence's tokens are cut into chunks of that many that run in parallel (each chunk's
     own sum from zero, the state carried across the chunks in order, then the outputs of every chunk from the
     state at its start), through the float32 scratch ``sums`` (sequences x chunks x heads x dim x vdim) and
-    ``decays`` (sequences x chunks x heads x dim), chunks = ceil(``max_new`` / chunk)."""
+    ``decays`` (sequences x chunks x heads x dim), chunks = ceil(``max_new`` / chunk).  Sequences of fewer than
+    ``min_new`` new tokens are walked in one go all the same.  With ``places`` the scratch holds that many (sequence,
+    chunk) pairs and no more, and the step takes as many passes as that needs; the results do not depend on it."""
     _need(proj, "proj", None, 2); _need(z, "z", torch.float32, 2); _need(z_bias, "z_bias", torch.float32, 1)
     _need(state, "state", torch.float32, 2); _need(out, "out", torch.float32, 2)
     _need(cu_new, "cu_new", torch.int32, 1); _need(seq_slot, "seq_slot", torch.int32, 1)
@@ -649,18 +664,12 @@ def gated_linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z:
         raise KernelError("gated_linear_scan: proj rows are too narrow")
     if state.shape[1] != n_heads * dim * vdim or not state.is_contiguous() or dim > SCAN_MAX_DIM:
         raise KernelError(f"gated_linear_scan: state rows of heads x dim x vdim, dim up to {SCAN_MAX_DIM}")
-    max_chunks = 0
-    if chunk > 0:
-        max_chunks = -(-max_new // chunk)
-        _need(sums, "sums", torch.float32); _need(decays, "decays", torch.float32)
-        if max_chunks < 1 or sums.numel() < B * max_chunks * n_heads * dim * vdim \
-                or decays.numel() < B * max_chunks * n_heads * dim:
-            raise KernelError("gated_linear_scan: the scratch of the chunked run is too small")
+    max_chunks, places = _scan_places(chunk, max_new, B, places, sums, decays, n_heads, dim, vdim, "gated_linear_scan")
     _check(_fn("recurrence_ops", "ssb_gated_linear_scan")(
         _ptr(proj), c_int(proj.stride(0)), c_int(dtype_code(proj.dtype)), c_int(q_off), c_int(k_off), c_int(v_off),
         _ptr(z), c_int(z.stride(0)), _ptr(z_bias), c_float(tau), c_float(q_scale), _ptr(state), _ptr(cu_new),
         _ptr(seq_slot), _ptr(out), c_int(out.stride(0)), c_int(B), c_int(T), c_int(n_heads), c_int(dim), c_int(vdim),
-        c_int(chunk), c_int(max_chunks), _ptr(sums), _ptr(decays), c_int(1 if pdl else 0), _stream()),
+        c_int(chunk), c_int(max_chunks), c_int(min_new), c_int(places), _ptr(sums), _ptr(decays), c_int(1 if pdl else 0), _stream()),
         "gated_linear_scan")
 
 
@@ -710,11 +719,12 @@ def gated_scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim:
 def tied_scan(proj: torch.Tensor, q_off: int, f_off: int, v_off: int, z_bias: torch.Tensor, lower: torch.Tensor,
               state: torch.Tensor, cu_new: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, n_heads: int, dim: int,
               vdim: int, norm_w: Optional[torch.Tensor] = None, eps: float = 0.0, pdl: bool = False, chunk: int = 0,
-              max_new: int = 0, sums: Optional[torch.Tensor] = None, decays: Optional[torch.Tensor] = None) -> None:
+              max_new: int = 0, sums: Optional[torch.Tensor] = None, decays: Optional[torch.Tensor] = None, min_new: int = 0,
+              places: Optional[int] = None) -> None:
     """Per sequence and head, over the sequence's new tokens in order, with the gate f = lower + (1 - lower) *
     sigmoid(z + z_bias) per head and channel:  S = diag(f) S + (1 - f) v^T;  o = S^T silu(q).  q and z (heads x dim)
-    and v (heads x vdim) are columns of ``proj``; ``state``, ``chunk``, ``sums`` and ``decays`` as in ``gated_linear_scan``.
-    ``out`` gets o (float32) or, with ``norm_w`` [vdim] (heads of up to ``tied_scan_cols`` values), o / rms(o) * norm_w per head."""
+    and v (heads x vdim) are columns of ``proj``; ``state``, ``chunk``, ``sums``, ``decays``, ``min_new`` and ``places``
+    as in ``gated_linear_scan``.  ``out`` gets o (float32) or, with ``norm_w`` [vdim] (heads of up to ``tied_scan_cols`` values), o / rms(o) * norm_w per head."""
     _tied_args(proj, q_off, f_off, v_off, z_bias, lower, state, cu_new, seq_slot, n_heads, dim, vdim, "tied_scan")
     _need(out, "out", proj.dtype if norm_w is not None else torch.float32, 2)
     T, B = proj.shape[0], seq_slot.shape[0]
@@ -724,18 +734,12 @@ def tied_scan(proj: torch.Tensor, q_off: int, f_off: int, v_off: int, z_bias: to
         _need(norm_w, "norm_w", torch.float32, 1)
         if norm_w.shape[0] != vdim or vdim > tied_scan_cols(dim, vdim):
             raise KernelError(f"tied_scan: a norm weight per value column, heads of up to {tied_scan_cols(dim, vdim)}")
-    max_chunks = 0
-    if chunk > 0:
-        max_chunks = -(-max_new // chunk)
-        _need(sums, "sums", torch.float32); _need(decays, "decays", torch.float32)
-        if max_chunks < 1 or sums.numel() < B * max_chunks * n_heads * dim * vdim \
-                or decays.numel() < B * max_chunks * n_heads * dim:
-            raise KernelError("tied_scan: the scratch of the chunked run is too small")
+    max_chunks, places = _scan_places(chunk, max_new, B, places, sums, decays, n_heads, dim, vdim, "tied_scan")
     _check(_fn("recurrence_ops", "ssb_tied_scan")(
         _ptr(proj), c_int(proj.stride(0)), c_int(dtype_code(proj.dtype)), c_int(q_off), c_int(f_off), c_int(v_off),
         _ptr(z_bias), _ptr(lower), _ptr(state), _ptr(cu_new), _ptr(seq_slot), _ptr(None if norm_w is not None else out),
         c_int(out.stride(0)), _ptr(norm_w), c_float(eps), _ptr(out if norm_w is not None else None), c_int(out.stride(0)),
-        c_int(B), c_int(T), c_int(n_heads), c_int(dim), c_int(vdim), c_int(chunk), c_int(max_chunks), _ptr(sums), _ptr(decays),
+        c_int(B), c_int(T), c_int(n_heads), c_int(dim), c_int(vdim), c_int(chunk), c_int(max_chunks), c_int(min_new), c_int(places), _ptr(sums), _ptr(decays),
         c_int(1 if pdl else 0), _stream()), "tied_scan")
 
 
@@ -822,17 +826,15 @@ SCAN_SCRATCH_BYTES = 1 << 30     # the most the chunk sums of a step may take
 
 
 def scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim: int):
-    """(chunk, floats of sums, floats of decays) for a step's recurrence; chunk 0: walk every sequence in one
-    go.  The chunk grows beyond SCAN_CHUNK where the sums of all chunks would not fit the scratch bound."""
+    """The cut of a recurrence whose sums a sequence's own length decides, as the options of ``gated_linear_scan`` and
+    ``tied_scan``, and the floats of sums and of decays: sequences of SCAN_CHUNK_MIN_NEW new tokens or more in chunks of
+    SCAN_CHUNK, the others walked in one go, whatever else is in the step.  The scratch is bounded: what does not fit runs in
+    several passes."""
     if max_new < SCAN_CHUNK_MIN_NEW:
-        return 0, 0, 0
+        return {}, 0, 0
     per = n_heads * dim * vdim
-    most = SCAN_SCRATCH_BYTES // (4 * per * n_seqs)
-    if most < 2:
-        return 0, 0, 0
-    chunk = max(SCAN_CHUNK, -(-max_new // most))
-    n = -(-max_new // chunk)
-    return chunk, n_seqs * n * per, n_seqs * n * n_heads * dim
+    places = min(n_seqs * (-(-max_new // SCAN_CHUNK)), max(SCAN_SCRATCH_BYTES // (4 * per), 1))
+    return {"chunk": SCAN_CHUNK, "min_new": SCAN_CHUNK_MIN_NEW, "places": places}, places * per, places * n_heads * dim
 
 
 def head_norm_gate(o: torch.Tensor, weight: torch.Tensor, eps: float, gate: Optional[torch.Tensor], out: torch.Tensor,

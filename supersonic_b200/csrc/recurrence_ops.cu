@@ -6,8 +6,10 @@
 // a_t = sigmoid(z_t)^(1/tau), evaluated as exp(log_sigmoid(z_t) / tau).  Everything that enters the
 // recurrence is float32; q, k and v are read in their storage type and widened.
 // The scan walks a sequence's new tokens in order, from the state the sequence's slot holds, and
-// leaves the state there; a block owns a tile of value columns of one head of one sequence, so no
-// sum depends on what else is in the batch.
+// leaves the state there; a block owns a tile of value columns of one head of one sequence.  A long run
+// may be cut into chunks that run in parallel, which adds the same terms in another order: whether and
+// where is the caller's choice, by the step's sizes or, with one chunk length and min_new, by the
+// sequence's own length, so that its sums do not depend on what else is in the batch.
 #include "common.cuh"
 #include <math.h>
 #include <type_traits>
@@ -37,11 +39,12 @@ __global__ void decay_kernel(float* __restrict__ z, int ldz, const float* __rest
 
 // Carries the state across a sequence's chunks: with S the state before chunk c, chunk c's place in
 // ``sums`` gets S (what the chunk starts from) and S <- decays[c] * S + sums[c]; the last S is the
-// sequence's state.  One thread per state element, chunks in order.
+// sequence's state.  One thread per state element, chunks in order: those that this pass holds, from chunk0 on.  Runs
+// of fewer than min_new tokens are walked in one go and have nothing to carry.
 __global__ void __launch_bounds__(256)
 gated_linear_carry_kernel(float* __restrict__ state, float* __restrict__ sums, const float* __restrict__ decays,
                           const int* __restrict__ cu_new, const int* __restrict__ seq_slot, int n_heads, int dim,
-                          int vdim, int chunk, int max_chunks) {
+                          int vdim, int chunk, int max_chunks, int chunk0, int min_new) {
     ssb_pdl_launch_dependents();
     ssb_pdl_wait();
     const int b = blockIdx.y, slot = seq_slot[b];
@@ -50,11 +53,12 @@ gated_linear_carry_kernel(float* __restrict__ state, float* __restrict__ sums, c
     const size_t e = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (e >= per) return;
     const size_t hi = e / vdim;                          // head * dim + channel
-    const int n_chunks = (cu_new[b + 1] - cu_new[b] + chunk - 1) / chunk;
+    const int n_new = cu_new[b + 1] - cu_new[b], n_chunks = min((n_new + chunk - 1) / chunk - chunk0, max_chunks);
+    if (n_new < min_new || n_chunks <= 0) return;
     float cur = state[(size_t)slot * per + e];
     float* sp = sums + (size_t)b * max_chunks * per + e;
     const float* dp = decays + (size_t)b * max_chunks * n_heads * dim + hi;
-    float loc = n_chunks > 0 ? sp[0] : 0.f, a = n_chunks > 0 ? dp[0] : 0.f;
+    float loc = sp[0], a = dp[0];
     for (int c = 0; c < n_chunks; ++c) {
         float loc_n = 0.f, a_n = 0.f;
         if (c + 1 < n_chunks) {
@@ -71,24 +75,25 @@ gated_linear_carry_kernel(float* __restrict__ state, float* __restrict__ sums, c
 
 static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
                       float q_scale, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo, int n_seqs,
-                      int n_heads, int dim, int vdim, int chunk, int max_chunks, float* sums, float* decays, bool pdl,
-                      cudaStream_t stream);
+                      int n_heads, int dim, int vdim, int chunk, int max_chunks, int min_new, int places, float* sums,
+                      float* decays, bool pdl, cudaStream_t stream);
 
 // proj [T, ld] holds q, k (n_heads x dim each) and v (n_heads x vdim) from the given columns;
 // z [T, ldz] float32 is the decay's pre-activation without its bias z_bias [n_heads x dim], and is overwritten
 // with the decays;
 // state [slots, n_heads, dim, vdim] float32; out [T, ldo] float32 gets o (n_heads x vdim).
-// chunk > 0: sequences are run in chunks of that many tokens, in parallel, through ``sums``
-// (n_seqs x max_chunks x n_heads x dim x vdim floats) and ``decays`` (n_seqs x max_chunks x n_heads x dim);
-// max_chunks = ceil(longest run of new tokens / chunk).
+// chunk > 0: sequences of min_new new tokens or more are run in chunks of that many tokens, in parallel, the others walked in
+// one go.  max_chunks = ceil(longest run of new tokens / chunk).  ``sums`` (places x n_heads x dim x vdim floats) and ``decays``
+// (places x n_heads x dim) hold so many (sequence, chunk) pairs at a time; with fewer than n_seqs x max_chunks the step
+// takes several passes, over sequences and over runs of chunks, and every sum is the same.
 SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off,
                                   float* z, int ldz, const float* z_bias, float tau, float q_scale,
                                   float* state, const int* cu_new, const int* seq_slot, float* out, int ldo,
                                   int n_seqs, int n_tokens, int n_heads, int dim, int vdim, int chunk, int max_chunks,
-                                  float* sums, float* decays, int pdl, cudaStream_t stream) {
+                                  int min_new, int places, float* sums, float* decays, int pdl, cudaStream_t stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (dim <= 0 || dim > SCAN_MAX_DIM || vdim <= 0 || !(tau > 0.f)) return SSB_ERR_BAD_SIZE;
-    if (chunk < 0 || (chunk > 0 && (max_chunks <= 0 || sums == nullptr || decays == nullptr))) return SSB_ERR_BAD_SIZE;
+    if (chunk < 0 || (chunk > 0 && (max_chunks <= 0 || places <= 0 || sums == nullptr || decays == nullptr))) return SSB_ERR_BAD_SIZE;
     const long long items = chunk > 0 ? (long long)n_seqs * max_chunks : n_seqs;
     if (items > 0x7fffffffll) return SSB_ERR_BAD_SIZE;
     if (n_heads > 65535 || (vdim + 31) / 32 > 65535 || n_seqs > 65535) return SSB_ERR_BAD_SIZE;
@@ -99,7 +104,7 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
     if (!rc) rc = ssb_launch_status();
     if (rc) return rc;
     return gated_walk(proj, ld, dtype, q_off, k_off, v_off, z, ldz, q_scale, state, cu_new, seq_slot, out, ldo, n_seqs,
-                      n_heads, dim, vdim, chunk, max_chunks, sums, decays, pdl != 0, stream);
+                      n_heads, dim, vdim, chunk, max_chunks, min_new, places, sums, decays, pdl != 0, stream);
 }
 
 // =======================================================================================
@@ -135,6 +140,7 @@ struct TiedArgs {
     float* out; int ldo;
     const float* norm_w; float eps; void* y; int ldy;
     int n_heads, dim, vdim, chunk, max_chunks;
+    int chunk0, min_new, places;                           // this pass's first chunk; runs that are cut; see ssb_gated_linear_scan
     float* sums; float* decays;
 };
 
@@ -157,14 +163,17 @@ tied_walk_kernel(const TiedArgs a) {
     const int slot = a.seq_slot[b];
     if (slot < 0) return;                                  // padding row
     int t0 = a.cu_new[b], t1 = a.cu_new[b + 1];
-    if (a.chunk > 0) {
-        t0 += ch * a.chunk;
+    const bool cut = a.chunk > 0 && t1 - t0 >= a.min_new;
+    if (cut) {
+        t0 += (a.chunk0 + ch) * a.chunk;
         t1 = min(t1, t0 + a.chunk);
+    } else if (a.chunk > 0 && (!OUT || a.chunk0 + ch > 0)) {
+        return;                                            // a short run beside long ones: one block walks all of it
     }
     if (t0 >= t1) return;
     const T* proj = reinterpret_cast<const T*>(a.proj);
-    float* S = a.chunk > 0 ? a.sums + (((size_t)blockIdx.x * a.n_heads + h) * dim) * vdim
-                           : a.state + ((size_t)slot * a.n_heads + h) * dim * vdim;
+    float* S = cut ? a.sums + (((size_t)blockIdx.x * a.n_heads + h) * dim) * vdim
+                   : a.state + ((size_t)slot * a.n_heads + h) * dim * vdim;
     const int col0 = warp * 8 + cg * 4;                    // this lane's four columns, within the block's
     const bool pieces = vdim % 4 == 0 && ((uintptr_t)S & 15) == 0;       // a lane's four columns in one access
     float s[R4][4][4];
@@ -303,7 +312,7 @@ tied_walk_kernel(const TiedArgs a) {
         __syncthreads();
         const int last = t0 + (t1 - t0 - 1) / TW_TOKENS * TW_TOKENS;
         finish(last, buf ^ 1);
-        if (a.chunk > 0) return;                           // the state was carried by the carry kernel
+        if (cut) return;                                   // the state was carried by the carry kernel
     }
 #pragma unroll
     for (int g = 0; g < R4; ++g)
@@ -326,7 +335,7 @@ tied_walk_kernel(const TiedArgs a) {
 }
 
 template <typename T, int R4, int NT, bool GATED = false>
-static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_t stream) {
+static int launch_tied_pass(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_t stream) {
     constexpr int DIMP = 64 * R4, COLS = NT / 4;
     constexpr size_t smem = (size_t)TW_TOKENS * ((GATED ? 6 : 4) * DIMP + 4 * COLS) * sizeof(float);
     const long long items = a.chunk > 0 ? (long long)n_seqs * a.max_chunks : n_seqs;
@@ -347,7 +356,8 @@ static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
         if (rc) return rc;
         const size_t per = (size_t)a.n_heads * a.dim * a.vdim;
         rc = ssb_launch(gated_linear_carry_kernel, dim3((unsigned)((per + 255) / 256), n_seqs), dim3(256), 0, stream, pdl, a.state,
-                        a.sums, (const float*)a.decays, a.cu_new, a.seq_slot, a.n_heads, a.dim, a.vdim, a.chunk, a.max_chunks);
+                        a.sums, (const float*)a.decays, a.cu_new, a.seq_slot, a.n_heads, a.dim, a.vdim, a.chunk, a.max_chunks,
+                        a.chunk0, a.min_new);
         if (!rc) rc = ssb_launch_status();
         if (rc) return rc;
     }
@@ -355,14 +365,32 @@ static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
     return rc ? rc : ssb_launch_status();
 }
 
+// All of a step: in one pass where every (sequence, chunk) pair has its place in the scratch, else sequences in groups and their
+// chunks in runs, one after another.
+template <typename T, int R4, int NT, bool GATED = false>
+static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_t stream) {
+    if (a.chunk <= 0 || (long long)n_seqs * a.max_chunks <= a.places) return launch_tied_pass<T, R4, NT, GATED>(a, n_seqs, pdl, stream);
+    const int group = n_seqs < a.places ? n_seqs : a.places, run = a.places / group;
+    for (int b = 0; b < n_seqs; b += group)
+        for (int c = 0; c < a.max_chunks; c += run) {
+            TiedArgs p = a;
+            p.cu_new += b; p.seq_slot += b;
+            p.chunk0 = c;
+            p.max_chunks = a.max_chunks - c < run ? a.max_chunks - c : run;
+            const int rc = launch_tied_pass<T, R4, NT, GATED>(p, n_seqs - b < group ? n_seqs - b : group, pdl, stream);
+            if (rc) return rc;
+        }
+    return 0;
+}
+
 static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
                            float q_scale, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo, int n_seqs,
-                           int n_heads, int dim, int vdim, int chunk, int max_chunks, float* sums, float* decays, bool pdl,
-                           cudaStream_t stream) {
+                           int n_heads, int dim, int vdim, int chunk, int max_chunks, int min_new, int places, float* sums,
+                           float* decays, bool pdl, cudaStream_t stream) {
     TiedArgs a = {};
     a.proj = proj; a.ld = ld; a.q_off = q_off; a.f_off = k_off; a.v_off = v_off; a.decay = decay; a.ldz = ldz; a.q_scale = q_scale;
     a.state = state; a.cu_new = cu_new; a.seq_slot = seq_slot; a.out = out; a.ldo = ldo; a.n_heads = n_heads; a.dim = dim;
-    a.vdim = vdim; a.chunk = chunk; a.max_chunks = max_chunks; a.sums = sums; a.decays = decays;
+    a.vdim = vdim; a.chunk = chunk; a.max_chunks = max_chunks; a.min_new = min_new; a.places = places; a.sums = sums; a.decays = decays;
 #define SSB_GW(T) \
     return dim <= 64 ? launch_tied_walk<T, 1, 256, true>(a, n_seqs, pdl, stream) \
          : dim <= 128 ? launch_tied_walk<T, 2, 256, true>(a, n_seqs, pdl, stream) \
@@ -374,20 +402,21 @@ static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off,
 
 // proj [T, ld] holds q and the gate's pre-activation (n_heads x dim each) and v (n_heads x vdim) from the given columns;
 // z_bias and lower [n_heads x dim]; state [slots, n_heads, dim, vdim] float32.  norm_w null: out [T, ldo] float32 gets o;
-// else (vdim up to 128, up to 64 where dim is above 128) y [T, ldy] of proj's type gets the normed heads.  chunk, max_chunks, sums and decays as ssb_gated_linear_scan's.
+// else (vdim up to 128, up to 64 where dim is above 128) y [T, ldy] of proj's type gets the normed heads.  chunk, max_chunks, min_new, places, sums and decays as ssb_gated_linear_scan's.
 SSB_API int ssb_tied_scan(const void* proj, int ld, int dtype, int q_off, int f_off, int v_off, const float* z_bias,
                           const float* lower, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo,
                           const float* norm_w, float eps, void* y, int ldy, int n_seqs, int n_tokens, int n_heads, int dim,
-                          int vdim, int chunk, int max_chunks, float* sums, float* decays, int pdl, cudaStream_t stream) {
+                          int vdim, int chunk, int max_chunks, int min_new, int places, float* sums, float* decays, int pdl,
+                          cudaStream_t stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (dim <= 0 || dim > 256 || vdim <= 0 || n_heads <= 0 || z_bias == nullptr || lower == nullptr) return SSB_ERR_BAD_SIZE;
-    if (chunk < 0 || (chunk > 0 && (max_chunks <= 0 || sums == nullptr || decays == nullptr))) return SSB_ERR_BAD_SIZE;
+    if (chunk < 0 || (chunk > 0 && (max_chunks <= 0 || places <= 0 || sums == nullptr || decays == nullptr))) return SSB_ERR_BAD_SIZE;
     if (norm_w != nullptr ? (y == nullptr || vdim > (dim > 128 ? 64 : 128)) : out == nullptr) return SSB_ERR_BAD_SIZE;
-    TiedArgs a;
+    TiedArgs a = {};
     a.proj = proj; a.ld = ld; a.q_off = q_off; a.f_off = f_off; a.v_off = v_off; a.z_bias = z_bias; a.lower = lower;
     a.state = state; a.cu_new = cu_new; a.seq_slot = seq_slot; a.out = out; a.ldo = ldo; a.norm_w = norm_w; a.eps = eps;
     a.y = y; a.ldy = ldy; a.n_heads = n_heads; a.dim = dim; a.vdim = vdim; a.chunk = chunk; a.max_chunks = max_chunks;
-    a.sums = sums; a.decays = decays;
+    a.min_new = min_new; a.places = places; a.sums = sums; a.decays = decays;
     const bool chain = pdl != 0;
 #define SSB_TW(T)                                                                                          \
     {                                                                                                      \

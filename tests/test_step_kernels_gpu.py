@@ -1,6 +1,7 @@
 """Kernels that a step takes by its size, each against the kernel it stands in for (the same bits, where it keeps every sum)
 or against a float64 statement, at the sizes where it can go wrong: edges of tiles and chunks, remainders, one row and the most."""
 import math
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -173,6 +174,53 @@ def test_gated_scan_in_register_tiles(H, d, dv):
                                 max_new=max(lens), sums=sums if chunk else None, decays=decays if chunk else None)
         assert float((out.double() - want.view(T, -1)).norm() / want.norm()) < 2e-6, chunk
         assert float((state.double().view(-1) - end.view(-1)).norm() / end.norm()) < 2e-6, chunk
+
+
+def step_of(lens, slots):
+    """What a kernel set reads of a step of new tokens, sequence ``i`` bringing ``lens[i]`` in ``slots[i]``."""
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    return SimpleNamespace(n_seqs=len(lens), n_tokens=sum(lens), max_new=max(lens), is_decode=max(lens) == 1, seq_slot=i32(slots),
+                           cu_new=i32([sum(lens[:i]) for i in range(len(lens) + 1)]))
+
+
+@pytest.mark.parametrize("form", ["gated", "tied", "tied wide"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_deterministic_sets_scan_depends_on_no_other_sequence(form, dtype, monkeypatch):
+    """Sequences of fewer tokens than are cut, of just as many and of more, alone, beside one another, and with a scratch that
+    holds fewer chunks than the step has: outputs and states are the same bits.  The serving set's own cut, which does depend
+    on the step, stays within float32 rounding of them."""
+    o, H, d, dv = ops(), 2, 64, 160 if form == "tied wide" else 64
+    from supersonic_b200.csrc.fast_sets import FastKernels
+    lens, slots = [200, 300, 1, 256, 255, 700, 60], [3, 0, 6, 1, 5, 2, 4]
+    T, width = sum(lens), 2 * H * d + H * dv
+    rows, z0, bias = rnd(T, width, seed=1, dtype=dtype), rnd(T, H * d, seed=2), rnd(H * d, seed=3) + 1.0
+    state0, lower, gain = rnd(7, H * d * dv, seed=4), torch.rand(H * d, device=DEV) * 0.9, rnd(dv, seed=5)
+
+    def run(which, deterministic=True):
+        ks, at = FastKernels(deterministic=deterministic), [sum(lens[:i]) for i in which]
+        take = torch.cat([torch.arange(a, a + lens[i]) for a, i in zip(at, which)]).to(DEV)
+        batch, state, proj = step_of([lens[i] for i in which], [slots[i] for i in which]), state0.clone(), rows[take]
+        if form == "gated":
+            out = torch.full((len(take), H * dv), math.nan, device=DEV)
+            ks.gated_linear_scan(proj, 0, H * d, 2 * H * d, z0[take], bias, 16.0, 0.25, state, batch, out, H, d, dv)
+        else:
+            out = torch.full((len(take), H * dv), math.nan, device=DEV, dtype=dtype)
+            ks.tied_scan(proj, 0, H * d, 2 * H * d, bias, lower, state, batch, gain, 1e-5, out, H, d, dv)
+        return list(out.split([lens[i] for i in which])), state
+    together, end = run(range(len(lens)))
+    for group in ([0], [1], [5], [0, 1], [4, 3, 6], [2, 5, 0], [6, 5]):
+        outs, states = run(group)
+        for i, out in zip(group, outs):
+            assert torch.equal(out, together[i]) and torch.equal(states[slots[i]], end[slots[i]]), (group, i)
+    for places in (7, 9, 3):
+        monkeypatch.setattr(o, "SCAN_SCRATCH_BYTES", 4 * H * d * dv * places)
+        outs, states = run(range(len(lens)))
+        assert all(torch.equal(a, b) for a, b in zip(outs, together)) and torch.equal(states, end), places
+    monkeypatch.undo()
+    outs, states = run(range(len(lens)), deterministic=False)
+    tol = 2e-6 if dtype == torch.float32 or form == "gated" else 2.0 ** -8
+    for a, b in zip(outs + [states], together + [end]):
+        assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm())
 
 
 @pytest.mark.parametrize("kind", ["window", "pooled", "all", "sigmoid"])
