@@ -415,7 +415,8 @@ class FastKernels(PlainKernels):
                                        torch.float32, q_abs.device)
         ops.latent_attention_mma(q_abs, cache, batch.cu_new, batch.seq_start, batch.seq_slot, batch.slot_of_token,
                                  page_table, out, sinks, batch.max_new, n_heads, dk, kv_rank, page_shift, window,
-                                 scale, splits, partial, pdl=self.pdl)
+                                 scale, splits, partial, pdl=self.pdl,
+                                 form=ops.LATENT_PROMPT_FORM if self.deterministic and not batch.is_decode else 0)
 
     def _scan_scratch(self, n, device):
         return self._buffer("unit_scan_chunks", n, torch.float32, device)
@@ -424,6 +425,11 @@ class FastKernels(PlainKernels):
         if self.deterministic:                 # cut by the sequence's own length, whatever else is in the step
             return ops.scan_chunking(batch.n_seqs, batch.max_new, n_heads, dim, vdim)
         return super()._tied_chunking(batch, n_heads, dim, vdim)
+
+    def _in_parallel(self, batch, min_new: int) -> bool:
+        if self.deterministic:                 # every prompt step, however short its runs: the longest one decides for no other
+            return not batch.is_decode
+        return super()._in_parallel(batch, min_new)
 
     def matrix_state_step(self, proj, r_off, k_off, v_off, g_off, a_off, z, z_bias, decay_kind, decay_scale, a_bias,
                           unit_eps, kind, bonus, state, batch, norm_w, eps, gate_kind, y, n_heads, dim, vdim) -> bool:

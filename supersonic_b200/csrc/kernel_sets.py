@@ -246,11 +246,16 @@ class PlainKernels:
         return False
 
     def gated_unit_scan(self, gates, bias_r, bias_i, rate, u, y, y_bias, state, batch, out, block):
-        scratch = None
-        if u.dtype == torch.bfloat16 and batch.max_new >= ops.GATED_UNIT_SPLIT_MIN_NEW:       # a long run: chunks in parallel
+        scratch, split = None, self._in_parallel(batch, ops.GATED_UNIT_SPLIT_MIN_NEW)
+        if u.dtype == torch.bfloat16 and split:          # a long run: chunks in parallel
             scratch = self._scan_scratch(ops.gated_unit_scan_scratch(batch.n_seqs, batch.max_new, state.shape[1]), out.device)
         ops.gated_unit_scan(gates, bias_r, bias_i, rate, u, y, y_bias, state, batch.cu_new, batch.seq_slot, out, block,
-                            max_new=batch.max_new, scratch=scratch, pdl=self._chain(batch.n_tokens))
+                            max_new=batch.max_new, scratch=scratch, pdl=self._chain(batch.n_tokens), split=split)
+
+    def _in_parallel(self, batch, min_new: int) -> bool:
+        """Whether a step's runs of new tokens are cut into chunks that run in parallel, a vector recurrence's worth of work
+        each: from a longest run of ``min_new`` tokens on."""
+        return batch.max_new >= min_new
 
     # ---- along a sequence --------------------------------------------------------------
     def pair_embed(self, ids, table, pair, prev, batch, out, buckets, mul_prev, mul_cur):
@@ -364,10 +369,10 @@ class PlainKernels:
 
     def mingru_scan(self, proj, z_bias, x_bias, state, batch, out, width, out_scale=1.0):
         scratch = None
-        if batch.max_new >= ops.MINGRU_CHUNKED_MIN_NEW:      # a prompt: every 64 tokens in a block of their own
+        if self._in_parallel(batch, ops.MINGRU_CHUNKED_MIN_NEW):      # a prompt: every 64 tokens in a block of their own
             scratch = self._scan_scratch(ops.mingru_scan_scratch(batch.n_seqs, batch.max_new, width), out.device)
         ops.mingru_scan(proj, z_bias, x_bias, state, batch.cu_new, batch.seq_slot, out, width, out_scale,
-                        tiled=batch.max_new >= ops.MINGRU_TILED_MIN_NEW, pdl=self._chain(batch.n_tokens),
+                        tiled=self._in_parallel(batch, ops.MINGRU_TILED_MIN_NEW), pdl=self._chain(batch.n_tokens),
                         max_new=batch.max_new, scratch=scratch)
 
     # ---- experts ---------------------------------------------------------------------

@@ -451,6 +451,9 @@ def latent_attention_mma_ok(q: torch.Tensor, cache: torch.Tensor, out: torch.Ten
             and q.data_ptr() % 16 == 0 and cache.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0)
 
 
+LATENT_PROMPT_FORM = 2           # the form of latent_attention_mma that prompts of more than 16 (token, head) rows take
+
+
 def latent_attention_mma(q: torch.Tensor, cache: torch.Tensor, cu_new: torch.Tensor, seq_start: torch.Tensor,
                          seq_slot: torch.Tensor, slot_of_token: torch.Tensor, page_table: torch.Tensor,
                          out: torch.Tensor, sinks: Optional[torch.Tensor], max_new: int, n_heads: int, dk: int,
@@ -461,7 +464,7 @@ def latent_attention_mma(q: torch.Tensor, cache: torch.Tensor, cu_new: torch.Ten
     bfloat16.  ``n_splits`` > 1 cuts a sequence's pages into that many parts whose results a second launch
     merges through ``partial`` (float32, tokens x heads x n_splits x (dv + 2)).  ``form``: 0 lets the kernel
     choose how a block's warps are laid out (one group of 16 rows when a sequence brings no more, else two);
-    1, 2, 3 ask for 1 x 8, 2 x 4, 2 x 8 (row groups x slices)."""
+    1, 2, 3 ask for 1 x 8, 2 x 4, 2 x 8 (row groups x slices): the slices' shares of a page merge in another order."""
     if not latent_attention_mma_ok(q, cache, out, n_heads, dk, dv, page_shift):
         raise KernelError("latent_attention_mma: operands it does not take")
     _need(cu_new, "cu_new", torch.int32, 1); _need(seq_start, "seq_start", torch.int32, 1)
@@ -974,11 +977,12 @@ def gated_unit_scan_scratch(n_seqs: int, max_new: int, channels: int) -> int:
 def gated_unit_scan(gates: torch.Tensor, bias_r: torch.Tensor, bias_i: torch.Tensor, rate: torch.Tensor,
                     u: torch.Tensor, y: torch.Tensor, y_bias: Optional[torch.Tensor], state: torch.Tensor,
                     cu_new: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, block: int,
-                    max_new: int = 1, scratch: Optional[torch.Tensor] = None, pdl: bool = False) -> None:
+                    max_new: int = 1, scratch: Optional[torch.Tensor] = None, pdl: bool = False,
+                    split: Optional[bool] = None) -> None:
     """Per sequence and channel over the new tokens: r = sigmoid(g_r + bias_r), i = sigmoid(g_i + bias_i),
     a = exp(rate * r), S = a S + sqrt(1 - a^2) i u, out = S * gelu_tanh(y + y_bias).  ``gates`` [T, 2 x channels]
     float32 holds [g_r | g_i] per block of ``block`` channels; S float32 lives in ``state[slot]``.  Runs of
-    ``GATED_UNIT_SPLIT_MIN_NEW`` and more new tokens in bfloat16, given ``scratch`` (float32,
+    ``GATED_UNIT_SPLIT_MIN_NEW`` and more new tokens (or as ``split`` says) in bfloat16, given ``scratch`` (float32,
     ``gated_unit_scan_scratch`` elements), take several launches: what does not depend on the state for all tokens at
     once (written over ``gates``, and the activation of ``y`` over ``y``), then the walk over chunks of 128 tokens in
     parallel (each chunk from zero, the chunks' ends in order, each chunk from its true start)."""
@@ -993,7 +997,9 @@ def gated_unit_scan(gates: torch.Tensor, bias_r: torch.Tensor, bias_i: torch.Ten
     if gates.shape[0] != T or gates.shape[1] < 2 * C or min(u.shape[1], y.shape[1], out.shape[1]) < C or y.shape[0] != T \
             or out.shape[0] != T or cu_new.shape[0] != B + 1 or C % block or not state.is_contiguous():
         raise KernelError("gated_unit_scan: sizes")
-    if u.dtype == torch.bfloat16 and max_new >= GATED_UNIT_SPLIT_MIN_NEW and scratch is not None:
+    if split is None:
+        split = max_new >= GATED_UNIT_SPLIT_MIN_NEW
+    if u.dtype == torch.bfloat16 and split and scratch is not None:
         _need(scratch, "scratch", torch.float32)
         if scratch.numel() < gated_unit_scan_scratch(B, max_new, C):
             raise KernelError("gated_unit_scan: the scratch of the chunked walk is too small")

@@ -223,6 +223,45 @@ def test_a_deterministic_sets_scan_depends_on_no_other_sequence(form, dtype, mon
         assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm())
 
 
+@pytest.mark.parametrize("what", ["vector state", "min gru", "latent attention"])
+def test_a_deterministic_sets_short_runs_depend_on_no_other_sequence(what):
+    """Runs too short for the forms that long ones take, alone and beside long ones: the same bits."""
+    from supersonic_b200.csrc.fast_sets import FastKernels
+    from test_sotavik_kernels_gpu import latent_case
+    ks, lens, slots, C, H, dk, dv = FastKernels(deterministic=True), [30, 3, 300, 64, 2, 129], [3, 0, 6, 1, 5, 2], 128, 4, 48, 32
+    T = sum(lens)
+    gates, z_bias, x_bias, rate = rnd(T, 2 * C, seed=1), rnd(C, seed=2), rnd(C, seed=3), -torch.rand(C, device=DEV)
+    u, y, proj = (rnd(T, w, seed=w + i, dtype=torch.bfloat16) for i, w in enumerate((C, C, 3 * C)))
+    state0 = rnd(7, C, seed=7)
+
+    def run(which):
+        take = torch.cat([torch.arange(sum(lens[:i]), sum(lens[:i + 1])) for i in which]).to(DEV)
+        batch, state = step_of([lens[i] for i in which], [slots[i] for i in which]), state0.clone()
+        out = torch.full((len(take), H * dv if what == "latent attention" else C), math.nan, dtype=torch.bfloat16, device=DEV)
+        if what == "vector state":
+            ks.gated_unit_scan(gates[take], z_bias, x_bias, rate, u[take], y[take], z_bias, state, batch, out, 64)
+        elif what == "min gru":
+            ks.mingru_scan(proj[take], z_bias, x_bias, state, batch, out, C)
+        else:
+            new, past = [lens[i] for i in which], 170
+            cache, batch, store, table, q, rows = latent_case([n + past for n in new], new, H, dk, dv, seed=5)
+            for i, at in zip(which, [sum(new[:j]) for j in range(len(new))]):       # a sequence's own rows, whatever its place
+                own = rnd(lens[i] + past, dk, seed=50 + i, dtype=torch.bfloat16)
+                pages = table[batch.seq_slot[which.index(i)].long(), : -(-(lens[i] + past) // 64)].long()
+                for j, page in enumerate(pages.tolist()):
+                    piece = own[64 * j:64 * j + 64]
+                    store[page, 0, : piece.shape[0]] = piece
+                q[at:at + lens[i]] = rnd(lens[i], H * dk, seed=90 + i, dtype=torch.bfloat16)
+            ks.latent_attention(q, store, batch, table, out, H, dv, dk - dv, 6, None, dk ** -0.5, None)
+        assert bool(torch.isfinite(out.float()).all())
+        return list(out.split([lens[i] for i in which])), state
+    together, end = run(list(range(len(lens))))
+    for group in ([0], [1], [4], [3], [0, 1], [1, 4], [5, 0], [2, 4]):
+        outs, states = run(group)
+        for i, out in zip(group, outs):
+            assert torch.equal(out, together[i]) and torch.equal(states[slots[i]], end[slots[i]]), (group, i)
+
+
 @pytest.mark.parametrize("kind", ["window", "pooled", "all", "sigmoid"])
 @pytest.mark.parametrize("dim", [128, 64])
 def test_a_cluster_of_blocks_shares_a_decode_steps_pages(kind, dim):
