@@ -380,9 +380,10 @@ static bool wv_ok(const WpArgs& a, int dim, int vdim) {
     if (((a.ld | a.v_off | a.ld_first) & 3) ||
         (((uintptr_t)a.qkv | (uintptr_t)a.k_cache | (uintptr_t)a.v_cache | (uintptr_t)a.pk_cache | (uintptr_t)a.pv_cache | (uintptr_t)a.v_first) & 7))
         return false;
-    if (a.cos_t == nullptr || a.rot_dims == 0 || a.interleaved) return true;
+    if (a.cos_t == nullptr || a.rot_dims == 0) return true;
+    // whole lanes turn: in one that turns in part, an infinity beside the rotation would come out as no number
     const int e = dim / 32, half = a.rot_dims / 2, apart = half / e;
-    return half % e == 0 && (apart & (apart - 1)) == 0;
+    return a.interleaved ? a.rot_dims % e == 0 : half % e == 0 && (apart & (apart - 1)) == 0;
 }
 
 SSB_API int ssb_qkv_prepare(void* qkv, int ld, int dtype, const float* q_w, const float* k_w, int norm_mode, float eps,

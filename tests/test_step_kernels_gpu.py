@@ -333,6 +333,23 @@ def test_rows_prepared_a_warp_a_head(dim, vdim, n_q, n_kv, n_v, norm, rot, inter
         assert (got[1][3].abs().sum((1, 2, 3)) > 0).tolist() == [False, True, True, False, True, False]
 
 
+@pytest.mark.parametrize("rot", [2, 6, 64])
+def test_coordinates_beside_an_interleaved_rotation_stay_as_they_are(rot):
+    """Heads of 128 of which a few leading coordinates turn in pairs: an infinity in the others stays where it is and spreads to
+    no neighbour, in queries and in cached keys."""
+    T, dim = 3, 128
+    qkv = rnd(T, 3 * dim, seed=rot, dtype=torch.bfloat16)
+    qkv[:, [rot + 1, rot + 8, dim + rot + 1]] = math.inf
+    rows = qkv.clone()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    cos, sin = torch.cos(rnd(64, rot // 2, seed=1)), torch.sin(rnd(64, rot // 2, seed=1))
+    k, v = (torch.zeros(1, 1, 64, dim, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ops().qkv_prepare(qkv, None, None, None, 1e-5, cos, sin, rot, True, None, None, False, i32([5, 6, 7]), i32([0, 0, 0]), i32([[0]]),
+                      k, v, 1, 1, dim, dim, 6)
+    assert torch.equal(qkv[:, rot:dim], rows[:, rot:dim]) and torch.equal(k[0, 0, 5:8, rot:], rows[:, dim + rot:2 * dim])
+    assert torch.equal(v[0, 0, 5:8], rows[:, 2 * dim:]) and bool(torch.isfinite(qkv[:, :rot].float()).all())
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 8, 64), (31, 40, 128), (33, 72, 64), (129, 264, 192), (257, 1000, 128), (300, 256, 512)])
 @pytest.mark.parametrize("tile", [64, 128, 256, "pair"])
 def test_products_leave_in_whole_rows(m, n, k, tile):
