@@ -350,7 +350,8 @@ def test_coordinates_beside_an_interleaved_rotation_stay_as_they_are(rot):
     assert torch.equal(v[0, 0, 5:8], rows[:, 2 * dim:]) and bool(torch.isfinite(qkv[:, :rot].float()).all())
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 8, 64), (31, 40, 128), (33, 72, 64), (129, 264, 192), (257, 1000, 128), (300, 256, 512)])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 64), (31, 40, 128), (33, 72, 64), (129, 264, 192), (257, 1000, 128), (300, 256, 512),
+                                   (8, 96, 64), (41, 96, 128)])
 @pytest.mark.parametrize("tile", [64, 128, 256, "pair"])
 def test_products_leave_in_whole_rows(m, n, k, tile):
     """Every way out of the tcgen05 product at ragged edges: the float32 sums stored, the same added to what is there (one
