@@ -1775,7 +1775,9 @@ def target_nll(logits: torch.Tensor, targets: torch.Tensor, out: torch.Tensor) -
 
 def sample(logits: torch.Tensor, temperature: float, top_k: int, top_p: float,
            slots: Optional[torch.Tensor], rng_state: torch.Tensor, out: torch.Tensor,
-           drawn_u: Optional[torch.Tensor] = None) -> None:
+           drawn_u: Optional[torch.Tensor] = None, form: int = 0) -> None:
+    """A token per row of ``logits``, from the row's generator.  ``form``: how a top-k cut is searched, 0 by the sizes, 1 over
+    the row, 2 over its candidates (``top_k`` 1 to 64); the token is the same."""
     _need(logits, "logits", torch.float32, 2); _need(out, "out", torch.int32, 1)
     _need(rng_state, "rng_state", torch.int64, 1)
     n = logits.shape[0]
@@ -1792,7 +1794,7 @@ def sample(logits: torch.Tensor, temperature: float, top_k: int, top_p: float,
     _check(_fn("sampling", "ssb_sample")(
         _ptr(logits), c_longlong(logits.stride(0)), c_int(n), c_int(logits.shape[1]),
         c_float(temperature), c_int(int(top_k)), c_float(top_p), _ptr(slots), _ptr(rng_state), _ptr(out),
-        _ptr(drawn_u), _stream()), "sample")
+        _ptr(drawn_u), c_int(form), _stream()), "sample")
 
 
 # ---- decode kernels --------------------------------------------------------------------

@@ -805,24 +805,29 @@ sample_top_kernel(const float* __restrict__ logits, long long ld, int vocab, flo
     sc_draw(sh, turn, rank, n, n_it, lo_i, u, out + row_id, weights, largest);
 }
 
+// form 0: chosen by the sizes; 1: never from candidates; 2: from candidates (top_k 1 to 64, vocabularies up to 524,288).  The
+// token does not depend on it.
 SSB_API int ssb_sample(const float* logits, long long ld, int n_rows, int vocab, float temperature,
                        int top_k, float top_p, const int* slots, unsigned long long* rng_state, int* out,
-                       float* drawn_u, cudaStream_t stream) {
+                       float* drawn_u, int form, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
-    if (vocab <= 0 || vocab >= 0x40000000 || !(temperature > 0.f)) return SSB_ERR_BAD_SIZE;
+    if (vocab <= 0 || vocab >= 0x40000000 || !(temperature > 0.f) || form < 0 || form > 2) return SSB_ERR_BAD_SIZE;
     const int per_cta = (vocab + SC_CTAS - 1) / SC_CTAS;
     const size_t slice = (size_t)per_cta * sizeof(float);
+    if (form == 2 && (top_k <= 0 || top_k > TOP_MAX_K || n_rows > 65535 || per_cta > ST_MAX_IT * ST_TILE)) return SSB_ERR_BAD_SIZE;
     // a cluster of 8 blocks per row while a slice has at most 32 stretches (vocabularies up to 524,288)
     if (n_rows <= 65535 && per_cta <= ST_MAX_IT * ST_TILE) {
         // temperature alone: nothing to search, the row stays where it is
-        if ((top_k <= 0 || top_k >= vocab) && !(top_p < 1.0f)) {
+        if ((top_k <= 0 || top_k >= vocab) && !(top_p < 1.0f) && form != 2) {
             sample_stream_kernel<<<dim3(SC_CTAS, n_rows), SC_THREADS, 0, stream>>>(
                 logits, ld, vocab, 1.0f / temperature, slots, rng_state, out, drawn_u);
             return ssb_launch_status();
         }
-        // both cuts over 128,256 tokens, k 40, p 0.9: 64 rows 103 us held and 49 from candidates, 1 row 39 and 29.  A top-k cut
-        // alone is four counting passes over slices that are held (64 rows 61 and 43): re-reading pays from large steps on
-        if (top_k > 0 && top_k <= TOP_MAX_K && (top_p < 1.0f || (n_rows >= 16 && vocab > 65536))) {
+        // Both cuts, k 40, p 0.9, us held and from candidates: 64 rows of 128,256 tokens 98 and 46, 1 row 40 and 30; 1 and 64
+        // rows of 8,192 25 and 23, 47 and 34.  A top-k cut alone is four counting passes over slices that are held while the
+        // clusters find room for them: 64 x 50,257 30 and 33, 16 x 128,256 29 and 29, 12 x 262,144 34 and 31; at four million
+        // logits 64 x 65,536 32 and 32, 32 x 128,256 31 and 30, 16 x 262,144 62 and 34; 64 x 128,256 58 and 44.
+        if (form == 2 || (form == 0 && top_k > 0 && top_k <= TOP_MAX_K && (top_p < 1.0f || (long long)n_rows * vocab >= 4000000))) {
             sample_top_kernel<<<dim3(SC_CTAS, n_rows), SC_THREADS, 0, stream>>>(
                 logits, ld, vocab, 1.0f / temperature, top_k, top_p, slots, rng_state, out, drawn_u);
             return ssb_launch_status();

@@ -124,10 +124,12 @@ def test_latent_attention_of_prompts_ends_with_its_last_sums():
 
 
 @pytest.mark.parametrize("top_k", [1, 5, 40, 64])
-def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top_k):
-    """A top-k cut of a large step is searched over candidates, of a small one over the row in shared memory: the same
-    tokens.  Rows with ties at the cut, everything tied, one huge token, few finite ones, not-a-numbers."""
-    n, vocab = 18, 70001
+@pytest.mark.parametrize("top_p,vocab", [(1.0, 70001), (0.9, 70001), (0.6, 70001), (0.0, 70001), (0.9, 50), (1.0, 65), (0.6, 4096), (0.9, 400000)])
+def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top_k, top_p, vocab):
+    """A cut of a large step is searched over candidates, of a small one over the row: the same tokens.  Rows with ties at the
+    cut, everything tied (more candidates than are kept: both cuts over the row, its weights made again in every pass), one
+    huge token, few finite ones, not-a-numbers."""
+    n = 18
     lg = rnd(n, vocab, seed=top_k, scale=2.5)
     lg[0] = (lg[0] * 2).round() / 2
     lg[1, :] = 1.25
@@ -135,15 +137,22 @@ def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top
     lg[3, 30:] = -math.inf
     lg[4, 17] = math.nan
     lg[5] = lg[5].sort(descending=True).values
+    lg[8] = 1.25 - (torch.arange(vocab, device=DEV) % 3 == 0).float()
     lg[6, :] = -math.inf
     lg[7, 9] = math.inf
     seeds = torch.arange(1, n + 1, dtype=torch.int64, device=DEV) * 0x1E3779B97F4A7C15
-    state, out = seeds.clone(), torch.empty(n, dtype=torch.int32, device=DEV)
-    ops().sample(lg, 0.7, top_k, 1.0, None, state, out)
+    drawn = []
+    for form in (1, 2, 0):
+        state, out, u = seeds.clone(), torch.empty(n, dtype=torch.int32, device=DEV), torch.empty(n, device=DEV)
+        for turn in range(3):
+            ops().sample(lg, 0.7, top_k, top_p, None, state, out, u, form=form)
+            drawn.append(torch.cat([out, u.view(torch.int32)]))
+    for turn in range(3):
+        assert torch.equal(drawn[turn], drawn[3 + turn]) and torch.equal(drawn[turn], drawn[6 + turn])
     for lo in range(0, n, 9):
         alone, got = seeds[lo:lo + 9].clone(), torch.empty(9, dtype=torch.int32, device=DEV)
-        ops().sample(lg[lo:lo + 9].contiguous(), 0.7, top_k, 1.0, None, alone, got)
-        assert torch.equal(got, out[lo:lo + 9])
+        ops().sample(lg[lo:lo + 9].contiguous(), 0.7, top_k, top_p, None, alone, got)
+        assert torch.equal(got, drawn[0][lo:lo + 9])
 
 
 @pytest.mark.parametrize("H,d,dv", [(4, 256, 512), (3, 40, 24), (2, 128, 72)])
