@@ -59,7 +59,18 @@ class PlainKernels:
                             # dependent kernel become resident while a long kernel before it still runs, and a prompt of
                             # 2,048 tokens whose recurrences take a millisecond each ran 8.1 ms chained and 5.1 ms unchained
 
-    F32_PROMPT_MIN_NEW = 8  # new tokens of a float32 prompt from which 64 (token, head) rows of a kv head share a block
+    @staticmethod
+    def _f32_rows_share(batch, n_q: int, n_kv: int, head_dim: int) -> bool:
+        """Whether 64 (token, head) rows of a float32 prompt share a block and its fetch of a key.  A block's time is its chain of
+        keys whatever it holds, so the rows have to fill the blocks: with few, a row a block (attention_plain) finishes all of
+        them in one such chain, a shorter one.  us a row a block and shared, 32 heads over 8, at 4,000 keys: heads of 64,
+        8 x 32 rows 385 and 404, 16 x 32 435 and 382, 32 x 32 540 and 384; of 128, 16 x 32 551 and 591, 32 x 32 825 and 592.
+        Short contexts have little to share: 32 tokens of their own, 32 x 32 rows 14 and 15 (64), 17 and 23 (128), 64 x 32 18
+        and 15, 21 and 20."""
+        group = n_q // n_kv
+        blocks = min(batch.n_seqs * -(-batch.max_new * group // 64), batch.n_tokens * group // 64 + batch.n_seqs) * n_kv
+        waves = -(-blocks // (ops.sm_count() * (2 if head_dim == 64 else 1)))       # an SM holds two blocks, or one
+        return batch.n_tokens * n_q >= (8 * head_dim if batch.max_total > 128 else 2048) * waves
 
     def _chain(self, rows) -> bool:
         return bool(self.pdl) and int(rows) <= self.PDL_MAX_ROWS
@@ -148,8 +159,9 @@ class PlainKernels:
     def attention(self, q, k_cache, v_cache, batch, page_table, out, n_q, n_kv, head_dim, page_shift,
                   window: Optional[int], scale: float):
         # a float32 prompt: 64 (token, head) rows share the fetch of a key, the same sums in the same order
-        if not window and not batch.is_decode and batch.max_new >= self.F32_PROMPT_MIN_NEW \
-                and ops.attention_f32_prompt_ok(q, k_cache, v_cache, out, head_dim, batch.n_seqs):
+        if not window and not batch.is_decode \
+                and ops.attention_f32_prompt_ok(q, k_cache, v_cache, out, head_dim, batch.n_seqs) \
+                and self._f32_rows_share(batch, n_q, n_kv, head_dim):
             ops.attention_f32_prompt(q, k_cache, v_cache, batch.cu_new, batch.seq_start, batch.seq_slot, page_table, out,
                                      batch.max_new, n_q, n_kv, head_dim, page_shift, scale)
             return

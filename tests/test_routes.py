@@ -15,13 +15,15 @@ def calls(monkeypatch):
     seen = []
     for name in ("latent_attention_mma", "latent_attention_tc", "attention_plain", "attention_f32_prompt"):
         monkeypatch.setattr(ops, name, lambda *a, _n=name, **k: seen.append(_n))
+    monkeypatch.setattr(ops, "sm_count", lambda *a: 148)
     return seen
 
 
-def batch_of(n_seqs, max_new, is_decode=False):
+def batch_of(n_seqs, max_new, n_tokens=None, max_total=4000, kv_pages=32):
     none = torch.empty(0, dtype=torch.int32)
-    return SimpleNamespace(n_seqs=n_seqs, max_new=max_new, is_decode=is_decode, n_tokens=max_new, kv_pages=1, cu_new=none,
-                           seq_start=none, seq_slot=none, slot_of_token=none, pos=none)
+    return SimpleNamespace(n_seqs=n_seqs, max_new=max_new, is_decode=max_new == 1, n_tokens=n_tokens or n_seqs * max_new,
+                           max_total=max_total, kv_pages=kv_pages, cu_new=none, seq_start=none, seq_slot=none,
+                           slot_of_token=none, pos=none)
 
 
 def test_latent_attention_of_more_row_tiles_than_a_grid_counts(calls):
@@ -41,6 +43,18 @@ def test_float32_prompts_of_more_sequences_than_a_grid_counts(calls):
     """Tiles of 64 (token, head) rows have a sequence each along the grid's z side, which counts to 65,535."""
     q, out = torch.empty(8, 128), torch.empty(8, 128)
     cache = torch.empty(1, 1, 64, 64)
-    for n_seqs in (2, 65535, 65536):
+    for n_seqs in (64, 65535, 65536):
         PlainKernels().attention(q, cache, cache, batch_of(n_seqs, 8), None, out, 2, 1, 64, 6, None, 1.0)
     assert calls == ["attention_f32_prompt", "attention_f32_prompt", "attention_plain"]
+
+
+@pytest.mark.parametrize("head_dim,batch,shared", [
+    (64, batch_of(1, 15), False), (64, batch_of(1, 16), True), (128, batch_of(1, 31), False), (128, batch_of(1, 32), True),
+    (64, batch_of(1, 32, max_total=128), False), (64, batch_of(4, 16, max_total=128), True),
+    (128, batch_of(64, 8, n_tokens=71), False),                      # one short prompt among 63 single tokens
+    (64, batch_of(3, 500, n_tokens=890), True), (128, batch_of(16, 2048, n_tokens=18000), True)])
+def test_float32_prompts_share_the_fetch_of_a_key_where_their_rows_fill_the_blocks(calls, head_dim, batch, shared):
+    q, out = torch.empty(8, 32 * head_dim), torch.empty(8, 32 * head_dim)
+    cache = torch.empty(1, 8, 64, head_dim)
+    PlainKernels().attention(q, cache, cache, batch, None, out, 32, 8, head_dim, 6, None, 1.0)
+    assert calls == ["attention_f32_prompt" if shared else "attention_plain"]
