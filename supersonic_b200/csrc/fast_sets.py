@@ -22,7 +22,6 @@ STREAM_ROWS = ops.GEMV_TC_MAX_ROWS   # steps of up to this many rows take the pr
 CLUSTER_CHUNK_PAGES = 8       # the most pages a chunk holds when a sequence's chunks run as a cluster
 EXPERT_NARROW_ROWS = 24       # mean rows an expert up to which its products take tiles of 64 rows ...
 EXPERT_MIDDLE_ROWS = 64       # ... and of 128
-LATENT_TC_MIN_ROWS = 128      # (token, head) rows of the longest prompt from which latent attention runs on tcgen05
 TC_ATTENTION_MIN_NEW = 96     # prompts at least this long take the tcgen05 attention (tiles of 128 rows)
 
 
@@ -390,6 +389,18 @@ class FastKernels(PlainKernels):
                            cache, n_heads, dim, rot_dim, rot_dims, kv_rank, page_shift, write_cache,
                            getattr(position, "interleaved", False), pdl=self.pdl, q_latent=q_latent)
 
+    @staticmethod
+    def _latent_on_tcgen05(batch, n_heads: int, dk: int) -> bool:
+        """Whether a prompt step's latent attention runs on tcgen05: from 128 (token, head) rows of one sequence on, a tile of it,
+        where the sequences span enough pages (a power of two of them, which a captured step's sizes fix) or the rows are more
+        than 32 an SM, as many as mma.sync takes at once.  A tcgen05 block costs more to start and less a page.  us on mma.sync
+        and tcgen05, prompts without a past: 16 heads over rows of 576, 1 x 64 tokens 9.8 and 11.5, 1 x 128 15.4 and 13.1,
+        8 x 32 10.4 and 11.7, 8 x 64 18.6 and 12.1; 8 over 288, 1 x 64 6.6 and 10.6, 1 x 192 12.1 and 13.5, 1 x 256 15.0 and
+        15.2, 1 x 512 27 and 22, 8 x 64 6.8 and 10.7, 8 x 128 13.3 and 11.9; 4 over 96, 1 x 256 9.6 and 10.3, 1 x 512 16.4
+        and 15.6, 8 x 128 6.6 and 8.0, 8 x 192 10.0 and 9.4."""
+        return batch.max_new * n_heads >= 128 and (batch.kv_pages >= (2 if dk >= 512 else 4)
+                                                   or batch.n_tokens * n_heads > 32 * ops.sm_count())
+
     def latent_attention(self, q_abs, cache, batch, page_table, out, n_heads, kv_rank, rot_dim, page_shift,
                          window, scale, sinks):
         dk = kv_rank + rot_dim
@@ -397,7 +408,7 @@ class FastKernels(PlainKernels):
             super().latent_attention(q_abs, cache, batch, page_table, out, n_heads, kv_rank, rot_dim, page_shift,
                                      window, scale, sinks)
             return
-        if not batch.is_decode and not self.deterministic and batch.max_new * n_heads >= LATENT_TC_MIN_ROWS \
+        if not batch.is_decode and not self.deterministic and self._latent_on_tcgen05(batch, n_heads, dk) \
                 and ops.latent_attention_tc_ok(q_abs, cache, out, n_heads, dk, kv_rank, page_shift, batch.max_new):
             ops.latent_attention_tc(q_abs, cache, batch.cu_new, batch.seq_start, batch.seq_slot, page_table, out, sinks,
                                     batch.max_new, n_heads, dk, kv_rank, page_shift, window, scale)

@@ -39,6 +39,21 @@ def test_latent_attention_of_more_row_tiles_than_a_grid_counts(calls):
     assert not ops.latent_attention_tc_ok(q, cache, out, heads, rank + rot, rank, 6, 65536)
 
 
+@pytest.mark.parametrize("heads,rank,rot,batch,tc", [
+    (16, 512, 64, batch_of(1, 7, kv_pages=32), False), (16, 512, 64, batch_of(1, 8, kv_pages=2), True),
+    (16, 512, 64, batch_of(1, 64, kv_pages=1), False), (16, 512, 64, batch_of(8, 64, kv_pages=1), True),
+    (8, 256, 32, batch_of(1, 64, kv_pages=2), False), (8, 256, 32, batch_of(1, 16, kv_pages=4), True),
+    (8, 256, 32, batch_of(8, 64, kv_pages=1), False), (8, 256, 32, batch_of(8, 128, kv_pages=2), True),
+    (8, 256, 32, batch_of(700, 1, kv_pages=32), False)])
+def test_latent_attention_goes_to_tcgen05_where_pages_or_rows_pay_for_its_start(calls, heads, rank, rot, batch, tc):
+    bf16 = lambda *shape: torch.empty(shape, dtype=torch.bfloat16)  # noqa: E731
+    q, cache, out = bf16(1, heads * (rank + rot)), bf16(1, 1, 64, rank + rot), bf16(1, heads * rank)
+    for kernels in (FastKernels(), FastKernels(deterministic=True)):
+        kernels._buffer = lambda *a, **k: None
+        kernels.latent_attention(q, cache, batch, None, out, heads, rank, rot, 6, None, 1.0, None)
+    assert calls == ["latent_attention_tc" if tc else "latent_attention_mma", "latent_attention_mma"]
+
+
 def test_float32_prompts_of_more_sequences_than_a_grid_counts(calls):
     """Tiles of 64 (token, head) rows have a sequence each along the grid's z side, which counts to 65,535."""
     q, out = torch.empty(8, 128), torch.empty(8, 128)
