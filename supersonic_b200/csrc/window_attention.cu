@@ -217,7 +217,7 @@ struct WpArgs {
     const bf16* v_first; int ld_first; float v_lambda;
 };
 constexpr int WV_MAX_WARPS = 16, WV_MAX_PER_WARP = 4;     // warps a block; heads a warp
-constexpr int WV_MANY_TOKENS = 296;                       // two a streaming multiprocessor
+constexpr int WV_MANY_WARPS = 2064;                       // warps that share the step's tokens at a head a warp: see below
 
 template <int E>
 __device__ __forceinline__ void wv_load(const bf16* src, float (&x)[E]) {
@@ -414,9 +414,12 @@ SSB_API int ssb_qkv_prepare(void* qkv, int ld, int dtype, const float* q_w, cons
         a.v_first = (const bf16*)v_first; a.ld_first = v_first ? ld_first : 0; a.v_lambda = v_lambda;
         if (wv_ok(a, dim, vdim)) {
             // few tokens: a warp a head, the shortest chain; many: four heads a warp, whose loads share the latency of a block's
-            // chain slot - position - page, and several times the tokens resident (6,400 tokens, 16 heads of 128: 122 us a warp a head, 42 so, 79 in the kernel above;
-            // 32 heads of 64: 118, 69 and 79).
-            const int most = max(n_q, max(n_kv, n_v)), each = n_tokens >= WV_MANY_TOKENS ? WV_MAX_PER_WARP : 1;
+            // chain slot - position - page, and several times the tokens resident.  us at a head and at four heads a warp:
+            // 16 heads of 128 (blocks of 16 warps), 64 tokens 3.7 and 4.6, 129 4.8 and 4.7, 200 6.0 and 4.8, 296 8.0 and 5.0,
+            // 6,400 127 and 47 (the kernel above 79); 32 of 64, 129 tokens 4.7 and 4.6, 6,400 128 and 77 (79); 8 of 64 (8
+            // warps), 200 tokens 3.8 and 4.3, 256 4.3 and 4.4, 296 4.6 and 4.4, 400 5.6 and 4.4
+            const int most = max(n_q, max(n_kv, n_v));
+            const int each = (long long)n_tokens * min(WV_MAX_WARPS, most) >= WV_MANY_WARPS ? WV_MAX_PER_WARP : 1;
             const int threads = 32 * min(WV_MAX_WARPS, (most + each - 1) / each);
             auto kern = dim == 64 ? (vdim == 64 ? qkv_prepare_vec_kernel<2, 2> : qkv_prepare_vec_kernel<2, 4>)
                                   : (vdim == 64 ? qkv_prepare_vec_kernel<4, 2> : qkv_prepare_vec_kernel<4, 4>);

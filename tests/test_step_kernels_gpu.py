@@ -312,7 +312,7 @@ def test_a_cluster_of_blocks_shares_a_decode_steps_pages(kind, dim):
 
 @pytest.mark.parametrize("dim,vdim,n_q,n_kv,n_v", [(128, 128, 16, 4, 4), (64, 64, 32, 8, 8), (64, 128, 40, 20, 10), (128, 64, 3, 1, 1)])
 @pytest.mark.parametrize("norm,rot,interleaved", [("head", 64, False), ("row", 32, True), (None, 0, False), ("head", 16, False)])
-@pytest.mark.parametrize("T", [7, 300])
+@pytest.mark.parametrize("T", [7, 128, 129, 300])
 def test_rows_prepared_a_warp_a_head(dim, vdim, n_q, n_kv, n_v, norm, rot, interleaved, T):
     """Against the kernel that takes any width (which rows at an odd address still get): queries, cached keys and values, and
     the pooled rows of tokens that end a run; float32 in between, so one step of bfloat16 apart at the most."""
