@@ -518,7 +518,7 @@ class FastKernels(PlainKernels):
             decays = self._buffer("scan_decays", n_decays, torch.float32, out.device)
         ops.gated_linear_scan(proj, q_off, k_off, v_off, z, z_bias, tau, q_scale, state, batch.cu_new,
                               batch.seq_slot, out, n_heads, dim, vdim, pdl=self.pdl, max_new=batch.max_new, sums=sums,
-                              decays=decays, **cut)
+                              decays=decays, form=1 if self.deterministic else 0, **cut)
 
     def route_table(self, token_ids, table, n_experts, expert_of, pair_weight):
         ops.route_table(token_ids, table, n_experts, expert_of, pair_weight, pdl=self.pdl)

@@ -206,7 +206,7 @@ class PlainKernels:
             sums = torch.empty(n_sums, dtype=torch.float32, device=out.device)
             decays = torch.empty(n_decays, dtype=torch.float32, device=out.device)
         ops.gated_linear_scan(proj, q_off, k_off, v_off, z, z_bias, tau, q_scale, state, batch.cu_new,
-                              batch.seq_slot, out, n_heads, dim, vdim, max_new=batch.max_new, sums=sums, decays=decays, **cut)
+                              batch.seq_slot, out, n_heads, dim, vdim, max_new=batch.max_new, sums=sums, decays=decays, form=1, **cut)
 
     def head_norm_gate(self, o, weight, eps, gate, out, n_heads, vdim, gate_kind="silu"):
         ops.head_norm_gate(o, weight, eps, gate, out, n_heads, vdim, pdl=self._chain(o.shape[0]), gate_kind=gate_kind)

@@ -645,7 +645,7 @@ def gated_linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z:
                       cu_new: torch.Tensor, seq_slot: torch.Tensor, out: torch.Tensor, n_heads: int, dim: int,
                       vdim: int, pdl: bool = False, chunk: int = 0, max_new: int = 0,
                       sums: Optional[torch.Tensor] = None, decays: Optional[torch.Tensor] = None, min_new: int = 0,
-                      places: Optional[int] = None) -> None:
+                      places: Optional[int] = None, form: int = 0) -> None:
     """Per sequence and head, over the sequence's new tokens in order:
     S = diag(sigmoid(z + z_bias)^(1/tau)) S + k v^T;  out = S^T (q * q_scale), with S [dim, vdim] float32 read
     from and left in ``state[slot]``.  q, k (heads x dim) and v (heads x vdim) are columns of ``proj``; ``z`` is
@@ -655,7 +655,8 @@ def gated_linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z:
     state at its start), through the float32 scratch ``sums`` (sequences x chunks x heads x dim x vdim) and
     ``decays`` (sequences x chunks x heads x dim), chunks = ceil(``max_new`` / chunk).  Sequences of fewer than
     ``min_new`` new tokens are walked in one go all the same.  With ``places`` the scratch holds that many (sequence,
-    chunk) pairs and no more, and the step takes as many passes as that needs; the results do not depend on it."""
+    chunk) pairs and no more, and the step takes as many passes as that needs; the results do not depend on it.
+    ``form``: lanes that share a column's rows, 1: 16, 2: 32 (of more than 64 rows), 0: by the step's sizes."""
     _need(proj, "proj", None, 2); _need(z, "z", torch.float32, 2); _need(z_bias, "z_bias", torch.float32, 1)
     _need(state, "state", torch.float32, 2); _need(out, "out", torch.float32, 2)
     _need(cu_new, "cu_new", torch.int32, 1); _need(seq_slot, "seq_slot", torch.int32, 1)
@@ -672,7 +673,7 @@ def gated_linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z:
         _ptr(proj), c_int(proj.stride(0)), c_int(dtype_code(proj.dtype)), c_int(q_off), c_int(k_off), c_int(v_off),
         _ptr(z), c_int(z.stride(0)), _ptr(z_bias), c_float(tau), c_float(q_scale), _ptr(state), _ptr(cu_new),
         _ptr(seq_slot), _ptr(out), c_int(out.stride(0)), c_int(B), c_int(T), c_int(n_heads), c_int(dim), c_int(vdim),
-        c_int(chunk), c_int(max_chunks), c_int(min_new), c_int(places), _ptr(sums), _ptr(decays), c_int(1 if pdl else 0), _stream()),
+        c_int(chunk), c_int(max_chunks), c_int(min_new), c_int(places), c_int(form), _ptr(sums), _ptr(decays), c_int(1 if pdl else 0), _stream()),
         "gated_linear_scan")
 
 
@@ -708,12 +709,17 @@ def tied_scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim: 
 
 def gated_scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim: int, sms: int):
     """(chunk, floats of sums, floats of decays) for ``gated_linear_scan``: as many chunks as give the SMs two blocks each
-    (blocks own 64 value columns of a head); one walk a sequence where that is no more than two chunks."""
-    blocks = n_seqs * n_heads * (-(-vdim // 64))
+    (blocks own 64 value columns of a head), of 64 tokens or more, or three of 40 or more where an SM each is left for them;
+    one walk a sequence where that is no more than two chunks.  4 heads of 256 x 512, us in one walk and in three chunks: 100
+    tokens 51 and 52, 130 84 and 55, 190 118 and 74; four such sequences 150 tokens 97 and 171."""
+    blocks = max(n_seqs * n_heads * (-(-vdim // 64)), 1)
     per = n_heads * dim * vdim
-    n = min(2 * sms // max(blocks, 1), max_new // 64, SCAN_SCRATCH_BYTES // (4 * per * n_seqs))
+    most = SCAN_SCRATCH_BYTES // (4 * per * n_seqs)
+    n = min(2 * sms // blocks, max_new // 64, most)
     if n < 3:
-        return 0, 0, 0
+        if max_new < 120 or 3 * blocks > sms or most < 3:
+            return 0, 0, 0
+        n = 3
     chunk = -(-(-(-max_new // n)) // 8) * 8           # whole turns of eight tokens
     n = -(-max_new // chunk)
     return chunk, n_seqs * n * per, n_seqs * n * n_heads * dim

@@ -75,7 +75,7 @@ gated_linear_carry_kernel(float* __restrict__ state, float* __restrict__ sums, c
 
 static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
                       float q_scale, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo, int n_seqs,
-                      int n_heads, int dim, int vdim, int chunk, int max_chunks, int min_new, int places, float* sums,
+                      int n_heads, int dim, int vdim, int chunk, int max_chunks, int min_new, int places, int form, float* sums,
                       float* decays, bool pdl, cudaStream_t stream);
 
 // proj [T, ld] holds q, k (n_heads x dim each) and v (n_heads x vdim) from the given columns;
@@ -85,14 +85,16 @@ static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off,
 // chunk > 0: sequences of min_new new tokens or more are run in chunks of that many tokens, in parallel, the others walked in
 // one go.  max_chunks = ceil(longest run of new tokens / chunk).  ``sums`` (places x n_heads x dim x vdim floats) and ``decays``
 // (places x n_heads x dim) hold so many (sequence, chunk) pairs at a time; with fewer than n_seqs x max_chunks the step
-// takes several passes, over sequences and over runs of chunks, and every sum is the same.
+// takes several passes, over sequences and over runs of chunks, and every sum is the same.  form: lanes that share a column's
+// rows, 1: 16, 2: 32 (dim above 64), 0: by the step's sizes; the sums over the rows differ in order.
 SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off,
                                   float* z, int ldz, const float* z_bias, float tau, float q_scale,
                                   float* state, const int* cu_new, const int* seq_slot, float* out, int ldo,
                                   int n_seqs, int n_tokens, int n_heads, int dim, int vdim, int chunk, int max_chunks,
-                                  int min_new, int places, float* sums, float* decays, int pdl, cudaStream_t stream) {
+                                  int min_new, int places, int form, float* sums, float* decays, int pdl,
+                                  cudaStream_t stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
-    if (dim <= 0 || dim > SCAN_MAX_DIM || vdim <= 0 || !(tau > 0.f)) return SSB_ERR_BAD_SIZE;
+    if (dim <= 0 || dim > SCAN_MAX_DIM || vdim <= 0 || !(tau > 0.f) || form < 0 || form > 2) return SSB_ERR_BAD_SIZE;
     if (chunk < 0 || (chunk > 0 && (max_chunks <= 0 || places <= 0 || sums == nullptr || decays == nullptr))) return SSB_ERR_BAD_SIZE;
     const long long items = chunk > 0 ? (long long)n_seqs * max_chunks : n_seqs;
     if (items > 0x7fffffffll) return SSB_ERR_BAD_SIZE;
@@ -104,7 +106,7 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
     if (!rc) rc = ssb_launch_status();
     if (rc) return rc;
     return gated_walk(proj, ld, dtype, q_off, k_off, v_off, z, ldz, q_scale, state, cu_new, seq_slot, out, ldo, n_seqs,
-                      n_heads, dim, vdim, chunk, max_chunks, min_new, places, sums, decays, pdl != 0, stream);
+                      n_heads, dim, vdim, chunk, max_chunks, min_new, places, form, sums, decays, pdl != 0, stream);
 }
 
 // =======================================================================================
@@ -121,9 +123,9 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
 //   OUT = false: chunk sums, from zero, with the product of the chunk's decays;
 //   OUT = true: outputs from the state at the start (the slot's, or what the carry kernel left for the chunk).
 // GATED: the gated linear attention at the top of this file on the same tiles, S <- a S + k v with decays that a kernel before
-// this one made, o = S^T (q_scale q).  (A kernel of its own, a
-// column a thread with the sums through shared memory, took 1,011 us for 4 heads of 256 x 512 and 2,048 tokens where this
-// takes 518, 412 us for 128 x 256 where this takes 133, and 128 us for one token of 64 sequences where this takes 112.)
+// this one made, o = S^T (q_scale q).  (A kernel of its own, a column a thread with the sums through shared memory, took 1,011 us
+// for 4 heads of 256 x 512 and 2,048 tokens where this takes 518, 412 us for 128 x 256 where this takes 133, and 128 us for one
+// token of 64 sequences where this takes 112.)
 // norm_w given (one block holds all of the head's columns): the head norm is taken where the outputs meet in shared
 // memory, y = o / rms(o) * norm_w, a warp a token; else o itself goes out in float32.
 // =======================================================================================
@@ -144,10 +146,11 @@ struct TiedArgs {
     float* sums; float* decays;
 };
 
-template <typename T, int R4, int NT, bool OUT, bool GATED>
+template <typename T, int R4, int NT, bool OUT, bool GATED, int RL>      // RL: lanes that share a column's rows, 16 or 32
 __global__ void __launch_bounds__(NT)
 tied_walk_kernel(const TiedArgs a) {
-    constexpr int DIMP = 64 * R4, COLS = NT / 4;          // padded rows; columns a block owns
+    constexpr int DIMP = 64 * R4, WCOLS = 128 / RL, COLS = NT / 32 * WCOLS;  // padded rows; columns of a warp, of a block
+    constexpr int RG = DIMP / (4 * RL);                    // groups of four rows a lane
     constexpr int KI = TW_TOKENS * DIMP / NT, VI = TW_TOKENS * COLS / NT;
     extern __shared__ __align__(16) float tw_sm[];
     float* k_s = tw_sm;                                    // [2][TW_TOKENS][DIMP]
@@ -157,7 +160,7 @@ tied_walk_kernel(const TiedArgs a) {
     float* d_s = o_s + 2 * TW_TOKENS * COLS;               // GATED: [2][TW_TOKENS][DIMP]
     const int dim = a.dim, vdim = a.vdim, h = blockIdx.y, j0 = blockIdx.z * COLS;
     const int b = a.chunk > 0 ? blockIdx.x / a.max_chunks : blockIdx.x, ch = a.chunk > 0 ? blockIdx.x % a.max_chunks : 0;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane & 15, cg = lane >> 4;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane % RL, cg = lane / RL;
     ssb_pdl_launch_dependents();
     ssb_pdl_wait();
     const int slot = a.seq_slot[b];
@@ -174,14 +177,14 @@ tied_walk_kernel(const TiedArgs a) {
     const T* proj = reinterpret_cast<const T*>(a.proj);
     float* S = cut ? a.sums + (((size_t)blockIdx.x * a.n_heads + h) * dim) * vdim
                    : a.state + ((size_t)slot * a.n_heads + h) * dim * vdim;
-    const int col0 = warp * 8 + cg * 4;                    // this lane's four columns, within the block's
+    const int col0 = warp * WCOLS + cg * 4;                    // this lane's four columns, within the block's
     const bool pieces = vdim % 4 == 0 && ((uintptr_t)S & 15) == 0;       // a lane's four columns in one access
-    float s[R4][4][4];
+    float s[RG][4][4];
 #pragma unroll
-    for (int g = 0; g < R4; ++g)
+    for (int g = 0; g < RG; ++g)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const int i = (g * 16 + rg) * 4 + r, j = j0 + col0;
+            const int i = (g * RL + rg) * 4 + r, j = j0 + col0;
             float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
             if (OUT && i < dim && j < vdim) {
                 const float* src = S + (size_t)i * vdim + j;
@@ -190,9 +193,9 @@ tied_walk_kernel(const TiedArgs a) {
             }
             s[g][r][0] = x.x; s[g][r][1] = x.y; s[g][r][2] = x.z; s[g][r][3] = x.w;
         }
-    float prod[R4][4];
+    float prod[RG][4];
 #pragma unroll
-    for (int g = 0; g < R4; ++g)
+    for (int g = 0; g < RG; ++g)
 #pragma unroll
         for (int r = 0; r < 4; ++r) prod[g][r] = 1.f;
     // this thread's channels among the staged items are the same in every turn: DIMP divides NT or is divided by it
@@ -265,7 +268,7 @@ tied_walk_kernel(const TiedArgs a) {
         __syncthreads();
         if (t + TW_TOKENS < t1) fetch(t + TW_TOKENS);
         if (OUT && t > t0) finish(t - TW_TOKENS, buf ^ 1);
-        if (j0 + warp * 8 < vdim) {
+        if (j0 + warp * WCOLS < vdim) {
             const int n_tok = min(TW_TOKENS, t1 - t);
 #pragma unroll 2
             for (int tt = 0; tt < n_tok; ++tt) {
@@ -273,16 +276,16 @@ tied_walk_kernel(const TiedArgs a) {
                 const float v[4] = {v4.x, v4.y, v4.z, v4.w};
                 float o[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int g = 0; g < R4; ++g) {
-                    const float4 k4 = *reinterpret_cast<const float4*>(kb + tt * DIMP + (g * 16 + rg) * 4);
+                for (int g = 0; g < RG; ++g) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(kb + tt * DIMP + (g * RL + rg) * 4);
                     const float k[4] = {k4.x, k4.y, k4.z, k4.w};
                     float q[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {1.f, 1.f, 1.f, 1.f};
                     if (GATED) {
-                        const float4 d4 = *reinterpret_cast<const float4*>(d_s + (buf * TW_TOKENS + tt) * DIMP + (g * 16 + rg) * 4);
+                        const float4 d4 = *reinterpret_cast<const float4*>(d_s + (buf * TW_TOKENS + tt) * DIMP + (g * RL + rg) * 4);
                         d[0] = d4.x; d[1] = d4.y; d[2] = d4.z; d[3] = d4.w;
                     }
                     if (OUT) {
-                        const float4 q4 = *reinterpret_cast<const float4*>(qb + tt * DIMP + (g * 16 + rg) * 4);
+                        const float4 q4 = *reinterpret_cast<const float4*>(qb + tt * DIMP + (g * RL + rg) * 4);
                         q[0] = q4.x; q[1] = q4.y; q[2] = q4.z; q[3] = q4.w;
                     }
 #pragma unroll
@@ -296,14 +299,15 @@ tied_walk_kernel(const TiedArgs a) {
                     }
                 }
                 if (OUT) {
-                    // sums over the sixteen lanes of a column group; a lane ends with one of the four columns
-                    const bool hi8 = (lane & 8) != 0, hi4 = (lane & 4) != 0;
-                    const float p0 = (hi8 ? o[2] : o[0]) + __shfl_xor_sync(0xffffffffu, hi8 ? o[0] : o[2], 8);
-                    const float p1 = (hi8 ? o[3] : o[1]) + __shfl_xor_sync(0xffffffffu, hi8 ? o[1] : o[3], 8);
-                    float p = (hi4 ? p1 : p0) + __shfl_xor_sync(0xffffffffu, hi4 ? p0 : p1, 4);
-                    p += __shfl_xor_sync(0xffffffffu, p, 2);
-                    p += __shfl_xor_sync(0xffffffffu, p, 1);
-                    if ((lane & 3) == 0) ob[tt * COLS + col0 + (hi8 ? 2 : 0) + (hi4 ? 1 : 0)] = p;
+                    // sums over the lanes of a column group; a lane ends with one of the four columns
+                    constexpr int H2 = RL / 2, H1 = RL / 4;
+                    const bool hi2 = (lane & H2) != 0, hi1 = (lane & H1) != 0;
+                    const float p0 = (hi2 ? o[2] : o[0]) + __shfl_xor_sync(0xffffffffu, hi2 ? o[0] : o[2], H2);
+                    const float p1 = (hi2 ? o[3] : o[1]) + __shfl_xor_sync(0xffffffffu, hi2 ? o[1] : o[3], H2);
+                    float p = (hi1 ? p1 : p0) + __shfl_xor_sync(0xffffffffu, hi1 ? p0 : p1, H1);
+#pragma unroll
+                    for (int m = H1 / 2; m > 0; m >>= 1) p += __shfl_xor_sync(0xffffffffu, p, m);
+                    if ((lane & (H1 - 1)) == 0) ob[tt * COLS + col0 + (hi2 ? 2 : 0) + (hi1 ? 1 : 0)] = p;
                 }
             }
         }
@@ -315,10 +319,10 @@ tied_walk_kernel(const TiedArgs a) {
         if (cut) return;                                   // the state was carried by the carry kernel
     }
 #pragma unroll
-    for (int g = 0; g < R4; ++g)
+    for (int g = 0; g < RG; ++g)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const int i = (g * 16 + rg) * 4 + r, j = j0 + col0;
+            const int i = (g * RL + rg) * 4 + r, j = j0 + col0;
             if (i < dim && j < vdim) {
                 float* dst = S + (size_t)i * vdim + j;
                 if (pieces) {
@@ -334,16 +338,16 @@ tied_walk_kernel(const TiedArgs a) {
         }
 }
 
-template <typename T, int R4, int NT, bool GATED = false>
+template <typename T, int R4, int NT, bool GATED, int RL>
 static int launch_tied_pass(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_t stream) {
-    constexpr int DIMP = 64 * R4, COLS = NT / 4;
+    constexpr int DIMP = 64 * R4, COLS = NT / 32 * (128 / RL);
     constexpr size_t smem = (size_t)TW_TOKENS * ((GATED ? 6 : 4) * DIMP + 4 * COLS) * sizeof(float);
     const long long items = a.chunk > 0 ? (long long)n_seqs * a.max_chunks : n_seqs;
     const dim3 grid((unsigned)items, a.n_heads, (a.vdim + COLS - 1) / COLS);
     if (items > 0x7fffffffll || grid.y > 65535 || grid.z > 65535 || n_seqs > 65535) return SSB_ERR_BAD_SIZE;
     static_assert(smem <= 200 * 1024, "");
-    auto sums = tied_walk_kernel<T, R4, NT, false, GATED>;
-    auto outs = tied_walk_kernel<T, R4, NT, true, GATED>;
+    auto sums = tied_walk_kernel<T, R4, NT, false, GATED, RL>;
+    auto outs = tied_walk_kernel<T, R4, NT, true, GATED, RL>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(outs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -367,9 +371,9 @@ static int launch_tied_pass(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
 
 // All of a step: in one pass where every (sequence, chunk) pair has its place in the scratch, else sequences in groups and their
 // chunks in runs, one after another.
-template <typename T, int R4, int NT, bool GATED = false>
+template <typename T, int R4, int NT, bool GATED = false, int RL = 16>
 static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_t stream) {
-    if (a.chunk <= 0 || (long long)n_seqs * a.max_chunks <= a.places) return launch_tied_pass<T, R4, NT, GATED>(a, n_seqs, pdl, stream);
+    if (a.chunk <= 0 || (long long)n_seqs * a.max_chunks <= a.places) return launch_tied_pass<T, R4, NT, GATED, RL>(a, n_seqs, pdl, stream);
     const int group = n_seqs < a.places ? n_seqs : a.places, run = a.places / group;
     for (int b = 0; b < n_seqs; b += group)
         for (int c = 0; c < a.max_chunks; c += run) {
@@ -377,24 +381,35 @@ static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
             p.cu_new += b; p.seq_slot += b;
             p.chunk0 = c;
             p.max_chunks = a.max_chunks - c < run ? a.max_chunks - c : run;
-            const int rc = launch_tied_pass<T, R4, NT, GATED>(p, n_seqs - b < group ? n_seqs - b : group, pdl, stream);
+            const int rc = launch_tied_pass<T, R4, NT, GATED, RL>(p, n_seqs - b < group ? n_seqs - b : group, pdl, stream);
             if (rc) return rc;
         }
     return 0;
 }
 
+// Blocks of 64 columns up to which a column's rows are shared by 32 lanes instead of 16, with 32 columns a block: half the work a
+// warp and token, on twice the SMs.  us with 16 and 32 lanes (and in the kernel of a column a thread that was here before): 4
+// heads of 128 x 256, one sequence, 1 token 7.5 and 6.1 (6.2), 20 15.0 and 10.9 (12.3), 100 64 and 35 (40); 4 of 256 x 512, 1 token
+// 9.6 and 7.5 (6.1), 20 22.5 and 17.1 (15.7), 100 77 and 55 (56).  With more blocks it only adds shuffles: 8 sequences of 256 x
+// 512, 1 token 16.4 and 17.1.
+constexpr int GATED_FEW_BLOCKS = 74;
+
 static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
                            float q_scale, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo, int n_seqs,
-                           int n_heads, int dim, int vdim, int chunk, int max_chunks, int min_new, int places, float* sums,
-                           float* decays, bool pdl, cudaStream_t stream) {
+                           int n_heads, int dim, int vdim, int chunk, int max_chunks, int min_new, int places, int form,
+                           float* sums, float* decays, bool pdl, cudaStream_t stream) {
     TiedArgs a = {};
     a.proj = proj; a.ld = ld; a.q_off = q_off; a.f_off = k_off; a.v_off = v_off; a.decay = decay; a.ldz = ldz; a.q_scale = q_scale;
     a.state = state; a.cu_new = cu_new; a.seq_slot = seq_slot; a.out = out; a.ldo = ldo; a.n_heads = n_heads; a.dim = dim;
     a.vdim = vdim; a.chunk = chunk; a.max_chunks = max_chunks; a.min_new = min_new; a.places = places; a.sums = sums; a.decays = decays;
+    const long long blocks = (chunk > 0 ? (long long)n_seqs * max_chunks : n_seqs) * n_heads * ((vdim + 63) / 64);
+    const bool narrow = form == 2 || (form == 0 && blocks <= GATED_FEW_BLOCKS);
 #define SSB_GW(T) \
     return dim <= 64 ? launch_tied_walk<T, 1, 256, true>(a, n_seqs, pdl, stream) \
-         : dim <= 128 ? launch_tied_walk<T, 2, 256, true>(a, n_seqs, pdl, stream) \
-                      : launch_tied_walk<T, 4, 256, true>(a, n_seqs, pdl, stream)
+         : dim <= 128 ? (narrow ? launch_tied_walk<T, 2, 256, true, 32>(a, n_seqs, pdl, stream) \
+                                : launch_tied_walk<T, 2, 256, true>(a, n_seqs, pdl, stream)) \
+                      : (narrow ? launch_tied_walk<T, 4, 256, true, 32>(a, n_seqs, pdl, stream) \
+                                : launch_tied_walk<T, 4, 256, true>(a, n_seqs, pdl, stream))
     if (dtype == SSB_F32) SSB_GW(float);
     SSB_GW(bf16);
 #undef SSB_GW

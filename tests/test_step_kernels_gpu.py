@@ -155,7 +155,7 @@ def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top
         assert torch.equal(got, drawn[0][lo:lo + 9])
 
 
-@pytest.mark.parametrize("H,d,dv", [(4, 256, 512), (3, 40, 24), (2, 128, 72)])
+@pytest.mark.parametrize("H,d,dv", [(4, 256, 512), (3, 40, 24), (2, 128, 72), (1, 200, 30), (2, 65, 33)])
 def test_gated_scan_in_register_tiles(H, d, dv):
     """Runs long and short of whole turns of eight tokens, whole and in chunks, against the recurrence in float64; float32
     sums of d terms after hundreds of float32 state updates: 2e-6 relative."""
@@ -174,13 +174,13 @@ def test_gated_scan_in_register_tiles(H, d, dv):
             want[t] = torch.einsum("hdv,hd->hv", S, q[t]) * 0.25
         end[slot] = S
         at += n
-    for chunk in (0, 24, 64):
+    for chunk, form in ((0, 0), (24, 0), (64, 0), (0, 1), (24, 1)) + (((0, 2), (24, 2), (64, 2)) if d > 64 else ()):
         n = -(-max(lens) // chunk) if chunk else 0
         sums = torch.empty(max(B * n * H * d * dv, 1), device=DEV)
         decays = torch.empty(max(B * n * H * d, 1), device=DEV)
         state, z, out = state0.clone(), z0.clone(), torch.empty(T, H * dv, device=DEV)
         ops().gated_linear_scan(proj, 0, H * d, 2 * H * d, z, bias, 16.0, 0.25, state, cu, slots, out, H, d, dv, chunk=chunk,
-                                max_new=max(lens), sums=sums if chunk else None, decays=decays if chunk else None)
+                                max_new=max(lens), sums=sums if chunk else None, decays=decays if chunk else None, form=form)
         assert float((out.double() - want.view(T, -1)).norm() / want.norm()) < 2e-6, chunk
         assert float((state.double().view(-1) - end.view(-1)).norm() / end.norm()) < 2e-6, chunk
 
