@@ -457,26 +457,36 @@ class FastKernels(PlainKernels):
         """The most pages a sequence of this batch can span: the upper end of its bucket."""
         return 2 * batch.kv_pages - 1 if batch.kv_pages > 1 else 1
 
-    def _shares(self, batch, n_kv: int, pages: int) -> int:
-        """Blocks of a cluster that share the pages of a (sequence, kv head) in a decode step: as many as leave a block an SM
-        and a page or more a block; a sequence of fewer than four pages stays in one, the exchange costs more than it
-        saves there (a step of 8 Ronelorn sequences of two pages: 2.7 % slower shared).  Deterministic sets keep one order."""
+    def _shares(self, batch, n_kv: int, most: int, usual: Optional[int] = None, small: bool = False) -> int:
+        """Blocks of a cluster that share the pages of a (sequence, kv head) in a decode step.  ``most``: the most pages a sequence
+        spans; ``usual``: as many as it spans on average, where a mask makes that fewer; ``small``: an SM holds several of the
+        kernel's blocks.  A cluster costs its exchange (one page: 5.2 us unshared, 6.4 shared), so pairs want eight pages, more
+        blocks four, and all of them an SM each, or two thirds of the SMs where the usual sequence is shorter, or where eight
+        large blocks have to find room side by side.  us unshared and shared, window attention: pairs, 16 x 4 heads of 128, 5
+        pages 12.3 and 12.7, 10 pages 17.1 and 15.2; fours, 8 x 4 heads 17.0 and 11.9, 16 x 2 heads, 4 pages 10.9 and 9.2;
+        eights, 2 x 4 heads 16.8 and 10.9, 4 x 4 heads (16 clusters) 17.0 and 20.3, 2 x 8 heads of 64, 24 pages 26.0 and 10.5.
+        Sigmoid attention in blocks of 256 tokens, 1 and 4 pages: fours, 12 x 2 heads 5.2 and 6.5, 9.2 and 7.0, 16 x 2 heads 5.3
+        and 7.4, 9.2 and 8.0.  Deterministic sets keep one order."""
         if not batch.is_decode or self.deterministic:
             return 1
-        for c in (8, 4, 2):
-            if batch.n_seqs * n_kv * c <= ops.sm_count() and max(c, 4) <= pages:
+        usual = most if usual is None else usual
+        heads, sms = batch.n_seqs * n_kv, ops.sm_count()
+        for c, least in ((8, 8), (4, 4), (2, 8)):
+            if (usual >= least and heads * c <= (sms if c < 8 or small else 2 * sms // 3)) \
+                    or (most >= least and heads * c <= 2 * sms // 3):
                 return c
         return 1
 
     def sigmoid_attention(self, q, k_cache, v_cache, batch, page_table, bias, out, n_q, n_kv, dim, vdim, page_shift,
                           chunk, window, scale):
         if ops.sigmoid_attention_mma_ok(q, k_cache, v_cache, out, dim, vdim, page_shift):
-            pages = self._most_pages(batch)
+            most = self._most_pages(batch)
             if chunk or window:
-                pages = min(pages, -(-min(c for c in (chunk, window) if c) >> page_shift) + 1)
+                most = min(most, -(-min(c for c in (chunk, window) if c) >> page_shift) + 1)
+            usual = most if not chunk else min(most, (chunk >> page_shift) // 2 + 1)       # anywhere in its block of tokens
             ops.sigmoid_attention_mma(q, k_cache, v_cache, batch.cu_new, batch.seq_start, batch.seq_slot, page_table, bias,
                                       out, batch.max_new, n_q, n_kv, dim, vdim, page_shift, chunk, window, scale,
-                                      pdl=self._chain(batch.n_tokens), cluster=self._shares(batch, n_kv, pages))
+                                      pdl=self._chain(batch.n_tokens), cluster=self._shares(batch, n_kv, most, usual, small=True))
         else:
             super().sigmoid_attention(q, k_cache, v_cache, batch, page_table, bias, out, n_q, n_kv, dim, vdim, page_shift,
                                       chunk, window, scale)
@@ -503,7 +513,7 @@ class FastKernels(PlainKernels):
                                  batch.max_new, n_q, n_kv, dim, vdim, page_shift, window, keep_first, pool, scale, softcap,
                                  sinks, vcos, vsin, v_inter, out_scale, pdl=self._chain(batch.n_tokens), v_share=v_share,
                                  gate=gate, gate_elems=gate_elems, slopes=slopes, head_mul=head_mul,
-                                 cluster=self._shares(batch, n_kv, pages))
+                                 cluster=self._shares(batch, n_kv, pages, small=max(dim, vdim) <= 64))
 
     def gated_linear_scan(self, proj, q_off, k_off, v_off, z, z_bias, tau, q_scale, state, batch, out, n_heads,
                           dim, vdim):

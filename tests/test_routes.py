@@ -73,3 +73,13 @@ def test_float32_prompts_share_the_fetch_of_a_key_where_their_rows_fill_the_bloc
     cache = torch.empty(1, 8, 64, head_dim)
     PlainKernels().attention(q, cache, cache, batch, None, out, 32, 8, head_dim, 6, None, 1.0)
     assert calls == ["attention_f32_prompt" if shared else "attention_plain"]
+
+
+@pytest.mark.parametrize("n_seqs,n_kv,most,usual,blocks", [
+    (1, 4, 15, None, 8), (3, 4, 15, None, 8), (4, 4, 15, None, 4), (9, 4, 15, None, 4), (10, 4, 15, None, 2), (18, 4, 15, None, 2), (19, 4, 15, None, 1),
+    (1, 4, 7, None, 4), (10, 4, 7, None, 1), (1, 4, 3, None, 1), (8, 2, 5, 3, 4), (13, 2, 5, 3, 1), (2, 4, 9, 5, 8), (8, 4, 9, 5, 4)])
+def test_blocks_that_share_a_decode_steps_pages(calls, n_seqs, n_kv, most, usual, blocks):
+    assert FastKernels()._shares(batch_of(n_seqs, 1), n_kv, most, usual) == blocks
+    assert FastKernels()._shares(batch_of(2, 1), 8, 31, small=True) == 8 and FastKernels()._shares(batch_of(2, 1), 8, 31) == 4
+    assert FastKernels(deterministic=True)._shares(batch_of(n_seqs, 1), n_kv, most, usual) == 1
+    assert FastKernels()._shares(batch_of(n_seqs, 2), n_kv, most, usual) == 1
