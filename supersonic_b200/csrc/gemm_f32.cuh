@@ -430,23 +430,27 @@ static inline int gf_sms() {
     return sms;
 }
 
-// Which kernel takes a product: up to 16 rows, the one that streams the weights once for all of them.  Above, whichever is
-// done first by the time a chunk of 16 k takes it: the blocks run in waves over the SMs, and tiles that are too large leave
-// SMs idle where tiles that are too small fetch more often than they multiply.  Microseconds a chunk, measured for 1 and
-// for each further wave: 16 rows x 16 columns a block 0.13 + 0.10; tiles of 64 x 64 0.90 + 0.60, of 128 x 64 1.45 + 1.15,
-// of 128 x 128 2.24 + 2.24, with the sums in tensor memory 2.33 + 2.00.  Sides of the lines it draws (us; rows x columns, k
-// 2048): 128 x 2048 89 with 16 rows and 116 with tiles of 64; 100 x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072
-// 186 with 128 x 64, 192 with 64 x 64; 1000 x 2048 291 with 128 x 128, 299 with the sums in tensor memory, 321 with 128 x 64;
-// 1000 x 16384 2003, 1794 and 2148.
-static inline int gemm_f32_form(int n_batch, int M, int N) {
-    if (M <= 16) return M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
-    const long long sms = gf_sms();
+// Which kernel takes a product: the one that streams the weights once for up to 16 rows at a time, or one of the tiles, whichever
+// is done first by the time a chunk of 16 k takes it: the blocks run in waves over the SMs, and tiles that are too large leave
+// SMs idle where tiles that are too small fetch more often than they multiply.  Hundredths of a microsecond a chunk, measured
+// for 1 and for each further wave: up to 1, 2, 4, 8 and 16 rows x 16 columns a block 5 to 3 + 2.8, 3, 3.8, 5 and 10, whole turns
+// of 32 chunks whatever K is; tiles of 64 x 64 90 + 60, of 128 x 64 145 + 115, of 128 x 128 224 + 224, with the sums in tensor
+// memory 233 + 200, and 3 us to start and end.  Sides of the lines it draws (us; rows x columns, k 2048): 128 x 2048 89 with 16
+// rows and 116 with tiles of 64; 100 x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072 186 with 128 x 64, 192 with 64 x
+// 64; 1000 x 2048 291 with 128 x 128, 299 with the sums in tensor memory, 321 with 128 x 64; 1000 x 16384 2003, 1794 and 2148.
+// K 64: 300 x 64 5.3 with 16 rows, 6.5 with tiles of 64, 700 x 64 8.2 and 6.6; 1 x 32000 14.7 with 1 row, 13.1 with tiles, 16 x
+// 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.
+static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
+    const long long sms = gf_sms(), chunks = (K + 15) / 16, turns = (K + 511) / 512;
     const auto waves = [&](int rows, int cols) {
         return ((long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * n_batch + sms - 1) / sms;
     };
-    const int forms[5] = {16, 100, 101, 102, 103};
-    const long long cost[5] = {3 + 10 * waves(16, 16), 30 + 60 * waves(64, 64), 30 + 115 * waves(128, 64), 224 * waves(128, 128),
-                               33 + 200 * waves(128, 128)};
+    const int rows = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
+    const int first = rows < 16 ? 50 : 30, each = rows == 1 ? 28 : rows == 2 ? 30 : rows == 4 ? 38 : rows == 8 ? 50 : 100;
+    const int forms[5] = {rows, 100, 101, 102, 103};
+    const long long cost[5] = {32 * turns * (first + each * waves(rows, 16)), 3000 + 10 * chunks * (30 + 60 * waves(64, 64)),
+                               3000 + 10 * chunks * (30 + 115 * waves(128, 64)), 3000 + 10 * chunks * 224 * waves(128, 128),
+                               3000 + 10 * chunks * (33 + 200 * waves(128, 128))};
     int best = 0;
     for (int f = 1; f < 5; ++f)
         if (cost[f] < cost[best]) best = f;
@@ -458,7 +462,7 @@ static inline int gemm_f32_form(int n_batch, int M, int N) {
 static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, const float* W, int ldw, long long w_batch,
                                   float* C, int ldc, long long c_batch, int n_batch, int M, int N, int K, int accumulate,
                                   int form, cudaStream_t stream) {
-    if (form == 0) form = gemm_f32_form(n_batch, M, N);
+    if (form == 0) form = gemm_f32_form(n_batch, M, N, K);
 #define GF_CONFIGURE(kernel, smem) do { \
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)); \
         if (e != cudaSuccess) return (int)e; \

@@ -32,7 +32,8 @@ def off_by_one(t):
 # rows that every form takes (one to sixteen rows a group, tiles), around the edges of groups, tiles, turns of 512 and chunks of 16
 @pytest.mark.parametrize("m,n,k", [(1, 1, 4), (1, 9, 2052), (2, 130, 516), (3, 65, 20), (4, 8, 512), (5, 33, 1000), (8, 16, 528),
                                    (9, 200, 2048), (16, 64, 1028), (17, 100, 520), (33, 257, 300), (65, 130, 36), (129, 127, 44),
-                                   (300, 2500, 516), (257, 129, 64), (64, 3, 4), (1000, 129, 12), (1000, 16400, 36)])
+                                   (300, 2500, 516), (257, 129, 64), (64, 3, 4), (1000, 129, 12), (1000, 16400, 36),
+                                   (1, 30001, 32), (3, 9000, 1028), (7, 33000, 36), (16, 2500, 1028), (13, 8200, 516), (2, 5000, 2052)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, accumulate):
     a, w, c = rnd(m, k, seed=m), rnd(n, k, seed=n), rnd(m, n, seed=k)
