@@ -33,7 +33,7 @@ def off_by_one(t):
 @pytest.mark.parametrize("m,n,k", [(1, 1, 4), (1, 9, 2052), (2, 130, 516), (3, 65, 20), (4, 8, 512), (5, 33, 1000), (8, 16, 528),
                                    (9, 200, 2048), (16, 64, 1028), (17, 100, 520), (33, 257, 300), (65, 130, 36), (129, 127, 44),
                                    (300, 2500, 516), (257, 129, 64), (64, 3, 4), (1000, 129, 12), (1000, 16400, 36),
-                                   (1, 30001, 32), (3, 9000, 1028), (7, 33000, 36), (16, 2500, 1028), (13, 8200, 516), (2, 5000, 2052)])
+                                   (1, 30001, 32), (1, 2500, 1028), (8, 2500, 516), (3, 9000, 1028), (7, 33000, 36), (16, 2500, 1028), (13, 8200, 516), (2, 5000, 2052)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, accumulate):
     a, w, c = rnd(m, k, seed=m), rnd(n, k, seed=n), rnd(m, n, seed=k)
@@ -104,6 +104,52 @@ def test_latent_attention_of_prompts_on_tcgen05(H, dk, dv, window):
         o.check_device_errors(torch.device(DEV))
         err = float((out.double() - ref).norm() / ref.norm())
         assert err < 2.0 ** -9, (lengths, new, err)
+
+
+@pytest.mark.parametrize("H,dk,dv,window", [(16, 576, 512, None), (8, 288, 256, None), (5, 48, 32, None), (16, 576, 512, 150), (3, 96, 64, 100)])
+@pytest.mark.parametrize("sinked", [False, True])
+def test_latent_attention_moves_its_reference_with_scores_that_grow(H, dk, dv, window, sinked):
+    """Keys that grow along the sequence, at another pace for every head and token: a row's weights outgrow the maximum of its
+    first keys in several turns, in some rows of a warp and not in others, and what was summed against the old maximum is
+    scaled by a factor between zero and one.  Row by row against float64: the result's rounding to bfloat16, 2^-9 of every
+    element, and weights of 16 bits."""
+    from test_sotavik_kernels_gpu import latent_case
+    o, scale, lengths, new = ops(), dk ** -0.5, [420, 200, 64, 333], [300, 170, 64, 1]
+    cache, batch, store, table, q, rows = latent_case(lengths, new, H, dk, dv, seed=H + dk)
+    sinks = torch.linspace(-1.0, 6.0, H, device=DEV) if sinked else None
+    lean = rnd(dk, seed=3)
+    T = sum(new)
+    with_lean = torch.rand(T, H, 1, device=DEV, generator=torch.Generator(device=DEV).manual_seed(4)) * 3.0
+    q.copy_((q.view(T, H, dk).float() * 0.5 + with_lean * lean * dk ** -0.5 * 4.0).to(torch.bfloat16).view(T, H * dk))
+    moved, stayed, at = 0, 0, 0
+    out = torch.full((T, H * dv), math.nan, dtype=torch.bfloat16, device=DEV)
+    want = torch.empty(T, H, dv, dtype=torch.float64, device=DEV)
+    for b, (n, k) in enumerate(zip(lengths, new)):
+        p = torch.arange(n, device=DEV)
+        r = (rows[b].float() * 0.5 + (p[:, None] / 64.0).floor() * 0.5 * lean).to(torch.bfloat16)
+        slot = int(batch.seq_slot[b])
+        for page in range((n + 63) // 64):
+            piece = r[64 * page:64 * page + 64]
+            store[int(table[slot, page]), 0, : piece.shape[0]] = piece
+        s = torch.einsum("thd,kd->thk", q[at:at + k].double().view(k, H, dk), r.double()) * scale
+        pos = torch.arange(n - k, n, device=DEV)[:, None]
+        seen = (p[None] <= pos) & ((p[None] > pos - window) if window else (p[None] >= 0))
+        s = s.masked_fill(~seen[:, None], -math.inf)
+        w = torch.exp(s - s.amax(2, keepdim=True))
+        den = w.sum(2) + (torch.exp(sinks.double()[None] - s.amax(2)) if sinked else 0.0)
+        want[at:at + k] = torch.einsum("thk,kv->thv", w, r[:, :dv].double()) / den[:, :, None]
+        if n > 128:                                    # pages of the last tokens against the maximum of their first one
+            pages = torch.nn.functional.pad(s[-60:], (0, -n % 64), value=-math.inf).view(min(k, 60), H, -1, 64)
+            first = pages.amax(3).gather(2, torch.isfinite(pages.amax(3)).int().argmax(2, keepdim=True))
+            grown = (torch.exp(pages - first[..., None]).sum(3) > 256.0).any(2)
+            moved, stayed = moved + int(grown.sum()), stayed + int((~grown).sum())
+        at += k
+    assert moved > 20 and stayed > 20, (moved, stayed)
+    o.latent_attention_tc(q, store, batch.cu_new, batch.seq_start, batch.seq_slot, table, out, sinks, batch.max_new, H, dk, dv, 6,
+                          window, scale)
+    o.check_device_errors(torch.device(DEV))
+    err = (out.double().view(T, H, dv) - want).norm(dim=2) / want.norm(dim=2)
+    assert float(err.max()) < 2.0 ** -8, float(err.max())
 
 
 def test_latent_attention_of_prompts_ends_with_its_last_sums():
