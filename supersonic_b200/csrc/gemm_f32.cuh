@@ -31,7 +31,7 @@ __device__ __forceinline__ void gf_kahan(float& acc, float& lost, float part) {
 // of A; the chunks' sums go through shared memory, two turns deep, to further warps whose threads add them in order, one
 // result each: 32 additions of four dependent steps a turn, which nobody else waits for.  W and A come by cp.async, STAGES
 // turns deep, in one stream over all the tiles that a block of the grid walks.
-// Bound by the latency of a turn at one row (48 % of the issue slots, 42 % of the memory's time) and by the shared-memory reads
+// Bound by the latency of a turn at one row (41 % of the issue slots, 49 % of the memory's time) and by the shared-memory reads
 // of the products from 8 on; the general kernel read the weights again for every row and spent a dependent chain of 4 additions
 // per 16 products in every thread.  Weights of 16384 x 2048 (134 MB), us: 1 row 270 on the general kernel and 33 here, 8 rows
 // 270 and 54, 16 rows 270 and 91; of 2048 x 8192, 2 rows 805 and 23.  16 rows of W a block (R = 2): with 8, and a block a tile,

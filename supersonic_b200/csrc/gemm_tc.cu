@@ -106,7 +106,8 @@ __device__ __forceinline__ void tc_put32_bf16(float* stage, const float (&v)[32]
 // Sums that are added to a float32 result are added in memory, whether K is cut into parts or not: a load of what was there,
 // waited for before every store, was most of the epilogue (2,048 x 2,048 x 2,048, pairs: 35.6 us with loads and stores, 29.5 added
 // in memory row by row, 25.6 with the rows staged as above; results stored in bfloat16, 2,048 x 16,384 x 2,048: 128 and 113).
-// One addition an element either way, so a result without parts has the same bits.
+// One addition an element either way, so a result without parts has the bits of a load, an addition and a store, but for numbers
+// below 2^-126, which an addition in memory may take for zero.
 template <int BN>
 __device__ __forceinline__ void tc_epilogue(uint32_t acc, int quarter, int row, int n0, int M, int N, void* __restrict__ C,
                                             int ldc, int out_is_f32, int mode, float* stage, const TcRope& rope) {

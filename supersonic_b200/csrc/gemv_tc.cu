@@ -29,8 +29,10 @@ __host__ __device__ constexpr int gv_stages(int bnb) { return bnb <= 16 ? 6 : (b
 constexpr int GV_MAX_ROWS = 128;
 constexpr unsigned GV_ROT = 5;            // k-blocks by which neighbouring row tiles start apart (see the producer)
 // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5: epilogue; from 64 batch rows on warps 6-9 too, which take the second
-// half of the rows: a block's last step is serial to its products (a decode step of 64 sequences, 1B: 1,111 us with one group
-// of warps, 1,040 with two)
+// half of the rows: a block's last step is serial to its products.  us with one group of warps and with two: a decode step of 64
+// sequences, 1B 1,111 and 1,040; the tile of 128 rows (96 registers a thread then, 36 bytes of them spilled), products of 96 rows,
+// 1B gate/up 34.8 and 28.7, down 20.5 and 18.4, 8B gate/up 61.4 and 57.3, down 34.8 and 32.8; steps of 100 and 128 sequences, 1B
+// 1,284 and 1,151, 1,366 and 1,188, 8B 4,585 and 4,350, 4,930 and 4,630.
 __host__ __device__ constexpr int gv_groups(int bnb) { return bnb >= 64 ? 2 : 1; }
 __host__ __device__ constexpr int gv_threads(int bnb) { return 64 + 128 * gv_groups(bnb); }
 
