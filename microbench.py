@@ -6,7 +6,7 @@ so that weights come from DRAM), and reports bytes or FLOPs per second.
     python microbench.py attention_prefill --tokens 2048 --seqs 1 [--kernel tc]
     python microbench.py gemm --rows 2048 --n 28672 --k 4096 --tile 256
     python microbench.py sampling --rows 64 --vocab 128256 --temperature 0.7 --top-k 40 --top-p 0.9
-    python microbench.py latent_attention --tokens 2048 --heads 16 --k 576 --n 512
+    python microbench.py latent_attention --tokens 2048 --heads 16 --k 576 --n 512 [--kernel tc]
     python microbench.py latent_attention --tokens 1 --batch 64 --context 520 --splits 2 --heads 16 --k 576 --n 512
     python microbench.py grouped_gemm --tokens 2048 --experts 64 --top 6 --n 1408 --k 2048 --kernel swiglu
     python microbench.py gated_linear_scan --tokens 2048 --heads 4 --k 256 --n 512 --chunk 128
@@ -163,7 +163,8 @@ def attention_prefill(args):
 
 def latent_attention(args):
     """One prompt of --tokens tokens (or --batch decode rows over --context cached tokens with --splits) of
-    latent attention: --heads heads over one cached row of --k elements per token whose first --n are the values."""
+    latent attention: --heads heads over one cached row of --k elements per token whose first --n are the values;
+    prompts on tcgen05 with --kernel tc."""
     H, dk, dv = args.heads, args.k, args.n
     decode = args.tokens <= 1
     S, new, total = (args.batch, 1, args.context) if decode else (args.seqs, args.tokens, args.tokens)
@@ -179,10 +180,15 @@ def latent_attention(args):
     sinks = torch.zeros(H, device=DEV)
     splits = args.splits if decode else 1
     partial = torch.empty(S * new * H * splits * (dv + 2), device=DEV) if splits > 1 else None
-    us = _time(lambda i: ops.latent_attention_mma(q, cache, cu, start, slot, slot_tok, table, out, sinks, new, H, dk, dv, 6,
-                                                  None, dk ** -0.5, splits, partial, form=args.form), args.iters)
+    tc = args.kernel == "tc"
+    if tc:
+        us = _time(lambda i: ops.latent_attention_tc(q, cache, cu, start, slot, table, out, sinks, new, H, dk, dv, 6, None,
+                                                     dk ** -0.5), args.iters)
+    else:
+        us = _time(lambda i: ops.latent_attention_mma(q, cache, cu, start, slot, slot_tok, table, out, sinks, new, H, dk, dv, 6,
+                                                      None, dk ** -0.5, splits, partial, form=args.form), args.iters)
     keys = S * (total if decode else new * (new + 1) / 2)
-    return {"kernel": "latent_attention_mma", "seqs": S, "new": new, "context": total, "heads": H, "dk": dk, "dv": dv,
+    return {"kernel": "latent_attention_tc" if tc else "latent_attention_mma", "seqs": S, "new": new, "context": total, "heads": H, "dk": dk, "dv": dv,
             "splits": splits, "form": args.form, "us": round(us, 2), "TFLOP/s": round(2.0 * keys * H * (dk + dv) / us / 1e6, 1),
             "GB/s": round(S * total * dk * 2 / us / 1e3, 1)}
 
