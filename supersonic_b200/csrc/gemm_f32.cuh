@@ -6,6 +6,16 @@
 #pragma once
 #include "common.cuh"
 
+static inline int gf_sms() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
+        sms = n;
+    }
+    return sms;
+}
+
 constexpr int GF_CHUNK = 16;               // products of one FMA chain
 constexpr int GF_LD = GF_CHUNK + 4;        // a chunk's place in shared memory: 80 bytes, so that eight neighbouring chunks
                                            // (or rows) start in eight different groups of four banks
@@ -31,11 +41,9 @@ __device__ __forceinline__ void gf_kahan(float& acc, float& lost, float part) {
 // of A; the chunks' sums go through shared memory, two turns deep, to further warps whose threads add them in order, one
 // result each: 32 additions of four dependent steps a turn, which nobody else waits for.  W and A come by cp.async, STAGES
 // turns deep, in one stream over all the tiles that a block of the grid walks.
-// Bound by the latency of a turn at one row (41 % of the issue slots, 49 % of the memory's time) and by the shared-memory reads
-// of the products from 8 on; the general kernel read the weights again for every row and spent a dependent chain of 4 additions
-// per 16 products in every thread.  Weights of 16384 x 2048 (134 MB), us: 1 row 270 on the general kernel and 33 here, 8 rows
-// 270 and 54, 16 rows 270 and 91; of 2048 x 8192, 2 rows 805 and 23.  16 rows of W a block (R = 2): with 8, and a block a tile,
-// 1 row of 16384 x 2048 took 40 and of 128256 x 2048 246 where this takes 205.
+// Bound by the shared-memory reads of the products from 8 rows on; the general kernel read the weights again for every row and
+// spent a dependent chain of 4 additions per 16 products in every thread.  Weights of 16384 x 2048 (134 MB), us: 8 rows 270 on
+// the general kernel and 54 here, 16 rows 270 and 91.  Up to four rows take the kernel below, but where they are too long for it.
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int GF_PRODUCT_THREADS = 256;
 constexpr int GF_SKINNY_CHUNKS = 32;                                  // chunks a turn: one a lane
@@ -168,6 +176,179 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __rest
 #pragma unroll
             for (int m = 0; m < MB; ++m) sums[buf * SUMS + ((warp * R + r) * MB + m) * (CH + 1) + lane] = part[r][m];
         gf_bar_arrive(BAR_WRITTEN + buf, ALL);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Up to four rows (decode steps): a warp walks RW rows of W from end to end on its own.  32 / RW lanes a row take a chunk each,
+// hand the sums of a step to one another by shuffles and add them in k order, the step before while this one multiplies: no
+// barrier and no exchange through shared memory between the warps of a block.  W comes by cp.async into a ring of the warp's
+// own, its first turns before the dependency wait (no kernel of a step writes weights); A lies whole in shared memory.  16-byte
+// pieces are permuted within their chunk, so that the eight lanes of an access start in eight different groups of four banks.
+// Many columns are bound by the memory, few by a warp's chain: a step's fetches, 16 products, shuffles and additions (16
+// clocks a chunk), one after another, so that few columns take few rows a warp and long steps.  us on the kernel above and
+// here, 1, 2 and 4 rows: 128256 x 2048 202, 236, 301 and 153, 164, 205; 16384 x 2048 30, 34, 42 and 24, 27, 32; 3072 x 2048
+// 10.7, 12.0, 14.3 and 9.3, 10.0, 11.2; 1 and 2 rows, 2048 x 8192 18.0, 20.3 and 15.9, 16.8, 4096 x 14336 56, 64 and 38, 44.
+// Four rows of W a warp, 2 x 2048 x 8192: 22.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int GF_WALK_WARPS = 8, GF_WALK_STAGES = 4, GF_WALK_TURN = 1024;        // a turn: 1024 / RW columns of RW rows, two steps
+constexpr size_t GF_WALK_RING = sizeof(float) * GF_WALK_STAGES * GF_WALK_TURN;   // a warp's
+constexpr size_t GF_WALK_SMEM = 227 * 1024;
+static inline size_t gf_walk_rows(int mb, int K) { return sizeof(float) * (size_t)mb * (((size_t)K + 511) / 512 * 512); }
+// Whether the rows of A leave room for the rings of seven warps (4 x 2048 x 8192 with six: 31.7 us, 25.0 on the kernel above).
+static inline bool gf_walk_ok(int M, int K) {
+    return M <= 4 && gf_walk_rows(M <= 2 ? M : 4, K) + 7 * GF_WALK_RING <= GF_WALK_SMEM;
+}
+// Rows of W a warp: as many as leave six warps an SM something to do.
+static inline int gf_walk_width(int N) { return N > 24 * gf_sms() ? 4 : N > 12 * gf_sms() ? 2 : 1; }
+
+// The chunks' sums of a step, one of each of MB rows a lane, in; those of this lane's row (its chunk modulo MB) in k order out.
+template <int MB, int RW>
+__device__ __forceinline__ void gf_walk_exchange(const float (&part)[MB], float (&v)[32 / RW], int lane) {
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr int CL = 32 / RW;
+    const int n = lane % RW, c = lane / RW;
+    if constexpr (MB == 1) {
+#pragma unroll
+        for (int j = 0; j < CL; ++j) v[j] = __shfl_sync(ALL, part[0], j * RW + n);
+    } else if constexpr (MB == 2) {
+        const bool odd = c & 1;
+        const float got = __shfl_xor_sync(ALL, odd ? part[0] : part[1], RW);
+        const float t0 = odd ? got : part[0], t1 = odd ? part[1] : got;
+#pragma unroll
+        for (int p = 0; p < CL / 2; ++p) {
+            v[2 * p] = __shfl_sync(ALL, t0, (2 * p + (c & 1)) * RW + n);
+            v[2 * p + 1] = __shfl_sync(ALL, t1, (2 * p + (c & 1)) * RW + n);
+        }
+    } else {
+        const bool odd = c & 1, high = c & 2;
+        const float g0 = __shfl_xor_sync(ALL, odd ? part[0] : part[1], RW);
+        const float g1 = __shfl_xor_sync(ALL, odd ? part[2] : part[3], RW);
+        const float t0 = odd ? g0 : part[0], t1 = odd ? part[1] : g0;          // row c & 1, the pair's two chunks
+        const float u0 = odd ? g1 : part[2], u1 = odd ? part[3] : g1;          // row 2 + (c & 1)
+        const float h0 = __shfl_xor_sync(ALL, high ? t0 : u0, 2 * RW);
+        const float h1 = __shfl_xor_sync(ALL, high ? t1 : u1, 2 * RW);
+        const float w[4] = {high ? h0 : t0, high ? h1 : t1, high ? u0 : h0, high ? u1 : h1};
+#pragma unroll
+        for (int p = 0; p < CL / 4; ++p)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[4 * p + i] = __shfl_sync(ALL, w[i], (4 * p + (c & 3)) * RW + n);
+    }
+}
+
+// How a row's 16-byte pieces are permuted: a piece's place is its number xor this, of its chunk and row.
+template <int RW>
+__device__ __forceinline__ int gf_walk_key(int chunk, int row) {
+    return RW == 4 ? row : RW == 2 ? ((chunk >> 1) & 1) ^ (row << 1) : (chunk >> 1) & 3;
+}
+
+template <int MB, int RW>
+__global__ void __launch_bounds__(32 * GF_WALK_WARPS)
+gemm_f32_walk_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
+                     int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int accumulate) {
+    constexpr int CL = 32 / RW, STEP = CL * GF_CHUNK, SEG = GF_WALK_TURN / RW, ROW_LOADS = 8 / RW, STAGES = GF_WALK_STAGES;
+    static_assert(SEG == 2 * STEP && GF_WALK_TURN == 8 * 32 * 4, "two steps a turn, eight pieces a lane");
+    extern __shared__ __align__(16) float gf_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const int n = lane % RW, c = lane / RW, Kp = (K + 511) / 512 * 512;
+    float* a_s = gf_smem;                                              // [row of A][Kp], zeros from K on
+    float* ring = a_s + MB * Kp + warp * STAGES * GF_WALK_TURN;        // this warp's: [stage][row of W][SEG]
+    A += (size_t)blockIdx.z * a_batch;
+    W += (size_t)blockIdx.z * w_batch;
+    C += (size_t)blockIdx.z * c_batch;
+    const int tasks = (N + RW - 1) / RW, first = warp * (int)gridDim.x + (int)blockIdx.x, stride = warps * (int)gridDim.x;
+    const int turns = (K + SEG - 1) / SEG;
+    const int total = first < tasks ? (tasks - first + stride - 1) / stride * turns : 0;
+
+    int ahead_turn = 0, ahead_task = first, ahead_slot = 0;            // of the next load
+    auto load = [&]() {
+        const int k = ahead_turn * SEG + lane * 4, rows = N - ahead_task * RW;
+        const float* src = W + (size_t)ahead_task * RW * ldw + k;
+        float* dst = ring + ahead_slot * GF_WALK_TURN;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {                                  // what lies outside arrives as zeros
+            const int r = e / ROW_LOADS, s = e % ROW_LOADS * 32;       // row, and the row's piece lane + s
+            const bool in = r < rows && k + s * 4 < K;
+            gf_cp16(dst + r * SEG + ((s + lane) ^ gf_walk_key<RW>(lane / 4, r)) * 4, in ? src + (size_t)r * ldw + s * 4 : W, in ? 16 : 0);
+        }
+        if (++ahead_slot == STAGES) ahead_slot = 0;
+        if (++ahead_turn == turns) { ahead_turn = 0; ahead_task += stride; }
+    };
+    ssb_pdl_launch_dependents();
+#pragma unroll
+    for (int t = 0; t < STAGES - 1; ++t) {
+        if (t < total) load();
+        gf_commit();
+    }
+    ssb_pdl_wait();                                                    // A and C are the predecessor's
+    for (int p = tid; p < MB * (Kp / 4); p += blockDim.x) {
+        const int m = p / (Kp / 4), u = p % (Kp / 4);
+        const bool in = m < M && u * 4 < K;
+        gf_cp16(a_s + m * Kp + (u ^ gf_walk_key<1>(u / 4, 0)) * 4, in ? A + (size_t)m * lda + u * 4 : A, in ? 16 : 0);
+    }
+    gf_commit();
+    gf_wait<0>();
+    __syncthreads();
+
+    int w_at[4], a_at[4];                                              // this lane's chunk of a step: its pieces' places
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        w_at[q] = n * SEG + ((c * 4 + q) ^ gf_walk_key<RW>(c, n)) * 4;
+        a_at[q] = ((c * 4 + q) ^ gf_walk_key<1>(c, 0)) * 4;
+    }
+    float acc = 0.f, lost = 0.f, held[CL];                             // held: the step before's chunks of this lane's row of A
+#pragma unroll
+    for (int j = 0; j < CL; ++j) held[j] = 0.f;
+    int turn = 0, task = first, slot = 0;
+    for (int g = 0; g < total; ++g) {
+        gf_wait<STAGES - 2>();
+        __syncwarp();                                                  // the turn has landed; all lanes are done with the one before
+        if (g + STAGES - 1 < total) load();
+        gf_commit();
+        int here = 0;                                                  // chunks of the last step
+#pragma unroll
+        for (int st = 0; st < 2; ++st) {
+            const int k0 = turn * SEG + st * STEP;
+            if (k0 >= K) break;
+            here = (K - k0 + GF_CHUNK - 1) / GF_CHUNK;
+            const float* w_t = ring + slot * GF_WALK_TURN + st * STEP;
+            const float* a_t = a_s + k0;
+            float part[MB];
+#pragma unroll
+            for (int m = 0; m < MB; ++m) part[m] = 0.f;
+#pragma unroll
+            for (int q = 0; q < GF_CHUNK / 4; ++q) {
+                const float4 w = *reinterpret_cast<const float4*>(w_t + w_at[q]);
+#pragma unroll
+                for (int m = 0; m < MB; ++m) {
+                    const float4 a = *reinterpret_cast<const float4*>(a_t + m * Kp + a_at[q]);
+                    part[m] = fmaf(a.x, w.x, part[m]);
+                    part[m] = fmaf(a.y, w.y, part[m]);
+                    part[m] = fmaf(a.z, w.z, part[m]);
+                    part[m] = fmaf(a.w, w.w, part[m]);
+                }
+            }
+            // whole steps, and zeros before a row's first: adding a zero to the zeros it starts from changes nothing
+#pragma unroll
+            for (int j = 0; j < CL; ++j) gf_kahan(acc, lost, held[j]);
+            gf_walk_exchange<MB, RW>(part, held, lane);
+        }
+        if (++slot == STAGES) slot = 0;
+        if (++turn == turns) {                                         // the row's last step, which may have fewer chunks
+#pragma unroll
+            for (int j = 0; j < CL; ++j) {
+                if (j < here) gf_kahan(acc, lost, held[j]);
+                held[j] = 0.f;
+            }
+            const int col = task * RW + n;
+            if (c < MB && c < M && col < N) {
+                float* dst = C + (size_t)c * ldc + col;
+                *dst = accumulate ? *dst + acc : acc;
+            }
+            acc = lost = 0.f;
+            turn = 0;
+            task += stride;
+        }
     }
 }
 
@@ -420,48 +601,44 @@ static inline bool gemm_f32_ok(const void* A, int lda, long long a_batch, const 
     return !(((uintptr_t)A | (uintptr_t)W) & 15) && !((lda | ldw | K) & 3) && !((a_batch | w_batch) & 3);
 }
 
-static inline int gf_sms() {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
-        sms = n;
-    }
-    return sms;
-}
-
-// Which kernel takes a product: the one that streams the weights once for up to 16 rows at a time, or one of the tiles, whichever
+// Which kernel takes a product: one that streams the weights once for up to 16 rows at a time, or one of the tiles, whichever
 // is done first by the time a chunk of 16 k takes it: the blocks run in waves over the SMs, and tiles that are too large leave
 // SMs idle where tiles that are too small fetch more often than they multiply.  Hundredths of a microsecond a chunk, measured
-// for 1 and for each further wave: up to 1, 2, 4, 8 and 16 rows x 16 columns a block 5 to 3 + 2.8, 3, 3.8, 5 and 10, whole turns
-// of 32 chunks whatever K is; tiles of 64 x 64 90 + 60, of 128 x 64 145 + 115, of 128 x 128 224 + 224, with the sums in tensor
-// memory 233 + 200, and 3 us to start and end.  Sides of the lines it draws (us; rows x columns, k 2048): 128 x 2048 89 with 16
-// rows and 116 with tiles of 64; 100 x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072 186 with 128 x 64, 192 with 64 x
-// 64; 1000 x 2048 291 with 128 x 128, 299 with the sums in tensor memory, 321 with 128 x 64; 1000 x 16384 2003, 1794 and 2148.
-// K 64: 300 x 64 5.3 with 16 rows, 6.5 with tiles of 64, 700 x 64 8.2 and 6.6; 1 x 32000 14.7 with 1 row, 13.1 with tiles, 16 x
-// 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.
+// for 1 and for each further wave: up to 4, 8 and 16 rows x 16 columns a block 5 to 3 + 3.8, 5 and 10, whole turns of 32 chunks
+// whatever K is; tiles of 64 x 64 90 + 60, of 128 x 64 145 + 115, of 128 x 128 224 + 224, with the sums in tensor memory 233 +
+// 200, and 3 us to start and end.  A walking warp's turn: 4 rows of W 65, 70 and 85 (1, 2, 4 rows of A), 2 rows 80, 1 row 130,
+// and 3 us.  Sides of the lines it draws (us; rows x columns, k 2048): 128 x 2048 89 with 16 rows and 116 with tiles of 64; 100
+// x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072 186 with 128 x 64, 192 with 64 x 64; 1000 x 2048 291 with 128 x
+// 128, 299 with the sums in tensor memory, 321 with 128 x 64; 1000 x 16384 2003, 1794 and 2148.  K 64: 300 x 64 5.3 with 16
+// rows, 6.5 with tiles of 64, 700 x 64 8.2 and 6.6; 16 x 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.
 static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
     const long long sms = gf_sms(), chunks = (K + 15) / 16, turns = (K + 511) / 512;
     const auto waves = [&](int rows, int cols) {
         return ((long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * n_batch + sms - 1) / sms;
     };
-    const int rows = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
-    const int first = rows < 16 ? 50 : 30, each = rows == 1 ? 28 : rows == 2 ? 30 : rows == 4 ? 38 : rows == 8 ? 50 : 100;
-    const int forms[5] = {rows, 100, 101, 102, 103};
-    const long long cost[5] = {32 * turns * (first + each * waves(rows, 16)), 3000 + 10 * chunks * (30 + 60 * waves(64, 64)),
-                               3000 + 10 * chunks * (30 + 115 * waves(128, 64)), 3000 + 10 * chunks * 224 * waves(128, 128),
-                               3000 + 10 * chunks * (33 + 200 * waves(128, 128))};
+    const bool walk = gf_walk_ok(M, K);
+    const int rows = M <= 4 ? 4 : M <= 8 ? 8 : 16;
+    const int first = rows < 16 ? 50 : 30, each = rows == 4 ? 38 : rows == 8 ? 50 : 100;
+    const int forms[5] = {walk ? (M <= 2 ? M : 4) : M <= 4 ? 5 : rows, 100, 101, 102, 103};
+    long long cost[5] = {32 * turns * (first + each * waves(rows, 16)), 3000 + 10 * chunks * (30 + 60 * waves(64, 64)),
+                         3000 + 10 * chunks * (30 + 115 * waves(128, 64)), 3000 + 10 * chunks * 224 * waves(128, 128),
+                         3000 + 10 * chunks * (33 + 200 * waves(128, 128))};
+    if (walk) {
+        const int width = gf_walk_width(N), turn = width == 1 ? 1300 : width == 2 ? 800 : M <= 1 ? 650 : M <= 2 ? 700 : 850;
+        const long long held = sms * GF_WALK_WARPS, rounds = ((long long)((N + width - 1) / width) * n_batch + held - 1) / held;
+        cost[0] = 3000 + ((K + GF_WALK_TURN / width - 1) / (GF_WALK_TURN / width)) * rounds * turn;
+    }
     int best = 0;
     for (int f = 1; f < 5; ++f)
         if (cost[f] < cost[best]) best = f;
     return forms[best];
 }
 
-// form 0: chosen by the sizes; else one of the kernels: 1, 2, 4, 8, 16 (few rows, that many a group), 100, 101, 102, 103 (tiles
+// form 0: chosen by the sizes; else one of the kernels: 1, 2, 4 (a warp walks), 5, 8, 16 (few rows, 4, 8, 16 a group), 100, 101, 102, 103 (tiles
 // of 64 x 64, 128 x 64 and twice 128 x 128, the last with its sums in tensor memory)
 static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, const float* W, int ldw, long long w_batch,
                                   float* C, int ldc, long long c_batch, int n_batch, int M, int N, int K, int accumulate,
-                                  int form, cudaStream_t stream) {
+                                  int form, cudaStream_t stream, bool pdl = false) {
     if (form == 0) form = gemm_f32_form(n_batch, M, N, K);
 #define GF_CONFIGURE(kernel, smem) do { \
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)); \
@@ -489,10 +666,27 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         kernel<<<dim3((N + cols - 1) / cols, (M + rows - 1) / rows, n_batch), GF_TILE_THREADS, smem, stream>>>( \
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
     } while (0)
+#define GF_WALK(MB, RW) do { \
+        const size_t rows = gf_walk_rows(MB, K); \
+        auto kernel = gemm_f32_walk_kernel<MB, RW>; \
+        GF_CONFIGURE(kernel, GF_WALK_SMEM); \
+        const int tasks = (N + RW - 1) / RW, blocks = tasks < gf_sms() ? tasks : gf_sms(), room = (int)((GF_WALK_SMEM - rows) / GF_WALK_RING); \
+        int warps = (tasks + blocks - 1) / blocks; \
+        warps = warps > GF_WALK_WARPS ? GF_WALK_WARPS : warps; \
+        warps = warps > room ? room : warps; \
+        const int rc = ssb_launch(kernel, dim3((unsigned)blocks, 1, n_batch), dim3(32 * warps), rows + warps * GF_WALK_RING, \
+                                  stream, pdl, A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
+        if (rc) return rc; \
+    } while (0)
+#define GF_WALKS(MB) do { \
+        const int width = gf_walk_width(N); \
+        if (width == 4) GF_WALK(MB, 4); else if (width == 2) GF_WALK(MB, 2); else GF_WALK(MB, 1); \
+    } while (0)
     switch (form) {
-        case 1: GF_SKINNY(1, 2, 3); break;
-        case 2: GF_SKINNY(2, 2, 3); break;
-        case 4: GF_SKINNY(4, 2, 3); break;
+        case 1: GF_WALKS(1); break;
+        case 2: GF_WALKS(2); break;
+        case 4: GF_WALKS(4); break;
+        case 5: GF_SKINNY(4, 2, 3); break;
         case 8: GF_SKINNY(8, 2, 3); break;
         case 16: GF_SKINNY(16, 2, 2); break;
         case 100: GF_TILES(4, 4, 3); break;
@@ -502,6 +696,8 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         default: return SSB_ERR_BAD_SIZE;
     }
 #undef GF_SKINNY
+#undef GF_WALK
+#undef GF_WALKS
 #undef GF_TILES
 #undef GF_CONFIGURE
     return ssb_launch_status();

@@ -54,10 +54,13 @@ def as_tensor(x) -> torch.Tensor:
 class PlainKernels:
     name = "plain"
     capturable = False      # the float32 path launches every step eagerly: each launch's status is looked at
-    pdl = False             # no launch is a programmatic dependent of the one before
+    pdl = False             # whether launches of small steps are programmatic dependents of the one before
     PDL_MAX_ROWS = 128      # ... and in a set that does chain its launches, only those of small steps are: the blocks of a
                             # dependent kernel become resident while a long kernel before it still runs, and a prompt of
                             # 2,048 tokens whose recurrences take a millisecond each ran 8.1 ms chained and 5.1 ms unchained
+
+    def __init__(self, pdl: bool = False):
+        self.pdl = pdl
 
     @staticmethod
     def _f32_rows_share(batch, n_q: int, n_kv: int, head_dim: int) -> bool:
@@ -82,11 +85,12 @@ class PlainKernels:
         ops.embed_norm(ids, table, weight, eps, out, scale)
 
     def rmsnorm(self, x, weight, eps, out, rows=None):
-        ops.rmsnorm(x, weight, eps, out, rows)
+        ops.rmsnorm(x, weight, eps, out, rows, pdl=self._chain(out.shape[0]))
 
     def linear(self, x, weight, out, accumulate=False):
         """out (+)= x @ weight^T; ``x`` may be a :class:`NormedInput`."""
-        ops.gemm_nt_plain(as_tensor(x), weight, out, accumulate)
+        x = as_tensor(x)
+        ops.gemm_nt_plain(x, weight, out, accumulate, pdl=self._chain(x.shape[0]))
 
     def pack_gate_up(self, gate, up):
         """Gate and up weights as one matrix, in the layout ``gate_up_swiglu`` wants."""
@@ -148,7 +152,7 @@ class PlainKernels:
     def rope_append(self, qkv, cos, sin, batch, page_table, k_cache, v_cache, n_q, n_kv, head_dim,
                     rotary_dim, page_shift, write_cache=True, interleaved=False):
         ops.rope_append(qkv, cos, sin, batch.pos, batch.slot_of_token, page_table, k_cache, v_cache,
-                        n_q, n_kv, head_dim, rotary_dim, page_shift, write_cache, interleaved)
+                        n_q, n_kv, head_dim, rotary_dim, page_shift, write_cache, interleaved, pdl=self._chain(batch.n_tokens))
 
     def rope_attention(self, qkv, position, kv, batch, out, n_q, n_kv, head_dim, page_shift, window,
                        scale) -> bool:
@@ -166,7 +170,7 @@ class PlainKernels:
                                      batch.max_new, n_q, n_kv, head_dim, page_shift, scale)
             return
         ops.attention_plain(q, k_cache, v_cache, batch.pos, batch.slot_of_token, page_table, out,
-                            n_q, n_kv, head_dim, page_shift, window, scale)
+                            n_q, n_kv, head_dim, page_shift, window, scale, pdl=self._chain(batch.n_tokens))
 
     def swiglu(self, gate_up, out):
         ops.swiglu(gate_up, out)
@@ -460,6 +464,6 @@ def kernel_set_for(dtype: torch.dtype, prefer: Optional[str] = None, determinist
     """float32 always runs the plain set (which has no atomics on data); bfloat16 runs the fast set
     unless ``prefer='plain'``, with or without float atomics in its split projections."""
     if dtype == torch.float32 or prefer == "plain":
-        return PlainKernels()
+        return PlainKernels(pdl=dtype == torch.float32)
     from .fast_sets import FastKernels
     return FastKernels(deterministic=deterministic)

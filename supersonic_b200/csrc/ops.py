@@ -134,8 +134,9 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor
         c_int(dtype_code(out.dtype)), c_int(n), c_int(x.shape[1]), c_int(1 if pdl else 0), _stream()), "rmsnorm")
 
 
-def gemm_nt_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> None:
-    """out[m, n] (+)= sum_k a[m, k] w[n, k]; float32 accumulation in k order."""
+def gemm_nt_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, pdl: bool = False) -> None:
+    """out[m, n] (+)= sum_k a[m, k] w[n, k]; float32 accumulation in k order.  ``pdl``: ``w`` is written by no kernel of the
+    step."""
     _need(a, "a", None, 2); _need(w, "w", None, 2); _need(out, "out", None, 2)
     if a.dtype != w.dtype:
         raise KernelError(f"gemm: a is {a.dtype} but w is {w.dtype}")
@@ -146,14 +147,14 @@ def gemm_nt_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulat
     _check(_fn("plain_ops", "ssb_gemm_nt_plain")(
         _ptr(a), c_int(a.stride(0)), _ptr(w), c_int(w.stride(0)), c_int(dtype_code(a.dtype)), _ptr(out),
         c_int(out.stride(0)), c_int(dtype_code(out.dtype)), c_int(M), c_int(N), c_int(K),
-        c_int(1 if accumulate else 0), _stream()), "gemm_nt_plain")
+        c_int(1 if accumulate else 0), c_int(1 if pdl else 0), _stream()), "gemm_nt_plain")
 
 
 def rope_append(qkv: torch.Tensor, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor],
                 pos: torch.Tensor, slot: torch.Tensor, page_table: torch.Tensor,
                 k_cache: Optional[torch.Tensor], v_cache: Optional[torch.Tensor], n_q: int, n_kv: int,
                 head_dim: int, rotary_dim: int, page_shift: int, write_cache: bool = True,
-                interleaved: bool = False) -> None:
+                interleaved: bool = False, pdl: bool = False) -> None:
     """Rotate q (and k) of every token in place; write k and v into the paged cache entry.  Pairs are
     (i, i + rotary_dim/2), or with ``interleaved`` (2i, 2i + 1)."""
     _need(qkv, "qkv", None, 2); _need(pos, "pos", torch.int32, 1); _need(slot, "slot", torch.int32, 1)
@@ -180,13 +181,13 @@ def rope_append(qkv: torch.Tensor, cos: Optional[torch.Tensor], sin: Optional[to
         c_int(table_positions), _ptr(pos), _ptr(slot), _ptr(page_table), c_int(page_table.shape[1]),
         _ptr(k_cache), _ptr(v_cache), c_int(T), c_int(n_q), c_int(n_kv), c_int(head_dim),
         c_int(rotary_dim), c_int(page_shift), c_int(1 if write_cache else 0), c_int(1 if interleaved else 0),
-        _stream()), "rope_append")
+        c_int(1 if pdl else 0), _stream()), "rope_append")
 
 
 def attention_plain(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos: torch.Tensor,
                     slot: torch.Tensor, page_table: torch.Tensor, out: torch.Tensor, n_q: int, n_kv: int,
                     head_dim: int, page_shift: int, window: Optional[int], scale: float,
-                    value_dim: Optional[int] = None, sinks: Optional[torch.Tensor] = None) -> None:
+                    value_dim: Optional[int] = None, sinks: Optional[torch.Tensor] = None, pdl: bool = False) -> None:
     """Each token attends over keys [max(0, pos-window+1), pos] of its slot in the paged cache.
     ``value_dim``: width of a value and of a head's output when it differs from ``head_dim``;
     ``v_cache`` None: a token's value is the first ``value_dim`` elements of its key row.
@@ -215,7 +216,7 @@ def attention_plain(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
         _ptr(slot), _ptr(page_table), c_int(page_table.shape[1]), _ptr(out), c_int(out.stride(0)),
         c_int(T), c_int(n_q), c_int(n_kv), c_int(head_dim), c_int(page_shift),
         c_int(int(window) if window else 0), c_float(scale), c_int(v_dim), c_int(v_row), _ptr(sinks),
-        _stream()), "attention_plain")
+        c_int(1 if pdl else 0), _stream()), "attention_plain")
 
 
 def attention_f32_prompt_ok(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,

@@ -238,7 +238,7 @@ gemm_nt_plain_kernel(const TA* __restrict__ A, int lda, const TA* __restrict__ W
 // projections: a head's columns of a packed row, a head's own matrix); 1 and zeros: one product
 static int gemm_nt_plain_launch(const void* A, int lda, long long a_batch, const void* W, int ldw,
                                 long long w_batch, int in_dtype, void* C, int ldc, long long c_batch,
-                                int out_dtype, int n_batch, int M, int N, int K, int accumulate,
+                                int out_dtype, int n_batch, int M, int N, int K, int accumulate, bool pdl,
                                 cudaStream_t stream) {
     if (M <= 0 || N <= 0 || n_batch <= 0) return 0;
     if (K <= 0 || n_batch > 65535) return SSB_ERR_BAD_SIZE;
@@ -246,7 +246,7 @@ static int gemm_nt_plain_launch(const void* A, int lda, long long a_batch, const
     // float32 operands in whole 16-byte pieces: the same sums, bit for bit, from kernels made for their number of rows
     if (in_dtype == SSB_F32 && out_dtype == SSB_F32 && gemm_f32_ok(A, lda, a_batch, W, ldw, w_batch, K))
         return gemm_f32_launch((const float*)A, lda, a_batch, (const float*)W, ldw, w_batch, (float*)C, ldc, c_batch, n_batch,
-                               M, N, K, accumulate, 0, stream);
+                               M, N, K, accumulate, 0, stream, pdl);
     dim3 grid((N + 63) / 64, (M + 63) / 64, n_batch);
 #define SSB_GEMM(TA, TC, ACC) \
     gemm_nt_plain_kernel<TA, TC, ACC><<<grid, 256, 0, stream>>>( \
@@ -264,61 +264,75 @@ static int gemm_nt_plain_launch(const void* A, int lda, long long a_batch, const
     return ssb_launch_status();
 }
 
+// pdl: W is written by no kernel of the step, and the kernels of a few rows may start as dependents of the one before
 SSB_API int ssb_gemm_nt_plain(const void* A, int lda, const void* W, int ldw, int in_dtype, void* C,
-                              int ldc, int out_dtype, int M, int N, int K, int accumulate,
+                              int ldc, int out_dtype, int M, int N, int K, int accumulate, int pdl,
                               cudaStream_t stream) {
-    return gemm_nt_plain_launch(A, lda, 0, W, ldw, 0, in_dtype, C, ldc, 0, out_dtype, 1, M, N, K, accumulate, stream);
+    return gemm_nt_plain_launch(A, lda, 0, W, ldw, 0, in_dtype, C, ldc, 0, out_dtype, 1, M, N, K, accumulate, pdl != 0, stream);
 }
 
 SSB_API int ssb_gemm_nt_plain_batched(const void* A, int lda, long long a_batch, const void* W, int ldw,
                                       long long w_batch, int in_dtype, void* C, int ldc, long long c_batch,
                                       int out_dtype, int n_batch, int M, int N, int K, cudaStream_t stream) {
     return gemm_nt_plain_launch(A, lda, a_batch, W, ldw, w_batch, in_dtype, C, ldc, c_batch, out_dtype, n_batch,
-                                M, N, K, 0, stream);
+                                M, N, K, 0, false, stream);
 }
 
 // ---------------------------------------------------------------------------------------
 // rotary position encoding on q (in place) and k, then k and v into the paged cache
 // qkv row layout: [q heads | k heads | v heads], each head_dim wide
 // ---------------------------------------------------------------------------------------
+constexpr int RO_HEADS = 8;                              // heads (of q, k and v) a block: few tokens still make many blocks
+
 template <typename T>
-__global__ void rope_append_kernel(T* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
-                                   const float* __restrict__ sin_t, int table_positions,
-                                   const int* __restrict__ pos, const int* __restrict__ slot,
-                                   const int* __restrict__ page_table, int max_pages,
-                                   T* __restrict__ k_cache, T* __restrict__ v_cache, int n_q, int n_kv,
-                                   int head_dim, int rotary_dim, int page_shift, int write_cache,
-                                   int interleaved) {
-    const int t = blockIdx.x;
+__global__ void __launch_bounds__(256)
+rope_append_kernel(T* __restrict__ qkv, int ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                   int table_positions, const int* __restrict__ pos, const int* __restrict__ slot,
+                   const int* __restrict__ page_table, int max_pages, T* __restrict__ k_cache, T* __restrict__ v_cache, int n_q,
+                   int n_kv, int head_dim, int rotary_dim, int page_shift, int write_cache, int interleaved) {
+    ssb_pdl_launch_dependents();
+    ssb_pdl_wait();
+    const int t = blockIdx.x, h0 = blockIdx.y * RO_HEADS;
     const int s = slot[t];
     if (s < 0) return;                                   // padding row
     const int p = pos[t];
-    const int half = rotary_dim / 2;
+    const int half = rotary_dim / 2, rest = head_dim - rotary_dim;
     T* row = qkv + (size_t)t * ld;
     const bool have_table = (cos_t != nullptr) && p < table_positions;
     const float* c_row = have_table ? cos_t + (size_t)p * half : nullptr;
     const float* s_row = have_table ? sin_t + (size_t)p * half : nullptr;
-    const int n_rot_heads = write_cache ? n_q + n_kv : n_q;
-    // rotate q heads (and k heads): pairs (i, i + half) of the first rotary_dim elements, or
-    // (interleaved) pairs (2i, 2i + 1)
-    for (int e = threadIdx.x; e < n_rot_heads * half; e += blockDim.x) {
-        const int h = e / half, i = e % half;
+    size_t tok = 0;                                      // the token's row of kv head 0 in the cache entry
+    if (write_cache) tok = ssb_cache_row(page_table, max_pages, s, p, page_shift, n_kv, 0, 1);
+    const size_t head_rows = (size_t)1 << page_shift;
+    // rotate q heads (and k heads): pairs (i, i + half) of the first rotary_dim elements, or (interleaved) pairs
+    // (2i, 2i + 1); what a thread has rotated of a key it also appends
+    const int rot_end = min(h0 + RO_HEADS, write_cache ? n_q + n_kv : n_q);
+    for (int e = threadIdx.x; e < (rot_end - h0) * half; e += blockDim.x) {
+        const int h = h0 + e / half, i = e % half;
         T* x = row + (size_t)h * head_dim;
         const int ia = interleaved ? 2 * i : i, ib = interleaved ? 2 * i + 1 : i + half;
         const float c = have_table ? c_row[i] : 1.f, sn = have_table ? s_row[i] : 0.f;
         const float x1 = ssb_to_float(x[ia]), x2 = ssb_to_float(x[ib]);
-        x[ia] = ssb_from_float<T>(x1 * c - x2 * sn);
-        x[ib] = ssb_from_float<T>(x1 * sn + x2 * c);
+        const T y1 = ssb_from_float<T>(x1 * c - x2 * sn), y2 = ssb_from_float<T>(x1 * sn + x2 * c);
+        x[ia] = y1;
+        x[ib] = y2;
+        if (h >= n_q) {
+            T* dst = k_cache + (tok + (h - n_q) * head_rows) * head_dim;
+            dst[ia] = y1;
+            dst[ib] = y2;
+        }
     }
     if (!write_cache) return;
-    __syncthreads();
-    const T* k_src = row + (size_t)n_q * head_dim;
-    const T* v_src = k_src + (size_t)n_kv * head_dim;
-    for (int e = threadIdx.x; e < n_kv * head_dim; e += blockDim.x) {
-        const int h = e / head_dim, d = e % head_dim;
-        const size_t off = ssb_cache_row(page_table, max_pages, s, p, page_shift, n_kv, h, head_dim) + d;
-        k_cache[off] = k_src[e];
-        v_cache[off] = v_src[e];
+    // what is appended as it is: a key's elements behind the rotated ones, and values
+    const int k_first = max(h0, n_q), k_end = min(h0 + RO_HEADS, n_q + n_kv);
+    for (int e = threadIdx.x; e < (k_end - k_first) * rest; e += blockDim.x) {
+        const int h = k_first + e / rest, d = rotary_dim + e % rest;
+        k_cache[(tok + (h - n_q) * head_rows) * head_dim + d] = row[(size_t)h * head_dim + d];
+    }
+    const int v_first = max(h0, n_q + n_kv), v_end = min(h0 + RO_HEADS, n_q + 2 * n_kv);
+    for (int e = threadIdx.x; e < (v_end - v_first) * head_dim; e += blockDim.x) {
+        const int h = v_first + e / head_dim, d = e % head_dim;
+        v_cache[(tok + (h - n_q - n_kv) * head_rows) * head_dim + d] = row[(size_t)h * head_dim + d];
     }
 }
 
@@ -326,20 +340,24 @@ SSB_API int ssb_rope_append(void* qkv, int ld, int dtype, const float* cos_t, co
                             int table_positions, const int* pos, const int* slot,
                             const int* page_table, int max_pages, void* k_cache, void* v_cache,
                             int n_tokens, int n_q, int n_kv, int head_dim, int rotary_dim,
-                            int page_shift, int write_cache, int interleaved, cudaStream_t stream) {
+                            int page_shift, int write_cache, int interleaved, int pdl, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (rotary_dim % 2 || rotary_dim > head_dim || rotary_dim < 0) return SSB_ERR_BAD_SIZE;
+    const int heads = write_cache ? n_q + 2 * n_kv : n_q;
+    if (heads > RO_HEADS * 65535) return SSB_ERR_BAD_SIZE;
+    const dim3 grid(n_tokens, (heads + RO_HEADS - 1) / RO_HEADS);
+    int rc;
     if (dtype == SSB_F32)
-        rope_append_kernel<float><<<n_tokens, 256, 0, stream>>>(
-            (float*)qkv, ld, cos_t, sin_t, table_positions, pos, slot, page_table, max_pages,
-            (float*)k_cache, (float*)v_cache, n_q, n_kv, head_dim, rotary_dim, page_shift, write_cache, interleaved);
+        rc = ssb_launch(rope_append_kernel<float>, grid, dim3(256), 0, stream, pdl != 0, (float*)qkv, ld, cos_t, sin_t,
+                        table_positions, pos, slot, page_table, max_pages, (float*)k_cache, (float*)v_cache, n_q, n_kv, head_dim,
+                        rotary_dim, page_shift, write_cache, interleaved);
     else if (dtype == SSB_BF16)
-        rope_append_kernel<bf16><<<n_tokens, 256, 0, stream>>>(
-            (bf16*)qkv, ld, cos_t, sin_t, table_positions, pos, slot, page_table, max_pages,
-            (bf16*)k_cache, (bf16*)v_cache, n_q, n_kv, head_dim, rotary_dim, page_shift, write_cache, interleaved);
+        rc = ssb_launch(rope_append_kernel<bf16>, grid, dim3(256), 0, stream, pdl != 0, (bf16*)qkv, ld, cos_t, sin_t,
+                        table_positions, pos, slot, page_table, max_pages, (bf16*)k_cache, (bf16*)v_cache, n_q, n_kv, head_dim,
+                        rotary_dim, page_shift, write_cache, interleaved);
     else
         return SSB_ERR_BAD_DTYPE;
-    return ssb_launch_status();
+    return rc ? rc : ssb_launch_status();
 }
 
 // ---------------------------------------------------------------------------------------
@@ -465,11 +483,129 @@ attention_plain_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ k
     }
 }
 
+// The same sums for float32 rows of up to 128 elements in whole 16-byte pieces: a chunk's keys and values come by cp.async,
+// all of a chunk's values and the next chunk's keys while the scores and their sums are made, instead of eight values at a time
+// behind every eight additions; a key's place is looked up once.
+constexpr int AS_MAX_DIM = 128;
+static size_t attention_staged_smem(int head_dim, int v_dim) {
+    return sizeof(float) * (size_t)ATT_THREADS * (head_dim + 4 + v_dim);
+}
+
+__global__ void __launch_bounds__(ATT_THREADS)
+attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
+                        const int* __restrict__ pos, const int* __restrict__ slot, const int* __restrict__ page_table,
+                        int max_pages, float* __restrict__ out, int ldo, int n_q, int n_kv, int head_dim, int page_shift,
+                        int window, float scale, int v_dim, int v_row, const float* __restrict__ sinks) {
+    extern __shared__ __align__(16) float as_smem[];
+    __shared__ __align__(16) float q_s[AS_MAX_DIM];
+    __shared__ __align__(16) float p_s[ATT_THREADS];
+    __shared__ size_t tok_s[2][ATT_THREADS];             // a chunk's keys: their rows in the cache entry
+    __shared__ float red[ATT_THREADS / 32 + 1];
+    const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ld = head_dim + 4;
+    float* k_s = as_smem;                                // [key][head_dim + 4]
+    float* v_s = k_s + ATT_THREADS * ld;                 // [key][v_dim]
+    float* o = out + (size_t)t * ldo + (size_t)h * v_dim;
+    ssb_pdl_launch_dependents();
+    ssb_pdl_wait();
+    const int s = slot[t];
+    if (s < 0) {
+        for (int d = tid; d < v_dim; d += ATT_THREADS) o[d] = 0.f;
+        return;
+    }
+    const int p = pos[t];
+    const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
+    const int kvh = h / (n_q / n_kv);
+    const int kq = head_dim / 4, vq = v_dim / 4;
+    auto look_up = [&](int base, int buf) {
+        if (base + tid <= p) tok_s[buf][tid] = ssb_cache_row(page_table, max_pages, s, base + tid, page_shift, n_kv, kvh, 1);
+    };
+    auto fetch = [&](const float* src, int row, int quads, float* dst, int dst_ld, int base, int buf) {
+        const int n = min(ATT_THREADS, p - base + 1) * quads;
+        for (int e = tid; e < n; e += ATT_THREADS) {
+            const int r = e / quads, c = e % quads * 4;
+            gf_cp16(dst + r * dst_ld + c, src + tok_s[buf][r] * row + c, 16);
+        }
+        gf_commit();
+    };
+    look_up(lo, 0);
+    const float* qp = q + (size_t)t * ldq + (size_t)h * head_dim;
+    if (tid < head_dim) q_s[tid] = qp[tid];
+    __syncthreads();
+    fetch(k_cache, head_dim, kq, k_s, ld, lo, 0);
+    float m = -INFINITY, l = 0.f, acc = 0.f;
+    int buf = 0;
+    for (int base = lo; base <= p; base += ATT_THREADS, buf ^= 1) {
+        fetch(v_cache, v_row, vq, v_s, v_dim, base, buf);
+        look_up(base + ATT_THREADS, buf ^ 1);
+        gf_wait<1>();
+        __syncthreads();                                 // the keys have landed
+        float sc = -INFINITY;
+        if (base + tid <= p) {
+            const float* kr = k_s + tid * ld;
+            float dot = 0.f;
+#pragma unroll 8
+            for (int d = 0; d < head_dim; d += 4) {
+                const float4 k4 = *reinterpret_cast<const float4*>(kr + d);
+                const float4 q4 = *reinterpret_cast<const float4*>(q_s + d);
+                dot = fmaf(q4.x, k4.x, dot);
+                dot = fmaf(q4.y, k4.y, dot);
+                dot = fmaf(q4.z, k4.z, dot);
+                dot = fmaf(q4.w, k4.w, dot);
+            }
+            sc = dot * scale;
+        }
+        float cm = sc;
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, i));
+        if (lane == 0) red[warp] = cm;
+        __syncthreads();                                 // and everyone is done with the keys
+        if (base + ATT_THREADS <= p) fetch(k_cache, head_dim, kq, k_s, ld, base + ATT_THREADS, buf ^ 1);
+        else gf_commit();
+        const float m_new = fmaxf(m, fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3])));
+        p_s[tid] = (base + tid <= p) ? expf(sc - m_new) : 0.f;
+        __syncthreads();
+        if (warp == 0) {                                 // the tree of block_reduce_sum: i with i + 64, then i + 32, ...
+            float cs = (p_s[lane] + p_s[lane + 64]) + (p_s[lane + 32] + p_s[lane + 96]);
+#pragma unroll
+            for (int i = 16; i > 0; i >>= 1) cs += __shfl_down_sync(0xffffffffu, cs, i);
+            if (lane == 0) red[ATT_THREADS / 32] = cs;
+        }
+        gf_wait<1>();
+        __syncthreads();                                 // the values have landed, the sum is there
+        const float alpha = (m == -INFINITY) ? 0.f : expf(m - m_new);
+        l = l * alpha + red[ATT_THREADS / 32];
+        if (tid < v_dim) {
+            const int n_in = min(ATT_THREADS, p - base + 1);
+            acc *= alpha;
+            int j = 0;
+            for (; j + 8 <= n_in; j += 8) {
+                float v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = v_s[(j + i) * v_dim + tid];
+                const float4 a = *reinterpret_cast<const float4*>(p_s + j), b = *reinterpret_cast<const float4*>(p_s + j + 4);
+                acc = fmaf(a.x, v[0], acc); acc = fmaf(a.y, v[1], acc); acc = fmaf(a.z, v[2], acc); acc = fmaf(a.w, v[3], acc);
+                acc = fmaf(b.x, v[4], acc); acc = fmaf(b.y, v[5], acc); acc = fmaf(b.z, v[6], acc); acc = fmaf(b.w, v[7], acc);
+            }
+            for (; j < n_in; ++j) acc = fmaf(p_s[j], v_s[j * v_dim + tid], acc);
+        }
+        m = m_new;
+        __syncthreads();                                 // everyone is done with the values and the weights
+    }
+    float keep = 1.f;
+    if (sinks != nullptr) {
+        const float sk = sinks[h];
+        const float m_all = fmaxf(m, sk);
+        keep = (m == -INFINITY) ? 0.f : expf(m - m_all);
+        l = l * keep + expf(sk - m_all);
+    }
+    if (tid < v_dim) o[tid] = l > 0.f ? acc * keep / l : 0.f;
+}
+
 SSB_API int ssb_attention_plain(const void* q, int ldq, int dtype, const void* k_cache,
                                 const void* v_cache, const int* pos, const int* slot,
                                 const int* page_table, int max_pages, void* out, int ldo, int n_tokens,
                                 int n_q, int n_kv, int head_dim, int page_shift, int window, float scale,
-                                int v_dim, int v_row, const float* sinks, cudaStream_t stream) {
+                                int v_dim, int v_row, const float* sinks, int pdl, cudaStream_t stream) {
     // v_dim: width of a value and of a head's output; v_row: elements between the value rows of
     // consecutive tokens (values may be the first v_dim elements of the key rows: pass the key
     // store as v_cache and v_row = head_dim); sinks: one float per query head, or null
@@ -477,6 +613,17 @@ SSB_API int ssb_attention_plain(const void* q, int ldq, int dtype, const void* k
     if (head_dim > ATT_MAX_HEAD_DIM || head_dim <= 0 || n_kv <= 0 || n_q % n_kv) return SSB_ERR_BAD_SIZE;
     if (v_dim <= 0 || v_dim > ATT_MAX_HEAD_DIM || v_row < v_dim) return SSB_ERR_BAD_SIZE;
     dim3 grid(n_tokens, n_q);
+    if (dtype == SSB_F32 && head_dim <= AS_MAX_DIM && v_dim <= AS_MAX_DIM && !((head_dim | v_dim | v_row) & 3)
+        && !(((uintptr_t)k_cache | (uintptr_t)v_cache) & 15)) {
+        const size_t smem = attention_staged_smem(head_dim, v_dim);
+        const cudaError_t e = cudaFuncSetAttribute(attention_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)attention_staged_smem(AS_MAX_DIM, AS_MAX_DIM));
+        if (e != cudaSuccess) return (int)e;
+        const int rc = ssb_launch(attention_staged_kernel, grid, dim3(ATT_THREADS), smem, stream, pdl != 0, (const float*)q, ldq,
+                                  (const float*)k_cache, (const float*)v_cache, pos, slot, page_table, max_pages, (float*)out, ldo,
+                                  n_q, n_kv, head_dim, page_shift, window, scale, v_dim, v_row, sinks);
+        return rc ? rc : ssb_launch_status();
+    }
     if (dtype == SSB_F32)
         attention_plain_kernel<float><<<grid, ATT_THREADS, 0, stream>>>(
             (const float*)q, ldq, (const float*)k_cache, (const float*)v_cache, pos, slot, page_table,

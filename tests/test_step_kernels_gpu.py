@@ -33,7 +33,8 @@ def off_by_one(t):
 @pytest.mark.parametrize("m,n,k", [(1, 1, 4), (1, 9, 2052), (2, 130, 516), (3, 65, 20), (4, 8, 512), (5, 33, 1000), (8, 16, 528),
                                    (9, 200, 2048), (16, 64, 1028), (17, 100, 520), (33, 257, 300), (65, 130, 36), (129, 127, 44),
                                    (300, 2500, 516), (257, 129, 64), (64, 3, 4), (1000, 129, 12), (1000, 16400, 36),
-                                   (1, 30001, 32), (1, 2500, 1028), (8, 2500, 516), (3, 9000, 1028), (7, 33000, 36), (16, 2500, 1028), (13, 8200, 516), (2, 5000, 2052)])
+                                   (1, 30001, 32), (1, 2500, 1028), (8, 2500, 516), (3, 9000, 1028), (7, 33000, 36), (16, 2500, 1028), (13, 8200, 516), (2, 5000, 2052),
+                                   (2, 2500, 1028), (4, 2501, 516), (4, 9001, 2052), (4, 130, 8192), (2, 70, 9220), (1, 4000, 4)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, accumulate):
     a, w, c = rnd(m, k, seed=m), rnd(n, k, seed=n), rnd(m, n, seed=k)
@@ -54,6 +55,33 @@ def test_float32_head_products_are_the_general_kernels_bit_for_bit(T, H, K, N):
     ops().head_linear_plain(off_by_one(x.contiguous()), w, want)
     ops().head_linear_plain(x, w, got)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("hd,v_dim,window,with_sinks", [(64, 64, 0, False), (128, 128, 0, True), (32, 32, 200, False), (20, 12, 0, False),
+                                                        (128, 64, 129, True), (4, 4, 1, False)])
+def test_float32_attention_with_staged_keys_is_the_plain_kernels_bit_for_bit(hd, v_dim, window, with_sinks):
+    """Around whole chunks of 128 keys, rows of no slot, windows that start anywhere, values narrower than keys; pages that
+    belong to nobody are not numbers, and one row sees an infinite value."""
+    n_q, n_kv, pos, slots = 6, 2, [0, 126, 127, 128, 255, 256, 300, 5], [3, 0, 1, 2, 5, 4, 6, -1]
+    perm = torch.randperm(40, generator=torch.Generator().manual_seed(hd)).to(torch.int32)
+    table, at = torch.zeros(7, 6, dtype=torch.int32), 0
+    k, v = rnd(40, n_kv, 64, hd, seed=1), rnd(40, n_kv, 64, v_dim, seed=2)
+    for slot, p in zip(slots[:-1], pos):
+        table[slot, :p // 64 + 1] = perm[at:at + p // 64 + 1]
+        at += p // 64 + 1
+    v[int(table[1, 1]), 0, 63, 1] = math.inf
+    k[perm[at:].long()] = math.nan
+    v[perm[at:].long()] = math.nan
+    q = rnd(len(pos), n_q * hd, seed=3, scale=2.0)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    sinks = rnd(n_q, seed=4) if with_sinks else None
+    outs = []
+    for kc, vc in ((off_by_one(k), off_by_one(v)), (k, v)):
+        out = torch.full((len(pos), n_q * v_dim), 9.0, device=DEV)
+        ops().attention_plain(q, kc, vc, i32(pos), i32(slots), table.to(DEV), out, n_q, n_kv, hd, 6, window or None, hd ** -0.5,
+                              value_dim=v_dim, sinks=sinks)
+        outs.append(torch.nan_to_num(out, nan=7.0))
+    assert torch.equal(outs[0], outs[1]) and bool((outs[1][-1] == 0).all())
 
 
 @pytest.mark.parametrize("hd,n_q,n_kv", [(64, 8, 2), (128, 6, 2), (128, 3, 3), (64, 12, 1)])
