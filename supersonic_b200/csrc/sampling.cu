@@ -242,9 +242,9 @@ constexpr int ST_TILE = SC_THREADS * ST_EL;              // a stretch
 constexpr int ST_MAX_IT = 32;                            // stretches per slice: one per lane of the warp that scans them
 
 __device__ __forceinline__ unsigned sc_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void sc_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void sc_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void sc_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void sc_cluster_sync() { sc_cluster_arrive(); sc_cluster_wait(); }
 __device__ __forceinline__ unsigned sc_remote_addr(const void* local, unsigned rank) {
     unsigned addr = (unsigned)__cvta_generic_to_shared(local), remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
@@ -487,19 +487,15 @@ __device__ __forceinline__ void rx_add(unsigned (*hist)[256], bool takes_part, u
 // One byte of a cut.  Every thread has added its elements into rx.hist[buf] before.  Returns the bin b
 // with S(b) >= need > S(b + 1), S(b) being what bins b.. hold over the whole cluster, and lowers need by
 // S(b + 1).  top_fraction >= 0: need is first set to that fraction of everything counted (at least 1).
-// CLUSTER false: this block's bins alone (what every block of the cluster holds, it decides alike).
-template <bool COUNT, bool CLUSTER = true>
+template <bool COUNT>
 __device__ __forceinline__ int rx_byte(RxShared& rx, int buf, unsigned long long& need, float top_fraction) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     __syncthreads();
-    if (CLUSTER) sc_cluster_sync();                      // every block's bins are complete
+    sc_cluster_sync();                                   // every block's bins are complete
     unsigned long long g = 0, v = 0;
     if (tid < 256) {
-        if (!CLUSTER)
-            g = COUNT ? rx.hist[buf][0][tid] : (unsigned long long)rx.hist[buf][0][tid] +
-                ((unsigned long long)rx.hist[buf][1][tid] << 14) + ((unsigned long long)rx.hist[buf][2][tid] << 28);
 #pragma unroll
-        for (unsigned c = 0; CLUSTER && c < SC_CTAS; ++c) {
+        for (unsigned c = 0; c < SC_CTAS; ++c) {
             g += (unsigned long long)sc_remote_u32(&rx.hist[buf][0][tid], c);
             if (!COUNT)
                 g += ((unsigned long long)sc_remote_u32(&rx.hist[buf][1][tid], c) << 14) +
@@ -645,164 +641,355 @@ sample_cluster_kernel(const float* __restrict__ logits, long long ld, int vocab,
 }
 
 // ---- a small top-k cut: candidates instead of the row -----------------------------------------------
-// What is searched is made small first.  Every thread keeps the largest key of the elements it reads; the k-th largest of
-// a block's maxima has k elements of the row at or above it, so the largest of the eight blocks' bounds is at or below
-// the row's k-th key, and what lies at or above it is k elements and a few more.  They are collected in a second reading
-// of the slice (from L2), every block gets all of them through the cluster's shared memory, and both cuts are found in
-// the block alone; the draw looks only at the stretches that hold a candidate.  A row with more than TOP_CAP candidates
-// (many ties at the cut) takes the search over the whole row, its keys read again in every pass.
+// What is searched is made small first.  Every thread keeps the largest key of the elements it reads; a block sorts the maxima
+// of 128 groups of threads and hands eight of its first k, evenly spread, to every other block.  Where the eight blocks
+// together are known to have k elements at or above a key, the row's k-th key lies at or above it too, and what else does is a
+// few elements more: about 60 of a row for k 40.  Threads that hold one read theirs again (from L2) and send them to the first
+// block, which is alone with the rest: both cuts by counting, every candidate against all others, and the draw over the
+// shares of stretches that hold a candidate.  A row with more than TOP_CAP candidates (many ties at the cut) takes the search
+// over the whole row in all blocks, its keys read again in every pass.
 // The cuts, the weights and the order in which the draw adds them are those of sample_cluster_kernel: the same token.
+// Bound by the latencies of its phases (three meetings of the cluster and a dozen of a block), not by the row's bytes.  64
+// rows of 128,256 tokens, k 40, p 0.9: 25.5 us where radix passes over 350 candidates in every block and a draw in all of them
+// took 45; one row 20 and 30.
 constexpr int TOP_CAP = 2 * SC_THREADS;                  // candidates of a row: two a thread
-constexpr int TOP_MAX_K = 64;                            // up to here a row has about nine candidates per element kept: they fit
+constexpr int TOP_MAX_K = 64;
+constexpr int TOP_GROUPS = 128;                          // groups of threads whose maxima a block sorts
+constexpr int TOP_MARKS = 8;                             // of which it hands on this many
+constexpr int TOP_SHARES = ST_MAX_IT * SC_WARPS;         // shares (a warp's part of a stretch) of a slice
 
 struct TopShared {
-    unsigned mine[TOP_CAP];                              // this slice's candidates (keys), in any order
-    unsigned all[TOP_CAP];                               // the row's
-    unsigned char has[ST_MAX_IT * SC_WARPS];             // whether a warp's share of a stretch holds a candidate
-    unsigned bound, n;
+    unsigned long long cand[TOP_CAP];                    // candidates: weight bits (key, until the cut is known) << 32 | index
+    unsigned long long kept[TOP_CAP];                    // what the top-k cut keeps, as weights; later the draw's shares
+    float part[SC_CTAS * TOP_SHARES];                    // sums of the draw
+    unsigned used[SC_CTAS * TOP_SHARES / 32];            // shares that hold something
+    float it_before[SC_CTAS][ST_MAX_IT], it_sum[SC_CTAS][ST_MAX_IT], slice_sum[SC_CTAS];
+    unsigned maxima[TOP_GROUPS], sorted[TOP_GROUPS];
+    unsigned marks[SC_CTAS * TOP_MARKS], largest[SC_CTAS];        // every block's
+    unsigned block_max, bound, n, n_kept, n_shares, cut, w_cut;
+    int found;
+};
+// The search over the whole row and the draw's shares of weights do not meet.
+union TopScratch {
+    struct { ScShared sh; RxShared rx; } row;
+    float share[SC_WARPS][32 * ST_EL];
 };
 
-// A key that at least k elements of the slice reach: the k-th largest of the maxima of groups of threads, by one warp (its
-// low twelve bits left zero).  Groups are as large as leaves four times k of them; every thread passes its own maximum.
-__device__ __forceinline__ unsigned top_bound(unsigned best, int k, unsigned* maxima) {
-    const int tid = threadIdx.x;
-    int g = 1;
-    while (g < 16 && SC_THREADS / (2 * g) >= 4 * k) g *= 2;
-    for (int o = 1; o < g; o *= 2) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if ((tid & (g - 1)) == 0) maxima[tid / g] = best;
-    __syncthreads();
-    unsigned found = 0u;
-    if (tid < 32) {
-        const int per = SC_THREADS / g / 32;
-        unsigned v[SC_THREADS / 32];
-#pragma unroll
-        for (int i = 0; i < SC_THREADS / 32; ++i) v[i] = i < per ? maxima[i * 32 + tid] : 0u;
-        for (int bit = 31; bit >= 12; --bit) {
-            const unsigned c = found | (1u << bit);
-            int count = 0;
-#pragma unroll
-            for (int i = 0; i < SC_THREADS / 32; ++i)
-                if (i < per) count += __popc(__ballot_sync(0xffffffffu, v[i] >= c));
-            if (count >= k) found = c;
-        }
-    }
-    return found;                                        // of the first warp; the others' is zero
+__device__ __forceinline__ void sc_store_remote(void* local, unsigned rank, unsigned v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(sc_remote_addr(local, rank)), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sc_store_remote(void* local, unsigned rank, unsigned long long v) {
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(sc_remote_addr(local, rank)), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned sc_add_remote(unsigned* local, unsigned rank, unsigned v) {
+    unsigned old;
+    asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(sc_remote_addr(local, rank)), "r"(v) : "memory");
+    return old;
 }
 
-// One cut over the candidates, which every block holds: the radix selection of rx_cuts on two elements a thread.
-template <bool COUNT>
-__device__ __forceinline__ unsigned top_cut(RxShared& rx, unsigned a0, unsigned a1, bool in0, bool in1, unsigned long long q0,
-                                            unsigned long long q1, unsigned long long need, float top_fraction) {
+// Calls f(element, index) for every element of the slice that this thread reads, four at a time where they lie so.
+template <typename F>
+__device__ __forceinline__ void top_read(const float* slice, int n, F f) {
     const int tid = threadIdx.x;
-    unsigned prefix = 0u, mask = 0u;
-    int buf = 0;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int b = tid; b < (COUNT ? 1 : 3) * 256; b += SC_THREADS) rx.hist[buf][0][b] = 0u;
-        __syncthreads();
-        rx_add<COUNT>(rx.hist[buf], in0 && (a0 & mask) == prefix, (a0 >> shift) & 255u, q0);
-        rx_add<COUNT>(rx.hist[buf], in1 && (a1 & mask) == prefix, (a1 >> shift) & 255u, q1);
-        prefix |= (unsigned)rx_byte<COUNT, false>(rx, buf, need, shift == 24 ? top_fraction : -1.f) << shift;
-        mask |= 255u << shift;
-        buf ^= 1;
+    if (((uintptr_t)slice & 15) == 0) {
+        const float4* quads = reinterpret_cast<const float4*>(slice);
+        const int n4 = n / 4;
+        int i = tid;
+        for (; i + 3 * SC_THREADS < n4; i += 4 * SC_THREADS) {
+            float4 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = quads[i + j * SC_THREADS];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int at = 4 * (i + j * SC_THREADS);
+                f(x[j].x, at); f(x[j].y, at + 1); f(x[j].z, at + 2); f(x[j].w, at + 3);
+            }
+        }
+        for (; i < n4; i += SC_THREADS) {
+            const float4 x = quads[i];
+            f(x.x, 4 * i); f(x.y, 4 * i + 1); f(x.z, 4 * i + 2); f(x.w, 4 * i + 3);
+        }
+        if (4 * n4 + tid < n) f(slice[4 * n4 + tid], 4 * n4 + tid);
+    } else {
+#pragma unroll 8
+        for (int i = tid; i < n; i += SC_THREADS) f(slice[i], i);
     }
-    return prefix;
 }
 
 __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS, 4)
 sample_top_kernel(const float* __restrict__ logits, long long ld, int vocab, float inv_temperature, int top_k, float top_p,
                   const int* __restrict__ slots, unsigned long long* __restrict__ rng_state, int* __restrict__ out,
                   float* __restrict__ drawn_u) {
-    __shared__ ScShared sh;
-    __shared__ RxShared rx;
     __shared__ TopShared top;
-    const int tid = threadIdx.x, warp = tid >> 5, row_id = blockIdx.y;
+    __shared__ __align__(16) TopScratch scratch;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row_id = blockIdx.y;
     const unsigned rank = sc_rank();
     const float* row = logits + (size_t)row_id * ld;
     const int per_cta = (vocab + SC_CTAS - 1) / SC_CTAS;
     const int lo_i = min((int)rank * per_cta, vocab), hi_i = min(lo_i + per_cta, vocab), n = hi_i - lo_i;
-    const int n_it = (n + ST_TILE - 1) / ST_TILE;
-    int turn = 0;
-    if (tid == 0) { sh.found = 0x7fffffff; rx.bin = 0; rx.need_left = 0; top.n = 0u; }
-    for (int i = tid; i < ST_MAX_IT * SC_WARPS; i += SC_THREADS) top.has[i] = 0;
-
+    const float* slice = row + lo_i;
+    if (tid == 0) {
+        top.block_max = 0u; top.bound = 0u; top.n = 0u; top.n_kept = 0u; top.n_shares = 0u; top.cut = 0u; top.w_cut = 1u;
+        top.found = 0x7fffffff;
+    }
+    sc_cluster_arrive();                                 // nothing is sent to a block before it has started and set this up
     const int seq = slots ? slots[row_id] : row_id;
     unsigned long long state = rng_state[seq];
     state ^= state << 13; state ^= state >> 7; state ^= state << 17;
     const float u = (float)(state >> 40) / 16777216.0f;
 
-    const float* slice = row + lo_i;
     float mx = -INFINITY;
     unsigned best = 0u;
-#pragma unroll 8
-    for (int i = tid; i < n; i += SC_THREADS) {
-        const float x = slice[i] * inv_temperature;
+    top_read(slice, n, [&](float v, int) {
+        const float x = v * inv_temperature;
         mx = fmaxf(mx, x);
         best = max(best, float_order_key(x));
-    }
-    const unsigned mine = top_bound(best, top_k, top.all);
-    if (tid == 0) top.bound = mine;
-    mx = sc_max(mx, sh, turn);                           // its meeting publishes the bound as well
-    unsigned bound = 0u;
+    });
+    __syncthreads();
+    // the maxima of groups of threads, sorted: a value's rank is the number of those before it
+    unsigned mk = float_order_key(mx);
+    for (int o = 16; o > 0; o >>= 1) mk = max(mk, __shfl_xor_sync(ALL, mk, o));
+    if (lane == 0) atomicMax(&top.block_max, mk);
+    constexpr int G = SC_THREADS / TOP_GROUPS;
+    static_assert(G == 4 && TOP_GROUPS % (4 * G) == 0, "four threads a group, which share the counting of its rank");
+    unsigned group = max(best, __shfl_xor_sync(ALL, best, 1));
+    group = max(group, __shfl_xor_sync(ALL, group, 2));
+    if (tid % G == 0) top.maxima[tid / G] = group;
+    __syncthreads();
+    {
+        const int me = tid / G;
+        int before = 0;
 #pragma unroll
-    for (unsigned c = 0; c < SC_CTAS; ++c) bound = max(bound, sc_remote_u32(&top.bound, c));
-    if (rank == 0 && tid == 0) { rng_state[seq] = state; if (drawn_u) drawn_u[row_id] = u; }
-
-#pragma unroll 8
-    for (int i = tid; i < n; i += SC_THREADS) {
-        const unsigned key = float_order_key(slice[i] * inv_temperature);
-        if (key >= bound) {
-            const unsigned at = atomicAdd(&top.n, 1u);
-            if (at < TOP_CAP) top.mine[at] = key;
-            top.has[(i / ST_TILE) * SC_WARPS + (i % ST_TILE) / (32 * ST_EL)] = 1;
+        for (int j = 0; j < TOP_GROUPS / G / 4; ++j) {
+            const int at = 4 * (j * G + tid % G);
+            const uint4 o = *reinterpret_cast<const uint4*>(&top.maxima[at]);
+            before += (o.x > group || (o.x == group && at < me)) + (o.y > group || (o.y == group && at + 1 < me)) +
+                      (o.z > group || (o.z == group && at + 2 < me)) + (o.w > group || (o.w == group && at + 3 < me));
         }
+        before += __shfl_xor_sync(ALL, before, 1);
+        before += __shfl_xor_sync(ALL, before, 2);
+        if (tid % G == 0) top.sorted[before] = group;
     }
     __syncthreads();
-    sc_cluster_sync();                                   // every block's candidates are in place
-    unsigned n_of[SC_CTAS], total = 0u;
-#pragma unroll
-    for (unsigned c = 0; c < SC_CTAS; ++c) {
-        n_of[c] = sc_remote_u32(&top.n, c);
-        total += n_of[c];
+    sc_cluster_wait();
+    if (tid < SC_CTAS * TOP_MARKS) {                     // mark j: at least ceil(k (j + 1) / 8) elements of the slice reach it
+        const unsigned to = tid / TOP_MARKS, j = tid % TOP_MARKS;
+        sc_store_remote(&top.marks[rank * TOP_MARKS + j], to, top.sorted[(top_k * (j + 1) + TOP_MARKS - 1) / TOP_MARKS - 1]);
+        if (j == 0) sc_store_remote(&top.largest[rank], to, top.block_max);
     }
-    unsigned cut, w_cut = 1u;
-    if (total <= TOP_CAP) {                              // the same in every block
-        unsigned at = 0u;
+    sc_cluster_sync();                                   // every block has everyone's marks and maxima
+    if (tid < SC_CTAS * TOP_MARKS) {
+        const unsigned v = top.marks[tid];
+        int count = 0;
 #pragma unroll
-        for (unsigned c = 0; c < SC_CTAS; ++c) {
-            for (unsigned j = tid; j < n_of[c]; j += SC_THREADS) top.all[at + j] = sc_remote_u32(&top.mine[j], c);
-            at += n_of[c];
+        for (int c = 0; c < SC_CTAS; ++c) {
+            int of_block = 0;                            // a block's marks fall: the last one at or above v counts
+#pragma unroll
+            for (int j = 0; j < TOP_MARKS; ++j)
+                if (top.marks[c * TOP_MARKS + j] >= v) of_block = (top_k * (j + 1) + TOP_MARKS - 1) / TOP_MARKS;
+            count += of_block;
         }
+        if (count >= top_k) atomicMax(&top.bound, v);
+    }
+    {
+        unsigned all = 0u;
+#pragma unroll
+        for (int c = 0; c < SC_CTAS; ++c) all = max(all, top.largest[c]);
+        mx = __uint_as_float((all & 0x80000000u) ? (all & 0x7fffffffu) : ~all);
+    }
+    if (rank == 0 && tid == 0) { rng_state[seq] = state; if (drawn_u) drawn_u[row_id] = u; }
+    __syncthreads();
+    const unsigned bound = top.bound;
+    if (best >= bound)
+        top_read(slice, n, [&](float v, int i) {
+            const unsigned key = float_order_key(v * inv_temperature);
+            if (key >= bound) {
+                const unsigned at = sc_add_remote(&top.n, 0, 1u);
+                if (at < TOP_CAP) sc_store_remote(&top.cand[at], 0, (unsigned long long)key << 32 | (unsigned)(lo_i + i));
+            }
+        });
+    sc_cluster_sync();                                   // the first block has every candidate
+    const unsigned total = sc_remote_u32(&top.n, 0);
+    if (total > TOP_CAP) {                               // the same in every block
+        ScShared& sh = scratch.row.sh;
+        RxShared& rx = scratch.row.rx;
+        if (tid == 0) { sh.found = 0x7fffffff; rx.bin = 0; rx.need_left = 0; }
         __syncthreads();
-        const bool in0 = tid < total, in1 = tid + SC_THREADS < total;
-        const unsigned k0 = in0 ? top.all[tid] : 0u, k1 = in1 ? top.all[tid + SC_THREADS] : 0u;
-        cut = total > (unsigned)top_k ? top_cut<true>(rx, k0, k1, in0, in1, 1ull, 1ull, (unsigned long long)top_k, -1.f) : bound;
-        if (top_p < 1.0f) {
-            const unsigned b0 = in0 ? rx_weight(k0, cut, mx) : 0u, b1 = in1 ? rx_weight(k1, cut, mx) : 0u;
-            w_cut = max(1u, top_cut<false>(rx, b0, b1, b0 != 0u, b1 != 0u, rx_mass(b0), rx_mass(b1), 0ull, fmaxf(top_p, 0.f)));
-        }
-    } else {
-        for (int i = tid; i < ST_MAX_IT * SC_WARPS; i += SC_THREADS) top.has[i] = 1;
+        int turn = 0;
+        unsigned cut, w_cut;
         auto key_at = [&](int i) { return float_order_key(slice[i] * inv_temperature); };
         rx_cuts(rx, n, vocab, top_k, top_p, cut, w_cut, key_at, [](unsigned) {},
                 [&](int i) { return rx_weight(key_at(i), cut, mx); });
-    }
-    auto weights = [&](int it, float (&w)[ST_EL]) {
-        const int i0 = (it * SC_THREADS + tid) * ST_EL;
-        const bool any = top.has[it * SC_WARPS + warp];              // one answer for the warp
+        auto weights = [&](int it, float (&w)[ST_EL]) {
+            const int i0 = (it * SC_THREADS + tid) * ST_EL;
 #pragma unroll
-        for (int e = 0; e < ST_EL; ++e) {
-            const unsigned bits = any && i0 + e < n ? rx_weight(float_order_key(slice[i0 + e] * inv_temperature), cut, mx) : 0u;
-            w[e] = bits >= w_cut ? __uint_as_float(bits) : 0.f;
+            for (int e = 0; e < ST_EL; ++e) {
+                const unsigned bits = i0 + e < n ? rx_weight(key_at(i0 + e), cut, mx) : 0u;
+                w[e] = bits >= w_cut ? __uint_as_float(bits) : 0.f;
+            }
+        };
+        auto largest = [&](float& bv, int& bi) {
+            bv = -INFINITY; bi = 0x7fffffff;
+            for (int i = tid; i < n; i += SC_THREADS) {
+                const float x = slice[i] * inv_temperature;
+                if (x > bv) { bv = x; bi = lo_i + i; }
+            }
+        };
+        sc_draw(sh, turn, rank, n, (n + ST_TILE - 1) / ST_TILE, lo_i, u, out + row_id, weights, largest);
+        return;
+    }
+    // from here on the first block is alone; it waits for the others' look at its count before it leaves
+    if (rank != 0) return;
+    const int cands = (int)total;
+    // the key of the k-th largest: fewer than k lie above it, at least k at or above it
+    if (cands > top_k) {
+        for (int i = tid; i < cands; i += SC_THREADS) {
+            const unsigned key = (unsigned)(top.cand[i] >> 32);
+            int above = 0, reach = 0;
+            for (int j = 0; j < cands; ++j) {
+                const unsigned o = (unsigned)(top.cand[j] >> 32);
+                above += o > key;
+                reach += o >= key;
+            }
+            if (above < top_k && reach >= top_k) top.cut = key;
+        }
+    } else if (tid == 0) {
+        top.cut = bound;
+    }
+    for (int i = tid; i < SC_CTAS * TOP_SHARES; i += SC_THREADS) top.part[i] = 0.f;
+    if (tid < SC_CTAS * TOP_SHARES / 32) top.used[tid] = 0u;
+    __syncthreads();
+    for (int i = tid; i < cands; i += SC_THREADS) {
+        const unsigned long long c = top.cand[i];
+        const unsigned bits = rx_weight((unsigned)(c >> 32), top.cut, mx);
+        if (bits != 0u) top.kept[atomicAdd(&top.n_kept, 1u)] = (unsigned long long)bits << 32 | (unsigned)c;
+    }
+    __syncthreads();
+    const int n_kept = (int)top.n_kept;
+    if (top_p < 1.0f) {                                  // the weight at which the mass from the top reaches what is needed
+        for (int i = tid; i < n_kept; i += SC_THREADS) {
+            const unsigned bits = (unsigned)(top.kept[i] >> 32);
+            unsigned long long above = 0ull, reach = 0ull, all = 0ull;
+            for (int j = 0; j < n_kept; ++j) {
+                const unsigned o = (unsigned)(top.kept[j] >> 32);
+                const unsigned long long q = rx_mass(o);
+                above += o > bits ? q : 0ull;
+                reach += o >= bits ? q : 0ull;
+                all += q;
+            }
+            unsigned long long need = (unsigned long long)((double)fmaxf(top_p, 0.f) * (double)all);
+            need = need > 0 ? need : 1;
+            if (above < need && reach >= need) top.w_cut = bits;
+        }
+        __syncthreads();
+    }
+    // the draw: where element i of the row lies
+    auto place = [&](unsigned i, int& share, int& at) {
+        const int c = (int)i / per_cta, local = (int)i % per_cta, in = local % ST_TILE;
+        share = c * TOP_SHARES + local / ST_TILE * SC_WARPS + in / (32 * ST_EL);
+        at = in % (32 * ST_EL);
+    };
+    const unsigned w_cut = top.w_cut;
+    unsigned* shares = reinterpret_cast<unsigned*>(top.cand);          // of which some element is kept
+    for (int i = tid; i < n_kept; i += SC_THREADS)
+        if ((unsigned)(top.kept[i] >> 32) >= w_cut) {
+            int share, at;
+            place((unsigned)top.kept[i], share, at);
+            if (!(atomicOr(&top.used[share / 32], 1u << (share % 32)) >> (share % 32) & 1u)) shares[atomicAdd(&top.n_shares, 1u)] = share;
+        }
+    __syncthreads();
+    // this lane's four weights of a share, their sum, and the sums of the lanes up to this one
+    auto share_sums = [&](int share, float (&w)[ST_EL], float& v, float& incl) {
+        float* mine = scratch.share[warp];
+        *reinterpret_cast<float4*>(mine + lane * ST_EL) = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+        for (int i = lane; i < n_kept; i += 32) {
+            int of, at;
+            place((unsigned)top.kept[i], of, at);
+            const unsigned bits = (unsigned)(top.kept[i] >> 32);
+            if (of == share && bits >= w_cut) mine[at] = __uint_as_float(bits);
+        }
+        __syncwarp();
+        const float4 x = *reinterpret_cast<const float4*>(mine + lane * ST_EL);
+        __syncwarp();
+        w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
+        v = (w[0] + w[1]) + (w[2] + w[3]);
+        incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float q = __shfl_up_sync(ALL, incl, o);
+            if (lane >= o) incl += q;
         }
     };
-    auto largest = [&](float& bv, int& bi) {
-        bv = -INFINITY; bi = 0x7fffffff;
-        for (int i = tid; i < n; i += SC_THREADS) {
-            const float x = slice[i] * inv_temperature;
-            if (x > bv) { bv = x; bi = lo_i + i; }
+    for (int g = warp; g < (int)top.n_shares; g += SC_WARPS) {
+        float w[ST_EL], v, incl;
+        share_sums((int)shares[g], w, v, incl);
+        if (lane == 31) top.part[shares[g]] = incl;
+    }
+    __syncthreads();
+    const float* parts = top.part + min(warp, SC_CTAS - 1) * TOP_SHARES;        // warp = slice from here on
+    if (warp < SC_CTAS) {
+        float v = 0.f;
+        for (int w = 0; w < SC_WARPS; ++w) v += parts[lane * SC_WARPS + w];
+        float incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float q = __shfl_up_sync(ALL, incl, o);
+            if (lane >= o) incl += q;
         }
-    };
-    sc_draw(sh, turn, rank, n, n_it, lo_i, u, out + row_id, weights, largest);
+        top.it_before[warp][lane] = incl - v;
+        top.it_sum[warp][lane] = v;
+        if (lane == 31) top.slice_sum[warp] = incl;
+    }
+    __syncthreads();
+    float base = 0.f, kept = 0.f;
+    for (int c = 0; c < SC_CTAS; ++c) {
+        if (c == warp) base = kept;
+        kept += top.slice_sum[c];
+    }
+    if (!(kept > 0.f) || isinf(kept) || isnan(kept)) {   // nothing to draw from: the row's largest logit, lowest index first
+        float bv = -INFINITY;
+        int bi = 0x7fffffff;
+        for (int i = tid; i < vocab; i += SC_THREADS) {
+            const float x = row[i] * inv_temperature;
+            if (x > bv) { bv = x; bi = i; }
+        }
+        const float gm = block_max(bv, scratch.row.sh.red[0]);
+        if (bv == gm && bi != 0x7fffffff) atomicMin(&top.found, bi);
+    } else if (warp < SC_CTAS) {
+        const float r = u * kept, mine = top.slice_sum[warp];
+        if (mine > 0.f && base <= r && r <= base + mine) {                      // the slices tile [0, kept]
+            const unsigned at = __ballot_sync(ALL, top.it_sum[warp][lane] > 0.f && base + top.it_before[warp][lane] <= r);
+            const int it = at ? 31 - __clz(at) : 0;
+            float run = base + top.it_before[warp][it];
+            for (int w = 0; w < lane && w < SC_WARPS; ++w) run += parts[it * SC_WARPS + w];
+            const unsigned aw = __ballot_sync(ALL, lane < SC_WARPS && parts[it * SC_WARPS + min(lane, SC_WARPS - 1)] > 0.f && run <= r);
+            const int w_sel = aw ? 31 - __clz(aw) : 0;
+            const float before = __shfl_sync(ALL, run, w_sel);
+            float w[ST_EL], v, incl;
+            share_sums(warp * TOP_SHARES + it * SC_WARPS + w_sel, w, v, incl);
+            const float start = before + (incl - v);
+            const unsigned al = __ballot_sync(ALL, v > 0.f && start <= r);
+            if (al && lane == 31 - __clz(al)) {
+                const int i0 = warp * per_cta + ((it * SC_WARPS + w_sel) * 32 + lane) * ST_EL;
+                float cum = start;
+                int last = -1, hit = -1;
+#pragma unroll
+                for (int e = 0; e < ST_EL; ++e)
+                    if (hit < 0 && w[e] > 0.f) {
+                        last = i0 + e;
+                        cum += w[e];
+                        if (cum >= r) hit = i0 + e;
+                    }
+                if (hit < 0) hit = last;                 // rounding left r a hair above this lane's sum
+                if (hit >= 0) atomicMin(&top.found, hit);
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0) out[row_id] = (top.found == 0x7fffffff) ? 0 : top.found;
+    sc_cluster_sync();                                   // of the blocks that have not left yet: they have read the count
 }
 
 // form 0: chosen by the sizes; 1: never from candidates; 2: from candidates (top_k 1 to 64, vocabularies up to 524,288).  The
@@ -823,11 +1010,10 @@ SSB_API int ssb_sample(const float* logits, long long ld, int n_rows, int vocab,
                 logits, ld, vocab, 1.0f / temperature, slots, rng_state, out, drawn_u);
             return ssb_launch_status();
         }
-        // Both cuts, k 40, p 0.9, us held and from candidates: 64 rows of 128,256 tokens 98 and 46, 1 row 40 and 30; 1 and 64
-        // rows of 8,192 25 and 23, 47 and 34.  A top-k cut alone is four counting passes over slices that are held while the
-        // clusters find room for them: 64 x 50,257 30 and 33, 16 x 128,256 29 and 29, 12 x 262,144 34 and 31; at four million
-        // logits 64 x 65,536 32 and 32, 32 x 128,256 31 and 30, 16 x 262,144 62 and 34; 64 x 128,256 58 and 44.
-        if (form == 2 || (form == 0 && top_k > 0 && top_k <= TOP_MAX_K && (top_p < 1.0f || (long long)n_rows * vocab >= 4000000))) {
+        // us with the row held and from candidates, k 40: both cuts (p 0.9), 1 row of 8,192, 32,000 and 128,256 tokens 28, 32, 45 and
+        // 16, 18, 20, 64 rows 49, 55, 106 and 23, 25, 33; the top-k cut alone, 1 row 16, 19, 29 and 16, 16, 20, 64 rows 25, 29, 66 and
+        // 22, 25, 31.
+        if (form == 2 || (form == 0 && top_k > 0 && top_k <= TOP_MAX_K)) {
             sample_top_kernel<<<dim3(SC_CTAS, n_rows), SC_THREADS, 0, stream>>>(
                 logits, ld, vocab, 1.0f / temperature, top_k, top_p, slots, rng_state, out, drawn_u);
             return ssb_launch_status();
