@@ -266,17 +266,26 @@ class SequenceCache:
         the generator starts from a fixed state of the slot's own, never from zero (the fixed point
         of xorshift64) and never from what the slot's last sequence left."""
         slot = self._book.acquire()
-        for t in self._state.values():
-            t[slot].zero_()
-        self.seed(slot, rng_seed if rng_seed is not None else default_seed(slot))
+        self._set_up(slot, rng_seed if rng_seed is not None else default_seed(slot), list(self._state.values()))
         return slot
 
     def seed(self, slot: int, seed: int) -> None:
+        self._set_up(slot, seed, [])
+
+    def _set_up(self, slot: int, seed: int, states) -> None:
+        """Generator state of a slot, and rows of fixed state zeroed; on a device by one launch."""
         seed &= (1 << 64) - 1
         if seed == 0:
             seed = 0x9E3779B97F4A7C15       # xorshift needs a non-zero state (qwen36_moe_decode.rs:1091-1094)
         if seed >= 1 << 63:
             seed -= 1 << 64
+        if self.device.type == "cuda":
+            from ..csrc import ops
+            with torch.cuda.device(self.device):
+                ops.open_sequence(self.rng_state, slot, seed, states)
+            return
+        for t in states:
+            t[slot].zero_()
         self.rng_state[slot] = seed
 
     def release(self, slot: int) -> None:

@@ -82,6 +82,42 @@ def _fn(lib: str, name: str):
     return _lib_cache[key]
 
 
+# ---- what the host hands a step ----------------------------------------------------------
+PUT_INTS_MOST = 960
+
+
+def put_ints(values, out: torch.Tensor, before: Optional[torch.Tensor] = None) -> None:
+    """out = [before |] values: int32 values of the host (a contiguous numpy array) as kernel arguments, behind those of the
+    device tensor ``before``."""
+    _need(out, "out", torch.int32, 1)
+    n, n_before = len(values), 0 if before is None else before.numel()
+    if before is not None:
+        _need(before, "before", torch.int32, 1)
+    if values.dtype != "int32" or not values.flags.c_contiguous or out.shape[0] != n + n_before:
+        raise KernelError("put_ints: contiguous int32 values, one place for each")
+    fn, base = _fn("step_inputs", "ssb_put_ints"), values.ctypes.data
+    for lo in range(0, max(n, 1), PUT_INTS_MOST):
+        m, b = min(PUT_INTS_MOST, n - lo), n_before if lo == 0 else 0
+        _check(fn(c_void_p(base + 4 * lo), c_int(m), _ptr(before), c_int(b), c_void_p(out.data_ptr() + 4 * (lo + n_before - b)),
+                  _stream()), "put_ints")
+
+
+def open_sequence(rng_state: torch.Tensor, slot: int, seed: int, states) -> None:
+    """rng_state[slot] = seed (a signed 64-bit number); row ``slot`` of every tensor of ``states`` (four-byte elements) zeroed."""
+    _need(rng_state, "rng_state", torch.int64, 1)
+    if not 0 <= slot < rng_state.shape[0]:
+        raise KernelError(f"open_sequence: slot {slot} is outside {rng_state.shape[0]}")
+    for t in states:
+        _need(t, "state", None, 2)
+        if t.element_size() != 4 or slot >= t.shape[0] or t.shape[1] >= 1 << 31:
+            raise KernelError("open_sequence: states of four-byte elements, a row for every slot")
+    n = len(states)
+    rows = (c_void_p * max(n, 1))(*[t.data_ptr() + slot * t.stride(0) * 4 for t in states])
+    words = (c_int * max(n, 1))(*[t.shape[1] for t in states])
+    _check(_fn("step_inputs", "ssb_open_sequence")(c_void_p(rng_state.data_ptr() + 8 * slot), c_longlong(seed), rows, words,
+                                                   c_int(n), _stream()), "open_sequence")
+
+
 # ---- plain ops -------------------------------------------------------------------------
 def embed(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor, scale: float = 1.0,
           rounded: Optional[torch.Tensor] = None) -> None:

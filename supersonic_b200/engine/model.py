@@ -69,8 +69,8 @@ class DecodeGraph:
     """One captured decode step for a fixed number of sequences and key-page bucket.
 
     Token ids, positions and slots live in a fixed device buffer that each step
-    overwrites from pinned host memory; the captured kernels read them from there, so the
-    same graph serves any sequences at any positions within the bucket.  The reference has
+    overwrites by a kernel that carries them as arguments; the captured kernels read them from there,
+    so the same graph serves any sequences at any positions within the bucket.  The reference has
     no graphs: every op is a host call, several followed by a device synchronise
     (kernels/full_attention_bridge_cuda.cu:1905-1906)."""
 
@@ -78,10 +78,9 @@ class DecodeGraph:
         from ..csrc import ops
         B, dev = n_seqs, model.device
         self.n_seqs = B
-        # a ring of pinned staging buffers: the host may run several steps ahead of the device
-        self.hosts = [torch.zeros(3 * B, dtype=torch.int32).pin_memory() for _ in range(4)]
-        self.hosts_np = [h.numpy() for h in self.hosts]     # the same memory, cheap to fill from lists
-        self.copied = [None] * len(self.hosts)
+        self.staged = np.zeros(3 * B, dtype=np.int32)
+        # the host may run several steps ahead of the device, but not without end
+        self.started = [None] * 4
         self.turn = 0
         self.ints = torch.zeros(3 * B, dtype=torch.int32, device=dev)
         self.ints[2 * B:] = -1                              # warm-up rows are padding: nothing is written
@@ -112,25 +111,23 @@ class DecodeGraph:
     def run(self, tokens, positions, slots) -> torch.Tensor:
         """``tokens``: a host list, or an int32 device tensor (what a sampler just wrote: the step is then
         launched without the host ever seeing them)."""
+        from ..csrc import ops
         i = self.turn
-        self.turn = (i + 1) % len(self.hosts)
-        if self.copied[i] is not None:
-            self.copied[i].synchronize()                    # its last copy has left this buffer
-        h = self.hosts[i]
+        self.turn = (i + 1) % len(self.started)
+        if self.started[i] is not None:
+            self.started[i].synchronize()
         B = self.n_seqs
         if isinstance(tokens, torch.Tensor):
-            self.hosts_np[i][B:] = list(positions) + list(slots)
-            self.ints[B:].copy_(h[B:], non_blocking=True)
-            self.ints[:B].copy_(tokens.view(-1), non_blocking=True)
+            self.staged[B:] = list(positions) + list(slots)
+            ops.put_ints(self.staged[B:], self.ints, before=tokens.reshape(-1))
         else:
-            self.hosts_np[i][:] = list(tokens) + list(positions) + list(slots)     # a numpy view of the pinned buffer
-            self.ints.copy_(h, non_blocking=True)
-        if self.copied[i] is None:
-            self.copied[i] = torch.cuda.Event()
-        self.copied[i].record()
+            self.staged[:] = list(tokens) + list(positions) + list(slots)
+            ops.put_ints(self.staged, self.ints)
+        if self.started[i] is None:
+            self.started[i] = torch.cuda.Event()
+        self.started[i].record()
         self.graph.replay()
         if self.waiting_kernels:
-            from ..csrc import ops
             ops.note_bounded_wait_launches(self.waiting_kernels)
         return self.logits
 
@@ -148,7 +145,9 @@ class PromptGraph:
         from ..csrc import ops
         dev = model.device
         n = int(packed.flat.shape[0])
-        self.hosts = [torch.zeros(n, dtype=torch.int32).pin_memory() for _ in range(2)]
+        # few enough to come as kernel arguments, or through two pinned buffers in turn
+        self.by_launch = n <= 2 * ops.PUT_INTS_MOST
+        self.hosts = None if self.by_launch else [torch.zeros(n, dtype=torch.int32).pin_memory() for _ in range(2)]
         self.copied = [None, None]
         self.turn = 0
         self.ints = torch.zeros(n, dtype=torch.int32, device=dev)
@@ -168,8 +167,12 @@ class PromptGraph:
         self.turn = 1 - i
         if self.copied[i] is not None:
             self.copied[i].synchronize()
-        self.hosts[i].numpy()[:] = packed.flat
-        self.ints.copy_(self.hosts[i], non_blocking=True)
+        if self.by_launch:
+            from ..csrc import ops
+            ops.put_ints(np.ascontiguousarray(packed.flat, dtype=np.int32), self.ints)
+        else:
+            self.hosts[i].numpy()[:] = packed.flat
+            self.ints.copy_(self.hosts[i], non_blocking=True)
         if self.copied[i] is None:
             self.copied[i] = torch.cuda.Event()
         self.copied[i].record()
