@@ -242,10 +242,17 @@ __device__ __forceinline__ int gf_walk_key(int chunk, int row) {
     return RW == 4 ? row : RW == 2 ? ((chunk >> 1) & 1) ^ (row << 1) : (chunk >> 1) & 3;
 }
 
-template <int MB, int RW>
+// A gated unit's first product: W holds its gate rows, then as many up rows (N in all); a warp's rows are half of either, and
+// what is stored is ssb_gate of the two sums, times the row's factor.
+struct GfGate { int kind; float limit; const float* row_scale; };
+
+template <int MB, int RW, bool GATED = false>
 __global__ void __launch_bounds__(32 * GF_WALK_WARPS)
 gemm_f32_walk_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
-                     int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int accumulate) {
+                     int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int accumulate, GfGate gate) {
+    static_assert(!GATED || RW >= 2, "gate and up rows in one warp");
+    constexpr int OUT = GATED ? RW / 2 : RW;                           // columns of the result a warp makes
+    const int n_out = GATED ? N / 2 : N;
     constexpr int CL = 32 / RW, STEP = CL * GF_CHUNK, SEG = GF_WALK_TURN / RW, ROW_LOADS = 8 / RW, STAGES = GF_WALK_STAGES;
     static_assert(SEG == 2 * STEP && GF_WALK_TURN == 8 * 32 * 4, "two steps a turn, eight pieces a lane");
     extern __shared__ __align__(16) float gf_smem[];
@@ -256,20 +263,21 @@ gemm_f32_walk_kernel(const float* __restrict__ A, int lda, const float* __restri
     A += (size_t)blockIdx.z * a_batch;
     W += (size_t)blockIdx.z * w_batch;
     C += (size_t)blockIdx.z * c_batch;
-    const int tasks = (N + RW - 1) / RW, first = warp * (int)gridDim.x + (int)blockIdx.x, stride = warps * (int)gridDim.x;
+    const int tasks = (n_out + OUT - 1) / OUT, first = warp * (int)gridDim.x + (int)blockIdx.x, stride = warps * (int)gridDim.x;
     const int turns = (K + SEG - 1) / SEG;
     const int total = first < tasks ? (tasks - first + stride - 1) / stride * turns : 0;
 
     int ahead_turn = 0, ahead_task = first, ahead_slot = 0;            // of the next load
     auto load = [&]() {
-        const int k = ahead_turn * SEG + lane * 4, rows = N - ahead_task * RW;
-        const float* src = W + (size_t)ahead_task * RW * ldw + k;
+        const int k = ahead_turn * SEG + lane * 4, rows = n_out - ahead_task * OUT;
+        const float* src = W + (size_t)ahead_task * OUT * ldw + k;
         float* dst = ring + ahead_slot * GF_WALK_TURN;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {                                  // what lies outside arrives as zeros
             const int r = e / ROW_LOADS, s = e % ROW_LOADS * 32;       // row, and the row's piece lane + s
-            const bool in = r < rows && k + s * 4 < K;
-            gf_cp16(dst + r * SEG + ((s + lane) ^ gf_walk_key<RW>(lane / 4, r)) * 4, in ? src + (size_t)r * ldw + s * 4 : W, in ? 16 : 0);
+            const bool in = r % OUT < rows && k + s * 4 < K;
+            gf_cp16(dst + r * SEG + ((s + lane) ^ gf_walk_key<RW>(lane / 4, r)) * 4,
+                    in ? src + (size_t)(r % OUT + r / OUT * n_out) * ldw + s * 4 : W, in ? 16 : 0);
         }
         if (++ahead_slot == STAGES) ahead_slot = 0;
         if (++ahead_turn == turns) { ahead_turn = 0; ahead_task += stride; }
@@ -340,10 +348,12 @@ gemm_f32_walk_kernel(const float* __restrict__ A, int lda, const float* __restri
                 if (j < here) gf_kahan(acc, lost, held[j]);
                 held[j] = 0.f;
             }
-            const int col = task * RW + n;
-            if (c < MB && c < M && col < N) {
+            const float up = GATED ? __shfl_down_sync(0xffffffffu, acc, OUT) : 0.f;
+            const int col = task * OUT + n;
+            if (c < MB && c < M && n < OUT && col < n_out) {
                 float* dst = C + (size_t)c * ldc + col;
-                *dst = accumulate ? *dst + acc : acc;
+                if constexpr (GATED) *dst = ssb_gate(acc, up, gate.kind, gate.limit) * (gate.row_scale ? gate.row_scale[c] : 1.0f);
+                else *dst = accumulate ? *dst + acc : acc;
             }
             acc = lost = 0.f;
             turn = 0;
@@ -634,12 +644,16 @@ static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
     return forms[best];
 }
 
+// Whether a gated unit's first product is made by walking warps, which finish it.
+static inline bool gemm_f32_gated_ok(int M, int N, int K) { return N % 2 == 0 && gemm_f32_form(1, M, N, K) <= 4; }
+
 // form 0: chosen by the sizes; else one of the kernels: 1, 2, 4 (a warp walks), 5, 8, 16 (few rows, 4, 8, 16 a group), 100, 101, 102, 103 (tiles
 // of 64 x 64, 128 x 64 and twice 128 x 128, the last with its sums in tensor memory)
 static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, const float* W, int ldw, long long w_batch,
                                   float* C, int ldc, long long c_batch, int n_batch, int M, int N, int K, int accumulate,
-                                  int form, cudaStream_t stream, bool pdl = false) {
+                                  int form, cudaStream_t stream, bool pdl = false, const GfGate* gate = nullptr) {
     if (form == 0) form = gemm_f32_form(n_batch, M, N, K);
+    if (gate && (form > 4 || n_batch != 1 || N % 2)) return SSB_ERR_UNSUPPORTED;
 #define GF_CONFIGURE(kernel, smem) do { \
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)); \
         if (e != cudaSuccess) return (int)e; \
@@ -666,21 +680,22 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         kernel<<<dim3((N + cols - 1) / cols, (M + rows - 1) / rows, n_batch), GF_TILE_THREADS, smem, stream>>>( \
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
     } while (0)
-#define GF_WALK(MB, RW) do { \
+#define GF_WALK(MB, RW, ...) do { \
         const size_t rows = gf_walk_rows(MB, K); \
-        auto kernel = gemm_f32_walk_kernel<MB, RW>; \
+        auto kernel = gemm_f32_walk_kernel<MB, RW, ##__VA_ARGS__>; \
         GF_CONFIGURE(kernel, GF_WALK_SMEM); \
         const int tasks = (N + RW - 1) / RW, blocks = tasks < gf_sms() ? tasks : gf_sms(), room = (int)((GF_WALK_SMEM - rows) / GF_WALK_RING); \
         int warps = (tasks + blocks - 1) / blocks; \
         warps = warps > GF_WALK_WARPS ? GF_WALK_WARPS : warps; \
         warps = warps > room ? room : warps; \
         const int rc = ssb_launch(kernel, dim3((unsigned)blocks, 1, n_batch), dim3(32 * warps), rows + warps * GF_WALK_RING, \
-                                  stream, pdl, A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
+                                  stream, pdl, A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate, gate ? *gate : GfGate{}); \
         if (rc) return rc; \
     } while (0)
 #define GF_WALKS(MB) do { \
         const int width = gf_walk_width(N); \
-        if (width == 4) GF_WALK(MB, 4); else if (width == 2) GF_WALK(MB, 2); else GF_WALK(MB, 1); \
+        if (gate) { if (width == 4) GF_WALK(MB, 4, true); else GF_WALK(MB, 2, true); } \
+        else if (width == 4) GF_WALK(MB, 4); else if (width == 2) GF_WALK(MB, 2); else GF_WALK(MB, 1); \
     } while (0)
     switch (form) {
         case 1: GF_WALKS(1); break;

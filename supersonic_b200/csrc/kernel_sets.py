@@ -100,9 +100,12 @@ class PlainKernels:
         """out = silu(x @ gate^T) * (x @ up^T); ``act`` = (kind, limit) names another inner step of the gated unit
         (``ops.gated_activation``); ``row_scale``: one float32 factor per row of ``out``."""
         x = as_tensor(x)
+        kind, limit = act if act else ("silu", 0.0)
+        if layout == "halves" and x.dtype == torch.float32 and ops.gemm_f32_gated_ok(x, w_gate_up, out):
+            ops.gemm_f32_gated(x, w_gate_up, out, kind, limit, row_scale, pdl=self._chain(x.shape[0]))
+            return
         gate_up = torch.empty((x.shape[0], w_gate_up.shape[0]), dtype=x.dtype, device=x.device)
         self.linear(x, w_gate_up, gate_up)
-        kind, limit = act if act else ("silu", 0.0)
         ops.gated_activation(gate_up, out, kind, limit, interleaved=(layout == "interleaved"), row_scale=row_scale,
                              pdl=self._chain(x.shape[0]))
 
@@ -158,7 +161,16 @@ class PlainKernels:
                        scale) -> bool:
         """Position encoding, cache append and attention in one launch, if this set can do it
         for this case; False means the caller runs the two steps separately."""
-        return False
+        tables = getattr(position, "rotary_tables", None)
+        k_cache, v_cache, page_table, _ = kv
+        if not (batch.is_decode and tables) or getattr(position, "interleaved", False) \
+                or not ops.attention_f32_decode_ok(qkv, k_cache, v_cache, head_dim):
+            return False
+        cos, sin, rotary_dim = tables()
+        position.check_range(batch)
+        ops.attention_f32_decode(qkv, cos, sin, k_cache, v_cache, batch.pos, batch.slot_of_token, page_table, out, n_q, n_kv,
+                                 head_dim, rotary_dim, page_shift, window, scale, pdl=self._chain(batch.n_tokens))
+        return True
 
     def attention(self, q, k_cache, v_cache, batch, page_table, out, n_q, n_kv, head_dim, page_shift,
                   window: Optional[int], scale: float):

@@ -255,6 +255,37 @@ def attention_plain(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
         c_int(1 if pdl else 0), _stream()), "attention_plain")
 
 
+def attention_f32_decode_ok(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, head_dim: int) -> bool:
+    """Whether ``attention_f32_decode`` takes these: float32 heads of up to 128 elements, caches in whole 16-byte pieces."""
+    return (qkv.dtype == torch.float32 and head_dim <= 128 and head_dim % 4 == 0 and k_cache.dtype == torch.float32
+            and k_cache.is_contiguous() and v_cache.is_contiguous() and v_cache.shape == k_cache.shape
+            and (k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0)
+
+
+def attention_f32_decode(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
+                         pos: torch.Tensor, slot: torch.Tensor, page_table: torch.Tensor, out: torch.Tensor, n_q: int, n_kv: int,
+                         head_dim: int, rotary_dim: int, page_shift: int, window: Optional[int], scale: float,
+                         pdl: bool = False) -> None:
+    """``rope_append`` and ``attention_plain`` of a float32 decode step (one token a sequence) in one launch: the same bits.
+    ``qkv`` [T, q heads | k heads | v heads] is left unrotated."""
+    _need(qkv, "qkv", torch.float32, 2); _need(out, "out", torch.float32, 2)
+    _need(cos, "cos", torch.float32, 2); _need(sin, "sin", torch.float32, 2)
+    _need(pos, "pos", torch.int32, 1); _need(slot, "slot", torch.int32, 1); _need(page_table, "page_table", torch.int32, 2)
+    T = qkv.shape[0]
+    if not attention_f32_decode_ok(qkv, k_cache, v_cache, head_dim):
+        raise KernelError("attention_f32_decode: caches or head size are not supported")
+    if pos.shape[0] != T or slot.shape[0] != T or out.shape[0] != T or out.shape[1] < n_q * head_dim \
+            or qkv.shape[1] < (n_q + 2 * n_kv) * head_dim:
+        raise KernelError("attention_f32_decode: one position and one slot per token, rows of [q | k | v]")
+    if cos.shape != sin.shape or cos.shape[1] != rotary_dim // 2 or not cos.is_contiguous() or not sin.is_contiguous():
+        raise KernelError("attention_f32_decode: cos/sin must be [positions, rotary_dim/2], contiguous")
+    _check(_fn("plain_ops", "ssb_attention_f32_decode")(
+        _ptr(qkv), c_int(qkv.stride(0)), _ptr(cos), _ptr(sin), c_int(cos.shape[0]), c_int(rotary_dim), _ptr(k_cache),
+        _ptr(v_cache), _ptr(pos), _ptr(slot), _ptr(page_table), c_int(page_table.shape[1]), _ptr(out), c_int(out.stride(0)),
+        c_int(T), c_int(n_q), c_int(n_kv), c_int(head_dim), c_int(page_shift), c_int(int(window) if window else 0),
+        c_float(scale), c_int(1 if pdl else 0), _stream()), "attention_f32_decode")
+
+
 def attention_f32_prompt_ok(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor,
                             head_dim: int, n_seqs: int = 1) -> bool:
     """Whether ``attention_f32_prompt`` takes these: float32 rows and caches in whole 16-byte pieces, no more sequences than
@@ -318,6 +349,33 @@ def gated_activation(gate_up: torch.Tensor, out: torch.Tensor, kind: str = "silu
         _ptr(gate_up), c_int(gate_up.stride(0)), _ptr(out), c_int(out.stride(0)), c_int(dtype_code(out.dtype)), c_int(T),
         c_int(inter), c_int(1 if interleaved else 0), c_int(GATE_KINDS_FF[kind]), c_float(limit), _ptr(row_scale),
         c_int(1 if pdl else 0), _stream()), "gated_activation")
+
+
+def gemm_f32_gated_ok(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether ``gemm_f32_gated`` takes these: the few float32 rows whose product walking warps make."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32 and x.is_cuda
+            and x.dim() == 2 and w.dim() == 2 and x.stride(1) == 1 and w.stride(1) == 1
+            and bool(_fn("plain_ops", "ssb_gemm_f32_gated_ok")(
+                _ptr(x), c_int(x.stride(0)), _ptr(w), c_int(w.stride(0)), c_int(x.shape[0]), c_int(w.shape[0]), c_int(w.shape[1]))))
+
+
+def gemm_f32_gated(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: str = "silu", limit: float = 0.0,
+                   row_scale: Optional[torch.Tensor] = None, pdl: bool = False) -> None:
+    """``gemm_nt_plain`` by ``w`` [gate rows | up rows] and ``gated_activation`` behind it in one launch: the same bits."""
+    _need(x, "x", torch.float32, 2); _need(w, "w", torch.float32, 2); _need(out, "out", torch.float32, 2)
+    if kind not in GATE_KINDS_FF:
+        raise KernelError(f"gemm_f32_gated: kind {kind!r} is not known (known: {sorted(GATE_KINDS_FF)})")
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K or N % 2 or tuple(out.shape) != (M, N // 2):
+        raise KernelError(f"gemm_f32_gated: shapes x{tuple(x.shape)} w{tuple(w.shape)} out{tuple(out.shape)}")
+    if row_scale is not None:
+        _need(row_scale, "row_scale", torch.float32, 1)
+        if row_scale.shape[0] != M:
+            raise KernelError("gemm_f32_gated: one factor per row")
+    _check(_fn("plain_ops", "ssb_gemm_f32_gated")(
+        _ptr(x), c_int(x.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(out), c_int(out.stride(0)), c_int(M), c_int(N), c_int(K),
+        c_int(GATE_KINDS_FF[kind]), c_float(limit), _ptr(row_scale), c_int(1 if pdl else 0), _stream()), "gemm_f32_gated")
 
 
 def rms_add(residual: torch.Tensor, branch: torch.Tensor, weight: torch.Tensor, eps: float, clear: bool = False,

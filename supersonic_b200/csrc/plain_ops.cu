@@ -271,6 +271,18 @@ SSB_API int ssb_gemm_nt_plain(const void* A, int lda, const void* W, int ldw, in
     return gemm_nt_plain_launch(A, lda, 0, W, ldw, 0, in_dtype, C, ldc, 0, out_dtype, 1, M, N, K, accumulate, pdl != 0, stream);
 }
 
+// z = gate_fn(x gate^T, x up^T) * row_scale for a few float32 rows, in one launch; the bits of the product and the kernel behind it
+SSB_API int ssb_gemm_f32_gated_ok(const void* A, int lda, const void* W, int ldw, int M, int N, int K) {
+    return M > 0 && N > 0 && K > 0 && gemm_f32_ok(A, lda, 0, W, ldw, 0, K) && gemm_f32_gated_ok(M, N, K);
+}
+SSB_API int ssb_gemm_f32_gated(const float* A, int lda, const float* W, int ldw, float* z, int ldz, int M, int N, int K, int kind,
+                               float limit, const float* row_scale, int pdl, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (kind < 0 || kind > SSB_GATE_LAST || !ssb_gemm_f32_gated_ok(A, lda, W, ldw, M, N, K)) return SSB_ERR_BAD_SIZE;
+    const GfGate gate = {kind, limit, row_scale};
+    return gemm_f32_launch(A, lda, 0, W, ldw, 0, z, ldz, 0, 1, M, N, K, 0, 0, stream, pdl != 0, &gate);
+}
+
 SSB_API int ssb_gemm_nt_plain_batched(const void* A, int lda, long long a_batch, const void* W, int ldw,
                                       long long w_batch, int in_dtype, void* C, int ldc, long long c_batch,
                                       int out_dtype, int n_batch, int M, int N, int K, cudaStream_t stream) {
@@ -282,6 +294,12 @@ SSB_API int ssb_gemm_nt_plain_batched(const void* A, int lda, long long a_batch,
 // rotary position encoding on q (in place) and k, then k and v into the paged cache
 // qkv row layout: [q heads | k heads | v heads], each head_dim wide
 // ---------------------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ void rotate_pair(float x1, float x2, float c, float sn, T& y1, T& y2) {
+    y1 = ssb_from_float<T>(x1 * c - x2 * sn);
+    y2 = ssb_from_float<T>(x1 * sn + x2 * c);
+}
+
 constexpr int RO_HEADS = 8;                              // heads (of q, k and v) a block: few tokens still make many blocks
 
 template <typename T>
@@ -313,7 +331,8 @@ rope_append_kernel(T* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
         const int ia = interleaved ? 2 * i : i, ib = interleaved ? 2 * i + 1 : i + half;
         const float c = have_table ? c_row[i] : 1.f, sn = have_table ? s_row[i] : 0.f;
         const float x1 = ssb_to_float(x[ia]), x2 = ssb_to_float(x[ib]);
-        const T y1 = ssb_from_float<T>(x1 * c - x2 * sn), y2 = ssb_from_float<T>(x1 * sn + x2 * c);
+        T y1, y2;
+        rotate_pair(x1, x2, c, sn, y1, y2);
         x[ia] = y1;
         x[ib] = y2;
         if (h >= n_q) {
@@ -485,17 +504,21 @@ attention_plain_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ k
 
 // The same sums for float32 rows of up to 128 elements in whole 16-byte pieces: a chunk's keys and values come by cp.async,
 // all of a chunk's values and the next chunk's keys while the scores and their sums are made, instead of eight values at a time
-// behind every eight additions; a key's place is looked up once.
+// behind every eight additions; a key's place is looked up once.  ROPE (decode steps): q comes as the projection left it, [q | k |
+// v] in a row; the block rotates its query and its token's key (pairs i, i + rotary_dim / 2), and the first head of a kv head
+// appends key and value.
 constexpr int AS_MAX_DIM = 128;
+struct AsRope { const float *cos_t, *sin_t; int table_positions, rotary_dim; float *k_cache, *v_cache; };
 static size_t attention_staged_smem(int head_dim, int v_dim) {
     return sizeof(float) * (size_t)ATT_THREADS * (head_dim + 4 + v_dim);
 }
 
+template <bool ROPE>
 __global__ void __launch_bounds__(ATT_THREADS)
 attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
                         const int* __restrict__ pos, const int* __restrict__ slot, const int* __restrict__ page_table,
                         int max_pages, float* __restrict__ out, int ldo, int n_q, int n_kv, int head_dim, int page_shift,
-                        int window, float scale, int v_dim, int v_row, const float* __restrict__ sinks) {
+                        int window, float scale, int v_dim, int v_row, const float* __restrict__ sinks, AsRope rope) {
     extern __shared__ __align__(16) float as_smem[];
     __shared__ __align__(16) float q_s[AS_MAX_DIM];
     __shared__ __align__(16) float p_s[ATT_THREADS];
@@ -520,7 +543,7 @@ attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __res
         if (base + tid <= p) tok_s[buf][tid] = ssb_cache_row(page_table, max_pages, s, base + tid, page_shift, n_kv, kvh, 1);
     };
     auto fetch = [&](const float* src, int row, int quads, float* dst, int dst_ld, int base, int buf) {
-        const int n = min(ATT_THREADS, p - base + 1) * quads;
+        const int n = min(ATT_THREADS, p - base + (ROPE ? 0 : 1)) * quads;           // ROPE: the token's own is not there yet
         for (int e = tid; e < n; e += ATT_THREADS) {
             const int r = e / quads, c = e % quads * 4;
             gf_cp16(dst + r * dst_ld + c, src + tok_s[buf][r] * row + c, 16);
@@ -529,7 +552,34 @@ attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __res
     };
     look_up(lo, 0);
     const float* qp = q + (size_t)t * ldq + (size_t)h * head_dim;
-    if (tid < head_dim) q_s[tid] = qp[tid];
+    float own_k = 0.f, own_v = 0.f;                      // ROPE: an element of the token's key and value
+    if constexpr (ROPE) {
+        if (tid < head_dim) {
+            const float* row = q + (size_t)t * ldq;
+            const float* kp = row + (size_t)(n_q + kvh) * head_dim;
+            own_v = row[(size_t)(n_q + n_kv + kvh) * head_dim + tid];
+            float own_q = qp[tid];
+            own_k = kp[tid];
+            if (tid < rope.rotary_dim) {
+                const int half = rope.rotary_dim / 2, i = tid < half ? tid : tid - half;
+                const bool have = p < rope.table_positions;
+                const float c = have ? rope.cos_t[(size_t)p * half + i] : 1.f, sn = have ? rope.sin_t[(size_t)p * half + i] : 0.f;
+                float y1, y2;
+                rotate_pair(qp[i], qp[i + half], c, sn, y1, y2);
+                own_q = tid < half ? y1 : y2;
+                rotate_pair(kp[i], kp[i + half], c, sn, y1, y2);
+                own_k = tid < half ? y1 : y2;
+            }
+            q_s[tid] = own_q;
+            if (h % (n_q / n_kv) == 0) {
+                const size_t at = ssb_cache_row(page_table, max_pages, s, p, page_shift, n_kv, kvh, head_dim) + tid;
+                rope.k_cache[at] = own_k;
+                rope.v_cache[at] = own_v;
+            }
+        }
+    } else {
+        if (tid < head_dim) q_s[tid] = qp[tid];
+    }
     __syncthreads();
     fetch(k_cache, head_dim, kq, k_s, ld, lo, 0);
     float m = -INFINITY, l = 0.f, acc = 0.f;
@@ -537,6 +587,10 @@ attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __res
     for (int base = lo; base <= p; base += ATT_THREADS, buf ^= 1) {
         fetch(v_cache, v_row, vq, v_s, v_dim, base, buf);
         look_up(base + ATT_THREADS, buf ^ 1);
+        if (ROPE && p - base < ATT_THREADS && tid < head_dim) {
+            k_s[(p - base) * ld + tid] = own_k;
+            v_s[(p - base) * v_dim + tid] = own_v;
+        }
         gf_wait<1>();
         __syncthreads();                                 // the keys have landed
         float sc = -INFINITY;
@@ -601,6 +655,40 @@ attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __res
     if (tid < v_dim) o[tid] = l > 0.f ? acc * keep / l : 0.f;
 }
 
+static bool attention_staged_takes(const void* k_cache, const void* v_cache, int head_dim, int v_dim, int v_row) {
+    return head_dim <= AS_MAX_DIM && v_dim <= AS_MAX_DIM && !((head_dim | v_dim | v_row) & 3)
+        && !(((uintptr_t)k_cache | (uintptr_t)v_cache) & 15);
+}
+
+template <bool ROPE>
+static int attention_staged_launch(const float* q, int ldq, const float* k_cache, const float* v_cache, const int* pos, const int* slot,
+                                   const int* page_table, int max_pages, float* out, int ldo, int n_tokens, int n_q, int n_kv,
+                                   int head_dim, int page_shift, int window, float scale, int v_dim, int v_row, const float* sinks,
+                                   AsRope rope, bool pdl, cudaStream_t stream) {
+    const cudaError_t e = cudaFuncSetAttribute(attention_staged_kernel<ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)attention_staged_smem(AS_MAX_DIM, AS_MAX_DIM));
+    if (e != cudaSuccess) return (int)e;
+    const int rc = ssb_launch(attention_staged_kernel<ROPE>, dim3(n_tokens, n_q), dim3(ATT_THREADS), attention_staged_smem(head_dim, v_dim),
+                              stream, pdl, q, ldq, k_cache, v_cache, pos, slot, page_table, max_pages, out, ldo, n_q, n_kv, head_dim,
+                              page_shift, window, scale, v_dim, v_row, sinks, rope);
+    return rc ? rc : ssb_launch_status();
+}
+
+// A float32 decode step: rotation, append and attention of one token a sequence in one launch, the bits of ssb_rope_append and
+// ssb_attention_plain.  qkv: [q heads | k heads | v heads] a row, left as it is; rotary_dim even, up to head_dim.
+SSB_API int ssb_attention_f32_decode(const float* qkv, int ld, const float* cos_t, const float* sin_t, int table_positions,
+                                     int rotary_dim, float* k_cache, float* v_cache, const int* pos, const int* slot,
+                                     const int* page_table, int max_pages, float* out, int ldo, int n_tokens, int n_q, int n_kv,
+                                     int head_dim, int page_shift, int window, float scale, int pdl, cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (head_dim <= 0 || n_kv <= 0 || n_q % n_kv || n_q > 65535 || rotary_dim < 0 || rotary_dim % 2 || rotary_dim > head_dim
+        || (rotary_dim && (!cos_t || !sin_t)) || !attention_staged_takes(k_cache, v_cache, head_dim, head_dim, head_dim))
+        return SSB_ERR_BAD_SIZE;
+    const AsRope rope = {cos_t, sin_t, table_positions, rotary_dim, k_cache, v_cache};
+    return attention_staged_launch<true>(qkv, ld, k_cache, v_cache, pos, slot, page_table, max_pages, out, ldo, n_tokens, n_q, n_kv,
+                                         head_dim, page_shift, window, scale, head_dim, head_dim, nullptr, rope, pdl != 0, stream);
+}
+
 SSB_API int ssb_attention_plain(const void* q, int ldq, int dtype, const void* k_cache,
                                 const void* v_cache, const int* pos, const int* slot,
                                 const int* page_table, int max_pages, void* out, int ldo, int n_tokens,
@@ -613,17 +701,10 @@ SSB_API int ssb_attention_plain(const void* q, int ldq, int dtype, const void* k
     if (head_dim > ATT_MAX_HEAD_DIM || head_dim <= 0 || n_kv <= 0 || n_q % n_kv) return SSB_ERR_BAD_SIZE;
     if (v_dim <= 0 || v_dim > ATT_MAX_HEAD_DIM || v_row < v_dim) return SSB_ERR_BAD_SIZE;
     dim3 grid(n_tokens, n_q);
-    if (dtype == SSB_F32 && head_dim <= AS_MAX_DIM && v_dim <= AS_MAX_DIM && !((head_dim | v_dim | v_row) & 3)
-        && !(((uintptr_t)k_cache | (uintptr_t)v_cache) & 15)) {
-        const size_t smem = attention_staged_smem(head_dim, v_dim);
-        const cudaError_t e = cudaFuncSetAttribute(attention_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)attention_staged_smem(AS_MAX_DIM, AS_MAX_DIM));
-        if (e != cudaSuccess) return (int)e;
-        const int rc = ssb_launch(attention_staged_kernel, grid, dim3(ATT_THREADS), smem, stream, pdl != 0, (const float*)q, ldq,
-                                  (const float*)k_cache, (const float*)v_cache, pos, slot, page_table, max_pages, (float*)out, ldo,
-                                  n_q, n_kv, head_dim, page_shift, window, scale, v_dim, v_row, sinks);
-        return rc ? rc : ssb_launch_status();
-    }
+    if (dtype == SSB_F32 && attention_staged_takes(k_cache, v_cache, head_dim, v_dim, v_row))
+        return attention_staged_launch<false>((const float*)q, ldq, (const float*)k_cache, (const float*)v_cache, pos, slot,
+                                              page_table, max_pages, (float*)out, ldo, n_tokens, n_q, n_kv, head_dim, page_shift,
+                                              window, scale, v_dim, v_row, sinks, AsRope{}, pdl != 0, stream);
     if (dtype == SSB_F32)
         attention_plain_kernel<float><<<grid, ATT_THREADS, 0, stream>>>(
             (const float*)q, ldq, (const float*)k_cache, (const float*)v_cache, pos, slot, page_table,

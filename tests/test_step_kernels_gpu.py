@@ -84,6 +84,38 @@ def test_float32_attention_with_staged_keys_is_the_plain_kernels_bit_for_bit(hd,
     assert torch.equal(outs[0], outs[1]) and bool((outs[1][-1] == 0).all())
 
 
+@pytest.mark.parametrize("hd,rot,window", [(64, 64, 0), (128, 64, 0), (32, 32, 130), (20, 12, 0), (4, 0, 3), (128, 128, 128)])
+def test_float32_decode_attention_rotates_and_appends_the_same_bits(hd, rot, window):
+    """Against the two launches it stands in for: tokens at the edges of chunks and pages, one beyond the tables, one of no slot."""
+    n_q, n_kv, pos, slots = 6, 2, [0, 63, 64, 127, 128, 300, 5], [3, 0, 1, 2, 5, 4, -1]
+    table = torch.randperm(48, generator=torch.Generator().manual_seed(hd)).to(torch.int32)[:42].view(7, 6).to(DEV)
+    k, v = rnd(48, n_kv, 64, hd, seed=1), rnd(48, n_kv, 64, hd, seed=2)
+    cos, sin = rnd(290, rot // 2, seed=5), rnd(290, rot // 2, seed=6)
+    qkv = rnd(len(pos), (n_q + 2 * n_kv) * hd + 3, seed=3, scale=2.0)[:, : (n_q + 2 * n_kv) * hd]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    p, s, o = i32(pos), i32(slots), ops()
+    want_k, want_v, want_q, want = k.clone(), v.clone(), qkv.clone(), torch.empty(len(pos), n_q * hd, device=DEV)
+    o.rope_append(want_q, cos if rot else None, sin if rot else None, p, s, table, want_k, want_v, n_q, n_kv, hd, rot, 6)
+    o.attention_plain(want_q, want_k, want_v, p, s, table, want, n_q, n_kv, hd, 6, window or None, hd ** -0.5)
+    got, before = torch.full_like(want, 9.0), qkv.clone()
+    o.attention_f32_decode(qkv, cos, sin, k, v, p, s, table, got, n_q, n_kv, hd, rot, 6, window or None, hd ** -0.5)
+    assert torch.equal(got, want) and torch.equal(k, want_k) and torch.equal(v, want_v) and torch.equal(qkv, before)
+
+
+@pytest.mark.parametrize("m,inter,k", [(1, 5, 2052), (2, 2001, 520), (3, 901, 36), (4, 1000, 1028), (2, 8192, 2048), (1, 1801, 64)])
+@pytest.mark.parametrize("kind,limit", [("silu", 0.0), ("clamped_swish", 2.0), ("gelu_tanh", 0.0)])
+def test_float32_gated_products_are_the_two_launches_bit_for_bit(m, inter, k, kind, limit):
+    x, w, scale = rnd(m, k, seed=m), rnd(2 * inter, k, seed=inter, scale=0.1), rnd(m, seed=k)
+    if not ops().gemm_f32_gated_ok(x, w, torch.empty(m, inter, device=DEV)):
+        pytest.skip("another kernel makes this product")
+    both, want, got = torch.empty(m, 2 * inter, device=DEV), torch.empty(m, inter, device=DEV), torch.empty(m, inter, device=DEV)
+    for factor in (None, scale):
+        ops().gemm_nt_plain(x, w, both)
+        ops().gated_activation(both, want, kind, limit, row_scale=factor)
+        ops().gemm_f32_gated(x, w, got, kind, limit, factor)
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("hd,n_q,n_kv", [(64, 8, 2), (128, 6, 2), (128, 3, 3), (64, 12, 1)])
 def test_float32_prompt_attention_is_the_plain_kernels_bit_for_bit(hd, n_q, n_kv):
     """Prompts that continue a cache, of one token, of exactly a chunk of keys and a page; pages that belong to nobody are
