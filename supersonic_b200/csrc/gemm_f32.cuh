@@ -4,7 +4,7 @@
 // sums added in k order with compensation (Kahan).  Nothing here is re-associated, so a row's result does not depend on
 // which kernel took it, how many rows it came with or which tile it lay in.
 #pragma once
-#include "common.cuh"
+#include "packed_f32.cuh"
 
 static inline int gf_sms() {
     static int sms = 0;
@@ -371,27 +371,12 @@ gemm_f32_walk_kernel(const float* __restrict__ A, int lda, const float* __restri
 // 1000 rows, us on the general kernel and here: 2048 x 2048 504 and 291, 3072 x 2048 746 and 483, 16384 x 2048 3563 and 1794
 // (37.4 TFLOP/s), 2048 x 8192 2033 and 1145.
 // ---------------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long gf_twice(float x) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ unsigned long long gf_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ unsigned long long gf_add2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 // Two compensated additions; `kept` is what the last ones rounded away, with the sign it is added back with.
 __device__ __forceinline__ void gf_kahan2(unsigned long long& acc, unsigned long long& kept, unsigned long long part,
                                           unsigned long long minus_one) {
-    const unsigned long long y = gf_add2(part, kept);
-    const unsigned long long t = gf_add2(acc, y);
-    kept = gf_add2(y, gf_fma2(t, minus_one, acc));
+    const unsigned long long y = f2_add(part, kept);
+    const unsigned long long t = f2_add(acc, y);
+    kept = f2_add(y, f2_fma(t, minus_one, acc));
     acc = t;
 }
 
@@ -504,7 +489,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
 #pragma unroll
             for (int j = 0; j < RN / 2; ++j) { acc[i][j] = 0ull; kept[i][j] = 0ull; }
     }
-    const unsigned long long minus_one = gf_twice(-1.0f);
+    const unsigned long long minus_one = f2_twice(-1.0f);
 #pragma unroll
     for (int t = 0; t < GF_RAW - 1; ++t) {
         if (t < turns) fetch(t);
@@ -539,9 +524,9 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
             }
 #pragma unroll
             for (int i = 0; i < RM; ++i) {
-                const unsigned long long aa = gf_twice(a[i]);
+                const unsigned long long aa = f2_twice(a[i]);
 #pragma unroll
-                for (int j = 0; j < RN / 2; ++j) part[i][j] = gf_fma2(aa, w[j], part[i][j]);
+                for (int j = 0; j < RN / 2; ++j) part[i][j] = f2_fma(aa, w[j], part[i][j]);
             }
         }
         if constexpr (TMEM) {

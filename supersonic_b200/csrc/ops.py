@@ -743,8 +743,8 @@ def gated_linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z:
                       places: Optional[int] = None, form: int = 0) -> None:
     """Per sequence and head, over the sequence's new tokens in order:
     S = diag(sigmoid(z + z_bias)^(1/tau)) S + k v^T;  out = S^T (q * q_scale), with S [dim, vdim] float32 read
-    from and left in ``state[slot]``.  q, k (heads x dim) and v (heads x vdim) are columns of ``proj``; ``z`` is
-    overwritten with the decays.
+    from and left in ``state[slot]``.  q, k (heads x dim) and v (heads x vdim) are columns of ``proj``; ``z`` may
+    be overwritten with the decays.
     ``chunk`` > 0: every sequence's tokens are cut into chunks of that many that run in parallel (each chunk's
     own sum from zero, the state carried across the chunks in order, then the outputs of every chunk from the
     state at its start), through the float32 scratch ``sums`` (sequences x chunks x heads x dim x vdim) and

@@ -10,7 +10,7 @@
 // may be cut into chunks that run in parallel, which adds the same terms in another order: whether and
 // where is the caller's choice, by the step's sizes or, with one chunk length and min_new, by the
 // sequence's own length, so that its sums do not depend on what else is in the batch.
-#include "common.cuh"
+#include "packed_f32.cuh"
 #include <math.h>
 #include <type_traits>
 
@@ -73,20 +73,93 @@ gated_linear_carry_kernel(float* __restrict__ state, float* __restrict__ sums, c
     state[(size_t)slot * per + e] = cur;
 }
 
+// A token a sequence (a decode step): the state passes through once, row by row, and no lane owns a tile of it.  A block takes
+// COLS value columns of a head, four a lane; its warps share the rows, eight accesses in flight a lane, and the sums over the
+// rows meet in shared memory.  The decays are made here too.  (The walk loads a tile, then stores it, one block an SM: 64
+// sequences of 4 heads of 256 x 512, 268 MB of state in and out, took 112 us and a launch for the decays.)  A sequence may bring
+// several tokens (another none): it takes them one after another.
+template <typename T, int COLS>
+__global__ void __launch_bounds__(256)
+gated_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off, const float* __restrict__ z, int ldz,
+                  const float* __restrict__ z_bias, float inv_tau, float q_scale, float* __restrict__ state,
+                  const int* __restrict__ cu_new, const int* __restrict__ seq_slot, float* __restrict__ out, int ldo, int n_heads,
+                  int dim, int vdim) {
+    constexpr int LR = COLS / 4, RW = 32 / LR, PARTS = 8 * RW, DEEP = 8;         // lanes a row, rows of a warp's access
+    __shared__ float k_s[SCAN_MAX_DIM], q_s[SCAN_MAX_DIM], d_s[SCAN_MAX_DIM];
+    __shared__ __align__(16) float o_s[PARTS][COLS];
+    const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int part = warp * RW + lane / LR, at = lane % LR * 4, j = blockIdx.z * COLS + at;
+    ssb_pdl_launch_dependents();
+    ssb_pdl_wait();
+    const int slot = seq_slot[b];
+    if (slot < 0) return;                                  // padding row
+    float* S = state + ((size_t)slot * n_heads + h) * dim * vdim + j;
+    const bool mine = j < vdim;
+    const int t1 = cu_new[b + 1];
+    for (int t = cu_new[b]; t < t1; ++t) {
+        const T* row = proj + (size_t)t * ld;
+        float4 s[DEEP];
+        const int first = min(DEEP, (dim - part + PARTS - 1) / PARTS);           // of this lane's rows; the others come behind them
+#pragma unroll
+        for (int r = 0; r < DEEP; ++r)
+            if (r < first && mine) s[r] = *reinterpret_cast<const float4*>(S + (size_t)(part + r * PARTS) * vdim);
+        for (int i = tid; i < dim; i += 256) {
+            k_s[i] = ssb_to_float(row[k_off + h * dim + i]);
+            q_s[i] = ssb_to_float(row[q_off + h * dim + i]) * q_scale;
+            d_s[i] = expf(log_sigmoid(z[(size_t)t * ldz + h * dim + i] + z_bias[h * dim + i]) * inv_tau);
+        }
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f), o = v;
+        if (mine) {
+            const T* vp = row + v_off + (size_t)h * vdim + j;
+            v = make_float4(ssb_to_float(vp[0]), ssb_to_float(vp[1]), ssb_to_float(vp[2]), ssb_to_float(vp[3]));
+        }
+        __syncthreads();
+        if (mine) {
+            for (int i0 = part; i0 < dim; i0 += DEEP * PARTS) {
+                if (i0 != part) {
+#pragma unroll
+                    for (int r = 0; r < DEEP; ++r)
+                        if (i0 + r * PARTS < dim) s[r] = *reinterpret_cast<const float4*>(S + (size_t)(i0 + r * PARTS) * vdim);
+                }
+#pragma unroll
+                for (int r = 0; r < DEEP; ++r) {
+                    const int i = i0 + r * PARTS;
+                    if (i >= dim) break;
+                    const float k = k_s[i], q = q_s[i], d = d_s[i];
+                    const float4 x = make_float4(fmaf(d, s[r].x, k * v.x), fmaf(d, s[r].y, k * v.y), fmaf(d, s[r].z, k * v.z),
+                                                 fmaf(d, s[r].w, k * v.w));
+                    *reinterpret_cast<float4*>(S + (size_t)i * vdim) = x;
+                    o = make_float4(fmaf(x.x, q, o.x), fmaf(x.y, q, o.y), fmaf(x.z, q, o.z), fmaf(x.w, q, o.w));
+                }
+            }
+        }
+        *reinterpret_cast<float4*>(&o_s[part][at]) = o;
+        __syncthreads();
+        for (int c = tid; c < COLS; c += 256) {
+            float sum = 0.f;
+#pragma unroll
+            for (int p = 0; p < PARTS; ++p) sum += o_s[p][c];
+            if (blockIdx.z * COLS + c < vdim) out[(size_t)t * ldo + (size_t)h * vdim + blockIdx.z * COLS + c] = sum;
+        }
+        __syncthreads();
+    }
+}
+
 static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
                       float q_scale, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo, int n_seqs,
                       int n_heads, int dim, int vdim, int chunk, int max_chunks, int min_new, int places, int form, float* sums,
                       float* decays, bool pdl, cudaStream_t stream);
 
 // proj [T, ld] holds q, k (n_heads x dim each) and v (n_heads x vdim) from the given columns;
-// z [T, ldz] float32 is the decay's pre-activation without its bias z_bias [n_heads x dim], and is overwritten
+// z [T, ldz] float32 is the decay's pre-activation without its bias z_bias [n_heads x dim], and may be overwritten
 // with the decays;
 // state [slots, n_heads, dim, vdim] float32; out [T, ldo] float32 gets o (n_heads x vdim).
 // chunk > 0: sequences of min_new new tokens or more are run in chunks of that many tokens, in parallel, the others walked in
 // one go.  max_chunks = ceil(longest run of new tokens / chunk).  ``sums`` (places x n_heads x dim x vdim floats) and ``decays``
 // (places x n_heads x dim) hold so many (sequence, chunk) pairs at a time; with fewer than n_seqs x max_chunks the step
 // takes several passes, over sequences and over runs of chunks, and every sum is the same.  form: lanes that share a column's
-// rows, 1: 16, 2: 32 (dim above 64), 0: by the step's sizes; the sums over the rows differ in order.
+// rows, 1: the same for steps of any size (16, above 128 channels 32), 2: 32 (dim above 64), 3: a token at a time (whole runs, states in 16-byte pieces), 0: by the step's sizes; the
+// sums over the rows differ in order.
 SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off,
                                   float* z, int ldz, const float* z_bias, float tau, float q_scale,
                                   float* state, const int* cu_new, const int* seq_slot, float* out, int ldo,
@@ -94,12 +167,30 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
                                   int min_new, int places, int form, float* sums, float* decays, int pdl,
                                   cudaStream_t stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
-    if (dim <= 0 || dim > SCAN_MAX_DIM || vdim <= 0 || !(tau > 0.f) || form < 0 || form > 2) return SSB_ERR_BAD_SIZE;
+    if (dim <= 0 || dim > SCAN_MAX_DIM || vdim <= 0 || !(tau > 0.f) || form < 0 || form > 3) return SSB_ERR_BAD_SIZE;
     if (chunk < 0 || (chunk > 0 && (max_chunks <= 0 || places <= 0 || sums == nullptr || decays == nullptr))) return SSB_ERR_BAD_SIZE;
     const long long items = chunk > 0 ? (long long)n_seqs * max_chunks : n_seqs;
     if (items > 0x7fffffffll) return SSB_ERR_BAD_SIZE;
     if (n_heads > 65535 || (vdim + 31) / 32 > 65535 || n_seqs > 65535) return SSB_ERR_BAD_SIZE;
     if (dtype != SSB_F32 && dtype != SSB_BF16) return SSB_ERR_BAD_DTYPE;
+    const bool by_token = vdim % 4 == 0 && ((uintptr_t)state & 15) == 0 && chunk == 0;
+    if (form == 3 && !by_token) return SSB_ERR_BAD_SIZE;
+    if (by_token && (form == 3 || (form == 0 && n_tokens <= n_seqs))) {
+        // 128 columns a block where that gives the SMs two blocks each
+        const bool wide = (long long)n_seqs * n_heads * ((vdim + 127) / 128) >= 2 * 148;
+        const dim3 grid(n_seqs, n_heads, wide ? (vdim + 127) / 128 : (vdim + 31) / 32);
+#define SSB_GS(T, COLS)                                                                                                       \
+    do {                                                                                                                      \
+        const int st = ssb_launch(gated_step_kernel<T, COLS>, grid, dim3(256), 0, stream, pdl != 0, (const T*)proj, ld, q_off, k_off, \
+                                  v_off, (const float*)z, ldz, z_bias, 1.0f / tau, q_scale, state, cu_new, seq_slot, out, ldo, n_heads, \
+                                  dim, vdim);                                                                                 \
+        return st ? st : ssb_launch_status();                                                                                 \
+    } while (0)
+        if (dtype == SSB_F32) { if (wide) SSB_GS(float, 128); SSB_GS(float, 32); }
+        if (wide) SSB_GS(bf16, 128);
+        SSB_GS(bf16, 32);
+#undef SSB_GS
+    }
     const size_t total = (size_t)n_tokens * n_heads * dim;
     int rc = ssb_launch(decay_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, pdl != 0, z, ldz, z_bias,
                         1.0f / tau, n_heads * dim, total);
@@ -116,20 +207,21 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
 // rounding of 1 - f.
 //
 // A block takes one head of one sequence (or chunk of it) and up to 8 value columns a warp.  A lane owns a tile of the
-// state in registers, 4 columns by 4 R4 rows: sixteen lanes share four columns, so a token's k and q are read from
-// shared memory once for four columns, and the sums over rows are five shuffles for all four (the first two halve
-// the columns a lane still carries).  Eight tokens are staged per barrier, in two buffers, while the next eight are on
-// their way from memory.
+// state in registers, 4 columns by 4 rows and more, two rows a register pair: sixteen (or 32) lanes share four columns, so that a
+// token's k and q are read from shared memory once for four columns, and the multiply-adds go two rows an instruction
+// (packed_f32.cuh; each half rounds as the scalar one does).  Four tokens' sums over the lanes are taken together: of the 16
+// values a lane holds it hands on the half that the other keeps, four times, 15 shuffles where a token alone takes 5.  Eight
+// tokens are staged per barrier, in two buffers, while the next eight are on their way from memory.  4 heads of 256 x 512 and
+// 2,048 tokens 530 us in scalar multiply-adds and 5 shuffles a token, 455 so; 8 x 300 tokens 442 and 340.  Bound by what 8 to 16
+// warps an SM hide of the shared-memory reads (FMA pipe 36 %, issue slots 34 %).
 //   OUT = false: chunk sums, from zero, with the product of the chunk's decays;
 //   OUT = true: outputs from the state at the start (the slot's, or what the carry kernel left for the chunk).
 // GATED: the gated linear attention at the top of this file on the same tiles, S <- a S + k v with decays that a kernel before
-// this one made, o = S^T (q_scale q).  (A kernel of its own, a column a thread with the sums through shared memory, took 1,011 us
-// for 4 heads of 256 x 512 and 2,048 tokens where this takes 518, 412 us for 128 x 256 where this takes 133, and 128 us for one
-// token of 64 sequences where this takes 112.)
+// this one made, o = S^T (q_scale q).
 // norm_w given (one block holds all of the head's columns): the head norm is taken where the outputs meet in shared
 // memory, y = o / rms(o) * norm_w, a warp a token; else o itself goes out in float32.
 // =======================================================================================
-constexpr int TW_TOKENS = 8;
+constexpr int TW_TOKENS = 8, TW_GROUP = 4;                  // tokens staged together, and summed over lanes together
 
 // The written share 1 - f, from the gate's pre-activation (bias included) and the lower bound.
 __device__ __forceinline__ float tied_share(float z, float lower) { return (1.0f - lower) / (1.0f + expf(z)); }
@@ -147,7 +239,7 @@ struct TiedArgs {
 };
 
 template <typename T, int R4, int NT, bool OUT, bool GATED, int RL>      // RL: lanes that share a column's rows, 16 or 32
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, RL == 32 ? 2 : NT == 256 && R4 == 1 ? 3 : 1)
 tied_walk_kernel(const TiedArgs a) {
     constexpr int DIMP = 64 * R4, WCOLS = 128 / RL, COLS = NT / 32 * WCOLS;  // padded rows; columns of a warp, of a block
     constexpr int RG = DIMP / (4 * RL);                    // groups of four rows a lane
@@ -179,25 +271,31 @@ tied_walk_kernel(const TiedArgs a) {
                    : a.state + ((size_t)slot * a.n_heads + h) * dim * vdim;
     const int col0 = warp * WCOLS + cg * 4;                    // this lane's four columns, within the block's
     const bool pieces = vdim % 4 == 0 && ((uintptr_t)S & 15) == 0;       // a lane's four columns in one access
-    float s[RG][4][4];
+    unsigned long long s[RG][2][4];                            // two rows each, of four columns
 #pragma unroll
     for (int g = 0; g < RG; ++g)
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int i = (g * RL + rg) * 4 + r, j = j0 + col0;
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (OUT && i < dim && j < vdim) {
-                const float* src = S + (size_t)i * vdim + j;
-                if (pieces) x = *reinterpret_cast<const float4*>(src);
-                else x = make_float4(src[0], j + 1 < vdim ? src[1] : 0.f, j + 2 < vdim ? src[2] : 0.f, j + 3 < vdim ? src[3] : 0.f);
+        for (int r = 0; r < 2; ++r) {
+            float4 x[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int i = (g * RL + rg) * 4 + 2 * r + e, j = j0 + col0;
+                x[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (OUT && i < dim && j < vdim) {
+                    const float* src = S + (size_t)i * vdim + j;
+                    if (pieces) x[e] = *reinterpret_cast<const float4*>(src);
+                    else x[e] = make_float4(src[0], j + 1 < vdim ? src[1] : 0.f, j + 2 < vdim ? src[2] : 0.f, j + 3 < vdim ? src[3] : 0.f);
+                }
             }
-            s[g][r][0] = x.x; s[g][r][1] = x.y; s[g][r][2] = x.z; s[g][r][3] = x.w;
+            s[g][r][0] = f2_pair(x[0].x, x[1].x); s[g][r][1] = f2_pair(x[0].y, x[1].y);
+            s[g][r][2] = f2_pair(x[0].z, x[1].z); s[g][r][3] = f2_pair(x[0].w, x[1].w);
         }
-    float prod[RG][4];
+    unsigned long long prod[RG][2];
 #pragma unroll
     for (int g = 0; g < RG; ++g)
 #pragma unroll
-        for (int r = 0; r < 4; ++r) prod[g][r] = 1.f;
+        for (int r = 0; r < 2; ++r) prod[g][r] = f2_twice(1.f);
+    const unsigned long long minus_one = f2_twice(-1.f), one = f2_twice(1.f);
     // this thread's channels among the staged items are the same in every turn: DIMP divides NT or is divided by it
     float bias[KI], low[KI];
 #pragma unroll
@@ -270,44 +368,63 @@ tied_walk_kernel(const TiedArgs a) {
         if (OUT && t > t0) finish(t - TW_TOKENS, buf ^ 1);
         if (j0 + warp * WCOLS < vdim) {
             const int n_tok = min(TW_TOKENS, t1 - t);
-#pragma unroll 2
-            for (int tt = 0; tt < n_tok; ++tt) {
-                const float4 v4 = *reinterpret_cast<const float4*>(vb + tt * COLS + col0);
-                const float v[4] = {v4.x, v4.y, v4.z, v4.w};
-                float o[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int tt = 0; tt < n_tok; tt += TW_GROUP) {
+                unsigned long long o[TW_GROUP][4];         // of a group's tokens: the sums over even and over odd rows
 #pragma unroll
-                for (int g = 0; g < RG; ++g) {
-                    const float4 k4 = *reinterpret_cast<const float4*>(kb + tt * DIMP + (g * RL + rg) * 4);
-                    const float k[4] = {k4.x, k4.y, k4.z, k4.w};
-                    float q[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {1.f, 1.f, 1.f, 1.f};
-                    if (GATED) {
-                        const float4 d4 = *reinterpret_cast<const float4*>(d_s + (buf * TW_TOKENS + tt) * DIMP + (g * RL + rg) * 4);
-                        d[0] = d4.x; d[1] = d4.y; d[2] = d4.z; d[3] = d4.w;
-                    }
-                    if (OUT) {
-                        const float4 q4 = *reinterpret_cast<const float4*>(qb + tt * DIMP + (g * RL + rg) * 4);
-                        q[0] = q4.x; q[1] = q4.y; q[2] = q4.z; q[3] = q4.w;
-                    }
+                for (int u = 0; u < TW_GROUP; ++u)
 #pragma unroll
-                    for (int r = 0; r < 4; ++r) {
+                    for (int c = 0; c < 4; ++c) o[u][c] = 0ull;
+                auto token = [&](int u) {
+                    const float4 v4 = *reinterpret_cast<const float4*>(vb + (tt + u) * COLS + col0);
+                    const unsigned long long v[4] = {f2_twice(v4.x), f2_twice(v4.y), f2_twice(v4.z), f2_twice(v4.w)};
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            s[g][r][c] = GATED ? fmaf(d[r], s[g][r][c], k[r] * v[c]) : fmaf(k[r], v[c] - s[g][r][c], s[g][r][c]);
-                            if (OUT) o[c] = fmaf(s[g][r][c], q[r], o[c]);
+                    for (int g = 0; g < RG; ++g) {
+                        const int at = (tt + u) * DIMP + (g * RL + rg) * 4;
+                        const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(kb + at);
+                        ulonglong2 q = make_ulonglong2(0ull, 0ull), d = make_ulonglong2(one, one);
+                        if (GATED) d = *reinterpret_cast<const ulonglong2*>(d_s + buf * TW_TOKENS * DIMP + at);
+                        if (OUT) q = *reinterpret_cast<const ulonglong2*>(qb + at);
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            const unsigned long long kr = r ? k.y : k.x, dr = r ? d.y : d.x, qr = r ? q.y : q.x;
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) {
+                                s[g][r][c] = GATED ? f2_fma(dr, s[g][r][c], f2_mul(kr, v[c]))
+                                                   : f2_fma(kr, f2_fma(s[g][r][c], minus_one, v[c]), s[g][r][c]);
+                                if (OUT) o[u][c] = f2_fma(s[g][r][c], qr, o[u][c]);
+                            }
+                            if (!OUT && warp == 0) prod[g][r] = f2_mul(prod[g][r], GATED ? dr : f2_fma(kr, minus_one, one));
                         }
-                        if (!OUT && warp == 0) prod[g][r] *= GATED ? d[r] : 1.0f - k[r];
                     }
+                };
+                if (n_tok - tt >= TW_GROUP) {
+#pragma unroll
+                    for (int u = 0; u < TW_GROUP; ++u) token(u);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < TW_GROUP; ++u)
+                        if (u < n_tok - tt) token(u);
                 }
                 if (OUT) {
-                    // sums over the lanes of a column group; a lane ends with one of the four columns
-                    constexpr int H2 = RL / 2, H1 = RL / 4;
-                    const bool hi2 = (lane & H2) != 0, hi1 = (lane & H1) != 0;
-                    const float p0 = (hi2 ? o[2] : o[0]) + __shfl_xor_sync(0xffffffffu, hi2 ? o[0] : o[2], H2);
-                    const float p1 = (hi2 ? o[3] : o[1]) + __shfl_xor_sync(0xffffffffu, hi2 ? o[1] : o[3], H2);
-                    float p = (hi1 ? p1 : p0) + __shfl_xor_sync(0xffffffffu, hi1 ? p0 : p1, H1);
+                    // sums over the lanes of a column group: of the 16 values (token of the group, column) a lane holds, it hands
+                    // on the half that the other lane keeps, four times
+                    float w[4 * TW_GROUP];
 #pragma unroll
-                    for (int m = H1 / 2; m > 0; m >>= 1) p += __shfl_xor_sync(0xffffffffu, p, m);
-                    if ((lane & (H1 - 1)) == 0) ob[tt * COLS + col0 + (hi2 ? 2 : 0) + (hi1 ? 1 : 0)] = p;
+                    for (int u = 0; u < TW_GROUP; ++u)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) w[u * 4 + c] = f2_lo(o[u][c]) + f2_hi(o[u][c]);
+#pragma unroll
+                    for (int half = 2 * TW_GROUP, m = RL / 2; half > 0; half >>= 1, m >>= 1) {
+                        const bool hi = (lane & m) != 0;
+#pragma unroll
+                        for (int i = 0; i < half; ++i) {
+                            const float got = __shfl_xor_sync(0xffffffffu, hi ? w[i] : w[i + half], m);
+                            w[i] = (hi ? w[i + half] : w[i]) + got;
+                        }
+                    }
+                    if (RL == 32) w[0] += __shfl_xor_sync(0xffffffffu, w[0], 1);
+                    const int mine = rg / (RL / 16);       // token of the group, column
+                    if (rg % (RL / 16) == 0) ob[(tt + mine / 4) * COLS + col0 + mine % 4] = w[0];
                 }
             }
         }
@@ -323,18 +440,21 @@ tied_walk_kernel(const TiedArgs a) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int i = (g * RL + rg) * 4 + r, j = j0 + col0;
+            float x[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x[c] = r % 2 ? f2_hi(s[g][r / 2][c]) : f2_lo(s[g][r / 2][c]);
             if (i < dim && j < vdim) {
                 float* dst = S + (size_t)i * vdim + j;
                 if (pieces) {
-                    *reinterpret_cast<float4*>(dst) = make_float4(s[g][r][0], s[g][r][1], s[g][r][2], s[g][r][3]);
+                    *reinterpret_cast<float4*>(dst) = make_float4(x[0], x[1], x[2], x[3]);
                 } else {
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
-                        if (j + c < vdim) dst[c] = s[g][r][c];
+                        if (j + c < vdim) dst[c] = x[c];
                 }
             }
             if (!OUT && blockIdx.z == 0 && warp == 0 && cg == 0 && i < dim)
-                a.decays[((size_t)blockIdx.x * a.n_heads + h) * dim + i] = prod[g][r];
+                a.decays[((size_t)blockIdx.x * a.n_heads + h) * dim + i] = r % 2 ? f2_hi(prod[g][r / 2]) : f2_lo(prod[g][r / 2]);
         }
 }
 
@@ -387,11 +507,10 @@ static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
     return 0;
 }
 
-// Blocks of 64 columns up to which a column's rows are shared by 32 lanes instead of 16, with 32 columns a block: half the work a
-// warp and token, on twice the SMs.  us with 16 and 32 lanes (and in the kernel of a column a thread that was here before): 4
-// heads of 128 x 256, one sequence, 1 token 7.5 and 6.1 (6.2), 20 15.0 and 10.9 (12.3), 100 64 and 35 (40); 4 of 256 x 512, 1 token
-// 9.6 and 7.5 (6.1), 20 22.5 and 17.1 (15.7), 100 77 and 55 (56).  With more blocks it only adds shuffles: 8 sequences of 256 x
-// 512, 1 token 16.4 and 17.1.
+// Blocks of 64 columns up to which a column's rows are shared by 32 lanes instead of 16, with 32 columns a block, where a head has
+// up to 128 channels: half the work a warp and token, on twice the SMs.  us with 16 and 32 lanes, 4 heads of 128 x 256, one
+// sequence, 100 tokens 49 and 41, 8 of 300 111 and 120.  Above 128 channels 32 lanes always, two blocks an SM (126 registers a thread
+// instead of 245): 4 heads of 256 x 512, 100 tokens 73 and 56, 2,048 452 and 460, 64 sequences of 2 tokens 179 and 140.
 constexpr int GATED_FEW_BLOCKS = 74;
 
 static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
@@ -403,13 +522,12 @@ static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off,
     a.state = state; a.cu_new = cu_new; a.seq_slot = seq_slot; a.out = out; a.ldo = ldo; a.n_heads = n_heads; a.dim = dim;
     a.vdim = vdim; a.chunk = chunk; a.max_chunks = max_chunks; a.min_new = min_new; a.places = places; a.sums = sums; a.decays = decays;
     const long long blocks = (chunk > 0 ? (long long)n_seqs * max_chunks : n_seqs) * n_heads * ((vdim + 63) / 64);
-    const bool narrow = form == 2 || (form == 0 && blocks <= GATED_FEW_BLOCKS);
+    const bool narrow = form == 2 || (form != 1 && blocks <= GATED_FEW_BLOCKS);
 #define SSB_GW(T) \
     return dim <= 64 ? launch_tied_walk<T, 1, 256, true>(a, n_seqs, pdl, stream) \
          : dim <= 128 ? (narrow ? launch_tied_walk<T, 2, 256, true, 32>(a, n_seqs, pdl, stream) \
                                 : launch_tied_walk<T, 2, 256, true>(a, n_seqs, pdl, stream)) \
-                      : (narrow ? launch_tied_walk<T, 4, 256, true, 32>(a, n_seqs, pdl, stream) \
-                                : launch_tied_walk<T, 4, 256, true>(a, n_seqs, pdl, stream))
+                      : launch_tied_walk<T, 4, 256, true, 32>(a, n_seqs, pdl, stream)
     if (dtype == SSB_F32) SSB_GW(float);
     SSB_GW(bf16);
 #undef SSB_GW

@@ -281,7 +281,8 @@ def test_gated_scan_in_register_tiles(H, d, dv):
             want[t] = torch.einsum("hdv,hd->hv", S, q[t]) * 0.25
         end[slot] = S
         at += n
-    for chunk, form in ((0, 0), (24, 0), (64, 0), (0, 1), (24, 1)) + (((0, 2), (24, 2), (64, 2)) if d > 64 else ()):
+    for chunk, form in ((0, 0), (24, 0), (64, 0), (0, 1), (24, 1)) + (((0, 2), (24, 2), (64, 2)) if d > 64 else ()) + \
+            (((0, 3),) if dv % 4 == 0 else ()):
         n = -(-max(lens) // chunk) if chunk else 0
         sums = torch.empty(max(B * n * H * d * dv, 1), device=DEV)
         decays = torch.empty(max(B * n * H * d, 1), device=DEV)
@@ -290,6 +291,24 @@ def test_gated_scan_in_register_tiles(H, d, dv):
                                 max_new=max(lens), sums=sums if chunk else None, decays=decays if chunk else None, form=form)
         assert float((out.double() - want.view(T, -1)).norm() / want.norm()) < 2e-6, chunk
         assert float((state.double().view(-1) - end.view(-1)).norm() / end.norm()) < 2e-6, chunk
+
+
+@pytest.mark.parametrize("B,H,d,dv", [(3, 2, 256, 512), (80, 4, 100, 132), (1, 3, 33, 4), (75, 1, 256, 260)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gated_scan_of_one_token_a_sequence(B, H, d, dv, dtype):
+    """A decode step by rows of the state, in narrow and in wide blocks, a padding row among them, against the walk."""
+    proj, z0, bias = rnd(B, 2 * H * d + H * dv, seed=d, dtype=dtype), rnd(B, H * d, seed=1), rnd(H * d, seed=2) + 1.0
+    cu = torch.arange(B + 1, dtype=torch.int32, device=DEV)
+    slots = torch.randperm(B + 1, generator=torch.Generator().manual_seed(B)).to(torch.int32)[:B].to(DEV)
+    if B > 1:
+        slots[B // 2] = -1
+    state0, got = rnd(B + 1, H * d * dv, seed=3), []
+    for form in (1, 0):
+        state, out = state0.clone(), torch.zeros(B, H * dv, device=DEV)
+        ops().gated_linear_scan(proj, 0, H * d, 2 * H * d, z0.clone(), bias, 16.0, 0.25, state, cu, slots, out, H, d, dv, form=form)
+        got.append((out, state))
+    assert torch.equal(got[0][1], got[1][1])                       # a state's element is one product and one multiply-add
+    assert float((got[0][0] - got[1][0]).norm() / got[0][0].norm()) < 1e-6       # sums of d float32 products in another order
 
 
 def step_of(lens, slots):
