@@ -26,6 +26,11 @@ constexpr int GV_BM = 128;                // rows of W per block
 // stages of the ring: as many as let two blocks share an SM (no second wave for 149..296 blocks):
 // 18 KB a stage at up to 16 batch rows, 20 KB at 32, 24 KB at 64, 32 KB at 128
 __host__ __device__ constexpr int gv_stages(int bnb) { return bnb <= 16 ? 6 : (bnb <= 32 ? 5 : (bnb <= 64 ? 4 : 3)); }
+// ... and of a launch of no more blocks than SMs, one part of K each, where a second block an SM would only be the next
+// kernel's: us a decode step with two blocks' worth and with these, 1B, 40 rows 1,013 and 993, 64 977 and 961, 100 1,254 and
+// 1,225; 3B, 64 rows 2,264 and 2,233, 128 2,977 and 2,887.  Fewer rows lose more at the start of the next kernel (20 rows 815 and
+// 836 with nine stages).
+__host__ __device__ constexpr int gv_deep(int bnb) { return bnb <= 32 ? gv_stages(bnb) : bnb <= 64 ? 6 : 5; }
 constexpr int GV_MAX_ROWS = 128;
 constexpr unsigned GV_ROT = 5;            // k-blocks by which neighbouring row tiles start apart (see the producer)
 // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5: epilogue; from 64 batch rows on warps 6-9 too, which take the second
@@ -36,12 +41,11 @@ constexpr unsigned GV_ROT = 5;            // k-blocks by which neighbouring row 
 __host__ __device__ constexpr int gv_groups(int bnb) { return bnb >= 64 ? 2 : 1; }
 __host__ __device__ constexpr int gv_threads(int bnb) { return 64 + 128 * gv_groups(bnb); }
 
-template <int BNB>                        // batch rows per tile: 16, 32, 64 or 128
+template <int BNB, int GV_STAGES>         // batch rows per tile: 16, 32, 64 or 128; stages of the ring
 __global__ void __launch_bounds__(gv_threads(BNB), 2)
 gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                void* __restrict__ out, int ldo, int out_is_f32, int n_rows, int N, int K, int mode, int splits,
                float* __restrict__ partials, int* __restrict__ counters, int* __restrict__ error_word, int gate_kind, float gate_limit, const float* __restrict__ row_scale) {
-    constexpr int GV_STAGES = gv_stages(BNB);
     constexpr uint32_t W_BYTES = GV_BM * TC_BK * 2, X_BYTES = BNB * TC_BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
     constexpr int TMEM_COLS = BNB < 32 ? 32 : BNB;
     extern __shared__ unsigned char smem_raw[];
@@ -215,27 +219,33 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     own_sums(c0);
                 }
                 if (mode == TC_SWIGLU) {
-                    // rows come as [8 gate | 8 up] per 16: the up value of gate row r sits 8 lanes further
+                    // rows come as [8 gate | 8 up] per 16: a column's up value sits 8 lanes behind its gate value.  The two
+                    // lanes share the columns: the gate lane takes the even ones, the up lane the odd ones, each with what
+                    // the other hands it
                     const bool is_gate = (r & 15) < 8;
-                    const int n_out = n0 / 2 + (r >> 4) * 8 + (r & 7);
-                    // sixteen columns at a time, each step for all of them before the next: shuffle,
-                    // activation and store of one column are a chain of dependent instructions, and taken
-                    // column by column the 64 columns of a full tile took 9 us
+                    const int n_out = n0 / 2 + (r >> 4) * 8 + (r & 7), mine = is_gate ? 0 : 1;
+                    const bool in = n0 + (r & ~15) + 16 <= N;
+                    // eight columns at a time, each step for all of them before the next (shuffle, activation and store of
+                    // one column are a chain of dependent instructions), and none beyond the batch's last row.  Every
+                    // column of a tile by the gate lanes alone: a decode step of the 1B model 651 us at 1 row, 710 at 8, 856
+                    // at 32, 972 at 64
 #pragma unroll
-                    for (int j0 = 0; j0 < CW; j0 += 16) {
-                        float up[16], act[16];
+                    for (int j0 = 0; j0 < CW; j0 += 8) {
+                        if (c0 + j0 >= n_rows) break;
+                        float act[4];
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) up[j] = __shfl_down_sync(0xffffffffu, v[j0 + j], 8);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            act[j] = ssb_gate_fast(v[j0 + j], up[j], gate_kind, gate_limit);
-                            if (row_scale != nullptr && c0 + j0 + j < n_rows) act[j] *= row_scale[c0 + j0 + j];
+                        for (int j = 0; j < 4; ++j) {
+                            const float even = v[j0 + 2 * j], odd = v[j0 + 2 * j + 1];
+                            const float got = __shfl_xor_sync(0xffffffffu, is_gate ? odd : even, 8);
+                            act[j] = ssb_gate_fast(is_gate ? even : got, is_gate ? got : odd, gate_kind, gate_limit);
                         }
-                        if (is_gate && n + 8 < N) {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (c0 + j0 + j < n_rows)
-                                    ((bf16*)out)[(size_t)(c0 + j0 + j) * ldo + n_out] = __float2bfloat16_rn(act[j]);
+                        for (int j = 0; j < 4; ++j) {
+                            const int c = c0 + j0 + 2 * j + mine;
+                            if (in && c < n_rows) {
+                                if (row_scale != nullptr) act[j] *= row_scale[c];
+                                ((bf16*)out)[(size_t)c * ldo + n_out] = __float2bfloat16_rn(act[j]);
+                            }
                         }
                     }
                 } else if (n < N) {
@@ -260,13 +270,12 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
 }
 
-template <int BNB>
-static int launch_gv(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo, int out_is_f32, int n_rows,
+template <int BNB, int GV_STAGES>
+static int launch_gv_ring(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo, int out_is_f32, int n_rows,
                      int N, int K, int mode, int splits, float* partials, int* counters, int* error_word, bool pdl,
                      cudaStream_t stream, int gate_kind = 0, float gate_limit = 0.f, const float* row_scale = nullptr) {
-    constexpr int GV_STAGES = gv_stages(BNB);
     constexpr size_t smem = GV_STAGES * (GV_BM + BNB) * TC_BK * 2 + (2 * GV_STAGES + 1) * 8 + 32 + 1024;
-    auto kern = gemv_tc_kernel<BNB>;
+    auto kern = gemv_tc_kernel<BNB, GV_STAGES>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -277,6 +286,18 @@ static int launch_gv(const CUtensorMap& mw, const CUtensorMap& mx, void* out, in
                               out, ldo, out_is_f32, n_rows, N, K, mode, splits, partials, counters, error_word, gate_kind, gate_limit,
                               row_scale);
     return rc ? rc : ssb_launch_status();
+}
+
+template <int BNB>
+static int launch_gv(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo, int out_is_f32, int n_rows,
+                     int N, int K, int mode, int splits, float* partials, int* counters, int* error_word, bool pdl,
+                     cudaStream_t stream, int gate_kind = 0, float gate_limit = 0.f, const float* row_scale = nullptr) {
+    if constexpr (gv_deep(BNB) > gv_stages(BNB))
+        if (splits == 1 && (N + GV_BM - 1) / GV_BM <= 148 && K > 2 * gv_deep(BNB) * TC_BK)
+            return launch_gv_ring<BNB, gv_deep(BNB)>(mw, mx, out, ldo, out_is_f32, n_rows, N, K, mode, splits, partials, counters,
+                                                     error_word, pdl, stream, gate_kind, gate_limit, row_scale);
+    return launch_gv_ring<BNB, gv_stages(BNB)>(mw, mx, out, ldo, out_is_f32, n_rows, N, K, mode, splits, partials, counters,
+                                               error_word, pdl, stream, gate_kind, gate_limit, row_scale);
 }
 
 static inline int gv_bnb(int n_rows) { return n_rows <= 16 ? 16 : (n_rows <= 32 ? 32 : (n_rows <= 64 ? 64 : 128)); }
