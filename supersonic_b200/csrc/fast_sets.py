@@ -103,6 +103,8 @@ class FastKernels(PlainKernels):
                 # whatever else is in the step (decode steps pay for it: few blocks stream the weights)
                 ops.gemm_tc(x, weight, out, ops.TC_ACCUMULATE if accumulate else ops.TC_STORE,
                             tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else self._tile_n(rows, n), pdl=self._prompt_chain(rows))
+            elif not accumulate and ops.gemv_rows_tile(rows, n, k):
+                ops.gemv_rows(x, weight, out, ops.gemv_rows_tile(rows, n, k), pdl=self.pdl)
             elif rows <= STREAM_ROWS and accumulate:
                 # weights on the M side, K split over blocks that add with float atomics
                 ops.gemv_tc(x, weight, out, ops.TC_ACCUMULATE, splits=ops.gemv_tc_splits(n, k), pdl=self.pdl)
@@ -152,6 +154,8 @@ class FastKernels(PlainKernels):
         if self.deterministic:
             ops.gemm_tc_act(xt, weight, out, kind, scale,
                             tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else self._tile_n(rows, n))
+        elif ops.gemv_rows_tile(rows, n, k):
+            ops.gemv_rows(xt, weight, out, ops.gemv_rows_tile(rows, n, k), act=kind, scale=scale, pdl=self.pdl)
         elif rows <= STREAM_ROWS and n < 16384:
             sums = self._buffer("split_sums", rows * n, torch.float32, out.device, zero=True)[: rows * n].view(rows, n)
             ops.gemv_tc(xt, weight, sums, ops.TC_ACCUMULATE, splits=ops.gemv_tc_splits(n, k), pdl=self.pdl)

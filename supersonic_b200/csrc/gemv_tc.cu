@@ -300,6 +300,191 @@ static int launch_gv(const CUtensorMap& mw, const CUtensorMap& mx, void* out, in
                                                error_word, pdl, stream, gate_kind, gate_limit, row_scale);
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// Up to 16 rows and so few columns that tiles of 128 rows of W would fill a part of the SMs: tiles of 16, 32 or 64 rows that
+// take all of K, so that a result is finished where it is made.  (K cut over blocks of 128 rows adds float32 sums atomically into
+// a scratch that another launch rounds and clears.)  The products are mma.sync here: a tcgen05.mma takes some 70 clocks for 128
+// rows of W, used or not, and all of K is 128 of them for 2,048 columns (a decode step of the 1B model 10 % longer).  Warps
+// share a stage's k-blocks, and its 16-row pieces of W, and their sums meet in shared memory.  Bound by a launch's chain (x's
+// trip from L2, the products, the meeting, the store), as the small launches around it.  us a decode step with K cut and rounded,
+// and so: 1B, 4 and 8 rows 656 and 629, 682 and 656; 8B, 8 rows 2,857 and 2,820; Ronelorn 2,048 wide, 8 rows 202 and 193; Vufadra
+// 1,024 wide, 8 rows 203 and 180.  Sums added into the residual stay cut: a block streams too little of W at a time for the long
+// ones (1B, 8 rows 656 and 694).
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int GR_WARPS = 8, GR_THREADS = 32 * GR_WARPS + 32;  // the last warp feeds TMA
+constexpr int GR_ROWS = 16;                                   // rows of x
+__host__ __device__ constexpr int gr_kbs(int tm) { return 128 / tm; }                    // k-blocks a stage: a warp each, and 16 rows
+__host__ __device__ constexpr int gr_stages(int tm) { return tm == 16 ? 3 : 4; }
+__host__ __device__ constexpr uint32_t gr_stage_bytes(int tm) { return gr_kbs(tm) * (tm + GR_ROWS) * 128; }
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %4}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(z) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const CUtensorMap* map, uint32_t bar, int y, int z, uint64_t policy) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(y), "r"(z), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void gr_ldmatrix(uint32_t at, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void gr_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int TM>
+__global__ void __launch_bounds__(GR_THREADS, 2)
+gemv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, void* __restrict__ out, int ldo,
+                 int out_is_f32, int n_rows, int N, int K, int act, float scale, int* __restrict__ error_word) {
+    constexpr int KBS = gr_kbs(TM), STAGES = gr_stages(TM);
+    constexpr uint32_t STAGE_BYTES = gr_stage_bytes(TM), X_AT = KBS * TM * 128;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ float sums[GR_WARPS][GR_ROWS][17];                // of a warp: [row of x][row of W]
+    __shared__ uint64_t bars[2 * STAGES];
+    __shared__ volatile int abort_flag[2];                       // [0]: a role gave up; [1]: stays zero
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n0 = blockIdx.x * TM;
+    const int steps = (K / TC_BK + KBS - 1) / KBS;
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
+    if (tid == 32 * GR_WARPS) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, GR_WARPS); }
+        abort_flag[0] = 0;
+        abort_flag[1] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    ssb_pdl_launch_dependents();
+    __syncthreads();
+
+    if (warp == GR_WARPS) {
+        if (lane == 0) {
+            // as in gemv_tc_kernel: the ring's first weights before the dependency wait, blocks start at different places
+            const int rot = (int)(blockIdx.x % (unsigned)steps);
+            auto kb_of = [&](int i) { const int j = i + rot; return (j >= steps ? j - steps : j) * KBS; };
+            const uint64_t w_policy = ssb_policy_evict_first();
+            const int pre = min(steps, STAGES);
+            for (int i = 0; i < pre; ++i) {
+                mbar_expect_tx(full0 + 8 * i, STAGE_BYTES);
+                tma_load_3d_hint(smem_u32(smem + i * STAGE_BYTES), &map_w, full0 + 8 * i, n0, kb_of(i), w_policy);
+            }
+            ssb_pdl_wait();
+            for (int i = 0; i < pre; ++i) tma_load_3d(smem_u32(smem + i * STAGE_BYTES) + X_AT, &map_x, full0 + 8 * i, kb_of(i));
+            int issued = pre;
+            for (int i = pre; i < steps; ++i) {
+                const int s = i % STAGES;
+                if (!mbar_wait(empty0 + 8 * s, ((i / STAGES) & 1) ^ 1, abort_flag)) {
+                    *abort_flag = 1; atomicCAS(error_word, 0, TC_ERR_PRODUCER); break;
+                }
+                const uint32_t dst = smem_u32(smem + s * STAGE_BYTES);
+                mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+                tma_load_3d_hint(dst, &map_w, full0 + 8 * s, n0, kb_of(i), w_policy);
+                tma_load_3d(dst + X_AT, &map_x, full0 + 8 * s, kb_of(i));
+                issued = i + 1;
+            }
+            if (*abort_flag)
+                for (int i = max(0, issued - STAGES); i < issued; ++i)
+                    mbar_wait(full0 + 8 * (i % STAGES), (i / STAGES) & 1, abort_flag + 1);
+        }
+    } else {
+        // this warp's k-block of a stage and 16 rows of W; lanes' rows and 16-byte pieces (exchanged by the 128-byte swizzle)
+        const int kb = warp % KBS, piece = warp / KBS;
+        const int w_row = lane & 15, w_half = lane >> 4, x_row = (lane & 7) + (lane >> 4) * 8, x_half = (lane >> 3) & 1;
+        const bool wide = n_rows > 8;
+        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        for (int i = 0; i < steps; ++i) {
+            const int s = i % STAGES;
+            if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (i / STAGES) & 1, abort_flag))) {
+                if (lane == 0) { *abort_flag = 1; atomicCAS(error_word, 0, TC_ERR_MMA); }
+                break;
+            }
+            const uint32_t w_at = smem_u32(smem + s * STAGE_BYTES) + (kb * TM + piece * 16 + w_row) * 128;
+            const uint32_t x_at = smem_u32(smem + s * STAGE_BYTES) + X_AT + (kb * GR_ROWS + x_row) * 128;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {                        // k-blocks behind the last are zeros
+                uint32_t a[4], b[4];
+                gr_ldmatrix(w_at + (((2 * k + w_half) ^ (w_row & 7)) << 4), a);
+                gr_ldmatrix(x_at + (((2 * k + x_half) ^ (x_row & 7)) << 4), b);
+                gr_mma(acc[0], a, b[0], b[1]);
+                if (wide) gr_mma(acc[1], a, b[2], b[3]);
+            }
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty0 + 8 * s) : "memory");
+        }
+        const int r = lane >> 2, c = (lane & 3) * 2;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            sums[warp][h * 8 + c][r] = acc[h][0]; sums[warp][h * 8 + c + 1][r] = acc[h][1];
+            sums[warp][h * 8 + c][r + 8] = acc[h][2]; sums[warp][h * 8 + c + 1][r + 8] = acc[h][3];
+        }
+    }
+    __syncthreads();
+    if (warp == GR_WARPS || abort_flag[0]) return;
+    ssb_pdl_wait();                                              // out may still be the predecessor's
+    for (int e = tid; e < TM * n_rows; e += 32 * GR_WARPS) {
+        const int j = e / TM, r = e % TM, n = n0 + r;
+        if (n >= N) continue;
+        float x = 0.f;
+#pragma unroll
+        for (int k = 0; k < KBS; ++k) x += sums[r / 16 * KBS + k][j][r % 16];
+        const size_t o = (size_t)j * ldo + n;
+        if (act >= 0) x = ssb_activate(x, act) * scale;
+        if (out_is_f32) ((float*)out)[o] = x;
+        else ((bf16*)out)[o] = __float2bfloat16_rn(x);
+    }
+}
+
+// rows x K bfloat16 as (64 columns, rows, k-blocks): a box is box_rows rows of kbs k-blocks, each a tile of 128-byte rows
+static int gr_map(CUtensorMap* map, const void* base, int rows, int K, int ld, int box_rows, int kbs) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return SSB_ERR_UNSUPPORTED;
+    cuuint64_t dims[3] = {TC_BK, (cuuint64_t)rows, (cuuint64_t)(K / TC_BK)}, strides[2] = {(cuuint64_t)ld * 2, TC_BK * 2};
+    cuuint32_t box[3] = {TC_BK, (cuuint32_t)box_rows, (cuuint32_t)kbs}, elem[3] = {1, 1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : SSB_ERR_BAD_SIZE;
+}
+
+template <int TM>
+static int launch_gr(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, int out_is_f32, int n_rows, int N, int K, int act,
+                     float scale, int* error_word, bool pdl, cudaStream_t stream) {
+    constexpr size_t smem = gr_stages(TM) * gr_stage_bytes(TM) + 1024;
+    static_assert(smem + GR_WARPS * GR_ROWS * 17 * 4 + 128 <= 113 * 1024, "two blocks an SM");
+    auto kern = gemv_rows_kernel<TM>;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    CUtensorMap mw, mx;
+    int rc = gr_map(&mw, W, N, K, ldw, TM, gr_kbs(TM));
+    if (rc) return rc;
+    rc = gr_map(&mx, x, n_rows, K, ldx, GR_ROWS, gr_kbs(TM));
+    if (rc) return rc;
+    rc = ssb_launch(kern, dim3((N + TM - 1) / TM), dim3(GR_THREADS), smem, stream, pdl, mw, mx, out, ldo, out_is_f32, n_rows, N, K, act,
+                    scale, error_word);
+    return rc ? rc : ssb_launch_status();
+}
+
+// x: bfloat16 [n_rows <= 16, K], K in whole k-blocks of 64; W: bfloat16 [N, K].  act: -1 none, else activation act times scale.
+// tm: rows of W a block, 16, 32 or 64.
+SSB_API int ssb_gemv_rows(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, int out_dtype, int n_rows, int N, int K,
+                          int act, float scale, int tm, int* error_word, int pdl, cudaStream_t stream) {
+    if (n_rows <= 0 || N <= 0) return 0;
+    if (n_rows > GR_ROWS || K <= 0 || K % TC_BK || ldx % 8 || ldw % 8 || !error_word || N > 0x7fffff00) return SSB_ERR_BAD_SIZE;
+    if (((uintptr_t)x | (uintptr_t)W) & 15) return SSB_ERR_BAD_SIZE;
+    if (act < -1 || act > SSB_ACT_SILU) return SSB_ERR_BAD_SIZE;
+    if (out_dtype != SSB_F32 && out_dtype != SSB_BF16) return SSB_ERR_BAD_DTYPE;
+    const int f32o = out_dtype == SSB_F32;
+    if (tm == 16) return launch_gr<16>(x, ldx, W, ldw, out, ldo, f32o, n_rows, N, K, act, scale, error_word, pdl != 0, stream);
+    if (tm == 32) return launch_gr<32>(x, ldx, W, ldw, out, ldo, f32o, n_rows, N, K, act, scale, error_word, pdl != 0, stream);
+    if (tm == 64) return launch_gr<64>(x, ldx, W, ldw, out, ldo, f32o, n_rows, N, K, act, scale, error_word, pdl != 0, stream);
+    return SSB_ERR_BAD_SIZE;
+}
+
 static inline int gv_bnb(int n_rows) { return n_rows <= 16 ? 16 : (n_rows <= 32 ? 32 : (n_rows <= 64 ? 64 : 128)); }
 SSB_API int ssb_gemv_tc_max_rows() { return GV_MAX_ROWS; }
 

@@ -2467,6 +2467,35 @@ def gemv_tc_gate(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act=None, 
         _stream()), "gemv_tc_gate")
 
 
+GEMV_ROWS_MAX = 16
+
+
+def gemv_rows_tile(rows: int, n: int, k: int) -> int:
+    """Rows of W a block of :func:`gemv_rows` takes (0: not its sizes): as few as still make at most three blocks for two SMs.
+    us a decode step with up to 1, 1.5, 2 and 3 blocks an SM: 8B, 1 row 2,732, 2,648, 2,656, 2,759; 3B, 2 rows 1,500, 1,448, 1,446,
+    1,500; 1B, 8 rows 658, 656, 656, 655."""
+    if rows > GEMV_ROWS_MAX or k % 64:
+        return 0
+    return next((tm for tm in (16, 32, 64) if -(-n // tm) * 2 <= 3 * sm_count()), 0)
+
+
+def gemv_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile: int, act: Optional[str] = None, scale: float = 1.0,
+              pdl: bool = False) -> None:
+    """out = x @ w^T (or its activation, times ``scale``) for up to 16 rows, K in whole k-blocks of 64: tiles of ``tile`` (16, 32
+    or 64) rows of ``w`` that take all of K, so that no sum meets another."""
+    _need(x, "x", torch.bfloat16, 2); _need(w, "w", torch.bfloat16, 2); _need(out, "out", None, 2)
+    B, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K or tuple(out.shape) != (B, N) or (act is not None and act not in ACTIVATIONS):
+        raise KernelError(f"gemv_rows: shapes x{tuple(x.shape)} w{tuple(w.shape)} out{tuple(out.shape)}, activation {act!r}")
+    global _tc_unchecked
+    _tc_unchecked += 1
+    _check(_fn("gemv_tc", "ssb_gemv_rows")(
+        _ptr(x), c_int(x.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(out), c_int(out.stride(0)), c_int(dtype_code(out.dtype)),
+        c_int(B), c_int(N), c_int(K), c_int(-1 if act is None else ACTIVATIONS[act]), c_float(scale), c_int(tile),
+        _ptr(tc_error_word(x.device)), c_int(1 if pdl else 0), _stream()), "gemv_rows")
+
+
 # ---- vector element-wise kernels ------------------------------------------------------------------
 def rmsnorm_vec_ok(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> bool:
     return (out.dtype == torch.bfloat16 and x.dtype == torch.float32 and x.shape[1] % 4 == 0

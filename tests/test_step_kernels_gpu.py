@@ -230,6 +230,26 @@ def test_latent_attention_of_prompts_ends_with_its_last_sums():
         assert bool(torch.isfinite(first).all())
 
 
+@pytest.mark.parametrize("rows,n,k", [(1, 16, 64), (1, 3072, 2048), (7, 200, 448), (16, 33, 64), (16, 4736, 576), (3, 8200, 1088), (2, 1000, 8192),
+                                      (9, 12000, 192)])
+@pytest.mark.parametrize("tile", [16, 32, 64])
+def test_products_of_few_rows_in_narrow_tiles(rows, n, k, tile):
+    """Tiles of W that are not whole, stages whose last k-blocks do not exist, rows beyond the step's that must stay as they are:
+    float32 sums of bfloat16 products, 1e-5 of the result's norm, and one rounding where they are stored."""
+    x, w = rnd(rows, k, seed=rows, dtype=torch.bfloat16), rnd(n, k, seed=n, scale=0.05, dtype=torch.bfloat16)
+    x = torch.cat([x, torch.full((rows, 8), math.nan, dtype=torch.bfloat16, device=DEV)], dim=1)[:, :k]        # rows 16 bytes apart
+    want = x.double() @ w.double().T
+    o = ops()
+    got = torch.full((rows + 1, n), 3.0, device=DEV)
+    o.gemv_rows(x, w, got[:rows], tile)
+    assert float((got[:rows] - want).norm() / want.norm()) < 1e-5 and bool((got[rows] == 3.0).all())
+    got = torch.empty(rows, n + 8, dtype=torch.bfloat16, device=DEV)[:, :n]
+    o.gemv_rows(x, w, got, tile, act="relu_squared", scale=0.5)
+    ref = (0.5 * want.clamp(min=0) ** 2)
+    assert float((got.double() - ref).norm() / ref.norm()) < 2.0 ** -8          # half a unit in the last of eight bits, at most
+    o.check_device_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("top_k", [1, 5, 40, 64])
 @pytest.mark.parametrize("top_p,vocab", [(1.0, 70001), (0.9, 70001), (0.6, 70001), (0.0, 70001), (0.9, 50), (1.0, 65), (0.6, 4096), (0.9, 400000)])
 def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top_k, top_p, vocab):
