@@ -363,13 +363,12 @@ gemm_f32_walk_kernel(const float* __restrict__ A, int lda, const float* __restri
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Many rows (a prompt): tiles of 64 x 64 to 128 x 128, 4 x 4 to 8 x 8 results a thread, one chunk of k a turn.  A chunk comes
-// by cp.async as it lies in memory, GF_RAW deep, and is turned k-major in shared memory on the way to its two buffers, so that
-// a thread reads four neighbouring columns at a time and the multiply-adds go two columns an instruction (fma.rn.f32x2: each
-// half rounds as the scalar one does).  Bound by the FP32 pipes: a chunk's 16 multiply-adds of a result are followed by the
-// four steps of its compensated addition, so 4/5 of the peak is what this sum leaves.
-// 1000 rows, us on the general kernel and here: 2048 x 2048 504 and 291, 3072 x 2048 746 and 483, 16384 x 2048 3563 and 1794
-// (37.4 TFLOP/s), 2048 x 8192 2033 and 1145.
+// A few hundred rows, or few columns: tiles of 64 x 64 and 128 x 64, 4 x 4 and 8 x 4 results a thread, one chunk of k a turn, two or
+// three blocks an SM.  A chunk comes by cp.async as it lies in memory, GF_RAW deep, and is turned k-major in shared memory on the
+// way to its two buffers, so that a thread reads four neighbouring columns at a time and the multiply-adds go two columns an
+// instruction (fma.rn.f32x2: each half rounds as the scalar one does).  Bound by the FP32 pipes and the shared-memory reads beside
+// them: a chunk's 16 multiply-adds of a result are followed by the four steps of its compensated addition, so 4/5 of the peak
+// is what this sum leaves.  500 rows by 2048 x 2048, us on the general kernel and here: 257 and 181.
 // ---------------------------------------------------------------------------------------------------------------------
 // Two compensated additions; `kept` is what the last ones rounded away, with the sign it is added back with.
 __device__ __forceinline__ void gf_kahan2(unsigned long long& acc, unsigned long long& kept, unsigned long long part,
@@ -380,35 +379,12 @@ __device__ __forceinline__ void gf_kahan2(unsigned long long& acc, unsigned long
     acc = t;
 }
 
-// Sixteen words a lane of tensor memory, which a warp may also use as storage of its own lanes.
-__device__ __forceinline__ unsigned long long gf_pair(uint32_t lo, uint32_t hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ void gf_tld16(uint32_t at, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(at) : "memory");
-}
-// Every load issued so far has arrived; the registers of one of them are not read before.
-__device__ __forceinline__ void gf_tld_wait(uint32_t (&r)[16]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[i]));
-}
-__device__ __forceinline__ void gf_tst16(uint32_t at, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-                   "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(at) : "memory");
-}
-
 constexpr int GF_TILE_THREADS = 256, GF_RAW = 3;                     // GF_RAW: chunks on their way from memory, and at work
 
 template <int RM, int RN>
 constexpr size_t gf_tile_smem() { return sizeof(float) * (size_t)(2 + GF_RAW) * GF_CHUNK * 16 * (RM + RN); }
 
-template <int RM, int RN, int MIN_BLOCKS, bool TMEM = false>          // results a thread; tiles of 16 RM x 16 RN
+template <int RM, int RN, int MIN_BLOCKS>                // results a thread; tiles of 16 RM x 16 RN
 __global__ void __launch_bounds__(GF_TILE_THREADS, MIN_BLOCKS)
 gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C,
                      int ldc, int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int accumulate) {
@@ -460,35 +436,11 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
             dst[0] = x.x; dst[TN] = x.y; dst[2 * TN] = x.z; dst[3 * TN] = x.w;
         }
     };
-    constexpr int RES = RM * RN;
     unsigned long long acc[RM][RN / 2], kept[RM][RN / 2];             // two columns each
-    // TMEM: the running sums and what their additions rounded away, RES columns each of this warp's lanes of tensor memory; a
-    // thread then fits in 128 registers, and two blocks an SM
-    __shared__ uint32_t tmem_slot;
-    uint32_t t_acc = 0, t_kept = 0;
-    if constexpr (TMEM) {
-        if (warp == 0) {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                         ::"r"((uint32_t)__cvta_generic_to_shared(&tmem_slot)), "r"(4 * RES) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        t_acc = tmem_slot + ((uint32_t)(warp % 4 * 32) << 16) + warp / 4 * 2 * RES;
-        t_kept = t_acc + RES;
-        uint32_t zero[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) zero[i] = 0u;
+    for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int c = 0; c < 2 * RES; c += 16) gf_tst16(t_acc + c, zero);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-    } else {
-#pragma unroll
-        for (int i = 0; i < RM; ++i)
-#pragma unroll
-            for (int j = 0; j < RN / 2; ++j) { acc[i][j] = 0ull; kept[i][j] = 0ull; }
-    }
+        for (int j = 0; j < RN / 2; ++j) { acc[i][j] = 0ull; kept[i][j] = 0ull; }
     const unsigned long long minus_one = f2_twice(-1.0f);
 #pragma unroll
     for (int t = 0; t < GF_RAW - 1; ++t) {
@@ -529,51 +481,13 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
                 for (int j = 0; j < RN / 2; ++j) part[i][j] = f2_fma(aa, w[j], part[i][j]);
             }
         }
-        if constexpr (TMEM) {
 #pragma unroll
-            for (int c = 0; c < RES; c += 16) {
-                uint32_t x[16], y[16];
-                gf_tld16(t_acc + c, x);
-                gf_tld16(t_kept + c, y);
-                gf_tld_wait(x);
-                gf_tld_wait(y);
+        for (int i = 0; i < RM; ++i)
 #pragma unroll
-                for (int e = 0; e < 16; e += 2) {
-                    const int at = (c + e) / 2;
-                    unsigned long long sum = gf_pair(x[e], x[e + 1]), lost = gf_pair(y[e], y[e + 1]);
-                    gf_kahan2(sum, lost, part[at / (RN / 2)][at % (RN / 2)], minus_one);
-                    x[e] = (uint32_t)sum; x[e + 1] = (uint32_t)(sum >> 32);
-                    y[e] = (uint32_t)lost; y[e + 1] = (uint32_t)(lost >> 32);
-                }
-                gf_tst16(t_acc + c, x);
-                gf_tst16(t_kept + c, y);
-            }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        } else {
-#pragma unroll
-            for (int i = 0; i < RM; ++i)
-#pragma unroll
-                for (int j = 0; j < RN / 2; ++j) gf_kahan2(acc[i][j], kept[i][j], part[i][j], minus_one);
-        }
+            for (int j = 0; j < RN / 2; ++j) gf_kahan2(acc[i][j], kept[i][j], part[i][j], minus_one);
         gf_wait<GF_RAW - 2>();
         if (turn + 1 < turns) stage(turn + 1);
         __syncthreads();
-    }
-    if constexpr (TMEM) {
-#pragma unroll
-        for (int c = 0; c < RES; c += 16) {
-            uint32_t x[16];
-            gf_tld16(t_acc + c, x);
-            gf_tld_wait(x);
-#pragma unroll
-            for (int e = 0; e < 16; e += 2) acc[(c + e) / 2 / (RN / 2)][(c + e) / 2 % (RN / 2)] = gf_pair(x[e], x[e + 1]);
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (warp == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(4 * RES) : "memory");
-        }
     }
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
@@ -591,6 +505,145 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
+// Many rows, tiles of 128 x 128, one block an SM that walks its share of them.  Warps have roles: eight do nothing but multiply and
+// add, 8 x 8 results a thread in registers, and four others keep a ring of turns of 32 k ahead of them, k-major in shared memory.
+// Rows come as they lie, 128 bytes of one at a time, and are turned by scalar stores whose column is exchanged by the quarter
+// of k they belong to, so that neither the stores nor the reads meet on a bank.  Hardware barriers by number say when a turn is full
+// and when it is free; nothing waits in a loop.  Bound by the FP32 pipe: a chunk's 640 multiply-adds and compensated additions of a
+// warp in packed pairs take 2560 clocks an SM, 3200 are spent (a ninth of them in the meeting a turn).  With the same warps fetching,
+// turning and multiplying by turns: 1000 rows, 2048 x 2048 288 us and 217 here, 3072 x 2048 435 (64 x 64 tiles) and 430, 16384 x 2048
+// 1777 (two blocks an SM, their sums in tensor memory) and 1491, 45 TFLOP/s; 2048 x 8192 1142 and 850.  Turns of 64 k: 265 for the first.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int GF_ROLE_COMPUTE = 256, GF_ROLE_FETCH = 128, GF_ROLE_ALL = GF_ROLE_COMPUTE + GF_ROLE_FETCH, GF_ROLE_STAGES = 4, GF_ROLE_K = 32;
+template <int RM, int RN>
+constexpr size_t gf_role_smem() { return sizeof(float) * (size_t)GF_ROLE_STAGES * GF_ROLE_K * 16 * (RM + RN); }
+
+template <int RM, int RN>
+__global__ void __launch_bounds__(GF_ROLE_ALL, 1)
+gemm_f32_role_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
+                     int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int accumulate) {
+    constexpr int TM = 16 * RM, TN = 16 * RN, STAGES = GF_ROLE_STAGES, TK = GF_ROLE_K, STAGE = TK * (TM + TN);
+    constexpr int BAR_FULL = 1, BAR_FREE = 1 + STAGES;
+    extern __shared__ __align__(16) float gf_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    A += (size_t)blockIdx.z * a_batch;
+    W += (size_t)blockIdx.z * w_batch;
+    C += (size_t)blockIdx.z * c_batch;
+    const int m_tiles = (M + TM - 1) / TM, tiles = m_tiles * ((N + TN - 1) / TN), turns = (K + TK - 1) / TK;
+    if (warp >= GF_ROLE_COMPUTE / 32) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");        // 4 x 32 x 40 + 8 x 32 x 232 = 384 x 168, what the block has
+        const int f = tid - GF_ROLE_COMPUTE, q = f % 8, r0 = f / 8;      // 16 bytes of a row's 128; rows r0, r0 + 16, ...
+        int turn_no = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            const int m0 = tile % m_tiles * TM, n0 = tile / m_tiles * TN;
+            for (int turn = 0; turn < turns; ++turn, ++turn_no) {
+                const int s = turn_no % STAGES, k = turn * TK + q * 4;
+                float* a_s = gf_smem + s * STAGE;                        // [k][TM]
+                float* w_s = a_s + TK * TM;                              // [k][TN]
+                float4 x[TM / 16];
+#pragma unroll
+                for (int i = 0; i < TM / 16; ++i) {
+                    const int m = m0 + r0 + 16 * i;
+                    x[i] = m < M && k < K ? *reinterpret_cast<const float4*>(A + (size_t)m * lda + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                if (turn_no >= STAGES) gf_bar_sync(BAR_FREE + s, GF_ROLE_ALL);
+#pragma unroll
+                for (int i = 0; i < TM / 16; ++i) {
+                    float* dst = a_s + q * 4 * TM + ((r0 + 16 * i) ^ (q * 4));
+                    dst[0] = x[i].x; dst[TM] = x[i].y; dst[2 * TM] = x[i].z; dst[3 * TM] = x[i].w;
+                }
+                float4 y[TN / 16];
+#pragma unroll
+                for (int i = 0; i < TN / 16; ++i) {
+                    const int n = n0 + r0 + 16 * i;
+                    y[i] = n < N && k < K ? *reinterpret_cast<const float4*>(W + (size_t)n * ldw + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int i = 0; i < TN / 16; ++i) {
+                    float* dst = w_s + q * 4 * TN + ((r0 + 16 * i) ^ (q * 4));
+                    dst[0] = y[i].x; dst[TN] = y[i].y; dst[2 * TN] = y[i].z; dst[3 * TN] = y[i].w;
+                }
+                gf_bar_arrive(BAR_FULL + s, GF_ROLE_ALL);
+            }
+        }
+        return;
+    }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    const int tx = lane % 8 + 8 * (warp % 2), ty = lane / 8 + 4 * (warp / 2);    // columns 4 tx .. + 3 (and + 64); rows likewise
+    const unsigned long long minus_one = f2_twice(-1.0f);
+    const int all_turns = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * turns;
+    int turn_no = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int m0 = tile % m_tiles * TM, n0 = tile / m_tiles * TN;
+        unsigned long long acc[RM][RN / 2], kept[RM][RN / 2];            // two columns each
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN / 2; ++j) { acc[i][j] = 0ull; kept[i][j] = 0ull; }
+        for (int turn = 0; turn < turns; ++turn, ++turn_no) {
+            const int s = turn_no % STAGES;
+            const float* a_s = gf_smem + s * STAGE;
+            const float* w_s = a_s + TK * TM;
+            gf_bar_sync(BAR_FULL + s, GF_ROLE_ALL);
+#pragma unroll
+            for (int half = 0; half < TK / GF_CHUNK; ++half) {
+                if (turn * TK + half * GF_CHUNK >= K) break;
+                unsigned long long part[RM][RN / 2];
+#pragma unroll
+                for (int i = 0; i < RM; ++i)
+#pragma unroll
+                    for (int j = 0; j < RN / 2; ++j) part[i][j] = 0ull;
+#pragma unroll
+                for (int k4 = 0; k4 < GF_CHUNK / 4; ++k4) {
+                    const int swap = (half * 4 + k4) * 4;
+                    const float* ab = a_s + (half * GF_CHUNK + k4 * 4) * TM + ((4 * ty) ^ swap);
+                    const float* wb = w_s + (half * GF_CHUNK + k4 * 4) * TN + ((4 * tx) ^ swap);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        float a[RM];
+                        unsigned long long w[RN / 2];
+#pragma unroll
+                        for (int g = 0; g < RM / 4; ++g) {
+                            const float4 x = *reinterpret_cast<const float4*>(ab + k * TM + 64 * g);
+                            a[4 * g] = x.x; a[4 * g + 1] = x.y; a[4 * g + 2] = x.z; a[4 * g + 3] = x.w;
+                        }
+#pragma unroll
+                        for (int g = 0; g < RN / 4; ++g) {
+                            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(wb + k * TN + 64 * g);
+                            w[2 * g] = x.x; w[2 * g + 1] = x.y;
+                        }
+#pragma unroll
+                        for (int i = 0; i < RM; ++i) {
+                            const unsigned long long aa = f2_twice(a[i]);
+#pragma unroll
+                            for (int j = 0; j < RN / 2; ++j) part[i][j] = f2_fma(aa, w[j], part[i][j]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < RM; ++i)
+#pragma unroll
+                    for (int j = 0; j < RN / 2; ++j) gf_kahan2(acc[i][j], kept[i][j], part[i][j], minus_one);
+            }
+            if (turn_no + STAGES < all_turns) gf_bar_arrive(BAR_FREE + s, GF_ROLE_ALL);
+        }
+#pragma unroll
+        for (int i = 0; i < RM; ++i) {
+            const int m = m0 + 64 * (i / 4) + 4 * ty + i % 4;
+            if (m >= M) continue;
+#pragma unroll
+            for (int j = 0; j < RN / 2; ++j) {
+                const int n = n0 + 64 * (j / 2) + 4 * tx + 2 * (j % 2);
+                float* dst = C + (size_t)m * ldc + n;
+                const float lo = f2_lo(acc[i][j]), hi = f2_hi(acc[i][j]);
+                if (n < N) dst[0] = accumulate ? dst[0] + lo : lo;
+                if (n + 1 < N) dst[1] = accumulate ? dst[1] + hi : hi;
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
 // Whether the operands can be fetched in 16-byte pieces (rows of W and A start on 16-byte boundaries, K in whole pieces).
 static inline bool gemm_f32_ok(const void* A, int lda, long long a_batch, const void* W, int ldw, long long w_batch, int K) {
     return !(((uintptr_t)A | (uintptr_t)W) & 15) && !((lda | ldw | K) & 3) && !((a_batch | w_batch) & 3);
@@ -600,11 +653,10 @@ static inline bool gemm_f32_ok(const void* A, int lda, long long a_batch, const 
 // is done first by the time a chunk of 16 k takes it: the blocks run in waves over the SMs, and tiles that are too large leave
 // SMs idle where tiles that are too small fetch more often than they multiply.  Hundredths of a microsecond a chunk, measured
 // for 1 and for each further wave: up to 4, 8 and 16 rows x 16 columns a block 5 to 3 + 3.8, 5 and 10, whole turns of 32 chunks
-// whatever K is; tiles of 64 x 64 90 + 60, of 128 x 64 145 + 115, of 128 x 128 224 + 224, with the sums in tensor memory 233 +
-// 200, and 3 us to start and end.  A walking warp's turn: 4 rows of W 65, 70 and 85 (1, 2, 4 rows of A), 2 rows 80, 1 row 130,
+// whatever K is; tiles of 64 x 64 90 + 60, of 128 x 64 145 + 115, of 128 x 128 167 + 167, and 3 us to start and end.  A walking warp's turn: 4 rows of W 65, 70 and 85 (1, 2, 4 rows of A), 2 rows 80, 1 row 130,
 // and 3 us.  Sides of the lines it draws (us; rows x columns, k 2048): 128 x 2048 89 with 16 rows and 116 with tiles of 64; 100
-// x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072 186 with 128 x 64, 192 with 64 x 64; 1000 x 2048 291 with 128 x
-// 128, 299 with the sums in tensor memory, 321 with 128 x 64; 1000 x 16384 2003, 1794 and 2148.  K 64: 300 x 64 5.3 with 16
+// x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072 182 with 128 x 64, 189 with 64 x 64, 217 with 128 x 128; 500 x 3072
+// 217 with 128 x 128, 266 with 64 x 64; 500 x 2048 181 with 128 x 64, 217; 1000 x 2048 217 and 318.  K 64: 300 x 64 5.3 with 16
 // rows, 6.5 with tiles of 64, 700 x 64 8.2 and 6.6; 16 x 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.
 static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
     const long long sms = gf_sms(), chunks = (K + 15) / 16, turns = (K + 511) / 512;
@@ -614,17 +666,16 @@ static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
     const bool walk = gf_walk_ok(M, K);
     const int rows = M <= 4 ? 4 : M <= 8 ? 8 : 16;
     const int first = rows < 16 ? 50 : 30, each = rows == 4 ? 38 : rows == 8 ? 50 : 100;
-    const int forms[5] = {walk ? (M <= 2 ? M : 4) : M <= 4 ? 5 : rows, 100, 101, 102, 103};
-    long long cost[5] = {32 * turns * (first + each * waves(rows, 16)), 3000 + 10 * chunks * (30 + 60 * waves(64, 64)),
-                         3000 + 10 * chunks * (30 + 115 * waves(128, 64)), 3000 + 10 * chunks * 224 * waves(128, 128),
-                         3000 + 10 * chunks * (33 + 200 * waves(128, 128))};
+    const int forms[4] = {walk ? (M <= 2 ? M : 4) : M <= 4 ? 5 : rows, 100, 101, 102};
+    long long cost[4] = {32 * turns * (first + each * waves(rows, 16)), 3000 + 10 * chunks * (30 + 60 * waves(64, 64)),
+                         3000 + 10 * chunks * (30 + 115 * waves(128, 64)), 3000 + 10 * chunks * 167 * waves(128, 128)};
     if (walk) {
         const int width = gf_walk_width(N), turn = width == 1 ? 1300 : width == 2 ? 800 : M <= 1 ? 650 : M <= 2 ? 700 : 850;
         const long long held = sms * GF_WALK_WARPS, rounds = ((long long)((N + width - 1) / width) * n_batch + held - 1) / held;
         cost[0] = 3000 + ((K + GF_WALK_TURN / width - 1) / (GF_WALK_TURN / width)) * rounds * turn;
     }
     int best = 0;
-    for (int f = 1; f < 5; ++f)
+    for (int f = 1; f < 4; ++f)
         if (cost[f] < cost[best]) best = f;
     return forms[best];
 }
@@ -632,8 +683,8 @@ static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
 // Whether a gated unit's first product is made by walking warps, which finish it.
 static inline bool gemm_f32_gated_ok(int M, int N, int K) { return N % 2 == 0 && gemm_f32_form(1, M, N, K) <= 4; }
 
-// form 0: chosen by the sizes; else one of the kernels: 1, 2, 4 (a warp walks), 5, 8, 16 (few rows, 4, 8, 16 a group), 100, 101, 102, 103 (tiles
-// of 64 x 64, 128 x 64 and twice 128 x 128, the last with its sums in tensor memory)
+// form 0: chosen by the sizes; else one of the kernels: 1, 2, 4 (a warp walks), 5, 8, 16 (few rows, 4, 8, 16 a group), 100, 101, 102 (tiles of
+// 64 x 64, 128 x 64 and 128 x 128)
 static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, const float* W, int ldw, long long w_batch,
                                   float* C, int ldc, long long c_batch, int n_batch, int M, int N, int K, int accumulate,
                                   int form, cudaStream_t stream, bool pdl = false, const GfGate* gate = nullptr) {
@@ -682,6 +733,15 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         if (gate) { if (width == 4) GF_WALK(MB, 4, true); else GF_WALK(MB, 2, true); } \
         else if (width == 4) GF_WALK(MB, 4); else if (width == 2) GF_WALK(MB, 2); else GF_WALK(MB, 1); \
     } while (0)
+#define GF_ROLES(RM, RN) do { \
+        constexpr size_t smem = gf_role_smem<RM, RN>(); \
+        auto kernel = gemm_f32_role_kernel<RM, RN>; \
+        GF_CONFIGURE(kernel, smem); \
+        const long long tiles = (long long)((N + 16 * RN - 1) / (16 * RN)) * ((M + 16 * RM - 1) / (16 * RM)); \
+        if (tiles > 0x7fffffffLL) return SSB_ERR_BAD_SIZE; \
+        kernel<<<dim3((unsigned)(tiles < gf_sms() ? tiles : gf_sms()), 1, n_batch), GF_ROLE_ALL, smem, stream>>>( \
+            A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
+    } while (0)
     switch (form) {
         case 1: GF_WALKS(1); break;
         case 2: GF_WALKS(2); break;
@@ -691,13 +751,13 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         case 16: GF_SKINNY(16, 2, 2); break;
         case 100: GF_TILES(4, 4, 3); break;
         case 101: GF_TILES(8, 4, 2); break;
-        case 102: GF_TILES(8, 8, 1); break;
-        case 103: GF_TILES(8, 8, 2, true); break;
+        case 102: GF_ROLES(8, 8); break;
         default: return SSB_ERR_BAD_SIZE;
     }
 #undef GF_SKINNY
 #undef GF_WALK
 #undef GF_WALKS
+#undef GF_ROLES
 #undef GF_TILES
 #undef GF_CONFIGURE
     return ssb_launch_status();

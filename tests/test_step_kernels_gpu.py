@@ -34,7 +34,8 @@ def off_by_one(t):
                                    (9, 200, 2048), (16, 64, 1028), (17, 100, 520), (33, 257, 300), (65, 130, 36), (129, 127, 44),
                                    (300, 2500, 516), (257, 129, 64), (64, 3, 4), (1000, 129, 12), (1000, 16400, 36),
                                    (1, 30001, 32), (1, 2500, 1028), (8, 2500, 516), (3, 9000, 1028), (7, 33000, 36), (16, 2500, 1028), (13, 8200, 516), (2, 5000, 2052),
-                                   (2, 2500, 1028), (4, 2501, 516), (4, 9001, 2052), (4, 130, 8192), (2, 70, 9220), (1, 4000, 4)])
+                                   (2, 2500, 1028), (4, 2501, 516), (4, 9001, 2052), (4, 130, 8192), (2, 70, 9220), (1, 4000, 4),
+                                   (2000, 9001, 260), (901, 2050, 2052), (700, 8200, 48), (520, 5000, 4)])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, accumulate):
     a, w, c = rnd(m, k, seed=m), rnd(n, k, seed=n), rnd(m, n, seed=k)
@@ -48,7 +49,7 @@ def test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, accumulat
     assert bool((wide[:, n:] == 5.0).all())
 
 
-@pytest.mark.parametrize("T,H,K,N", [(1, 6, 64, 128), (133, 3, 128, 48), (70, 4, 24, 72), (8, 2, 16, 260)])
+@pytest.mark.parametrize("T,H,K,N", [(1, 6, 64, 128), (133, 3, 128, 48), (70, 4, 24, 72), (8, 2, 16, 260), (1000, 2, 68, 5000)])
 def test_float32_head_products_are_the_general_kernels_bit_for_bit(T, H, K, N):
     x, w = rnd(T, H, K + 4, seed=T)[:, :, :K], rnd(H, N, K, seed=N)
     want, got = torch.empty(T, H, N, device=DEV), torch.empty(T, H, N, device=DEV)
