@@ -45,6 +45,7 @@ constexpr int ADM_ROWS = 16;          // query heads per kv head, padded to the 
 // and four stages measured the same as two at every batch and context tried: with two blocks on every
 // SM the loads in flight already cover the memory's latency.
 __host__ __device__ constexpr int adm_stages(int /*head_dim*/) { return 2; }
+constexpr int ADM_MIN_CHUNK = 5, ADM_SIZES = 8;      // pages a chunk the kernel itself cuts has at least; sizes it looks at
 constexpr int ADM_MAX_SEQS = 1024;    // sequences a launch can take (their slots, positions and chunk counts sit in shared memory)
 // Transpose an 8 x 8 matrix of 16-bit values held across the warp (lane 4 r + c holds row r, columns 2 c, 2 c + 1).
 __device__ __forceinline__ uint32_t adm_transpose8(uint32_t a) {
@@ -121,7 +122,7 @@ attention_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, __nv_b
     __shared__ int sm_abort[2];                                  // [0]: a wait ran out; [1]: stays zero
     volatile int* abort_flag = sm_abort;
     const uint32_t full0 = smem_u32(full_bar);
-    __shared__ int warp_total[ADM_WARPS], warp_longest[ADM_WARPS], warp_live[ADM_WARPS];
+    __shared__ int warp_total[ADM_WARPS], warp_longest[ADM_WARPS], warp_live[ADM_WARPS], warp_items[ADM_WARPS][ADM_SIZES];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 
     ssb_pdl_launch_dependents();
@@ -143,11 +144,13 @@ attention_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, __nv_b
         return (p >> 6) - (key_lo >> 6) + 1;
     };
     // chunk_pages <= 0: the kernel sizes the chunks itself from the batch's pages; every block computes
-    // the same figure.  Sequences of about equal length: items about as many as the blocks (a fifth of
-    // them spare, for the items that rounding adds), since an item's fixed cost is worth some six pages
-    // of streaming.  Very unequal lengths (the longest more than one and a half times the mean) with
-    // enough work for it: two to three items a block, of at least eight pages, so that the blocks end
-    // together.  A caller that wants a sequence cut the same way in every batch gives chunk_pages itself.
+    // the same figure.  As fine as leaves every block one item (a second wave of items costs a second item's time, whatever
+    // few they are), but not below five pages, where what a cut saves is less than the meeting of its parts costs.  Very
+    // unequal lengths (the longest more than one and a half times the mean) with enough work for it: two to three items a
+    // block, of at least eight pages, so that the blocks end together.  us a decode step with items for four fifths of the
+    // blocks, which rounding may raise above their number, and so: 1B, 64 sequences of 1 to 512 tokens 1,032 and 960, 32 of 260
+    // 820 and 807, 40 of 1 to 1,829 1,175 and 1,050; 3B, 16 of 64 to 2,022 1,872 and 1,828.  A caller that wants a sequence cut
+    // the same way in every batch gives chunk_pages itself.
     const int n_cl = CL ? (int)adm_cluster_size() : 1;          // blocks of a cluster: the chunks of every sequence
     if (!CL && chunk_pages <= 0) {
         int local = 0, longest = 0, live = 0;
@@ -173,7 +176,34 @@ attention_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, __nv_b
         units *= n_kv;
         const long long coarse = max(1LL, (long long)gridDim.x * 4 / 5), fine = max(1LL, (long long)gridDim.x * 5 / 2);
         const long long fine_pages = (units + fine - 1) / fine;
-        chunk_pages = (unequal && fine_pages >= 8) ? (int)fine_pages : (int)max(2LL, (units + coarse - 1) / coarse);
+        if (unequal && fine_pages >= 8) {
+            chunk_pages = (int)fine_pages;
+        } else {
+            // the smallest of some sizes, the last of which cuts nothing, whose items the blocks take in one go
+            const int least = (int)max((long long)ADM_MIN_CHUNK, (units + gridDim.x - 1) / (long long)gridDim.x);
+            auto size_of = [&](int i) { return i == ADM_SIZES - 1 ? max(longest, 1) : least + (i < 5 ? i : 2 * i - 4); };
+            int items[ADM_SIZES];
+#pragma unroll
+            for (int i = 0; i < ADM_SIZES; ++i) items[i] = 0;
+            for (int b = threadIdx.x; b < n_seqs; b += ADM_THREADS) {
+                const int n = pages_of(b);
+#pragma unroll
+                for (int i = 0; i < ADM_SIZES; ++i) items[i] += (n + size_of(i) - 1) / size_of(i);
+            }
+#pragma unroll
+            for (int i = 0; i < ADM_SIZES; ++i) {
+                const int sum = __reduce_add_sync(0xffffffffu, items[i]);
+                if (lane == 0) warp_items[warp][i] = sum;
+            }
+            __syncthreads();
+            chunk_pages = (int)max((long long)ADM_MIN_CHUNK, (units + coarse - 1) / coarse);
+#pragma unroll
+            for (int i = ADM_SIZES - 1; i >= 0; --i) {
+                long long sum = 0;
+                for (int w = 0; w < ADM_WARPS; ++w) sum += warp_items[w][i];
+                if (sum * n_kv <= (long long)gridDim.x) chunk_pages = size_of(i);
+            }
+        }
         __syncthreads();                                         // warp_total is used again below
     }
     auto chunks_of = [&](int b) {

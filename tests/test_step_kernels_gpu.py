@@ -251,6 +251,39 @@ def test_products_of_few_rows_in_narrow_tiles(rows, n, k, tile):
     o.check_device_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("hd,lens", [(64, [300] * 60 + [450] * 14), (64, [20, 330] * 40), (128, [700] * 30), (128, [64 * 40] * 5 + [3]),
+                                     (64, [400] * 100), (128, [1, 64, 65, 320, 321, 384, 385])])
+def test_decode_attention_cuts_its_sequences_itself(hd, lens):
+    """One item a block where some size of chunk allows it, none does, five pages or fewer, a padding row: the outputs of the
+    same keys in fixed chunks of three pages, within the rounding of the weights to bfloat16 (2^-8 of a value)."""
+    o, n_q, n_kv, B = ops(), 8, 4, len(lens)
+    pages = [(n + 63) // 64 for n in lens]
+    most, at = max(pages), 0
+    perm = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(hd)).to(torch.int32)
+    table = torch.zeros(B, most, dtype=torch.int32)
+    for b, n in enumerate(pages):
+        table[b, :n] = perm[at:at + n]
+        at += n
+    k, v = rnd(sum(pages), n_kv, 64, hd, seed=1, dtype=torch.bfloat16), rnd(sum(pages), n_kv, 64, hd, seed=2, dtype=torch.bfloat16)
+    q = rnd(B, n_q * hd, seed=3, dtype=torch.bfloat16)
+    slots = list(range(B))
+    slots[1] = -1
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    outs = []
+    for chunk in (3, 0):
+        chunks = -(-most // 2)
+        nf, nc = o.attention_decode_chunked_scratch(B, n_q, n_kv, hd, chunks)
+        scratch, counters = torch.full((nf,), math.nan, device=DEV), torch.zeros(nc, dtype=torch.int32, device=DEV)
+        out = torch.full((B, n_q * hd), 9.0, dtype=torch.bfloat16, device=DEV)
+        o.attention_decode_chunked(q, k, v, i32([n - 1 for n in lens]), i32(slots), table.to(DEV), out, n_q, n_kv, hd, 6, None,
+                                   hd ** -0.5, chunk, chunks, scratch, counters)
+        assert bool((counters == 0).all())
+        outs.append(out.float())
+    assert bool((outs[1][1] == 0).all())
+    assert float((outs[0] - outs[1]).norm() / outs[0].norm()) < 2.0 ** -8
+    o.check_device_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("top_k", [1, 5, 40, 64])
 @pytest.mark.parametrize("top_p,vocab", [(1.0, 70001), (0.9, 70001), (0.6, 70001), (0.0, 70001), (0.9, 50), (1.0, 65), (0.6, 4096), (0.9, 400000)])
 def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top_k, top_p, vocab):
