@@ -263,6 +263,8 @@ class FastKernels(PlainKernels):
         step of 16 layers: batch 1 1,566 to 1,509 us, batch 2 1,564 to 1,531, batch 8 1,634 to 1,621."""
         if self.deterministic:
             return 0
+        if pages <= 3:                      # nothing to share, or a page each: us a step of one sequence in eights and so, 1B, 20
+            return 2 if pages > 1 and heads * 2 <= min(blocks, ops.sm_count()) else 0      # keys 635 and 626, 8B, 60 2,712 and 2,660
         for c in (8, 4, 2):
             if heads * c <= min(blocks, ops.sm_count()):
                 return c if pages <= CLUSTER_CHUNK_PAGES * c else 0
@@ -319,18 +321,35 @@ class FastKernels(PlainKernels):
         rows = batch.n_tokens
         if getattr(position, "interleaved", False):
             return False                      # the fused rotations pair (i, i + half)
-        if not (self.fuse_rope_prefill and tables and not batch.is_decode and rows > 64
+        if not (self.fuse_rope_prefill and tables and not batch.is_decode
                 and w_qkv.dtype == torch.bfloat16 and head_dim in (64, 128)):
             return False
         n, k = w_qkv.shape
-        if self._gemm_splits(rows, n, k, 256) > 1:
-            return False                      # a short prompt: K split over blocks is the faster way
+        stream = rows <= STREAM_ROWS and n < 16384
+        if stream and ops.gemv_rows_tile(rows, n, k):
+            return False
+        splits = self._gemm_splits(rows, n, k, 256)
         cos, sin, rotary_dim = tables()
         k_cache, v_cache, page_table, _ = kv
         x = as_tensor(x)
-        if rotary_dim != head_dim or not ops.gemm_tc_ok(x, w_qkv, qkv) or k_cache.dtype != torch.bfloat16:
+        if rotary_dim != head_dim or not ops.gemm_tc_ok(x, w_qkv, qkv) or k_cache.dtype != torch.bfloat16 \
+                or not (k_cache.is_contiguous() and v_cache.is_contiguous()):
+            return False
+        if not stream and (rows <= 64 or (rows <= STREAM_ROWS and splits > 1)):
             return False
         position.check_range(batch)
+        if stream or splits > 1:
+            # a short prompt: K split over blocks is the faster way (see ``linear``), and what rounds its sums rotates and
+            # appends in the same pass
+            chain = self._prompt_chain(rows)
+            sums = self._buffer("split_sums", rows * n, torch.float32, qkv.device, zero=True)[: rows * n].view(rows, n)
+            if stream:
+                ops.gemv_tc(x, w_qkv, sums, ops.TC_ACCUMULATE, splits=ops.gemv_tc_splits(n, k), pdl=self.pdl)
+            else:
+                ops.gemm_tc(x, w_qkv, sums, ops.TC_ACCUMULATE, tile_n=256, splits=splits, pdl=chain)
+            ops.rope_append_sums(sums, qkv, cos, sin, batch.pos, batch.slot_of_token, page_table, k_cache, v_cache, n_q, n_kv,
+                                 head_dim, page_shift, pdl=self.pdl)
+            return True
         ops.gemm_tc_rope_append(x, w_qkv, qkv, cos, sin, batch.pos, batch.slot_of_token, page_table, k_cache,
                                 v_cache, n_q, n_kv, head_dim, page_shift,
                                 tile_n=ops.TC_TILE_PAIR if self._pair_tiles(rows, n) else 256, pdl=self._prompt_chain(rows))

@@ -2556,3 +2556,24 @@ def rope_append_vec(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos
         _ptr(qkv), c_int(qkv.stride(0)), _ptr(cos), _ptr(sin), c_int(cos.shape[0]), _ptr(pos), _ptr(slot),
         _ptr(page_table), c_int(page_table.shape[1]), _ptr(k_cache), _ptr(v_cache), c_int(T), c_int(n_q),
         c_int(n_kv), c_int(head_dim), c_int(page_shift), c_int(1 if pdl else 0), _stream()), "rope_append_vec")
+
+
+def rope_append_sums(sums: torch.Tensor, qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: torch.Tensor,
+                     slot: torch.Tensor, page_table: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
+                     n_q: int, n_kv: int, head_dim: int, page_shift: int, pdl: bool = False) -> None:
+    """:func:`round_and_clear` of a projection's float32 sums [T, q | k | v] and :func:`rope_append_vec` behind it in one launch:
+    rotated queries in ``qkv``'s first columns (the others are left as they are), keys and values in the cache."""
+    _need(sums, "sums", torch.float32, 2); _need(qkv, "qkv", torch.bfloat16, 2)
+    _need(pos, "pos", torch.int32, 1); _need(slot, "slot", torch.int32, 1)
+    _need(page_table, "page_table", torch.int32, 2); _need(cos, "cos", torch.float32, 2); _need(sin, "sin", torch.float32, 2)
+    _need(k_cache, "k_cache", torch.bfloat16); _need(v_cache, "v_cache", torch.bfloat16)
+    T = qkv.shape[0]
+    if not sums.is_contiguous() or tuple(sums.shape) != (T, (n_q + 2 * n_kv) * head_dim) or qkv.shape[1] < n_q * head_dim \
+            or pos.shape[0] != T or slot.shape[0] != T or not (k_cache.is_contiguous() and v_cache.is_contiguous()):
+        raise KernelError("rope_append_sums: sums of whole contiguous rows, one position and slot per token")
+    if cos.shape != sin.shape or cos.shape[1] * 2 != head_dim or not (cos.is_contiguous() and sin.is_contiguous()):
+        raise KernelError("rope_append_sums: cos/sin must be [positions, head_dim/2], contiguous")
+    _check(_fn("elementwise_ops", "ssb_rope_append_sums")(
+        _ptr(sums), _ptr(qkv), c_int(qkv.stride(0)), _ptr(cos), _ptr(sin), c_int(cos.shape[0]), _ptr(pos), _ptr(slot),
+        _ptr(page_table), c_int(page_table.shape[1]), _ptr(k_cache), _ptr(v_cache), c_int(T), c_int(n_q),
+        c_int(n_kv), c_int(head_dim), c_int(page_shift), c_int(1 if pdl else 0), _stream()), "rope_append_sums")

@@ -284,6 +284,25 @@ def test_decode_attention_cuts_its_sequences_itself(hd, lens):
     o.check_device_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("hd,n_q,n_kv,T", [(64, 8, 2, 37), (128, 6, 3, 5), (64, 32, 8, 131), (8, 1, 1, 1)])
+def test_rotation_from_split_sums_is_the_two_launches_bit_for_bit(hd, n_q, n_kv, T):
+    """Rounding, rotation and append in one pass; a padding row's sums are cleared and nothing else."""
+    o, n = ops(), (n_q + 2 * n_kv) * hd
+    sums0, cos, sin = rnd(T, n, seed=1, scale=3.0), rnd(T + 5, hd // 2, seed=2), rnd(T + 5, hd // 2, seed=3)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos, slot = i32(list(range(5, T + 5))), i32([0 if t != 3 else -1 for t in range(T)])
+    table = torch.randperm(4, generator=torch.Generator().manual_seed(hd)).to(torch.int32).view(1, 4).to(DEV)
+    caches = [[rnd(4, n_kv, 64, hd, seed=4, dtype=torch.bfloat16) for _ in range(2)] for _ in range(2)]
+    sums, want, got = sums0.clone(), torch.empty(T, n, dtype=torch.bfloat16, device=DEV), torch.full((T, n), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.round_and_clear(sums, want)
+    o.rope_append_vec(want, cos, sin, pos, slot, table, *caches[0], n_q, n_kv, hd, 6)
+    sums = sums0.clone()
+    o.rope_append_sums(sums, got, cos, sin, pos, slot, table, *caches[1], n_q, n_kv, hd, 6)
+    live = (slot >= 0).cpu()
+    assert torch.equal(got[:, :n_q * hd].cpu()[live], want[:, :n_q * hd].cpu()[live]) and bool((got[:, n_q * hd:] == 7.0).all())
+    assert bool((sums == 0).all()) and all(torch.equal(a, b) for a, b in zip(*caches))
+
+
 @pytest.mark.parametrize("top_k", [1, 5, 40, 64])
 @pytest.mark.parametrize("top_p,vocab", [(1.0, 70001), (0.9, 70001), (0.6, 70001), (0.0, 70001), (0.9, 50), (1.0, 65), (0.6, 4096), (0.9, 400000)])
 def test_a_row_draws_the_same_token_from_its_candidates_as_from_the_held_row(top_k, top_p, vocab):
