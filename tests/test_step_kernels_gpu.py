@@ -716,3 +716,42 @@ def test_sums_of_a_few_rows_in_their_order(width, dtype):
             ops().stream_mix(off_by_one(streams), w[0].contiguous(), top, one)
             ops().stream_mix(streams, w[0].contiguous(), top, other)
             assert torch.equal(one, other)
+
+
+@pytest.mark.parametrize("n_seqs,longest,n_q,n_kv,hd,window",
+                         [(600, 90, 2, 1, 64, None), (40, 700, 6, 2, 128, None), (150, 300, 3, 1, 64, 100), (150, 300, 3, 3, 128, 65),
+                          (3, 400, 8, 2, 128, None), (2, 700, 5, 1, 64, None), (37, 512, 8, 4, 64, None)])
+def test_prompt_attention_over_many_units(n_seqs, longest, n_q, n_kv, hd, window):
+    """Blocks that stay for many units of a ragged batch, more sequences than a launch's table holds, sequences without a slot or
+    without tokens, one tile a unit and two.  Probabilities are rounded to bfloat16 (2^-9 of the largest value), and so is the
+    output (2^-9 again)."""
+    o, g = ops(), torch.Generator().manual_seed(n_seqs + longest)
+    lens, starts = torch.randint(1, longest + 1, (n_seqs,), generator=g), torch.randint(0, 200, (n_seqs,), generator=g)
+    lens[0], starts[0] = longest, 0
+    lens[n_seqs // 2] = 0 if n_seqs > 10 else 1
+    pages = (longest + 200 + 63) // 64
+    slot = torch.arange(n_seqs, dtype=torch.int32)
+    if n_seqs > 10:
+        slot[3::7] = -1
+    table = torch.randperm(n_seqs * pages, generator=g).to(torch.int32).view(n_seqs, pages).to(DEV)
+    k, v = (rnd(n_seqs * pages, n_kv, 64, hd, seed=s, dtype=torch.bfloat16) for s in (1, 2))
+    cu = torch.cat([torch.zeros(1, dtype=torch.int64), lens.cumsum(0)])
+    rows = int(cu[-1])
+    q = rnd(rows, (n_q + 2 * n_kv) * hd, seed=3, dtype=torch.bfloat16)
+    out = torch.full((rows, n_q * hd), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.attention_prefill_tc(q, k, v, cu.to(torch.int32).to(DEV), starts.to(torch.int32).to(DEV), slot.to(DEV), table, out, longest,
+                           n_q, n_kv, hd, 6, window, hd ** -0.5)
+    o.check_device_errors(torch.device(DEV))
+    for b in range(n_seqs):
+        r0, n, s = int(cu[b]), int(lens[b]), int(starts[b])
+        mine = out[r0:r0 + n].view(n, n_q, hd)
+        if slot[b] < 0:
+            assert bool((mine == 7.0).all())
+            continue
+        keys, values = (c[table[b].long()].transpose(0, 1).reshape(n_kv, -1, hd)[:, :s + n].double().repeat_interleave(n_q // n_kv, 0)
+                        for c in (k, v))
+        score = torch.einsum("nhd,hkd->hnk", q[r0:r0 + n, :n_q * hd].view(n, n_q, hd).double(), keys) * hd ** -0.5
+        at, key = torch.arange(s, s + n, device=DEV)[:, None], torch.arange(s + n, device=DEV)[None]
+        seen = (key <= at) & (key > at - window if window else key >= 0)
+        want = torch.softmax(score.masked_fill(~seen, -math.inf), -1) @ values
+        assert n == 0 or float((mine.double() - want.transpose(0, 1)).abs().max()) <= 2.0 ** -8 * 1.05 * float(values.abs().max())
