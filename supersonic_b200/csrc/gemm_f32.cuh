@@ -363,7 +363,7 @@ gemm_f32_walk_kernel(const float* __restrict__ A, int lda, const float* __restri
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// A few hundred rows, or few columns: tiles of 64 x 64 and 128 x 64, 4 x 4 and 8 x 4 results a thread, one chunk of k a turn, two or
+// A few hundred rows of many columns: tiles of 64 x 64 and 128 x 64, 4 x 4 and 8 x 4 results a thread, one chunk of k a turn, two or
 // three blocks an SM.  A chunk comes by cp.async as it lies in memory, GF_RAW deep, and is turned k-major in shared memory on the
 // way to its two buffers, so that a thread reads four neighbouring columns at a time and the multiply-adds go two columns an
 // instruction (fma.rn.f32x2: each half rounds as the scalar one does).  Bound by the FP32 pipes and the shared-memory reads beside
@@ -644,6 +644,125 @@ gemm_f32_role_kernel(const float* __restrict__ A, int lda, const float* __restri
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
+// 17 to 300 rows: too few for tiles of 64 columns to fill the SMs, too many to stream the weights 16 rows at a time.  A block's
+// warps take a chunk of k each of one tile of 8 RM x 4 RN results, RM x RN a lane, from rows as they lie in memory; the chunks' sums
+// go through shared memory to the threads that own the results, which add them in k order while the next turn is multiplied.
+// Bound by the shared-memory reads beside the multiply-adds (12 of 16 bytes for 128 multiply-adds a lane, then a chunk's sums
+// written and read).  us before (16 rows at a time, or tiles of 64 x 64) and here: tiles of 64 x 16, 64 x 2048 x 2048 51 and 34, 64 x
+// 2048 x 8192 193 and 125, 100 x 2048 x 8192 333 and 246, 300 x 2048 x 2048 181 and 155, 200 x 512 x 128 9.4 and 4.3; of 32 x 32, 32 x 16384 x 2048 170 and 152, 32 x 4096 x 4096 98 and 77.  Tiles of
+// 64 x 32, 8 x 8 results a lane: 72, and 284 for 64 x 16384 x 2048 (191 with tiles of 64 x 64, 219 of 64 x 16).
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int GF_PART_WARPS = 8, GF_PART_K = GF_PART_WARPS * GF_CHUNK, GF_PART_LD = GF_PART_K + 4, GF_PART_STAGES = 3;
+template <int RM, int RN>
+constexpr size_t gf_part_smem() {
+    return sizeof(float) * ((size_t)GF_PART_STAGES * (8 * RM + 4 * RN) * GF_PART_LD + (size_t)2 * GF_PART_WARPS * 32 * RM * RN);
+}
+
+template <int RM, int RN>
+__global__ void __launch_bounds__(32 * GF_PART_WARPS, 1)
+gemm_f32_part_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
+                     int M, int N, int K, long long a_batch, long long w_batch, long long c_batch, int accumulate) {
+    constexpr int TM = 8 * RM, TN = 4 * RN, TILE = TM * TN;
+    static_assert(TILE == 4 * 32 * GF_PART_WARPS, "a thread owns four results");
+    extern __shared__ __align__(16) float gf_smem[];
+    float* sums = gf_smem + GF_PART_STAGES * (TM + TN) * GF_PART_LD;     // [2][chunk of the turn][row][4 RN columns, exchanged]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane % 8, lc = lane / 8;
+    A += (size_t)blockIdx.z * a_batch;
+    W += (size_t)blockIdx.z * w_batch;
+    C += (size_t)blockIdx.z * c_batch;
+    const int m_tiles = (M + TM - 1) / TM, tiles = m_tiles * ((N + TN - 1) / TN);
+    const int chunks = (K + GF_CHUNK - 1) / GF_CHUNK, turns = (K + GF_PART_K - 1) / GF_PART_K;
+    const int all = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * turns;
+    int f_tile = blockIdx.x, f_turn = 0;                             // what is fetched next
+    auto fetch = [&](int stage) {
+        if (f_tile < tiles) {
+            const int m0 = f_tile % m_tiles * TM, n0 = f_tile / m_tiles * TN, k = f_turn * GF_PART_K + 4 * lane;
+            float* dst = gf_smem + stage * (TM + TN) * GF_PART_LD + warp * GF_PART_LD + 4 * lane;    // a warp fetches 512 bytes of a row
+#pragma unroll
+            for (int e = 0; e < (TM + TN) / GF_PART_WARPS; ++e) {
+                const int r = warp + e * GF_PART_WARPS;
+                const bool of_a = e < TM / GF_PART_WARPS;
+                const int row = of_a ? m0 + r : n0 + r - TM;
+                const bool in = k < K && row < (of_a ? M : N);
+                gf_cp16(dst + e * GF_PART_WARPS * GF_PART_LD, !in ? A : of_a ? A + (size_t)row * lda + k : W + (size_t)row * ldw + k, in ? 16 : 0);
+            }
+            if (++f_turn == turns) { f_turn = 0; f_tile += gridDim.x; }
+        }
+        gf_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < GF_PART_STAGES - 1; ++s) fetch(s);
+    const unsigned long long minus_one = f2_twice(-1.0f);
+    unsigned long long acc[2] = {0, 0}, kept[2] = {0, 0};            // four results
+    int a_tile = blockIdx.x, a_turn = 0, stage = 0;
+    auto add = [&](int buffer) {                                     // a turn's sums
+        const float* src = sums + buffer * GF_PART_WARPS * TILE + 4 * tid;
+        const int here = min(GF_PART_WARPS, chunks - a_turn * GF_PART_WARPS);
+#pragma unroll
+        for (int c = 0; c < GF_PART_WARPS; ++c) {
+            if (c >= here) break;
+            const ulonglong2 part = *reinterpret_cast<const ulonglong2*>(src + c * TILE);
+            gf_kahan2(acc[0], kept[0], part.x, minus_one);
+            gf_kahan2(acc[1], kept[1], part.y, minus_one);
+        }
+        if (++a_turn < turns) return;
+        // a row's results lie [column / 16][column % 4][column / 4 % 4]
+        const int m = a_tile % m_tiles * TM + 4 * tid / TN, place = 4 * tid % TN, n0 = a_tile / m_tiles * TN + place / 16 * 16 + place % 16 / 4;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float x = __uint_as_float((unsigned)(acc[e / 2] >> (32 * (e % 2))));
+            if (m < M && n0 + 4 * e < N) {
+                float* dst = C + (size_t)m * ldc + n0 + 4 * e;
+                *dst = accumulate ? *dst + x : x;
+            }
+        }
+        acc[0] = acc[1] = kept[0] = kept[1] = 0;
+        a_turn = 0;
+        a_tile += gridDim.x;
+    };
+    for (int turn = 0; turn < all; ++turn) {
+        gf_wait<GF_PART_STAGES - 2>();
+        __syncthreads();                                             // this turn has landed, the one before is multiplied
+        fetch(stage == 0 ? GF_PART_STAGES - 1 : stage - 1);
+        if (turn > 0) add((turn - 1) & 1);
+        float part[RM][RN];
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN; ++j) part[i][j] = 0.f;
+        const float* a_s = gf_smem + stage * (TM + TN) * GF_PART_LD + lr * GF_PART_LD + warp * GF_CHUNK;
+        const float* w_s = gf_smem + stage * (TM + TN) * GF_PART_LD + (TM + lc) * GF_PART_LD + warp * GF_CHUNK;
+#pragma unroll
+        for (int k = 0; k < GF_CHUNK; k += 4) {
+            float4 w[RN];
+#pragma unroll
+            for (int j = 0; j < RN; ++j) w[j] = *reinterpret_cast<const float4*>(w_s + j * 4 * GF_PART_LD + k);
+#pragma unroll
+            for (int i = 0; i < RM; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(a_s + i * 8 * GF_PART_LD + k);
+#pragma unroll
+                for (int j = 0; j < RN; ++j) {
+                    part[i][j] = fmaf(a.x, w[j].x, part[i][j]);
+                    part[i][j] = fmaf(a.y, w[j].y, part[i][j]);
+                    part[i][j] = fmaf(a.z, w[j].z, part[i][j]);
+                    part[i][j] = fmaf(a.w, w[j].w, part[i][j]);
+                }
+            }
+        }
+        float* dst = sums + ((turn & 1) * GF_PART_WARPS + warp) * TILE + lr * TN + 4 * lc;
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < RN; j += 4)
+                *reinterpret_cast<float4*>(dst + i * 8 * TN + 4 * j) = make_float4(part[i][j], part[i][j + 1], part[i][j + 2], part[i][j + 3]);
+        stage = stage + 1 == GF_PART_STAGES ? 0 : stage + 1;
+    }
+    __syncthreads();
+    add((all - 1) & 1);
+    gf_wait<0>();
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
 // Whether the operands can be fetched in 16-byte pieces (rows of W and A start on 16-byte boundaries, K in whole pieces).
 static inline bool gemm_f32_ok(const void* A, int lda, long long a_batch, const void* W, int ldw, long long w_batch, int K) {
     return !(((uintptr_t)A | (uintptr_t)W) & 15) && !((lda | ldw | K) & 3) && !((a_batch | w_batch) & 3);
@@ -653,11 +772,13 @@ static inline bool gemm_f32_ok(const void* A, int lda, long long a_batch, const 
 // is done first by the time a chunk of 16 k takes it: the blocks run in waves over the SMs, and tiles that are too large leave
 // SMs idle where tiles that are too small fetch more often than they multiply.  Hundredths of a microsecond a chunk, measured
 // for 1 and for each further wave: up to 4, 8 and 16 rows x 16 columns a block 5 to 3 + 3.8, 5 and 10, whole turns of 32 chunks
-// whatever K is; tiles of 64 x 64 90 + 60, of 128 x 64 145 + 115, of 128 x 128 167 + 167, and 3 us to start and end.  A walking warp's turn: 4 rows of W 65, 70 and 85 (1, 2, 4 rows of A), 2 rows 80, 1 row 130,
-// and 3 us.  Sides of the lines it draws (us; rows x columns, k 2048): 128 x 2048 89 with 16 rows and 116 with tiles of 64; 100
-// x 3072 118 with tiles of 64, 124 with 16 rows; 300 x 3072 182 with 128 x 64, 189 with 64 x 64, 217 with 128 x 128; 500 x 3072
-// 217 with 128 x 128, 266 with 64 x 64; 500 x 2048 181 with 128 x 64, 217; 1000 x 2048 217 and 318.  K 64: 300 x 64 5.3 with 16
-// rows, 6.5 with tiles of 64, 700 x 64 8.2 and 6.6; 16 x 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.
+// whatever K is; tiles of 64 x 64 90 + 60, of 128 x 64 145 + 115, of 128 x 128 167 + 167, of 64 x 16 and 32 x 32 by chunks 24 and 29 (whole turns of 8),
+// and 3 us to start and end.  A walking warp's turn: 4 rows of W 65, 70 and 85 (1, 2, 4 rows of A), 2 rows 80, 1 row 130,
+// and 3 us.  Sides of the lines it draws (us; rows x columns, k 2048): 32 x 2048 27 with 16 rows and 33 by chunks of 64 x 16; 64 x 2048
+// 51 and 34; 64 x 16384 219 by chunks and 191 with tiles of 64; 128 x 3072 95 by chunks, 114 with tiles of 64; 300 x 2048 155 by
+// chunks, 181 with 128 x 64; 300 x 3072 182 with 128 x 64, 189 with 64 x 64, 217 with 128 x 128; 500 x 3072 217 with 128 x 128, 266
+// with 64 x 64; 500 x 2048 181 with 128 x 64, 217; 1000 x 2048 217 and 318.  K 64: 300 x 64 5.3 with 16 rows, 6.5 with tiles of
+// 64; 16 x 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.
 static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
     const long long sms = gf_sms(), chunks = (K + 15) / 16, turns = (K + 511) / 512;
     const auto waves = [&](int rows, int cols) {
@@ -666,16 +787,18 @@ static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
     const bool walk = gf_walk_ok(M, K);
     const int rows = M <= 4 ? 4 : M <= 8 ? 8 : 16;
     const int first = rows < 16 ? 50 : 30, each = rows == 4 ? 38 : rows == 8 ? 50 : 100;
-    const int forms[4] = {walk ? (M <= 2 ? M : 4) : M <= 4 ? 5 : rows, 100, 101, 102};
-    long long cost[4] = {32 * turns * (first + each * waves(rows, 16)), 3000 + 10 * chunks * (30 + 60 * waves(64, 64)),
-                         3000 + 10 * chunks * (30 + 115 * waves(128, 64)), 3000 + 10 * chunks * 167 * waves(128, 128)};
+    const int forms[6] = {walk ? (M <= 2 ? M : 4) : M <= 4 ? 5 : rows, 100, 101, 102, 103, 104};
+    const long long parts = (chunks + GF_PART_WARPS - 1) / GF_PART_WARPS * GF_PART_WARPS;
+    long long cost[6] = {32 * turns * (first + each * waves(rows, 16)), 3000 + 10 * chunks * (30 + 60 * waves(64, 64)),
+                         3000 + 10 * chunks * (30 + 115 * waves(128, 64)), 3000 + 10 * chunks * 167 * waves(128, 128),
+                         3000 + 10 * parts * 24 * waves(64, 16), 3000 + 10 * parts * 29 * waves(32, 32)};
     if (walk) {
         const int width = gf_walk_width(N), turn = width == 1 ? 1300 : width == 2 ? 800 : M <= 1 ? 650 : M <= 2 ? 700 : 850;
         const long long held = sms * GF_WALK_WARPS, rounds = ((long long)((N + width - 1) / width) * n_batch + held - 1) / held;
         cost[0] = 3000 + ((K + GF_WALK_TURN / width - 1) / (GF_WALK_TURN / width)) * rounds * turn;
     }
     int best = 0;
-    for (int f = 1; f < 4; ++f)
+    for (int f = 1; f < 6; ++f)
         if (cost[f] < cost[best]) best = f;
     return forms[best];
 }
@@ -684,7 +807,7 @@ static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
 static inline bool gemm_f32_gated_ok(int M, int N, int K) { return N % 2 == 0 && gemm_f32_form(1, M, N, K) <= 4; }
 
 // form 0: chosen by the sizes; else one of the kernels: 1, 2, 4 (a warp walks), 5, 8, 16 (few rows, 4, 8, 16 a group), 100, 101, 102 (tiles of
-// 64 x 64, 128 x 64 and 128 x 128)
+// 64 x 64, 128 x 64 and 128 x 128), 103, 104 (a tile of 64 x 16, 32 x 32 by chunks of k)
 static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, const float* W, int ldw, long long w_batch,
                                   float* C, int ldc, long long c_batch, int n_batch, int M, int N, int K, int accumulate,
                                   int form, cudaStream_t stream, bool pdl = false, const GfGate* gate = nullptr) {
@@ -742,6 +865,15 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         kernel<<<dim3((unsigned)(tiles < gf_sms() ? tiles : gf_sms()), 1, n_batch), GF_ROLE_ALL, smem, stream>>>( \
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
     } while (0)
+#define GF_PARTS(RM, RN) do { \
+        constexpr size_t smem = gf_part_smem<RM, RN>(); \
+        auto kernel = gemm_f32_part_kernel<RM, RN>; \
+        GF_CONFIGURE(kernel, smem); \
+        const long long tiles = (long long)((N + 4 * RN - 1) / (4 * RN)) * ((M + 8 * RM - 1) / (8 * RM)); \
+        if (tiles > 0x7fffffffLL) return SSB_ERR_BAD_SIZE; \
+        kernel<<<dim3((unsigned)(tiles < gf_sms() ? tiles : gf_sms()), 1, n_batch), 32 * GF_PART_WARPS, smem, stream>>>( \
+            A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
+    } while (0)
     switch (form) {
         case 1: GF_WALKS(1); break;
         case 2: GF_WALKS(2); break;
@@ -752,12 +884,15 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         case 100: GF_TILES(4, 4, 3); break;
         case 101: GF_TILES(8, 4, 2); break;
         case 102: GF_ROLES(8, 8); break;
+        case 103: GF_PARTS(8, 4); break;
+        case 104: GF_PARTS(4, 8); break;
         default: return SSB_ERR_BAD_SIZE;
     }
 #undef GF_SKINNY
 #undef GF_WALK
 #undef GF_WALKS
 #undef GF_ROLES
+#undef GF_PARTS
 #undef GF_TILES
 #undef GF_CONFIGURE
     return ssb_launch_status();

@@ -49,6 +49,15 @@ def test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, accumulat
     assert bool((wide[:, n:] == 5.0).all())
 
 
+# tiles of 64 x 16 and of 32 x 32 whose chunks of k are shared out over warps: edges of tiles, turns of 8 chunks and chunks, blocks
+# that walk several tiles
+@pytest.mark.parametrize("m,n,k", [(64, 2100, 2052), (65, 2047, 20), (100, 1030, 516), (200, 2048, 1028), (17, 4700, 132), (32, 4700, 1028),
+                                   (31, 9001, 148), (64, 3072, 128), (20, 16390, 264)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_float32_products_by_chunks_are_the_general_kernels_bit_for_bit(m, n, k, accumulate):
+    test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, accumulate)
+
+
 @pytest.mark.parametrize("T,H,K,N", [(1, 6, 64, 128), (133, 3, 128, 48), (70, 4, 24, 72), (8, 2, 16, 260), (1000, 2, 68, 5000)])
 def test_float32_head_products_are_the_general_kernels_bit_for_bit(T, H, K, N):
     x, w = rnd(T, H, K + 4, seed=T)[:, :, :K], rnd(H, N, K, seed=N)
