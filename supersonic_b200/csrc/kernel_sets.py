@@ -66,10 +66,11 @@ class PlainKernels:
     def _f32_rows_share(batch, n_q: int, n_kv: int, head_dim: int) -> bool:
         """Whether 64 (token, head) rows of a float32 prompt share a block and its fetch of a key.  A block's time is its chain of
         keys whatever it holds, so the rows have to fill the blocks: with few, a row a block (attention_plain) finishes all of
-        them in one such chain, a shorter one.  us a row a block and shared, 32 heads over 8, at 4,000 keys: heads of 64,
-        8 x 32 rows 385 and 404, 16 x 32 435 and 382, 32 x 32 540 and 384; of 128, 16 x 32 551 and 591, 32 x 32 825 and 592.
-        Short contexts have little to share: 32 tokens of their own, 32 x 32 rows 14 and 15 (64), 17 and 23 (128), 64 x 32 18
-        and 15, 21 and 20."""
+        them in a shorter chain.  us a row a block and shared, 32 heads over 8, at 4,000 keys: heads of 64, 16 x 32 rows 257 and
+        374, 24 x 32 305 and 398, 32 x 32 404 and 376; of 128, 8 x 32 341 and 625, 16 x 32 680 and 580, 32 x 32 1,194 and 583.
+        Short contexts have little to share: tokens of their own, 16 x 32 rows 6.4 and 10.7 (64), 11.7 and 16.5 (128), 32 x 32
+        9.8 and 11.8, 22.9 and 17.7, 64 x 32 18.3 and 13.4, 50.7 and 20.3.  The lines are from before a row a block staged its
+        keys: at 4,000 keys they now lie at 28 tokens of such a model for heads of 64 (16 in the rule) and 14 for 128 (32)."""
         group = n_q // n_kv
         blocks = min(batch.n_seqs * -(-batch.max_new * group // 64), batch.n_tokens * group // 64 + batch.n_seqs) * n_kv
         waves = -(-blocks // (ops.sm_count() * (2 if head_dim == 64 else 1)))       # an SM holds two blocks, or one
