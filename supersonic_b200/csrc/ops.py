@@ -806,7 +806,7 @@ def gated_scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim:
     """(chunk, floats of sums, floats of decays) for ``gated_linear_scan``: as many chunks as give the SMs two blocks each
     (blocks own 64 value columns of a head), of 64 tokens or more, or three of 40 or more where an SM each is left for them;
     one walk a sequence where that is no more than two chunks.  4 heads of 256 x 512, us in one walk and in three chunks: 100
-    tokens 51 and 52, 130 84 and 55, 190 118 and 74; four such sequences 150 tokens 97 and 171."""
+    tokens 46 and 53, 130 57 and 60, 190 79 and 74; four such sequences are slower in three chunks (every chunk walks twice)."""
     blocks = max(n_seqs * n_heads * (-(-vdim // 64)), 1)
     per = n_heads * dim * vdim
     most = SCAN_SCRATCH_BYTES // (4 * per * n_seqs)
