@@ -232,8 +232,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                         const int p0 = q.start + tile * FT_BM, rows = item < n_items ? min(FT_BM, q.n_new - tile * FT_BM) : 0;
                         t_head[x] = kvh * group + item % group;
                         t_row[x] = q.row0 + tile * FT_BM;
-                        // tile 0 is never the later one
-                        if (x == 0) kb_lo = (window > 0 && p0 - window + 1 > 0) ? (p0 - window + 1) >> 6 : 0;
+                        // Keys begin at the page that the first tile of the pair (never the later one) sees first, for a tile
+                        // that is alone too: a row's turns, and with them its sums, are the same in a unit of either size
+                        if (x == 0) {
+                            const int first = q.start + (item & ~1) / group * FT_BM;
+                            kb_lo = (window > 0 && first - window + 1 > 0) ? (first - window + 1) >> 6 : 0;
+                        }
                         nb[x] = rows > 0 ? (((p0 + rows - 1) >> 6) - kb_lo + 2) >> 1 : 0;    // turns, from page kb_lo on
                         nb_max = max(nb_max, nb[x]);
                         q_tiles += nb[x] > 0;

@@ -764,3 +764,24 @@ def test_prompt_attention_over_many_units(n_seqs, longest, n_q, n_kv, hd, window
         seen = (key <= at) & (key > at - window if window else key >= 0)
         want = torch.softmax(score.masked_fill(~seen, -math.inf), -1) @ values
         assert n == 0 or float((mine.double() - want.transpose(0, 1)).abs().max()) <= 2.0 ** -8 * 1.05 * float(values.abs().max())
+
+
+@pytest.mark.parametrize("n_q,n_kv,hd,window,n,start", [(3, 1, 64, 65, 300, 0), (1, 1, 128, 65, 260, 0), (5, 1, 64, 100, 700, 30), (6, 2, 128, 129, 400, 200),
+                                                        (3, 1, 64, None, 300, 0)])
+def test_windowed_prompt_attention_is_the_same_bits_in_every_batch(n_q, n_kv, hd, window, n, start):
+    """An odd number of query heads a kv head: the second tile of a unit may lie in the next row tile.  A prompt alone (one tile
+    a unit) and among others that make enough units for two."""
+    o, pages = ops(), (n + start + 63) // 64
+    others = o.sm_count() // n_kv                                   # at least two units each: more than one a multiprocessor
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    k, v = (rnd(pages, n_kv, 64, hd, seed=s, dtype=torch.bfloat16) for s in (1, 2))
+    q = rnd(n, (n_q + 2 * n_kv) * hd, seed=3, dtype=torch.bfloat16)
+
+    def run(seqs):                                                  # the same prompt in every place, over the same pages
+        out = torch.empty(seqs * n, n_q * hd, dtype=torch.bfloat16, device=DEV)
+        o.attention_prefill_tc(q.repeat(seqs, 1), k, v, i32([i * n for i in range(seqs + 1)]), i32([start] * seqs), i32([0] * seqs),
+                               i32([list(range(pages))]), out, n, n_q, n_kv, hd, 6, window, hd ** -0.5)
+        o.check_device_errors(torch.device(DEV))
+        return out.view(seqs, n, -1)
+    alone, among = run(1)[0], run(others + 1)
+    assert all(torch.equal(alone, row) for row in among)
