@@ -92,8 +92,9 @@ def put_ints(values, out: torch.Tensor, before: Optional[torch.Tensor] = None) -
     _need(out, "out", torch.int32, 1)
     n, n_before = len(values), 0 if before is None else before.numel()
     if before is not None:
-        _need(before, "before", torch.int32, 1)
-    if values.dtype != "int32" or not values.flags.c_contiguous or out.shape[0] != n + n_before:
+        _need(before, "before", torch.int32, 1, rows_contiguous=False)          # one value has whatever stride
+    if values.dtype != "int32" or not values.flags.c_contiguous or out.shape[0] != n + n_before \
+            or (before is not None and not before.is_contiguous()):
         raise KernelError("put_ints: contiguous int32 values, one place for each")
     fn, base = _fn("step_inputs", "ssb_put_ints"), values.ctypes.data
     for lo in range(0, max(n, 1), PUT_INTS_MOST):

@@ -119,7 +119,7 @@ class DecodeGraph:
         B = self.n_seqs
         if isinstance(tokens, torch.Tensor):
             self.staged[B:] = list(positions) + list(slots)
-            ops.put_ints(self.staged[B:], self.ints, before=tokens.reshape(-1))
+            ops.put_ints(self.staged[B:], self.ints, before=tokens.reshape(-1).contiguous())
         else:
             self.staged[:] = list(tokens) + list(positions) + list(slots)
             ops.put_ints(self.staged, self.ints)

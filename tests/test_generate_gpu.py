@@ -502,3 +502,22 @@ def test_prompt_steps_of_recurring_sizes_are_captured_and_stay_right(model_folde
         assert np.abs(got[0] - want).max() < 2e-2 * np.abs(want).max()
         m2.close_sequence(s)
     assert m2.prompt_graph_replays >= 4
+
+
+def test_a_step_ahead_takes_tokens_as_they_lie(model_folders):
+    """A column of a wider matrix, a row of it, a matrix of one column: the same logits as from tokens that lie together."""
+    from supersonic_b200.engine import Model, StepEntry
+    d, pc, pw = model_folders["E"]
+    m = Model.from_dir(d, dtype="bfloat16", max_tokens=2048, deterministic=True)
+    dev = m.device
+    wide = torch.from_numpy(np.random.default_rng(5).integers(0, pc["vocab_size"], (3, 4))).to(torch.int32).to(dev)
+    for tokens in (wide[:, 1], wide[:1, 2], wide[:, 2:3], wide[0, :3], wide[1, 3]):
+        logits = []
+        for t in (tokens.clone(memory_format=torch.contiguous_format), tokens):
+            slots = [m.open_sequence() for _ in range(tokens.numel())]
+            m.step([StepEntry(s, [3, 1, 4 + i], [2]) for i, s in enumerate(slots)])
+            logits.append(m.step_ahead(slots, t))
+            for s in slots:
+                m.close_sequence(s)
+        assert torch.equal(*logits), tokens.shape
+    m.check_errors()
