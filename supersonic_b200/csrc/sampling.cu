@@ -18,6 +18,7 @@
 // sum walks tokens in index order instead of probability order (the distribution is the same).
 // Each sequence owns its generator state, so a draw does not depend on what else is in the batch.
 #include "common.cuh"
+#include <stddef.h>
 #include <math.h>
 
 constexpr int SAMPLE_THREADS = 1024;
@@ -664,11 +665,13 @@ struct TopShared {
     float part[SC_CTAS * TOP_SHARES];                    // sums of the draw
     unsigned used[SC_CTAS * TOP_SHARES / 32];            // shares that hold something
     float it_before[SC_CTAS][ST_MAX_IT], it_sum[SC_CTAS][ST_MAX_IT], slice_sum[SC_CTAS];
-    unsigned maxima[TOP_GROUPS], sorted[TOP_GROUPS];
+    alignas(16) unsigned maxima[TOP_GROUPS];             // read four at a time
+    unsigned sorted[TOP_GROUPS];
     unsigned marks[SC_CTAS * TOP_MARKS], largest[SC_CTAS];        // every block's
     unsigned block_max, bound, n, n_kept, n_shares, cut, w_cut;
     int found;
 };
+static_assert(alignof(TopShared) % 16 == 0 && offsetof(TopShared, maxima) % 16 == 0, "maxima lie on 16-byte boundaries");
 // The search over the whole row and the draw's shares of weights do not meet.
 union TopScratch {
     struct { ScShared sh; RxShared rx; } row;
