@@ -785,3 +785,35 @@ def test_windowed_prompt_attention_is_the_same_bits_in_every_batch(n_q, n_kv, hd
         return out.view(seqs, n, -1)
     alone, among = run(1)[0], run(others + 1)
     assert all(torch.equal(alone, row) for row in among)
+
+
+@pytest.mark.parametrize("n", [0, 1, 128, 129, 960, 961, 1920, 2500])
+@pytest.mark.parametrize("n_before", [0, 1, 300])
+def test_a_steps_integers_come_in_their_places(n, n_before):
+    """Around the sizes of one launch's arguments and of one launch, with and without a device tensor in front; what lies beside
+    the destination stays as it is."""
+    values = torch.arange(n, dtype=torch.int32).add(7).numpy()
+    before = torch.arange(n_before, dtype=torch.int32, device=DEV).sub(500) if n_before else None
+    room = torch.full((n + n_before + 8,), -9, dtype=torch.int32, device=DEV)
+    ops().put_ints(values, room[4:4 + n + n_before], before=before)
+    values[:] = 0                                                   # taken at the call
+    want = torch.cat([torch.full((4,), -9), torch.arange(n_before) - 500, torch.arange(n) + 7, torch.full((4,), -9)])
+    assert torch.equal(room.cpu().long(), want)
+
+
+@pytest.mark.parametrize("n_states", [0, 1, 96, 97, 200])
+def test_an_opened_sequence_starts_from_zeros(n_states):
+    """No state rows, a launch's worth of them and more, rows from one word to more than a block's share; other slots keep theirs."""
+    rng = torch.arange(5, dtype=torch.int64, device=DEV)
+    states = [torch.full((5, 1 + 37 * i if i != 1 else 300001), 3.0, device=DEV) for i in range(n_states)]
+    ops().open_sequence(rng, 2, -1234567890123456789, states)
+    assert rng.tolist() == [0, 1, -1234567890123456789, 3, 4]
+    keep = torch.tensor([0, 1, 3, 4], device=DEV)
+    assert all(bool((t[2] == 0).all()) and bool((t[keep] == 3).all()) for t in states)
+    with pytest.raises(ops().KernelError, match="slot"):
+        ops().open_sequence(rng, 5, 1, states)
+
+
+def test_the_host_and_the_kernel_agree_on_the_integers_a_launch_takes():
+    from supersonic_b200.csrc.build import load_library
+    assert load_library("step_inputs").ssb_put_ints_most() == ops().PUT_INTS_MOST
