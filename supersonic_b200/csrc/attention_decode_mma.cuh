@@ -179,8 +179,11 @@ attention_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, __nv_b
         if (unequal && fine_pages >= 8) {
             chunk_pages = (int)fine_pages;
         } else {
-            // the smallest of some sizes, the last of which cuts nothing, whose items the blocks take in one go
+            // the smallest of some sizes, the last of which cuts nothing, whose items the blocks take in one go.  Cutting nothing
+            // is for sequences that two waves of the coarse size would not be done with sooner: 31 sequences of 100 tokens and one
+            // of 8,000, heads of 128, uncut 106 us, in chunks of seven pages 16
             const int least = (int)max((long long)ADM_MIN_CHUNK, (units + gridDim.x - 1) / (long long)gridDim.x);
+            const int two_waves = (int)max((long long)ADM_MIN_CHUNK, (units + coarse - 1) / coarse);
             auto size_of = [&](int i) { return i == ADM_SIZES - 1 ? max(longest, 1) : least + (i < 5 ? i : 2 * i - 4); };
             int items[ADM_SIZES];
 #pragma unroll
@@ -196,12 +199,12 @@ attention_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, __nv_b
                 if (lane == 0) warp_items[warp][i] = sum;
             }
             __syncthreads();
-            chunk_pages = (int)max((long long)ADM_MIN_CHUNK, (units + coarse - 1) / coarse);
+            chunk_pages = two_waves;
 #pragma unroll
             for (int i = ADM_SIZES - 1; i >= 0; --i) {
                 long long sum = 0;
                 for (int w = 0; w < ADM_WARPS; ++w) sum += warp_items[w][i];
-                if (sum * n_kv <= (long long)gridDim.x) chunk_pages = size_of(i);
+                if (sum * n_kv <= (long long)gridDim.x && size_of(i) <= 2 * two_waves + 6) chunk_pages = size_of(i);
             }
         }
         __syncthreads();                                         // warp_total is used again below

@@ -293,6 +293,26 @@ def test_decode_attention_cuts_its_sequences_itself(hd, lens):
     o.check_device_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("hd,n_q,n_kv", [(64, 32, 8), (128, 32, 8), (128, 24, 8)])
+def test_decode_attention_cuts_a_long_sequence_beside_short_ones(hd, n_q, n_kv):
+    """So many short sequences that only uncut items would be taken in one go: the long one's parts still meet through the
+    scratch (uncut it keeps one block busy six times as long as the others take together)."""
+    o = ops()
+    B = o.sm_count() * 2 // n_kv - 5                                # of two blocks a multiprocessor, all but a few have an item
+    lens = [100] * (B - 1) + [8000]
+    k, v = (rnd(125, n_kv, 64, hd, seed=s, dtype=torch.bfloat16) for s in (1, 2))
+    table = torch.arange(125, dtype=torch.int32, device=DEV).repeat(B, 1)
+    q, out = rnd(B, n_q * hd, seed=3, dtype=torch.bfloat16), torch.empty(B, n_q * hd, dtype=torch.bfloat16, device=DEV)
+    chunks = o.sm_count() * 2 // n_kv
+    nf, nc = o.attention_decode_chunked_scratch(B, n_q, n_kv, hd, chunks)
+    scratch, counters = torch.full((nf,), math.nan, device=DEV), torch.zeros(nc, dtype=torch.int32, device=DEV)
+    o.attention_decode_chunked(q, k, v, torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV),
+                               torch.arange(B, dtype=torch.int32, device=DEV), table, out, n_q, n_kv, hd, 6, None, hd ** -0.5, 0, chunks,
+                               scratch, counters)
+    o.check_device_errors(torch.device(DEV))
+    assert bool((~scratch.isnan()).any())
+
+
 @pytest.mark.parametrize("hd,n_q,n_kv,T", [(64, 8, 2, 37), (128, 6, 3, 5), (64, 32, 8, 131), (8, 1, 1, 1)])
 def test_rotation_from_split_sums_is_the_two_launches_bit_for_bit(hd, n_q, n_kv, T):
     """Rounding, rotation and append in one pass; a padding row's sums are cleared and nothing else."""
