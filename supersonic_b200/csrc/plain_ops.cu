@@ -300,20 +300,22 @@ __device__ __forceinline__ void rotate_pair(float x1, float x2, float c, float s
     y2 = ssb_from_float<T>(x1 * sn + x2 * c);
 }
 
-constexpr int RO_HEADS = 8;                              // heads (of q, k and v) a block: few tokens still make many blocks
+// Heads (of q, k and v) a block where tokens are few, so that they make many: all of a token's where that makes more than eight
+// blocks an SM.  us with all and with eight, 48 heads of 64 in all: 1 token 3.3 and 1.8, 131 3.5 and 3.1, 900 7.1 and 10.1, 8,000 55
+// and 82; 48 of 128: 5.2 and 2.2, 5.3 and 3.9, 11.9 and 13.7, 102 and 124.
+constexpr int RO_HEADS = 8;
 
 template <typename T>
 __global__ void __launch_bounds__(256)
 rope_append_kernel(T* __restrict__ qkv, int ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                    int table_positions, const int* __restrict__ pos, const int* __restrict__ slot,
                    const int* __restrict__ page_table, int max_pages, T* __restrict__ k_cache, T* __restrict__ v_cache, int n_q,
-                   int n_kv, int head_dim, int rotary_dim, int page_shift, int write_cache, int interleaved) {
+                   int n_kv, int head_dim, int rotary_dim, int page_shift, int write_cache, int interleaved, int per_block) {
     ssb_pdl_launch_dependents();
     ssb_pdl_wait();
-    const int t = blockIdx.x, h0 = blockIdx.y * RO_HEADS;
-    const int s = slot[t];
+    const int t = blockIdx.x, h0 = blockIdx.y * per_block;
+    const int s = slot[t], p = pos[t];
     if (s < 0) return;                                   // padding row
-    const int p = pos[t];
     const int half = rotary_dim / 2, rest = head_dim - rotary_dim;
     T* row = qkv + (size_t)t * ld;
     const bool have_table = (cos_t != nullptr) && p < table_positions;
@@ -324,7 +326,7 @@ rope_append_kernel(T* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
     const size_t head_rows = (size_t)1 << page_shift;
     // rotate q heads (and k heads): pairs (i, i + half) of the first rotary_dim elements, or (interleaved) pairs
     // (2i, 2i + 1); what a thread has rotated of a key it also appends
-    const int rot_end = min(h0 + RO_HEADS, write_cache ? n_q + n_kv : n_q);
+    const int rot_end = min(h0 + per_block, write_cache ? n_q + n_kv : n_q);
     for (int e = threadIdx.x; e < (rot_end - h0) * half; e += blockDim.x) {
         const int h = h0 + e / half, i = e % half;
         T* x = row + (size_t)h * head_dim;
@@ -343,12 +345,12 @@ rope_append_kernel(T* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
     }
     if (!write_cache) return;
     // what is appended as it is: a key's elements behind the rotated ones, and values
-    const int k_first = max(h0, n_q), k_end = min(h0 + RO_HEADS, n_q + n_kv);
+    const int k_first = max(h0, n_q), k_end = min(h0 + per_block, n_q + n_kv);
     for (int e = threadIdx.x; e < (k_end - k_first) * rest; e += blockDim.x) {
         const int h = k_first + e / rest, d = rotary_dim + e % rest;
         k_cache[(tok + (h - n_q) * head_rows) * head_dim + d] = row[(size_t)h * head_dim + d];
     }
-    const int v_first = max(h0, n_q + n_kv), v_end = min(h0 + RO_HEADS, n_q + 2 * n_kv);
+    const int v_first = max(h0, n_q + n_kv), v_end = min(h0 + per_block, n_q + 2 * n_kv);
     for (int e = threadIdx.x; e < (v_end - v_first) * head_dim; e += blockDim.x) {
         const int h = v_first + e / head_dim, d = e % head_dim;
         v_cache[(tok + (h - n_q - n_kv) * head_rows) * head_dim + d] = row[(size_t)h * head_dim + d];
@@ -364,16 +366,17 @@ SSB_API int ssb_rope_append(void* qkv, int ld, int dtype, const float* cos_t, co
     if (rotary_dim % 2 || rotary_dim > head_dim || rotary_dim < 0) return SSB_ERR_BAD_SIZE;
     const int heads = write_cache ? n_q + 2 * n_kv : n_q;
     if (heads > RO_HEADS * 65535) return SSB_ERR_BAD_SIZE;
-    const dim3 grid(n_tokens, (heads + RO_HEADS - 1) / RO_HEADS);
+    const int groups = (heads + RO_HEADS - 1) / RO_HEADS, per_block = (long long)n_tokens * groups <= 8 * gf_sms() ? RO_HEADS : heads;
+    const dim3 grid(n_tokens, (heads + per_block - 1) / per_block);
     int rc;
     if (dtype == SSB_F32)
         rc = ssb_launch(rope_append_kernel<float>, grid, dim3(256), 0, stream, pdl != 0, (float*)qkv, ld, cos_t, sin_t,
                         table_positions, pos, slot, page_table, max_pages, (float*)k_cache, (float*)v_cache, n_q, n_kv, head_dim,
-                        rotary_dim, page_shift, write_cache, interleaved);
+                        rotary_dim, page_shift, write_cache, interleaved, per_block);
     else if (dtype == SSB_BF16)
         rc = ssb_launch(rope_append_kernel<bf16>, grid, dim3(256), 0, stream, pdl != 0, (bf16*)qkv, ld, cos_t, sin_t,
                         table_positions, pos, slot, page_table, max_pages, (bf16*)k_cache, (bf16*)v_cache, n_q, n_kv, head_dim,
-                        rotary_dim, page_shift, write_cache, interleaved);
+                        rotary_dim, page_shift, write_cache, interleaved, per_block);
     else
         return SSB_ERR_BAD_DTYPE;
     return rc ? rc : ssb_launch_status();

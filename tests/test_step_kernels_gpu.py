@@ -837,3 +837,25 @@ def test_an_opened_sequence_starts_from_zeros(n_states):
 def test_the_host_and_the_kernel_agree_on_the_integers_a_launch_takes():
     from supersonic_b200.csrc.build import load_library
     assert load_library("step_inputs").ssb_put_ints_most() == ops().PUT_INTS_MOST
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n_q,n_kv,hd,rot,interleaved,T", [(6, 3, 64, 64, False, 700), (5, 1, 24, 8, True, 1400), (17, 2, 32, 0, False, 500)])
+def test_rotation_of_many_tokens_is_that_of_a_few(dtype, n_q, n_kv, hd, rot, interleaved, T):
+    """So many tokens that a block takes all of one's heads, and the same tokens seven at a time (eight heads a block)."""
+    o = ops()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos, slot = i32([t // 2 for t in range(T)]), i32([-1 if t % 50 == 7 else t % 2 for t in range(T)])
+    pages = T // 128 + 1
+    table = torch.randperm(2 * pages, generator=torch.Generator().manual_seed(T)).to(torch.int32).view(2, pages).to(DEV)
+    cos, sin = rnd(T // 2 - 3, rot // 2, seed=5), rnd(T // 2 - 3, rot // 2, seed=6)
+    qkv = rnd(T, (n_q + 2 * n_kv) * hd, seed=3, dtype=dtype)
+    got = []
+    for step in (T, 7):
+        x, k, v = qkv.clone(), torch.zeros(2 * pages, n_kv, 64, hd, dtype=dtype, device=DEV), torch.zeros(2 * pages, n_kv, 64, hd, dtype=dtype, device=DEV)
+        for a in range(0, T, step):
+            b = slice(a, a + step)
+            o.rope_append(x[b], cos if rot else None, sin if rot else None, pos[b], slot[b], table, k, v, n_q, n_kv, hd, rot, 6,
+                          interleaved=interleaved)
+        got.append((x, k, v))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and not torch.equal(got[0][1], torch.zeros_like(got[0][1]))
