@@ -25,6 +25,17 @@ enum {
 
 static inline int ssb_launch_status() { return (int)cudaGetLastError(); }
 
+// Multiprocessors of the current device (of the first one that asked: a process's devices are alike).
+static inline int ssb_sm_count() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
+        sms = n;
+    }
+    return sms;
+}
+
 __device__ __forceinline__ float ssb_to_float(float x) { return x; }
 __device__ __forceinline__ float ssb_to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
 template <typename T> __device__ __forceinline__ T ssb_from_float(float x);

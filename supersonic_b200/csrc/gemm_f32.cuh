@@ -6,16 +6,6 @@
 #pragma once
 #include "packed_f32.cuh"
 
-static inline int gf_sms() {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
-        sms = n;
-    }
-    return sms;
-}
-
 constexpr int GF_CHUNK = 16;               // products of one FMA chain
 constexpr int GF_LD = GF_CHUNK + 4;        // a chunk's place in shared memory: 80 bytes, so that eight neighbouring chunks
                                            // (or rows) start in eight different groups of four banks
@@ -200,7 +190,7 @@ static inline bool gf_walk_ok(int M, int K) {
     return M <= 4 && gf_walk_rows(M <= 2 ? M : 4, K) + 7 * GF_WALK_RING <= GF_WALK_SMEM;
 }
 // Rows of W a warp: as many as leave six warps an SM something to do.
-static inline int gf_walk_width(int N) { return N > 24 * gf_sms() ? 4 : N > 12 * gf_sms() ? 2 : 1; }
+static inline int gf_walk_width(int N) { return N > 24 * ssb_sm_count() ? 4 : N > 12 * ssb_sm_count() ? 2 : 1; }
 
 // The chunks' sums of a step, one of each of MB rows a lane, in; those of this lane's row (its chunk modulo MB) in k order out.
 template <int MB, int RW>
@@ -780,7 +770,7 @@ static inline bool gemm_f32_ok(const void* A, int lda, long long a_batch, const 
 // with 64 x 64; 500 x 2048 181 with 128 x 64, 217; 1000 x 2048 217 and 318.  K 64: 300 x 64 5.3 with 16 rows, 6.5 with tiles of
 // 64; 16 x 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.
 static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
-    const long long sms = gf_sms(), chunks = (K + 15) / 16, turns = (K + 511) / 512;
+    const long long sms = ssb_sm_count(), chunks = (K + 15) / 16, turns = (K + 511) / 512;
     const auto waves = [&](int rows, int cols) {
         return ((long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols) * n_batch + sms - 1) / sms;
     };
@@ -825,7 +815,7 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         const long long tiles = (long long)groups * ((N + 8 * R - 1) / (8 * R)); \
         if (tiles > 0x7fffffffLL) return SSB_ERR_BAD_SIZE; \
         /* as many blocks as are resident at once (by shared memory), each walking its share of the tiles */ \
-        const long long held = gf_sms() * (228 * 1024 / (long long)(smem + 1024)); \
+        const long long held = ssb_sm_count() * (228 * 1024 / (long long)(smem + 1024)); \
         const long long blocks = tiles < held ? tiles : held; \
         kernel<<<dim3((unsigned)blocks, 1, n_batch), GF_PRODUCT_THREADS + gf_adders(MB, R), smem, stream>>>( \
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, groups, accumulate); \
@@ -843,7 +833,7 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         const size_t rows = gf_walk_rows(MB, K); \
         auto kernel = gemm_f32_walk_kernel<MB, RW, ##__VA_ARGS__>; \
         GF_CONFIGURE(kernel, GF_WALK_SMEM); \
-        const int tasks = (N + RW - 1) / RW, blocks = tasks < gf_sms() ? tasks : gf_sms(), room = (int)((GF_WALK_SMEM - rows) / GF_WALK_RING); \
+        const int tasks = (N + RW - 1) / RW, blocks = tasks < ssb_sm_count() ? tasks : ssb_sm_count(), room = (int)((GF_WALK_SMEM - rows) / GF_WALK_RING); \
         int warps = (tasks + blocks - 1) / blocks; \
         warps = warps > GF_WALK_WARPS ? GF_WALK_WARPS : warps; \
         warps = warps > room ? room : warps; \
@@ -862,7 +852,7 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         GF_CONFIGURE(kernel, smem); \
         const long long tiles = (long long)((N + 16 * RN - 1) / (16 * RN)) * ((M + 16 * RM - 1) / (16 * RM)); \
         if (tiles > 0x7fffffffLL) return SSB_ERR_BAD_SIZE; \
-        kernel<<<dim3((unsigned)(tiles < gf_sms() ? tiles : gf_sms()), 1, n_batch), GF_ROLE_ALL, smem, stream>>>( \
+        kernel<<<dim3((unsigned)(tiles < ssb_sm_count() ? tiles : ssb_sm_count()), 1, n_batch), GF_ROLE_ALL, smem, stream>>>( \
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
     } while (0)
 #define GF_PARTS(RM, RN) do { \
@@ -871,7 +861,7 @@ static inline int gemm_f32_launch(const float* A, int lda, long long a_batch, co
         GF_CONFIGURE(kernel, smem); \
         const long long tiles = (long long)((N + 4 * RN - 1) / (4 * RN)) * ((M + 8 * RM - 1) / (8 * RM)); \
         if (tiles > 0x7fffffffLL) return SSB_ERR_BAD_SIZE; \
-        kernel<<<dim3((unsigned)(tiles < gf_sms() ? tiles : gf_sms()), 1, n_batch), 32 * GF_PART_WARPS, smem, stream>>>( \
+        kernel<<<dim3((unsigned)(tiles < ssb_sm_count() ? tiles : ssb_sm_count()), 1, n_batch), 32 * GF_PART_WARPS, smem, stream>>>( \
             A, lda, W, ldw, C, ldc, M, N, K, a_batch, w_batch, c_batch, accumulate); \
     } while (0)
     switch (form) {

@@ -293,7 +293,7 @@ static int launch_gv(const CUtensorMap& mw, const CUtensorMap& mx, void* out, in
                      int N, int K, int mode, int splits, float* partials, int* counters, int* error_word, bool pdl,
                      cudaStream_t stream, int gate_kind = 0, float gate_limit = 0.f, const float* row_scale = nullptr) {
     if constexpr (gv_deep(BNB) > gv_stages(BNB))
-        if (splits == 1 && (N + GV_BM - 1) / GV_BM <= 148 && K > 2 * gv_deep(BNB) * TC_BK)
+        if (splits == 1 && (N + GV_BM - 1) / GV_BM <= ssb_sm_count() && K > 2 * gv_deep(BNB) * TC_BK)
             return launch_gv_ring<BNB, gv_deep(BNB)>(mw, mx, out, ldo, out_is_f32, n_rows, N, K, mode, splits, partials, counters,
                                                      error_word, pdl, stream, gate_kind, gate_limit, row_scale);
     return launch_gv_ring<BNB, gv_stages(BNB)>(mw, mx, out, ldo, out_is_f32, n_rows, N, K, mode, splits, partials, counters,

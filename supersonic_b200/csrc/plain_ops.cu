@@ -366,7 +366,7 @@ SSB_API int ssb_rope_append(void* qkv, int ld, int dtype, const float* cos_t, co
     if (rotary_dim % 2 || rotary_dim > head_dim || rotary_dim < 0) return SSB_ERR_BAD_SIZE;
     const int heads = write_cache ? n_q + 2 * n_kv : n_q;
     if (heads > RO_HEADS * 65535) return SSB_ERR_BAD_SIZE;
-    const int groups = (heads + RO_HEADS - 1) / RO_HEADS, per_block = (long long)n_tokens * groups <= 8 * gf_sms() ? RO_HEADS : heads;
+    const int groups = (heads + RO_HEADS - 1) / RO_HEADS, per_block = (long long)n_tokens * groups <= 8 * ssb_sm_count() ? RO_HEADS : heads;
     const dim3 grid(n_tokens, (heads + per_block - 1) / per_block);
     int rc;
     if (dtype == SSB_F32)

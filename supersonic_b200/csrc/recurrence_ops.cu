@@ -177,7 +177,7 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
     if (form == 3 && !by_token) return SSB_ERR_BAD_SIZE;
     if (by_token && (form == 3 || (form == 0 && n_tokens <= n_seqs))) {
         // 128 columns a block where that gives the SMs two blocks each
-        const bool wide = (long long)n_seqs * n_heads * ((vdim + 127) / 128) >= 2 * 148;
+        const bool wide = (long long)n_seqs * n_heads * ((vdim + 127) / 128) >= 2 * ssb_sm_count();
         const dim3 grid(n_seqs, n_heads, wide ? (vdim + 127) / 128 : (vdim + 31) / 32);
 #define SSB_GS(T, COLS)                                                                                                       \
     do {                                                                                                                      \
