@@ -505,13 +505,46 @@ attention_plain_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ k
     }
 }
 
-// The same sums for float32 rows of up to 128 elements in whole 16-byte pieces: a chunk's keys and values come by cp.async,
-// all of a chunk's values and the next chunk's keys while the scores and their sums are made, instead of eight values at a time
-// behind every eight additions; a key's place is looked up once.  ROPE (decode steps): q comes as the projection left it, [q | k |
-// v] in a row; the block rotates its query and its token's key (pairs i, i + rotary_dim / 2), and the first head of a kv head
-// appends key and value.
+// The same sums for float32 rows of up to 128 elements in whole 16-byte pieces, which come through shared memory; a key's place is
+// looked up once.  ROPE (decode steps): q comes as the projection left it, [q | k | v] in a row; the block rotates its query and its
+// token's key (pairs i, i + rotary_dim / 2), and the first head of a kv head appends key and value.
 constexpr int AS_MAX_DIM = 128;
 struct AsRope { const float *cos_t, *sin_t; int table_positions, rotary_dim; float *k_cache, *v_cache; };
+
+// The block's query, rotated where ROPE, and this thread's element of the token's own key and value.
+template <bool ROPE>
+__device__ __forceinline__ void attention_own_rows(const float* __restrict__ q, int ldq, int t, int h, int s, int p, int n_q, int n_kv,
+                                                   int head_dim, const int* __restrict__ page_table, int max_pages, int page_shift,
+                                                   const AsRope& rope, float* q_s, float& own_k, float& own_v) {
+    const int tid = threadIdx.x, kvh = h / (n_q / n_kv);
+    const float* qp = q + (size_t)t * ldq + (size_t)h * head_dim;
+    if (tid >= head_dim) return;
+    float own_q = qp[tid];
+    if constexpr (ROPE) {
+        const float* row = q + (size_t)t * ldq;
+        const float* kp = row + (size_t)(n_q + kvh) * head_dim;
+        own_v = row[(size_t)(n_q + n_kv + kvh) * head_dim + tid];
+        own_k = kp[tid];
+        if (tid < rope.rotary_dim) {
+            const int half = rope.rotary_dim / 2, i = tid < half ? tid : tid - half;
+            const bool have = p < rope.table_positions;
+            const float c = have ? rope.cos_t[(size_t)p * half + i] : 1.f, sn = have ? rope.sin_t[(size_t)p * half + i] : 0.f;
+            float y1, y2;
+            rotate_pair(qp[i], qp[i + half], c, sn, y1, y2);
+            own_q = tid < half ? y1 : y2;
+            rotate_pair(kp[i], kp[i + half], c, sn, y1, y2);
+            own_k = tid < half ? y1 : y2;
+        }
+        if (h % (n_q / n_kv) == 0) {
+            const size_t at = ssb_cache_row(page_table, max_pages, s, p, page_shift, n_kv, kvh, head_dim) + tid;
+            rope.k_cache[at] = own_k;
+            rope.v_cache[at] = own_v;
+        }
+    }
+    q_s[tid] = own_q;
+}
+
+// Where rows are few: all of a chunk's values and the next chunk's keys are on their way while the scores and their sums are made.
 static size_t attention_staged_smem(int head_dim, int v_dim) {
     return sizeof(float) * (size_t)ATT_THREADS * (head_dim + 4 + v_dim);
 }
@@ -554,35 +587,8 @@ attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __res
         gf_commit();
     };
     look_up(lo, 0);
-    const float* qp = q + (size_t)t * ldq + (size_t)h * head_dim;
     float own_k = 0.f, own_v = 0.f;                      // ROPE: an element of the token's key and value
-    if constexpr (ROPE) {
-        if (tid < head_dim) {
-            const float* row = q + (size_t)t * ldq;
-            const float* kp = row + (size_t)(n_q + kvh) * head_dim;
-            own_v = row[(size_t)(n_q + n_kv + kvh) * head_dim + tid];
-            float own_q = qp[tid];
-            own_k = kp[tid];
-            if (tid < rope.rotary_dim) {
-                const int half = rope.rotary_dim / 2, i = tid < half ? tid : tid - half;
-                const bool have = p < rope.table_positions;
-                const float c = have ? rope.cos_t[(size_t)p * half + i] : 1.f, sn = have ? rope.sin_t[(size_t)p * half + i] : 0.f;
-                float y1, y2;
-                rotate_pair(qp[i], qp[i + half], c, sn, y1, y2);
-                own_q = tid < half ? y1 : y2;
-                rotate_pair(kp[i], kp[i + half], c, sn, y1, y2);
-                own_k = tid < half ? y1 : y2;
-            }
-            q_s[tid] = own_q;
-            if (h % (n_q / n_kv) == 0) {
-                const size_t at = ssb_cache_row(page_table, max_pages, s, p, page_shift, n_kv, kvh, head_dim) + tid;
-                rope.k_cache[at] = own_k;
-                rope.v_cache[at] = own_v;
-            }
-        }
-    } else {
-        if (tid < head_dim) q_s[tid] = qp[tid];
-    }
+    attention_own_rows<ROPE>(q, ldq, t, h, s, p, n_q, n_kv, head_dim, page_table, max_pages, page_shift, rope, q_s, own_k, own_v);
     __syncthreads();
     fetch(k_cache, head_dim, kq, k_s, ld, lo, 0);
     float m = -INFINITY, l = 0.f, acc = 0.f;
@@ -658,23 +664,197 @@ attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __res
     if (tid < v_dim) o[tid] = l > 0.f ? acc * keep / l : 0.f;
 }
 
+// Where rows are many: a chunk's keys come in slices of SL dims, then its values in as many bytes a time, through a ring of STAGES
+// of them that runs across chunks, 32 to 96 KB where whole chunks take 66 (heads of 64) or 132 (128), so that two to six blocks
+// share an SM.  A block that is alone on its SM takes longer so: a meeting of the block and the addresses of a fetch for every slice
+// (one sequence of 1,000 tokens, 32 heads of 128, 56 us and 46).  Bound by what L2 delivers where rows are many (64 sequences of
+// 4,000 tokens, 32 heads of 128: 8.4 GB in 1,224 us), by a chunk's chain of products and meetings where few.
+template <bool ROPE, int SL, int STAGES>
+__global__ void __launch_bounds__(ATT_THREADS)
+attention_ring_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
+                        const int* __restrict__ pos, const int* __restrict__ slot, const int* __restrict__ page_table,
+                        int max_pages, float* __restrict__ out, int ldo, int n_q, int n_kv, int head_dim, int page_shift,
+                        int window, float scale, int v_dim, int v_row, const float* __restrict__ sinks, AsRope rope) {
+    static_assert(SL % 32 == 0, "pieces are exchanged so that eight neighbouring keys' start in eight groups of banks");
+    constexpr int STAGE = ATT_THREADS * SL, PIECES = SL / 4;
+    extern __shared__ __align__(16) float ar_smem[];     // [stage]: keys as [key][SL], values as [key][v_dim]
+    __shared__ __align__(16) float q_s[AS_MAX_DIM];
+    __shared__ __align__(16) float p_s[ATT_THREADS];
+    __shared__ size_t tok_s[2][ATT_THREADS];             // a chunk's keys: their rows in the cache entry
+    __shared__ float red[ATT_THREADS / 32 + 1];
+    const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* o = out + (size_t)t * ldo + (size_t)h * v_dim;
+    ssb_pdl_launch_dependents();
+    ssb_pdl_wait();
+    const int s = slot[t], p = pos[t];
+    if (s < 0) {
+        for (int d = tid; d < v_dim; d += ATT_THREADS) o[d] = 0.f;
+        return;
+    }
+    const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
+    const int kvh = h / (n_q / n_kv);
+    auto look_up = [&](int base, int buf) {
+        if (base + tid <= p) tok_s[buf][tid] = ssb_cache_row(page_table, max_pages, s, base + tid, page_shift, n_kv, kvh, 1);
+    };
+    look_up(lo, 0);
+    float own_k = 0.f, own_v = 0.f;                      // ROPE: an element of the token's key and value
+    attention_own_rows<ROPE>(q, ldq, t, h, s, p, n_q, n_kv, head_dim, page_table, max_pages, page_shift, rope, q_s, own_k, own_v);
+    __syncthreads();
+
+    int v_keys = ATT_THREADS;                            // keys a stage of values holds: a multiple of 8
+    while (v_keys * v_dim > STAGE) v_keys >>= 1;
+    const int k_stages = (head_dim + SL - 1) / SL, v_stages = ATT_THREADS / v_keys, quads = v_dim / 4;
+    auto place = [&](int key, int piece) {               // of a slice of a key's elements
+        return key * SL + ((piece ^ (key & 7)) << 2);
+    };
+    int ahead_base = lo, ahead_stage = 0, ahead_slot = 0, ahead_buf = 0;          // the stage that is fetched next
+    auto fetch = [&]() {
+        // the chunk's keys, and those of them that are in the cache (ROPE: the token's own is not there yet)
+        const int n = min(ATT_THREADS, p - ahead_base + 1), cached = ROPE ? min(n, p - ahead_base) : n;
+        const int j0 = (ahead_stage - k_stages) * v_keys;
+        if (n > 0 && j0 < n) {
+            float* dst = ar_smem + ahead_slot * STAGE;
+            if (j0 < 0) {
+                if (ahead_stage == 0) look_up(ahead_base + ATT_THREADS, ahead_buf ^ 1);        // read from the next turn on
+                const int d0 = ahead_stage * SL;
+                for (int e = tid; e < cached * PIECES; e += ATT_THREADS) {
+                    const int r = e / PIECES, c = e % PIECES;
+                    if (d0 + c * 4 < head_dim) gf_cp16(dst + place(r, c), k_cache + tok_s[ahead_buf][r] * head_dim + d0 + c * 4, 16);
+                }
+                if (ROPE && cached < n && tid >= d0 && tid < min(d0 + SL, head_dim)) dst[place(cached, (tid - d0) / 4) + tid % 4] = own_k;
+            } else {
+                const int here = min(v_keys, cached - j0);
+                for (int e = tid; e < here * quads; e += ATT_THREADS) {
+                    const int r = e / quads, c = e % quads * 4;
+                    gf_cp16(dst + r * v_dim + c, v_cache + tok_s[ahead_buf][j0 + r] * v_row + c, 16);
+                }
+                if (ROPE && cached < n && cached - j0 < v_keys && tid < v_dim) dst[(cached - j0) * v_dim + tid] = own_v;
+            }
+        }
+        gf_commit();
+        if (++ahead_slot == STAGES) ahead_slot = 0;
+        if (++ahead_stage == k_stages + v_stages) { ahead_stage = 0; ahead_base += ATT_THREADS; ahead_buf ^= 1; }
+    };
+#pragma unroll 1
+    for (int i = 0; i < STAGES - 1; ++i) {
+        fetch();
+        __syncthreads();                                 // the next chunk's places, where one was begun
+    }
+    int at = 0;                                          // the stage in work
+    auto turn = [&]() -> const float* {
+        gf_wait<STAGES - 2>();
+        __syncthreads();                                 // it has landed, and everyone is done with the one before
+        fetch();
+        const float* src = ar_smem + at * STAGE;
+        if (++at == STAGES) at = 0;
+        return src;
+    };
+    float m = -INFINITY, l = 0.f, acc = 0.f;
+    for (int base = lo; base <= p; base += ATT_THREADS) {
+        const int n_in = min(ATT_THREADS, p - base + 1);
+        float dot = 0.f;
+        for (int st = 0; st < k_stages; ++st) {
+            const float* src = turn();
+            const float* qs = q_s + st * SL;
+            if (tid < n_in) {
+                auto add = [&](int c) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(src + place(tid, c));
+                    const float4 q4 = *reinterpret_cast<const float4*>(qs + c * 4);
+                    dot = fmaf(q4.x, k4.x, dot);
+                    dot = fmaf(q4.y, k4.y, dot);
+                    dot = fmaf(q4.z, k4.z, dot);
+                    dot = fmaf(q4.w, k4.w, dot);
+                };
+                if (head_dim - st * SL >= SL) {
+#pragma unroll 8
+                    for (int c = 0; c < PIECES; ++c) add(c);
+                } else {
+                    for (int c = 0; c < (head_dim - st * SL) / 4; ++c) add(c);
+                }
+            }
+        }
+        const float sc = tid < n_in ? dot * scale : -INFINITY;
+        float cm = sc;
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, i));
+        if (lane == 0) red[warp] = cm;
+        __syncthreads();
+        const float m_new = fmaxf(m, fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3])));
+        p_s[tid] = tid < n_in ? expf(sc - m_new) : 0.f;
+        __syncthreads();
+        if (warp == 0) {                                 // the tree of block_reduce_sum: i with i + 64, then i + 32, ...
+            float cs = (p_s[lane] + p_s[lane + 64]) + (p_s[lane + 32] + p_s[lane + 96]);
+#pragma unroll
+            for (int i = 16; i > 0; i >>= 1) cs += __shfl_down_sync(0xffffffffu, cs, i);
+            if (lane == 0) red[ATT_THREADS / 32] = cs;
+        }
+        const float alpha = (m == -INFINITY) ? 0.f : expf(m - m_new);
+        acc *= alpha;
+        for (int st = 0; st < v_stages; ++st) {
+            const int j0 = st * v_keys, here = min(v_keys, n_in - j0);
+            if (here <= 0) break;                        // the last chunk's keys
+            const float* src = turn() + tid;
+            if (st == 0) l = l * alpha + red[ATT_THREADS / 32];
+            if (tid < v_dim) {
+                int j = 0;
+                for (; j + 8 <= here; j += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] = src[(j + i) * v_dim];
+                    const float4 a = *reinterpret_cast<const float4*>(p_s + j0 + j), b = *reinterpret_cast<const float4*>(p_s + j0 + j + 4);
+                    acc = fmaf(a.x, v[0], acc); acc = fmaf(a.y, v[1], acc); acc = fmaf(a.z, v[2], acc); acc = fmaf(a.w, v[3], acc);
+                    acc = fmaf(b.x, v[4], acc); acc = fmaf(b.y, v[5], acc); acc = fmaf(b.z, v[6], acc); acc = fmaf(b.w, v[7], acc);
+                }
+                for (; j < here; ++j) acc = fmaf(p_s[j0 + j], src[j * v_dim], acc);
+            }
+        }
+        m = m_new;
+    }
+    gf_wait<0>();
+    float keep = 1.f;
+    if (sinks != nullptr) {
+        const float sk = sinks[h];
+        const float m_all = fmaxf(m, sk);
+        keep = (m == -INFINITY) ? 0.f : expf(m - m_all);
+        l = l * keep + expf(sk - m_all);
+    }
+    if (tid < v_dim) o[tid] = l > 0.f ? acc * keep / l : 0.f;
+}
+
 static bool attention_staged_takes(const void* k_cache, const void* v_cache, int head_dim, int v_dim, int v_row) {
     return head_dim <= AS_MAX_DIM && v_dim <= AS_MAX_DIM && !((head_dim | v_dim | v_row) & 3)
         && !(((uintptr_t)k_cache | (uintptr_t)v_cache) & 15);
 }
 
+// Whole chunks while the device holds all the blocks at once, else the ring, as deep as leaves the blocks of an SM room.  us of a
+// decode step's launch, 1,000 tokens a sequence, 32 heads of 64 / 128, of a plain row a block (and its rotation), whole chunks and
+// the ring: 4 sequences 91, 40, 37 / 109, 46, 60; 8 101, 41, 37 / 122, 92, 64; 16 120, 70, 56 / 203, 184, 103; 64 360, 193, 167 /
+// 474, 643, 309.  Where heads of 64 still fit, the ring gains on long contexts and loses on short ones (8 sequences of 5 tokens
+// 3.3 and 3.6).
 template <bool ROPE>
 static int attention_staged_launch(const float* q, int ldq, const float* k_cache, const float* v_cache, const int* pos, const int* slot,
                                    const int* page_table, int max_pages, float* out, int ldo, int n_tokens, int n_q, int n_kv,
                                    int head_dim, int page_shift, int window, float scale, int v_dim, int v_row, const float* sinks,
                                    AsRope rope, bool pdl, cudaStream_t stream) {
-    const cudaError_t e = cudaFuncSetAttribute(attention_staged_kernel<ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)attention_staged_smem(AS_MAX_DIM, AS_MAX_DIM));
-    if (e != cudaSuccess) return (int)e;
-    const int rc = ssb_launch(attention_staged_kernel<ROPE>, dim3(n_tokens, n_q), dim3(ATT_THREADS), attention_staged_smem(head_dim, v_dim),
-                              stream, pdl, q, ldq, k_cache, v_cache, pos, slot, page_table, max_pages, out, ldo, n_q, n_kv, head_dim,
-                              page_shift, window, scale, v_dim, v_row, sinks, rope);
-    return rc ? rc : ssb_launch_status();
+#define AS_LAUNCH(MOST, SMEM, ...) do { \
+        auto kernel = __VA_ARGS__; \
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MOST)); \
+        if (e != cudaSuccess) return (int)e; \
+        const int rc = ssb_launch(kernel, dim3(n_tokens, n_q), dim3(ATT_THREADS), SMEM, stream, pdl, q, ldq, k_cache, v_cache, pos, slot, \
+                                  page_table, max_pages, out, ldo, n_q, n_kv, head_dim, page_shift, window, scale, v_dim, v_row, sinks, rope); \
+        return rc ? rc : ssb_launch_status(); \
+    } while (0)
+#define AS_RING(SL, STAGES) AS_LAUNCH(STAGES * ATT_THREADS * SL * 4, STAGES * ATT_THREADS * SL * 4, attention_ring_kernel<ROPE, SL, STAGES>)
+    const size_t whole = attention_staged_smem(head_dim, v_dim);
+    const long long blocks = (long long)n_tokens * n_q, sms = ssb_sm_count(), room = (227 * 1024) / (whole + 4 * 1024);
+    if (blocks <= room * sms)
+        AS_LAUNCH(attention_staged_smem(AS_MAX_DIM, AS_MAX_DIM), whole, attention_staged_kernel<ROPE>);
+    if (blocks <= 2 * sms) AS_RING(64, 3);
+    if (blocks <= 3 * sms) AS_RING(64, 2);
+    if (blocks <= 4 * sms) AS_RING(32, 3);
+    AS_RING(32, 2);
+#undef AS_RING
+#undef AS_LAUNCH
 }
 
 // A float32 decode step: rotation, append and attention of one token a sequence in one launch, the bits of ssb_rope_append and

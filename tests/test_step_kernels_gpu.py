@@ -112,6 +112,50 @@ def test_float32_decode_attention_rotates_and_appends_the_same_bits(hd, rot, win
     assert torch.equal(got, want) and torch.equal(k, want_k) and torch.equal(v, want_v) and torch.equal(qkv, before)
 
 
+# blocks (a token and a head each) for two, three, four and more a multiprocessor: rings of every depth, slices and stages that are
+# not full, heads that keep whole chunks while they fit
+@pytest.mark.parametrize("blocks", [2, 3, 4, 7])
+@pytest.mark.parametrize("hd,v_dim,window,with_sinks", [(64, 64, 0, False), (128, 128, 0, True), (128, 64, 129, False), (96, 96, 0, False), (64, 100, 1, True),
+                                                        (36, 20, 200, False)])
+def test_float32_attention_of_many_rows_is_the_plain_kernels_bit_for_bit(blocks, hd, v_dim, window, with_sinks):
+    o, n_q, n_kv, slots = ops(), 6, 2, 7
+    T = o.sm_count() * blocks // n_q - 3
+    pages = 6
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos, slot = i32([(t * 37 + 126) % 380 for t in range(T)]), i32([-1 if t % 40 == 11 else t % slots for t in range(T)])
+    table = torch.randperm(slots * pages, generator=torch.Generator().manual_seed(hd)).to(torch.int32).view(slots, pages).to(DEV)
+    k, v = rnd(slots * pages, n_kv, 64, hd, seed=1), rnd(slots * pages, n_kv, 64, v_dim, seed=2)
+    v[int(table[1, 5]), 0, 63, 1] = math.inf
+    q, sinks = rnd(T, n_q * hd, seed=3, scale=2.0), rnd(n_q, seed=4) if with_sinks else None
+    outs = []
+    for kc, vc in ((off_by_one(k), off_by_one(v)), (k, v)):
+        out = torch.full((T, n_q * v_dim), 9.0, device=DEV)
+        o.attention_plain(q, kc, vc, pos, slot, table, out, n_q, n_kv, hd, 6, window or None, hd ** -0.5, value_dim=v_dim, sinks=sinks)
+        outs.append(torch.nan_to_num(out, nan=7.0))
+    assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("blocks", [2, 3, 4, 7])
+@pytest.mark.parametrize("hd,rot,window", [(64, 64, 0), (128, 64, 0), (96, 12, 130), (36, 0, 3)])
+def test_float32_decode_attention_of_many_sequences_rotates_and_appends_the_same_bits(blocks, hd, rot, window):
+    """Against the two launches it stands in for, around whole chunks and pages, with rows of no slot."""
+    o, n_q, n_kv = ops(), 6, 2
+    T = o.sm_count() * blocks // n_q - 3
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    edges = [0, 31, 32, 63, 64, 127, 128, 159, 255, 256, 300, 319]
+    pos, slot = i32([edges[t % len(edges)] for t in range(T)]), i32([-1 if t % 40 == 11 else t for t in range(T)])
+    table = torch.randperm(5 * T, generator=torch.Generator().manual_seed(hd)).to(torch.int32).view(T, 5).to(DEV)
+    k, v = rnd(5 * T, n_kv, 64, hd, seed=1), rnd(5 * T, n_kv, 64, hd, seed=2)
+    cos, sin = rnd(310, rot // 2, seed=5), rnd(310, rot // 2, seed=6)
+    qkv = rnd(T, (n_q + 2 * n_kv) * hd, seed=3, scale=2.0)
+    want_k, want_v, want_q, want = k.clone(), v.clone(), qkv.clone(), torch.empty(T, n_q * hd, device=DEV)
+    o.rope_append(want_q, cos if rot else None, sin if rot else None, pos, slot, table, want_k, want_v, n_q, n_kv, hd, rot, 6)
+    o.attention_plain(want_q, off_by_one(want_k), off_by_one(want_v), pos, slot, table, want, n_q, n_kv, hd, 6, window or None, hd ** -0.5)
+    got, before = torch.full_like(want, 9.0), qkv.clone()
+    o.attention_f32_decode(qkv, cos, sin, k, v, pos, slot, table, got, n_q, n_kv, hd, rot, 6, window or None, hd ** -0.5)
+    assert torch.equal(got, want) and torch.equal(k, want_k) and torch.equal(v, want_v) and torch.equal(qkv, before)
+
+
 @pytest.mark.parametrize("m,inter,k", [(1, 5, 2052), (2, 2001, 520), (3, 901, 36), (4, 1000, 1028), (2, 8192, 2048), (1, 1801, 64)])
 @pytest.mark.parametrize("kind,limit", [("silu", 0.0), ("clamped_swish", 2.0), ("gelu_tanh", 0.0)])
 def test_float32_gated_products_are_the_two_launches_bit_for_bit(m, inter, k, kind, limit):
