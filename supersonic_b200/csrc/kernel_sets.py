@@ -64,17 +64,19 @@ class PlainKernels:
 
     @staticmethod
     def _f32_rows_share(batch, n_q: int, n_kv: int, head_dim: int) -> bool:
-        """Whether 64 (token, head) rows of a float32 prompt share a block and its fetch of a key.  A block's time is its chain of
-        keys whatever it holds, so the rows have to fill the blocks: with few, a row a block (attention_plain) finishes all of
-        them in a shorter chain.  us a row a block and shared, 32 heads over 8, at 4,000 keys: heads of 64, 16 x 32 rows 257 and
-        374, 24 x 32 305 and 398, 32 x 32 404 and 376; of 128, 8 x 32 341 and 625, 16 x 32 680 and 580, 32 x 32 1,194 and 583.
-        Short contexts have little to share: tokens of their own, 16 x 32 rows 6.4 and 10.7 (64), 11.7 and 16.5 (128), 32 x 32
-        9.8 and 11.8, 22.9 and 17.7, 64 x 32 18.3 and 13.4, 50.7 and 20.3.  The lines are from before a row a block staged its
-        keys: at 4,000 keys they now lie at 28 tokens of such a model for heads of 64 (16 in the rule) and 14 for 128 (32)."""
-        group = n_q // n_kv
+        """Whether 64 (token, head) rows of a float32 prompt share a block and its fetch of a key.  A shared block's time is its chain
+        of keys whatever it holds, so the rows have to be many: the fewer, the longer the contexts.  us a row a block and shared, 32
+        heads over 8, on both sides of the lines: heads of 64, at 4,000 keys 32 x 32 rows 366 and 377, 40 x 32 420 and 400, 64 of
+        their own behind 64 keys 23 and 17, of their own 48 x 32 10 and 12, 64 x 32 14 and 13; of 128, at 4,000 keys 24 x 32 532 and
+        630, 32 x 32 672 and 585, of their own 56 x 32 18 and 19, 64 x 32 21 and 20, 2 x 32 x 32 16 and 17.  Blocks that do not fit at
+        once take twice as long (128 wide: one an SM), or 1.6 times where two share an SM (64 wide, 100 x 16 rows of 10 sequences
+        over 16 at 4,000 keys 501 and 633)."""
+        group, sms = n_q // n_kv, ops.sm_count()
         blocks = min(batch.n_seqs * -(-batch.max_new * group // 64), batch.n_tokens * group // 64 + batch.n_seqs) * n_kv
-        waves = -(-blocks // (ops.sm_count() * (2 if head_dim == 64 else 1)))       # an SM holds two blocks, or one
-        return batch.n_tokens * n_q >= (8 * head_dim if batch.max_total > 128 else 2048) * waves
+        waves = -(-blocks // sms) if head_dim != 64 or blocks <= sms else 1.6 * -(-blocks // (2 * sms))
+        lines = ((64, 1792), (128, 1280), (None, 1152)) if head_dim == 64 else ((32, 2304), (64, 2048), (128, 1280), (None, 1024))
+        rows = next(n for longest, n in lines if longest is None or batch.max_total <= longest)
+        return batch.n_tokens * n_q >= rows * waves
 
     def _chain(self, rows) -> bool:
         return bool(self.pdl) and int(rows) <= self.PDL_MAX_ROWS

@@ -59,12 +59,12 @@ def test_float32_prompts_of_more_sequences_than_a_grid_counts(calls):
     q, out = torch.empty(8, 128), torch.empty(8, 128)
     cache = torch.empty(1, 1, 64, 64)
     for n_seqs in (64, 65535, 65536):
-        PlainKernels().attention(q, cache, cache, batch_of(n_seqs, 8), None, out, 2, 1, 64, 6, None, 1.0)
+        PlainKernels().attention(q, cache, cache, batch_of(n_seqs, 16), None, out, 2, 1, 64, 6, None, 1.0)
     assert calls == ["attention_f32_prompt", "attention_f32_prompt", "attention_plain"]
 
 
 @pytest.mark.parametrize("head_dim,batch,shared", [
-    (64, batch_of(1, 15), False), (64, batch_of(1, 16), True), (128, batch_of(1, 31), False), (128, batch_of(1, 32), True),
+    (64, batch_of(1, 35), False), (64, batch_of(1, 36), True), (128, batch_of(1, 31), False), (128, batch_of(1, 32), True),
     (64, batch_of(1, 32, max_total=128), False), (64, batch_of(4, 16, max_total=128), True),
     (128, batch_of(64, 8, n_tokens=71), False),                      # one short prompt among 63 single tokens
     (64, batch_of(3, 500, n_tokens=890), True), (128, batch_of(16, 2048, n_tokens=18000), True)])
