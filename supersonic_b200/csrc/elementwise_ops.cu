@@ -172,7 +172,9 @@ rope_append_vec_kernel(bf16* __restrict__ qkv, int ld, const float* __restrict__
 
 // The same from the float32 sums of a projection whose K was split (round_and_clear_kernel's input, zeroed behind the read): q, k
 // and v are rounded to bfloat16, q and k rotated and rounded again, q goes to qkv's first columns, k and v to the cache alone.
-// One launch for two: 131 tokens of the 1B model 3.8 + 4.2 us of a layer and 4.6.
+// One launch for two, a piece a thread: with a token a block, whose threads took up to four pieces one after another, it was slower
+// than the two from 200 tokens of heads of 128 on.  us with the projection, two launches, a token a block and so: 131 tokens of 48
+// heads of 64 17.0, 13.4, 13.5; 256 of 40 of 128 23.9, 26.8, 21.1; 128 of 48 of 128 23.2, 23.6, 19.5.
 __global__ void __launch_bounds__(256)
 rope_append_sums_kernel(float* __restrict__ sums, bf16* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
                         const float* __restrict__ sin_t, const int* __restrict__ pos, const int* __restrict__ slot,
@@ -185,7 +187,8 @@ rope_append_sums_kernel(float* __restrict__ sums, bf16* __restrict__ qkv, int ld
     float* row = sums + (size_t)t * (n_q + 2 * n_kv) * head_dim;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     if (s < 0) {
-        for (int e = threadIdx.x; e < (n_q + 2 * n_kv) * head_dim / 4; e += 256) reinterpret_cast<float4*>(row)[e] = zero;
+        for (int e = blockIdx.y * 256 + threadIdx.x; e < (n_q + 2 * n_kv) * head_dim / 4; e += 256 * gridDim.y)
+            reinterpret_cast<float4*>(row)[e] = zero;
         return;
     }
     const int page = page_table[(size_t)s * max_pages + (p >> page_shift)];
@@ -201,26 +204,27 @@ rope_append_sums_kernel(float* __restrict__ sums, bf16* __restrict__ qkv, int ld
         const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
         return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
     };
-    for (int e = threadIdx.x; e < (n_q + n_kv) * hq; e += 256) {
-        const int h = e / hq, i4 = e % hq;
-        float4* x = reinterpret_cast<float4*>(row + (size_t)h * head_dim);
-        const float4 a = rounded(x[i4]), b = rounded(x[i4 + hq]), c = c_row[i4], sn = s_row[i4];
-        x[i4] = zero;
-        x[i4 + hq] = zero;
-        const uint2 lo = pack(a.x * c.x - b.x * sn.x, a.y * c.y - b.y * sn.y, a.z * c.z - b.z * sn.z, a.w * c.w - b.w * sn.w);
-        const uint2 hi = pack(a.x * sn.x + b.x * c.x, a.y * sn.y + b.y * c.y, a.z * sn.z + b.z * c.z, a.w * sn.w + b.w * c.w);
-        uint2* dst = reinterpret_cast<uint2*>(h < n_q ? qkv + (size_t)t * ld + (size_t)h * head_dim
-                                                      : k_cache + ((tok_base + ((size_t)(h - n_q) << page_shift)) + in_page) * head_dim);
-        dst[i4] = lo;
-        dst[i4 + hq] = hi;
-    }
-    const int v4 = head_dim / 4;
-    for (int e = threadIdx.x; e < n_kv * v4; e += 256) {
-        const int h = e / v4, j = e % v4;
-        float4* src = reinterpret_cast<float4*>(row + (size_t)(n_q + n_kv + h) * head_dim) + j;
-        const float4 x = *src;
-        *src = zero;
-        reinterpret_cast<uint2*>(v_cache + ((tok_base + ((size_t)h << page_shift)) + in_page) * head_dim)[j] = pack(x.x, x.y, x.z, x.w);
+    const int v4 = head_dim / 4, turned = (n_q + n_kv) * hq, all = turned + n_kv * v4;
+    for (int e = blockIdx.y * 256 + threadIdx.x; e < all; e += 256 * gridDim.y) {
+        if (e < turned) {
+            const int h = e / hq, i4 = e % hq;
+            float4* x = reinterpret_cast<float4*>(row + (size_t)h * head_dim);
+            const float4 a = rounded(x[i4]), b = rounded(x[i4 + hq]), c = c_row[i4], sn = s_row[i4];
+            x[i4] = zero;
+            x[i4 + hq] = zero;
+            const uint2 lo = pack(a.x * c.x - b.x * sn.x, a.y * c.y - b.y * sn.y, a.z * c.z - b.z * sn.z, a.w * c.w - b.w * sn.w);
+            const uint2 hi = pack(a.x * sn.x + b.x * c.x, a.y * sn.y + b.y * c.y, a.z * sn.z + b.z * c.z, a.w * sn.w + b.w * c.w);
+            uint2* dst = reinterpret_cast<uint2*>(h < n_q ? qkv + (size_t)t * ld + (size_t)h * head_dim
+                                                          : k_cache + ((tok_base + ((size_t)(h - n_q) << page_shift)) + in_page) * head_dim);
+            dst[i4] = lo;
+            dst[i4 + hq] = hi;
+        } else {
+            const int h = (e - turned) / v4, j = (e - turned) % v4;
+            float4* src = reinterpret_cast<float4*>(row + (size_t)(n_q + n_kv + h) * head_dim) + j;
+            const float4 x = *src;
+            *src = zero;
+            reinterpret_cast<uint2*>(v_cache + ((tok_base + ((size_t)h << page_shift)) + in_page) * head_dim)[j] = pack(x.x, x.y, x.z, x.w);
+        }
     }
 }
 
@@ -233,7 +237,8 @@ SSB_API int ssb_rope_append_sums(float* sums, void* qkv, int ld, const float* co
     if (head_dim % 8 || ld % 8 || !cos_t || !sin_t || table_positions <= 0) return SSB_ERR_BAD_SIZE;
     if (((uintptr_t)sums | (uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15)
         return SSB_ERR_BAD_SIZE;
-    const int rc = ssb_launch(rope_append_sums_kernel, dim3(n_tokens), dim3(256), 0, stream, pdl != 0, sums, (bf16*)qkv, ld, cos_t, sin_t, pos,
+    const int pieces = (n_q + n_kv) * head_dim / 8 + n_kv * head_dim / 4;
+    const int rc = ssb_launch(rope_append_sums_kernel, dim3(n_tokens, (pieces + 255) / 256), dim3(256), 0, stream, pdl != 0, sums, (bf16*)qkv, ld, cos_t, sin_t, pos,
                               slot, page_table, max_pages, (bf16*)k_cache, (bf16*)v_cache, n_q, n_kv, head_dim, page_shift);
     return rc ? rc : ssb_launch_status();
 }
