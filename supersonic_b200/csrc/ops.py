@@ -2474,8 +2474,10 @@ GEMV_ROWS_MAX = 16
 def gemv_rows_tile(rows: int, n: int, k: int) -> int:
     """Rows of W a block of :func:`gemv_rows` takes (0: not its sizes): as few as still make at most three blocks for two SMs.
     us a decode step with up to 1, 1.5, 2 and 3 blocks an SM: 8B, 1 row 2,732, 2,648, 2,656, 2,759; 3B, 2 rows 1,500, 1,448, 1,446,
-    1,500; 1B, 8 rows 658, 656, 656, 655."""
-    if rows > GEMV_ROWS_MAX or k % 64:
+    1,500; 1B, 8 rows 658, 656, 656, 655.  Up to 4,096 columns: a block streams all of K alone, and longer ones lose to K cut over
+    blocks.  us with K cut and rounded, and so, 4 rows: 3072 x 2048 5.1 and 4.0, 3072 x 4096 6.9 and 6.8, 5120 x 4096 8.7 and 8.3,
+    5120 x 5120 10.1 and 13.6, 3072 x 6144 8.5 and 11.1, 8192 x 8192 22.7 and 25.3, 2048 x 12288 10.3 and 11.6."""
+    if rows > GEMV_ROWS_MAX or k % 64 or k > 4096:
         return 0
     return next((tm for tm in (16, 32, 64) if -(-n // tm) * 2 <= 3 * sm_count()), 0)
 
