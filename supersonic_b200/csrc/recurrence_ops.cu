@@ -238,8 +238,11 @@ struct TiedArgs {
     float* sums; float* decays;
 };
 
-template <typename T, int R4, int NT, bool OUT, bool GATED, int RL>      // RL: lanes that share a column's rows, 16 or 32
-__global__ void __launch_bounds__(NT, RL == 32 ? 2 : NT == 256 && R4 == 1 ? 3 : 1)
+// Blocks an SM that the registers of a form leave room for
+constexpr int tw_sm_blocks(int r4, int nt, int rl) { return rl == 32 || (nt == 256 && r4 == 1) ? 2 : 1; }
+
+template <typename T, int R4, int NT, bool OUT, bool GATED, int RL, int SM_BLOCKS>      // RL: lanes that share a column's rows, 16 or 32
+__global__ void __launch_bounds__(NT, SM_BLOCKS)
 tied_walk_kernel(const TiedArgs a) {
     constexpr int DIMP = 64 * R4, WCOLS = 128 / RL, COLS = NT / 32 * WCOLS;  // padded rows; columns of a warp, of a block
     constexpr int RG = DIMP / (4 * RL);                    // groups of four rows a lane
@@ -458,19 +461,23 @@ tied_walk_kernel(const TiedArgs a) {
         }
 }
 
-template <typename T, int R4, int NT, bool GATED, int RL>
+template <typename T, int R4, int NT, bool GATED, int RL, int SM_BLOCKS>
 static int launch_tied_pass(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_t stream) {
     constexpr int DIMP = 64 * R4, COLS = NT / 32 * (128 / RL);
-    constexpr size_t smem = (size_t)TW_TOKENS * ((GATED ? 6 : 4) * DIMP + 4 * COLS) * sizeof(float);
+    // A block that may have an SM to itself asks for more than half of its shared memory: two would share one while others stand
+    // still (us, 4 heads of 128 x 256: 190 tokens 43 and 33, 4 x 150 47 and 39; of 256 x 512, 20 tokens 17.1 and 13.6)
+    constexpr size_t needed = (size_t)TW_TOKENS * ((GATED ? 6 : 4) * DIMP + 4 * COLS) * sizeof(float), alone = 116 * 1024,
+                     most = needed < alone ? alone : needed;
     const long long items = a.chunk > 0 ? (long long)n_seqs * a.max_chunks : n_seqs;
     const dim3 grid((unsigned)items, a.n_heads, (a.vdim + COLS - 1) / COLS);
     if (items > 0x7fffffffll || grid.y > 65535 || grid.z > 65535 || n_seqs > 65535) return SSB_ERR_BAD_SIZE;
-    static_assert(smem <= 200 * 1024, "");
-    auto sums = tied_walk_kernel<T, R4, NT, false, GATED, RL>;
-    auto outs = tied_walk_kernel<T, R4, NT, true, GATED, RL>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(outs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static_assert(most <= 200 * 1024, "");
+    const size_t smem = (long long)grid.x * grid.y * grid.z <= ssb_sm_count() ? most : needed;
+    auto sums = tied_walk_kernel<T, R4, NT, false, GATED, RL, SM_BLOCKS>;
+    auto outs = tied_walk_kernel<T, R4, NT, true, GATED, RL, SM_BLOCKS>;
+    {
+        cudaError_t e = cudaFuncSetAttribute(sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(outs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         if (e != cudaSuccess) return (int)e;
     }
     int rc;
@@ -491,9 +498,9 @@ static int launch_tied_pass(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
 
 // All of a step: in one pass where every (sequence, chunk) pair has its place in the scratch, else sequences in groups and their
 // chunks in runs, one after another.
-template <typename T, int R4, int NT, bool GATED = false, int RL = 16>
+template <typename T, int R4, int NT, bool GATED = false, int RL = 16, int SM_BLOCKS = tw_sm_blocks(R4, NT, RL)>
 static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_t stream) {
-    if (a.chunk <= 0 || (long long)n_seqs * a.max_chunks <= a.places) return launch_tied_pass<T, R4, NT, GATED, RL>(a, n_seqs, pdl, stream);
+    if (a.chunk <= 0 || (long long)n_seqs * a.max_chunks <= a.places) return launch_tied_pass<T, R4, NT, GATED, RL, SM_BLOCKS>(a, n_seqs, pdl, stream);
     const int group = n_seqs < a.places ? n_seqs : a.places, run = a.places / group;
     for (int b = 0; b < n_seqs; b += group)
         for (int c = 0; c < a.max_chunks; c += run) {
@@ -501,7 +508,7 @@ static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
             p.cu_new += b; p.seq_slot += b;
             p.chunk0 = c;
             p.max_chunks = a.max_chunks - c < run ? a.max_chunks - c : run;
-            const int rc = launch_tied_pass<T, R4, NT, GATED, RL>(p, n_seqs - b < group ? n_seqs - b : group, pdl, stream);
+            const int rc = launch_tied_pass<T, R4, NT, GATED, RL, SM_BLOCKS>(p, n_seqs - b < group ? n_seqs - b : group, pdl, stream);
             if (rc) return rc;
         }
     return 0;
@@ -510,7 +517,10 @@ static int launch_tied_walk(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
 // Blocks of 64 columns up to which a column's rows are shared by 32 lanes instead of 16, with 32 columns a block, where a head has
 // up to 128 channels: half the work a warp and token, on twice the SMs.  us with 16 and 32 lanes, 4 heads of 128 x 256, one
 // sequence, 100 tokens 49 and 41, 8 of 300 111 and 120.  Above 128 channels 32 lanes always, two blocks an SM (126 registers a thread
-// instead of 245): 4 heads of 256 x 512, 100 tokens 73 and 56, 2,048 452 and 460, 64 sequences of 2 tokens 179 and 140.
+// instead of 245): 4 heads of 256 x 512, 100 tokens 73 and 56, 2,048 452 and 460.  Between:
+// 16 lanes, with all the registers of an SM for a block (184) while there is an SM for each, else two blocks an SM (128): 4 heads of
+// 128 x 256, 2 x 190 tokens in chunks (96 blocks) 42 and 43, 8 x 300 98 and 103, 2,048 tokens in chunks (288 blocks) 138 and 116, 4 x
+// 1,000 269 and 223.
 constexpr int GATED_FEW_BLOCKS = 74;
 
 static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* decay, int ldz,
@@ -526,7 +536,8 @@ static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off,
 #define SSB_GW(T) \
     return dim <= 64 ? launch_tied_walk<T, 1, 256, true>(a, n_seqs, pdl, stream) \
          : dim <= 128 ? (narrow ? launch_tied_walk<T, 2, 256, true, 32>(a, n_seqs, pdl, stream) \
-                                : launch_tied_walk<T, 2, 256, true>(a, n_seqs, pdl, stream)) \
+                         : blocks <= ssb_sm_count() ? launch_tied_walk<T, 2, 256, true>(a, n_seqs, pdl, stream) \
+                                                    : launch_tied_walk<T, 2, 256, true, 16, 2>(a, n_seqs, pdl, stream)) \
                       : launch_tied_walk<T, 4, 256, true, 32>(a, n_seqs, pdl, stream)
     if (dtype == SSB_F32) SSB_GW(float);
     SSB_GW(bf16);

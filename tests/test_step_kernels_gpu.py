@@ -457,6 +457,48 @@ def test_gated_scan_of_one_token_a_sequence(B, H, d, dv, dtype):
     assert float((got[0][0] - got[1][0]).norm() / got[0][0].norm()) < 1e-6       # sums of d float32 products in another order
 
 
+@pytest.mark.parametrize("H,d,dv,lens", [(4, 100, 132, [5] * 80), (3, 128, 64, [1, 9, 30, 2] * 15), (1, 65, 260, [12] * 40)])
+def test_gated_scan_is_the_same_bits_whatever_shares_a_multiprocessor(H, d, dv, lens):
+    """So many sequences that two blocks share a multiprocessor, and each of them alone, in the form that does not go by the sizes."""
+    o, width = ops(), 2 * H * d + H * dv
+    T, at = sum(lens), [sum(lens[:i]) for i in range(len(lens) + 1)]
+    proj, z, bias = rnd(T, width, seed=1, dtype=torch.bfloat16), rnd(T, H * d, seed=2), rnd(H * d, seed=3) + 1.0
+    state0 = rnd(len(lens), H * d * dv, seed=4)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+
+    def run(which):
+        rows = slice(at[which[0]], at[which[-1] + 1])
+        state, out = state0.clone(), torch.full((rows.stop - rows.start, H * dv), math.nan, device=DEV)
+        o.gated_linear_scan(proj[rows], 0, H * d, 2 * H * d, z[rows].clone(), bias, 16.0, 0.25, state, i32([at[i] - rows.start for i in which] + [rows.stop - rows.start]),
+                            i32(which), out, H, d, dv, form=1)
+        return out, state
+    together, end = run(list(range(len(lens))))
+    for i in range(0, len(lens), 7):
+        out, state = run([i])
+        assert torch.equal(out, together[at[i]:at[i + 1]]) and torch.equal(state[i], end[i])
+
+
+@pytest.mark.parametrize("H,d,dv,lens", [(4, 256, 512, [2]), (2, 100, 132, [2, 1, 2]), (1, 40, 24, [1, 2] * 40), (3, 65, 30, [2, 2])])
+def test_gated_scan_of_two_tokens_a_sequence(H, d, dv, lens):
+    """The serving set's choice for them against the recurrence in 64 bits: sums of d products in float32 (2^-24 each)."""
+    from supersonic_b200.csrc.fast_sets import FastKernels
+    T, batch = sum(lens), step_of(lens, list(range(len(lens)))[::-1])
+    proj, z, bias = rnd(T, 2 * H * d + H * dv, seed=1, dtype=torch.bfloat16), rnd(T, H * d, seed=2), rnd(H * d, seed=3) + 1.0
+    state, out = rnd(len(lens), H * d * dv, seed=4), torch.full((T, H * dv), math.nan, device=DEV)
+    S, want, t = state.double().view(-1, H, d, dv).clone(), torch.empty(T, H, dv, dtype=torch.float64, device=DEV), 0
+    q, k, v = (x.double() for x in (proj[:, :H * d].view(T, H, d), proj[:, H * d:2 * H * d].view(T, H, d), proj[:, 2 * H * d:].view(T, H, dv)))
+    decay = torch.sigmoid(z.double() + bias.double()).pow(1 / 16.0).view(T, H, d)
+    for i, n in enumerate(lens):
+        s = len(lens) - 1 - i
+        for t in range(t, t + n):
+            S[s] = decay[t][..., None] * S[s] + k[t][..., None] * v[t][:, None]
+            want[t] = torch.einsum("hd,hdv->hv", 0.25 * q[t], S[s])
+        t += 1
+    FastKernels().gated_linear_scan(proj, 0, H * d, 2 * H * d, z, bias, 16.0, 0.25, state, batch, out, H, d, dv)
+    assert float((out.double() - want.view(T, -1)).norm() / want.norm()) < d ** 0.5 * 2.0 ** -23
+    assert float((state.double() - S.view_as(state)).norm() / S.norm()) < 2.0 ** -21
+
+
 def step_of(lens, slots):
     """What a kernel set reads of a step of new tokens, sequence ``i`` bringing ``lens[i]`` in ``slots[i]``."""
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
