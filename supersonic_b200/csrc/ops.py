@@ -806,14 +806,15 @@ def tied_scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim: 
 def gated_scan_chunking(n_seqs: int, max_new: int, n_heads: int, dim: int, vdim: int, sms: int):
     """(chunk, floats of sums, floats of decays) for ``gated_linear_scan``: as many chunks as give the SMs two blocks each
     (blocks own 64 value columns of a head), of 64 tokens or more, or three of 40 or more where an SM each is left for them;
-    one walk a sequence where that is no more than two chunks.  4 heads of 256 x 512, us in one walk and in three chunks: 100
-    tokens 46 and 53, 130 57 and 60, 190 79 and 74; four such sequences are slower in three chunks (every chunk walks twice)."""
+    one walk a sequence where that is no more than two chunks.  us in one walk and in three chunks, 4 heads of 256 x 512: 130 tokens
+    55 and 56, 150 62 and 64, 170 70 and 71, 190 77 and 71; of 128 x 256: 100 26 and 24, 150 38 and 30; 2 of 64 x 64: 100 27 and 21.
+    Four sequences of 256 x 512 are slower in three chunks (every chunk walks twice)."""
     blocks = max(n_seqs * n_heads * (-(-vdim // 64)), 1)
     per = n_heads * dim * vdim
     most = SCAN_SCRATCH_BYTES // (4 * per * n_seqs)
     n = min(2 * sms // blocks, max_new // 64, most)
     if n < 3:
-        if max_new < 120 or 3 * blocks > sms or most < 3:
+        if max_new < (176 if dim > 128 else 100) or 3 * blocks > sms or most < 3:
             return 0, 0, 0
         n = 3
     chunk = -(-(-(-max_new // n)) // 8) * 8           # whole turns of eight tokens
