@@ -90,6 +90,73 @@ __device__ __forceinline__ float2 adm_ld_cluster2(const float* local, unsigned r
     return v;
 }
 
+// Pages that hold keys of a sequence; a padding row is no work item.
+__device__ __forceinline__ int adm_pages(int slot, int p, int window) {
+    const int key_lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
+    return slot < 0 ? 0 : (p >> 6) - (key_lo >> 6) + 1;
+}
+
+// The pages of a chunk, from the batch's (slots and positions in shared memory); every block finds the same, and its three arrays
+// of a word a warp are free again when all threads are back.  As fine as leaves every block one item (a second wave of items
+// costs a second item's time, whatever few they are), but not below five pages, where what a cut saves is less than the meeting
+// of its parts costs.  Very unequal lengths (the longest more than one and a half times the mean) with enough work for it: two to
+// three items a block, of at least eight pages, so that the blocks end together.  us a decode step with items for four fifths of
+// the blocks, which rounding may raise above their number, and so: 1B, 64 sequences of 1 to 512 tokens 1,032 and 960, 32 of 260
+// 820 and 807, 40 of 1 to 1,829 1,175 and 1,050; 3B, 16 of 64 to 2,022 1,872 and 1,828.  A caller that wants a sequence cut
+// the same way in every batch gives its pages itself.  A step's device time, us, with all eight sizes weighed by every launch and 64-bit
+// divisions, and so: 1B, 64 sequences of 20 tokens 832 and 814; 3B, 128 of 20 2,470 and 2,425, 20 of 520 1,802 and 1,785; 1B, 40 of
+// 4,000 1,765 and 1,818.
+__device__ __forceinline__ int adm_chunk_pages(const int* sm_slot, const int* sm_pos, int n_seqs, int n_kv, int window, int* warp_total,
+                                               int* warp_longest, int* warp_live) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, blocks = (int)gridDim.x;
+    int local = 0, longest = 0, live = 0;
+    for (int b = threadIdx.x; b < n_seqs; b += ADM_THREADS) {
+        const int n = adm_pages(sm_slot[b], sm_pos[b], window);
+        local += n;
+        longest = max(longest, n);
+        live += n > 0;
+    }
+    local = __reduce_add_sync(0xffffffffu, local);
+    live = __reduce_add_sync(0xffffffffu, live);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (lane == 0) { warp_total[warp] = local; warp_longest[warp] = longest; warp_live[warp] = live; }
+    __syncthreads();
+    long long pages = 0;
+    int seqs = 0;
+    for (int w = 0; w < ADM_WARPS; ++w) { pages += warp_total[w]; seqs += warp_live[w]; longest = max(longest, warp_longest[w]); }
+    __syncthreads();
+    const bool unequal = 2LL * longest * seqs > 3LL * pages;                // longest > 1.5 x mean
+    const unsigned units = (unsigned)min(pages * n_kv, 1LL << 31), coarse = max(1, blocks * 4 / 5), fine = max(1, blocks * 5 / 2);
+    const unsigned fine_pages = (units + fine - 1) / fine;
+    if (unequal && fine_pages >= 8) return (int)fine_pages;
+    const int two_waves = max(ADM_MIN_CHUNK, (int)((units + coarse - 1) / coarse));
+    // Nothing to look for where every sequence is one item of any size, or the sequences alone are more than the blocks take in one
+    // go.
+    if (longest <= ADM_MIN_CHUNK || (long long)seqs * n_kv > blocks) return two_waves;
+    // the smallest of some sizes, the last of which cuts nothing, whose items the blocks take in one go; every warp finds the same.
+    // Cutting nothing is for sequences that two waves of the coarse size would not be done with sooner: 31 sequences of 100 tokens
+    // and one of 8,000, heads of 128, uncut 106 us, in chunks of seven pages 16
+    const int least = max(ADM_MIN_CHUNK, (int)((units + blocks - 1) / blocks));
+    auto size_of = [&](int i) { return i == ADM_SIZES - 1 ? longest : least + (i < 5 ? i : 2 * i - 4); };
+    int items[ADM_SIZES];
+    float inverse[ADM_SIZES];
+#pragma unroll
+    for (int i = 0; i < ADM_SIZES; ++i) { items[i] = 0; inverse[i] = 1.0f / (float)size_of(i); }
+    for (int b = lane; b < n_seqs; b += 32) {
+        // ceil(n / size) = floor((n - 1/2) / size) + 1, exact for up to a million pages
+        const int n = adm_pages(sm_slot[b], sm_pos[b], window);
+#pragma unroll
+        for (int i = 0; i < ADM_SIZES; ++i) items[i] += n > 0 ? (int)(((float)n - 0.5f) * inverse[i]) + 1 : 0;
+    }
+    int chunk = two_waves;
+#pragma unroll
+    for (int i = ADM_SIZES - 1; i >= 0; --i) {
+        const long long all = __reduce_add_sync(0xffffffffu, items[i]);
+        if (all * n_kv <= blocks && size_of(i) <= 2 * two_waves + 6) chunk = size_of(i);
+    }
+    return chunk;
+}
+
 template <int HD, bool FUSE, bool CL, int NT>   // NT: tiles of 8 query heads per kv head (1: up to 8 heads, 2: up to 16)
 __global__ void __launch_bounds__(ADM_THREADS)
 attention_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, __nv_bfloat16* k_cache,
@@ -122,7 +189,7 @@ attention_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, __nv_b
     __shared__ int sm_abort[2];                                  // [0]: a wait ran out; [1]: stays zero
     volatile int* abort_flag = sm_abort;
     const uint32_t full0 = smem_u32(full_bar);
-    __shared__ int warp_total[ADM_WARPS], warp_longest[ADM_WARPS], warp_live[ADM_WARPS], warp_items[ADM_WARPS][ADM_SIZES];
+    __shared__ int warp_total[ADM_WARPS], warp_longest[ADM_WARPS], warp_live[ADM_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 
     ssb_pdl_launch_dependents();
@@ -137,78 +204,9 @@ attention_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, __nv_b
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
-    auto pages_of = [&](int b) {
-        if (sm_slot[b] < 0) return 0;                            // a padding row is no work item (zeros below)
-        const int p = sm_pos[b];
-        const int key_lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
-        return (p >> 6) - (key_lo >> 6) + 1;
-    };
-    // chunk_pages <= 0: the kernel sizes the chunks itself from the batch's pages; every block computes
-    // the same figure.  As fine as leaves every block one item (a second wave of items costs a second item's time, whatever
-    // few they are), but not below five pages, where what a cut saves is less than the meeting of its parts costs.  Very
-    // unequal lengths (the longest more than one and a half times the mean) with enough work for it: two to three items a
-    // block, of at least eight pages, so that the blocks end together.  us a decode step with items for four fifths of the
-    // blocks, which rounding may raise above their number, and so: 1B, 64 sequences of 1 to 512 tokens 1,032 and 960, 32 of 260
-    // 820 and 807, 40 of 1 to 1,829 1,175 and 1,050; 3B, 16 of 64 to 2,022 1,872 and 1,828.  A caller that wants a sequence cut
-    // the same way in every batch gives chunk_pages itself.
+    auto pages_of = [&](int b) { return adm_pages(sm_slot[b], sm_pos[b], window); };
     const int n_cl = CL ? (int)adm_cluster_size() : 1;          // blocks of a cluster: the chunks of every sequence
-    if (!CL && chunk_pages <= 0) {
-        int local = 0, longest = 0, live = 0;
-        for (int b = threadIdx.x; b < n_seqs; b += ADM_THREADS) {
-            const int n = pages_of(b);
-            local += n;
-            longest = max(longest, n);
-            live += n > 0;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            local += __shfl_xor_sync(0xffffffffu, local, o);
-            live += __shfl_xor_sync(0xffffffffu, live, o);
-            longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
-        }
-        if (lane == 0) { warp_total[warp] = local; warp_longest[warp] = longest; warp_live[warp] = live; }
-        __syncthreads();
-        long long units = 0;
-        int seqs = 0;
-        longest = 0;
-        for (int w = 0; w < ADM_WARPS; ++w) { units += warp_total[w]; seqs += warp_live[w]; longest = max(longest, warp_longest[w]); }
-        const bool unequal = 2LL * longest * seqs > 3LL * units;            // longest > 1.5 x mean
-        units *= n_kv;
-        const long long coarse = max(1LL, (long long)gridDim.x * 4 / 5), fine = max(1LL, (long long)gridDim.x * 5 / 2);
-        const long long fine_pages = (units + fine - 1) / fine;
-        if (unequal && fine_pages >= 8) {
-            chunk_pages = (int)fine_pages;
-        } else {
-            // the smallest of some sizes, the last of which cuts nothing, whose items the blocks take in one go.  Cutting nothing
-            // is for sequences that two waves of the coarse size would not be done with sooner: 31 sequences of 100 tokens and one
-            // of 8,000, heads of 128, uncut 106 us, in chunks of seven pages 16
-            const int least = (int)max((long long)ADM_MIN_CHUNK, (units + gridDim.x - 1) / (long long)gridDim.x);
-            const int two_waves = (int)max((long long)ADM_MIN_CHUNK, (units + coarse - 1) / coarse);
-            auto size_of = [&](int i) { return i == ADM_SIZES - 1 ? max(longest, 1) : least + (i < 5 ? i : 2 * i - 4); };
-            int items[ADM_SIZES];
-#pragma unroll
-            for (int i = 0; i < ADM_SIZES; ++i) items[i] = 0;
-            for (int b = threadIdx.x; b < n_seqs; b += ADM_THREADS) {
-                const int n = pages_of(b);
-#pragma unroll
-                for (int i = 0; i < ADM_SIZES; ++i) items[i] += (n + size_of(i) - 1) / size_of(i);
-            }
-#pragma unroll
-            for (int i = 0; i < ADM_SIZES; ++i) {
-                const int sum = __reduce_add_sync(0xffffffffu, items[i]);
-                if (lane == 0) warp_items[warp][i] = sum;
-            }
-            __syncthreads();
-            chunk_pages = two_waves;
-#pragma unroll
-            for (int i = ADM_SIZES - 1; i >= 0; --i) {
-                long long sum = 0;
-                for (int w = 0; w < ADM_WARPS; ++w) sum += warp_items[w][i];
-                if (sum * n_kv <= (long long)gridDim.x && size_of(i) <= 2 * two_waves + 6) chunk_pages = size_of(i);
-            }
-        }
-        __syncthreads();                                         // warp_total is used again below
-    }
+    if (!CL && chunk_pages <= 0) chunk_pages = adm_chunk_pages(sm_slot, sm_pos, n_seqs, n_kv, window, warp_total, warp_longest, warp_live);
     auto chunks_of = [&](int b) {
         const int n = pages_of(b);
         return n == 0 ? 0 : min((n + chunk_pages - 1) / chunk_pages, max_chunks);
