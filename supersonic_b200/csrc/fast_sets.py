@@ -263,8 +263,11 @@ class FastKernels(PlainKernels):
         step of 16 layers: batch 1 1,566 to 1,509 us, batch 2 1,564 to 1,531, batch 8 1,634 to 1,621."""
         if self.deterministic:
             return 0
-        if pages <= 3:                      # nothing to share, or a page each: us a step of one sequence in eights and so, 1B, 20
-            return 2 if pages > 1 and heads * 2 <= min(blocks, ops.sm_count()) else 0      # keys 635 and 626, 8B, 60 2,712 and 2,660
+        # nothing to share on one page; two or three are a block's or two.  us a step, in eights and so (a page: 20 and 60 keys): 1B,
+        # one sequence, 20 keys 635 and 626, 180 630 and 624, 2 of 130 621 and 634, 8 of 130 638 and 638; 3B, 2 of 130 1,448 and
+        # 1,441; 8B, one of 60 2,712 and 2,660, of 100 2,707 and 2,672, 4 of 180 2,707 and 2,689, 9 of 130 2,739 and 2,740
+        if pages <= 3:
+            return 2 if pages > 1 and heads * 2 <= min(blocks, ops.sm_count()) else 0
         for c in (8, 4, 2):
             if heads * c <= min(blocks, ops.sm_count()):
                 return c if pages <= CLUSTER_CHUNK_PAGES * c else 0

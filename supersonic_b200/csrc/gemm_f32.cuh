@@ -638,9 +638,11 @@ gemm_f32_role_kernel(const float* __restrict__ A, int lda, const float* __restri
 // warps take a chunk of k each of one tile of 8 RM x 4 RN results, RM x RN a lane, from rows as they lie in memory; the chunks' sums
 // go through shared memory to the threads that own the results, which add them in k order while the next turn is multiplied.
 // Bound by the shared-memory reads beside the multiply-adds (12 of 16 bytes for 128 multiply-adds a lane, then a chunk's sums
-// written and read).  us before (16 rows at a time, or tiles of 64 x 64) and here: tiles of 64 x 16, 64 x 2048 x 2048 51 and 34, 64 x
-// 2048 x 8192 193 and 125, 100 x 2048 x 8192 333 and 246, 300 x 2048 x 2048 181 and 155, 200 x 512 x 128 9.4 and 4.3; of 32 x 32, 32 x 16384 x 2048 170 and 152, 32 x 4096 x 4096 98 and 77.  Tiles of
-// 64 x 32, 8 x 8 results a lane: 72, and 284 for 64 x 16384 x 2048 (191 with tiles of 64 x 64, 219 of 64 x 16).
+// written and read).  us before (16 rows at a time, or tiles of 64 x 64) and here, rows x columns x k:
+//   tiles of 64 x 16: 64 x 2048 x 2048 51 and 34, 64 x 2048 x 8192 193 and 125, 100 x 2048 x 8192 333 and 246, 300 x 2048 x 2048 181
+//   and 155, 200 x 512 x 128 9.4 and 4.3;
+//   tiles of 32 x 32: 32 x 16384 x 2048 170 and 152, 32 x 4096 x 4096 98 and 77.
+// Tiles of 64 x 32, 8 x 8 results a lane: 64 x 2048 x 2048 72, 64 x 16384 x 2048 284 (191 with tiles of 64 x 64, 219 of 64 x 16).
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int GF_PART_WARPS = 8, GF_PART_K = GF_PART_WARPS * GF_CHUNK, GF_PART_LD = GF_PART_K + 4, GF_PART_STAGES = 3;
 template <int RM, int RN>

@@ -1005,8 +1005,8 @@ def matrix_state_scan(proj: torch.Tensor, r_off: int, k_off: int, v_off: int, de
                       n_heads: int, dim: int, vdim: int, unit: Optional[torch.Tensor] = None,
                       bonus: Optional[torch.Tensor] = None, pdl: bool = False) -> None:
     """Per sequence and head over the sequence's new tokens in order, S [dim, vdim] float32 read from and left in
-    ``state[slot]`` (kept there as [heads, vdim, dim]: a value column's rows together).  ``"delta"``: S = diag(w) S - (a u)(u^T S) + k v^T, out = S^T r, with ``unit`` = [u | a u] as
-    ``state_scan_prepare`` leaves it; ``"bonus"``: out = (S + diag(bonus) k v^T)^T r, then S = diag(w) S + k v^T.
+    ``state[slot]`` (kept there as [heads, vdim, dim]: a value column's rows together).  ``"delta"``: S = diag(w) S - (a u)(u^T S) +
+    k v^T, out = S^T r, with ``unit`` = [u | a u] as ``state_scan_prepare`` leaves it; ``"bonus"``: out = (S + diag(bonus) k v^T)^T r, then S = diag(w) S + k v^T.
     ``decay`` [T, heads x dim] float32 holds w, or log w if ``proj`` is float32 (that path takes the exponential in
     double and carries the state of a step's tokens in double); r, k (heads x dim) and v (heads x vdim) are columns of ``proj``."""
     _need(proj, "proj", None, 2); _need(decay, "decay", torch.float32, 2); _need(state, "state", torch.float32, 2)

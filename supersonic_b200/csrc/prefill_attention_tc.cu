@@ -550,7 +550,8 @@ SSB_API int ssb_attention_prefill_tc(const void* q, int ldq, int n_rows_q, const
     const int sms = ssb_sm_count();
     // One tile a unit while pairs would leave SMs without a block: us for a prompt of (query heads, size, tokens) with two tiles and
     // one, (24, 128, 700) 21.1 and 18.9, (32, 128, 512) 19.1 and 16.3, 1,000 (128 pairs) 27.1 and 25.1, 300 behind 8,192 152 and
-    // 133; beyond, the shared fetch wins: 2,048 (256 pairs) 45.8 and 50.0, 4,096 138 and 147.  Same results either way.
+    // 133; beyond, the shared fetch wins: 2,048 (256 pairs) 45.8 and 50.0, 4,096 138 and 147.  The same bits either way: a tile's
+    // turns begin where its pair's do.
     const int tiles = (long long)n_kv * n_seqs * pairs <= sms ? 1 : 2;
     const int levels = tiles == 1 ? ((max_new + FT_BM - 1) / FT_BM) * group : pairs;
 #define SSB_FT(HD_, T_) do { \

@@ -651,8 +651,8 @@ sample_cluster_kernel(const float* __restrict__ logits, long long ld, int vocab,
 // over the whole row in all blocks, its keys read again in every pass.
 // The cuts, the weights and the order in which the draw adds them are those of sample_cluster_kernel: the same token.
 // Bound by the latencies of its phases (three meetings of the cluster and a dozen of a block), not by the row's bytes.  64
-// rows of 128,256 tokens, k 40, p 0.9: 25.5 us where radix passes over 350 candidates in every block and a draw in all of them
-// took 45; one row 20 and 30.
+// rows of 128,256 tokens, k 40, p 0.9, in captured launches: 25.5 us where radix passes over 350 candidates in every block and a
+// draw in all of them took 45; one row 13.
 constexpr int TOP_CAP = 2 * SC_THREADS;                  // candidates of a row: two a thread
 constexpr int TOP_MAX_K = 64;
 constexpr int TOP_GROUPS = 128;                          // groups of threads whose maxima a block sorts
@@ -1013,9 +1013,9 @@ SSB_API int ssb_sample(const float* logits, long long ld, int n_rows, int vocab,
                 logits, ld, vocab, 1.0f / temperature, slots, rng_state, out, drawn_u);
             return ssb_launch_status();
         }
-        // us with the row held and from candidates, k 40: both cuts (p 0.9), 1 row of 8,192, 32,000 and 128,256 tokens 28, 32, 45 and
-        // 16, 18, 20, 64 rows 49, 55, 106 and 23, 25, 33; the top-k cut alone, 1 row 16, 19, 29 and 16, 16, 20, 64 rows 25, 29, 66 and
-        // 22, 25, 31.
+        // us with the row held and from candidates, k 40, in captured launches: both cuts (p 0.9), 1 row of 8,192, 32,000 and 128,256
+        // tokens 22, 24, 36 and 11, 11, 13, 64 rows 44, 48, 100 and 18, 19, 25; the top-k cut alone, 1 row 11, 13, 20 and 10, 11, 12, 64
+        // rows 19, 23, 58 and 17, 19, 24.
         if (form == 2 || (form == 0 && top_k > 0 && top_k <= TOP_MAX_K)) {
             sample_top_kernel<<<dim3(SC_CTAS, n_rows), SC_THREADS, 0, stream>>>(
                 logits, ld, vocab, 1.0f / temperature, top_k, top_p, slots, rng_state, out, drawn_u);
