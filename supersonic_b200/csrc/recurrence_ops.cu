@@ -73,18 +73,22 @@ gated_linear_carry_kernel(float* __restrict__ state, float* __restrict__ sums, c
     state[(size_t)slot * per + e] = cur;
 }
 
+// Shared memory of which one block fits an SM, and two
+constexpr int TW_ALONE = 116 * 1024, TW_PAIR = 70 * 1024;
+
 // A token a sequence (a decode step): the state passes through once, row by row, and no lane owns a tile of it.  A block takes
 // COLS value columns of a head, four a lane; its warps share the rows, eight accesses in flight a lane, and the sums over the
-// rows meet in shared memory.  The decays are made here too.  (The walk loads a tile, then stores it, one block an SM: 64
-// sequences of 4 heads of 256 x 512, 268 MB of state in and out, took 112 us and a launch for the decays.)  A sequence may bring
-// several tokens (another none): it takes them one after another.
+// rows (in a tree, so that they are no further from 64 bits than the walk's) meet in shared memory.  The decays are made here
+// too.  (The walk loads a tile, then stores it, one block an SM: 64 sequences of 4 heads of 256 x 512, 268 MB of state in and out,
+// took 112 us and a launch for the decays.)  A sequence may bring several tokens (another none): it takes them one after another.
 template <typename T, int COLS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 gated_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off, const float* __restrict__ z, int ldz,
                   const float* __restrict__ z_bias, float inv_tau, float q_scale, float* __restrict__ state,
                   const int* __restrict__ cu_new, const int* __restrict__ seq_slot, float* __restrict__ out, int ldo, int n_heads,
                   int dim, int vdim) {
     constexpr int LR = COLS / 4, RW = 32 / LR, PARTS = 8 * RW, DEEP = 8;         // lanes a row, rows of a warp's access
+    constexpr int ACC = COLS >= 128 ? 2 : 1;               // sums of a lane
     __shared__ float k_s[SCAN_MAX_DIM], q_s[SCAN_MAX_DIM], d_s[SCAN_MAX_DIM];
     __shared__ __align__(16) float o_s[PARTS][COLS];
     const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -108,7 +112,7 @@ gated_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, int 
             q_s[i] = ssb_to_float(row[q_off + h * dim + i]) * q_scale;
             d_s[i] = expf(log_sigmoid(z[(size_t)t * ldz + h * dim + i] + z_bias[h * dim + i]) * inv_tau);
         }
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f), o = v;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f), o[ACC] = {};
         if (mine) {
             const T* vp = row + v_off + (size_t)h * vdim + j;
             v = make_float4(ssb_to_float(vp[0]), ssb_to_float(vp[1]), ssb_to_float(vp[2]), ssb_to_float(vp[3]));
@@ -129,17 +133,27 @@ gated_step_kernel(const T* __restrict__ proj, int ld, int q_off, int k_off, int 
                     const float4 x = make_float4(fmaf(d, s[r].x, k * v.x), fmaf(d, s[r].y, k * v.y), fmaf(d, s[r].z, k * v.z),
                                                  fmaf(d, s[r].w, k * v.w));
                     *reinterpret_cast<float4*>(S + (size_t)i * vdim) = x;
-                    o = make_float4(fmaf(x.x, q, o.x), fmaf(x.y, q, o.y), fmaf(x.z, q, o.z), fmaf(x.w, q, o.w));
+                    float4& sum = o[r % ACC];
+                    sum = make_float4(fmaf(x.x, q, sum.x), fmaf(x.y, q, sum.y), fmaf(x.z, q, sum.z), fmaf(x.w, q, sum.w));
                 }
             }
         }
-        *reinterpret_cast<float4*>(&o_s[part][at]) = o;
+#pragma unroll
+        for (int half = ACC / 2; half > 0; half /= 2)
+#pragma unroll
+            for (int r = 0; r < half; ++r)
+                o[r] = make_float4(o[r].x + o[r + half].x, o[r].y + o[r + half].y, o[r].z + o[r + half].z, o[r].w + o[r + half].w);
+        *reinterpret_cast<float4*>(&o_s[part][at]) = o[0];
         __syncthreads();
         for (int c = tid; c < COLS; c += 256) {
-            float sum = 0.f;
+            float sum[PARTS];
 #pragma unroll
-            for (int p = 0; p < PARTS; ++p) sum += o_s[p][c];
-            if (blockIdx.z * COLS + c < vdim) out[(size_t)t * ldo + (size_t)h * vdim + blockIdx.z * COLS + c] = sum;
+            for (int p = 0; p < PARTS; ++p) sum[p] = o_s[p][c];
+#pragma unroll
+            for (int half = PARTS / 2; half > 0; half /= 2)
+#pragma unroll
+                for (int p = 0; p < half; ++p) sum[p] += sum[p + half];
+            if (blockIdx.z * COLS + c < vdim) out[(size_t)t * ldo + (size_t)h * vdim + blockIdx.z * COLS + c] = sum[0];
         }
         __syncthreads();
     }
@@ -158,8 +172,8 @@ static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off,
 // one go.  max_chunks = ceil(longest run of new tokens / chunk).  ``sums`` (places x n_heads x dim x vdim floats) and ``decays``
 // (places x n_heads x dim) hold so many (sequence, chunk) pairs at a time; with fewer than n_seqs x max_chunks the step
 // takes several passes, over sequences and over runs of chunks, and every sum is the same.  form: lanes that share a column's
-// rows, 1: the same for steps of any size (16, above 128 channels 32), 2: 32 (dim above 64), 3: a token at a time (whole runs, states in 16-byte pieces), 0: by the step's sizes; the
-// sums over the rows differ in order.
+// rows, 1: the same for steps of any size (16, above 128 channels 32), 2: 32 (dim above 64), 3: a token at a time (whole runs,
+// states in 16-byte pieces), 0: by the step's sizes; the sums over the rows differ in order.
 SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off,
                                   float* z, int ldz, const float* z_bias, float tau, float q_scale,
                                   float* state, const int* cu_new, const int* seq_slot, float* out, int ldo,
@@ -179,9 +193,14 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
         // 128 columns a block where that gives the SMs two blocks each
         const bool wide = (long long)n_seqs * n_heads * ((vdim + 127) / 128) >= 2 * ssb_sm_count();
         const dim3 grid(n_seqs, n_heads, wide ? (vdim + 127) / 128 : (vdim + 31) / 32);
+        // one block an SM, or two, where that is all it takes: more would share one while others stand still
+        const long long blocks = (long long)grid.x * grid.y * grid.z;
+        const size_t smem = blocks <= ssb_sm_count() ? TW_ALONE : blocks <= 2 * ssb_sm_count() ? TW_PAIR : 0;
 #define SSB_GS(T, COLS)                                                                                                       \
     do {                                                                                                                      \
-        const int st = ssb_launch(gated_step_kernel<T, COLS>, grid, dim3(256), 0, stream, pdl != 0, (const T*)proj, ld, q_off, k_off, \
+        const cudaError_t e = cudaFuncSetAttribute(gated_step_kernel<T, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, TW_ALONE); \
+        if (e != cudaSuccess) return (int)e;                                                                                  \
+        const int st = ssb_launch(gated_step_kernel<T, COLS>, grid, dim3(256), smem, stream, pdl != 0, (const T*)proj, ld, q_off, k_off, \
                                   v_off, (const float*)z, ldz, z_bias, 1.0f / tau, q_scale, state, cu_new, seq_slot, out, ldo, n_heads, \
                                   dim, vdim);                                                                                 \
         return st ? st : ssb_launch_status();                                                                                 \
@@ -212,8 +231,8 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
 // (packed_f32.cuh; each half rounds as the scalar one does).  Four tokens' sums over the lanes are taken together: of the 16
 // values a lane holds it hands on the half that the other keeps, four times, 15 shuffles where a token alone takes 5.  Eight
 // tokens are staged per barrier, in two buffers, while the next eight are on their way from memory.  4 heads of 256 x 512 and
-// 2,048 tokens 530 us in scalar multiply-adds and 5 shuffles a token, 455 so; 8 x 300 tokens 442 and 340.  Bound by what 8 to 16
-// warps an SM hide of the shared-memory reads (FMA pipe 36 %, issue slots 34 %).
+// 2,048 tokens 530 us in scalar multiply-adds and 5 shuffles a token, 455 so; 8 x 300 tokens 442 and 340.  Bound by what 16 warps an
+// SM hide of the shared-memory reads (multiply-add pipe 26 %, issue slots 50 %).
 //   OUT = false: chunk sums, from zero, with the product of the chunk's decays;
 //   OUT = true: outputs from the state at the start (the slot's, or what the carry kernel left for the chunk).
 // GATED: the gated linear attention at the top of this file on the same tiles, S <- a S + k v with decays that a kernel before
@@ -466,8 +485,8 @@ static int launch_tied_pass(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
     constexpr int DIMP = 64 * R4, COLS = NT / 32 * (128 / RL);
     // A block that may have an SM to itself asks for more than half of its shared memory: two would share one while others stand
     // still (us, 4 heads of 128 x 256: 190 tokens 43 and 33, 4 x 150 47 and 39; of 256 x 512, 20 tokens 17.1 and 13.6)
-    constexpr size_t needed = (size_t)TW_TOKENS * ((GATED ? 6 : 4) * DIMP + 4 * COLS) * sizeof(float), alone = 116 * 1024,
-                     most = needed < alone ? alone : needed;
+    constexpr size_t needed = (size_t)TW_TOKENS * ((GATED ? 6 : 4) * DIMP + 4 * COLS) * sizeof(float),
+                     most = needed < TW_ALONE ? TW_ALONE : needed;
     const long long items = a.chunk > 0 ? (long long)n_seqs * a.max_chunks : n_seqs;
     const dim3 grid((unsigned)items, a.n_heads, (a.vdim + COLS - 1) / COLS);
     if (items > 0x7fffffffll || grid.y > 65535 || grid.z > 65535 || n_seqs > 65535) return SSB_ERR_BAD_SIZE;
@@ -546,7 +565,8 @@ static int gated_walk(const void* proj, int ld, int dtype, int q_off, int k_off,
 
 // proj [T, ld] holds q and the gate's pre-activation (n_heads x dim each) and v (n_heads x vdim) from the given columns;
 // z_bias and lower [n_heads x dim]; state [slots, n_heads, dim, vdim] float32.  norm_w null: out [T, ldo] float32 gets o;
-// else (vdim up to 128, up to 64 where dim is above 128) y [T, ldy] of proj's type gets the normed heads.  chunk, max_chunks, min_new, places, sums and decays as ssb_gated_linear_scan's.
+// else (vdim up to 128, up to 64 where dim is above 128) y [T, ldy] of proj's type gets the normed heads.  chunk, max_chunks,
+// min_new, places, sums and decays as ssb_gated_linear_scan's.
 SSB_API int ssb_tied_scan(const void* proj, int ld, int dtype, int q_off, int f_off, int v_off, const float* z_bias,
                           const float* lower, float* state, const int* cu_new, const int* seq_slot, float* out, int ldo,
                           const float* norm_w, float eps, void* y, int ldy, int n_seqs, int n_tokens, int n_heads, int dim,
@@ -1131,8 +1151,8 @@ matrix_state_scan_async_kernel(const bf16* __restrict__ proj, int ld, int r_off,
 }
 
 // proj [T, ld]: r, k (n_heads x dim) and v (n_heads x vdim) from the given columns; decay [T, ldd] float32
-// (n_heads x dim), for float32 rows their logarithms (what the prepare kernel leaves in either case); kind 0 (delta rule): unit [T, ldu] float32 = [u | a * u]; kind 1: bonus [n_heads x dim]
-// float32 or null; state [slots, n_heads, vdim, dim] float32 (a value column's key rows lie together, so that the eight
+// (n_heads x dim), for float32 rows their logarithms (what the prepare kernel leaves in either case); kind 0 (delta rule): unit
+// [T, ldu] float32 = [u | a * u]; kind 1: bonus [n_heads x dim] float32 or null; state [slots, n_heads, vdim, dim] float32 (a value column's key rows lie together, so that the eight
 // lanes of a column read and write it in one piece); out [T, ldo] float32 (n_heads x vdim).
 SSB_API int ssb_matrix_state_scan(const void* proj, int ld, int dtype, int r_off, int k_off, int v_off,
                                   const float* decay, int ldd, int kind, const float* unit, int ldu, const float* bonus,
