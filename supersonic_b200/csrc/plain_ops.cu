@@ -667,8 +667,9 @@ attention_staged_kernel(const float* __restrict__ q, int ldq, const float* __res
 // Where rows are many: a chunk's keys come in slices of SL dims, then its values in as many bytes a time, through a ring of STAGES
 // of them that runs across chunks, 32 to 96 KB where whole chunks take 66 (heads of 64) or 132 (128), so that two to six blocks
 // share an SM.  A block that is alone on its SM takes longer so: a meeting of the block and the addresses of a fetch for every slice
-// (one sequence of 1,000 tokens, 32 heads of 128, 56 us and 46).  Bound by what L2 delivers where rows are many (64 sequences of
-// 4,000 tokens, 32 heads of 128: 8.4 GB in 1,224 us), by a chunk's chain of products and meetings where few.
+// (one sequence of 1,000 tokens, 32 heads of 128, 56 us and 46).  Bound by the issue slots where rows are many (64 sequences of
+// 1,000 tokens, 32 heads over 8 of 128: 77 % busy, 47 % of the shared memory's cycles, 9.2 TB/s from L2), by a chunk's chain of
+// products and meetings where few.
 template <bool ROPE, int SL, int STAGES>
 __global__ void __launch_bounds__(ATT_THREADS)
 attention_ring_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
