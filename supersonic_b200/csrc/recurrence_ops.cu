@@ -198,8 +198,10 @@ SSB_API int ssb_gated_linear_scan(const void* proj, int ld, int dtype, int q_off
         const size_t smem = blocks <= ssb_sm_count() ? TW_ALONE : blocks <= 2 * ssb_sm_count() ? TW_PAIR : 0;
 #define SSB_GS(T, COLS)                                                                                                       \
     do {                                                                                                                      \
-        const cudaError_t e = cudaFuncSetAttribute(gated_step_kernel<T, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, TW_ALONE); \
-        if (e != cudaSuccess) return (int)e;                                                                                  \
+        if (smem > 0) {                                                                                                       \
+            const cudaError_t e = cudaFuncSetAttribute(gated_step_kernel<T, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, TW_ALONE); \
+            if (e != cudaSuccess) return (int)e;                                                                              \
+        }                                                                                                                     \
         const int st = ssb_launch(gated_step_kernel<T, COLS>, grid, dim3(256), smem, stream, pdl != 0, (const T*)proj, ld, q_off, k_off, \
                                   v_off, (const float*)z, ldz, z_bias, 1.0f / tau, q_scale, state, cu_new, seq_slot, out, ldo, n_heads, \
                                   dim, vdim);                                                                                 \
@@ -494,7 +496,7 @@ static int launch_tied_pass(const TiedArgs& a, int n_seqs, bool pdl, cudaStream_
     const size_t smem = (long long)grid.x * grid.y * grid.z <= ssb_sm_count() ? most : needed;
     auto sums = tied_walk_kernel<T, R4, NT, false, GATED, RL, SM_BLOCKS>;
     auto outs = tied_walk_kernel<T, R4, NT, true, GATED, RL, SM_BLOCKS>;
-    {
+    if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(outs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         if (e != cudaSuccess) return (int)e;
@@ -1152,7 +1154,8 @@ matrix_state_scan_async_kernel(const bf16* __restrict__ proj, int ld, int r_off,
 
 // proj [T, ld]: r, k (n_heads x dim) and v (n_heads x vdim) from the given columns; decay [T, ldd] float32
 // (n_heads x dim), for float32 rows their logarithms (what the prepare kernel leaves in either case); kind 0 (delta rule): unit
-// [T, ldu] float32 = [u | a * u]; kind 1: bonus [n_heads x dim] float32 or null; state [slots, n_heads, vdim, dim] float32 (a value column's key rows lie together, so that the eight
+// [T, ldu] float32 = [u | a * u]; kind 1: bonus [n_heads x dim] float32 or null; state [slots, n_heads, vdim, dim] float32 (a value
+// column's key rows lie together, so that the eight
 // lanes of a column read and write it in one piece); out [T, ldo] float32 (n_heads x vdim).
 SSB_API int ssb_matrix_state_scan(const void* proj, int ld, int dtype, int r_off, int k_off, int v_off,
                                   const float* decay, int ldd, int kind, const float* unit, int ldu, const float* bonus,
