@@ -770,7 +770,9 @@ static inline bool gemm_f32_ok(const void* A, int lda, long long a_batch, const 
 // 51 and 34; 64 x 16384 219 by chunks and 191 with tiles of 64; 128 x 3072 95 by chunks, 114 with tiles of 64; 300 x 2048 155 by
 // chunks, 181 with 128 x 64; 300 x 3072 182 with 128 x 64, 189 with 64 x 64, 217 with 128 x 128; 500 x 3072 217 with 128 x 128, 266
 // with 64 x 64; 500 x 2048 181 with 128 x 64, 217; 1000 x 2048 217 and 318.  K 64: 300 x 64 5.3 with 16 rows, 6.5 with tiles of
-// 64; 16 x 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.
+// 64; 16 x 8192 14.3 and 6.1.  16 x 128256, k 256 155 and 141, k 512 171 and 274.  Blocks of 16 rows that stay for many waves take 9.3
+// a wave and 4.2 us in all (of whole chunks; k 1500 is 10 % above that): 32 x 6144, k 4096 146 and 153 with 32 x 32, 32 x 3072 75 and
+// 78, 33 x 5120, k 8192 330 and 366 by chunks of 64 x 16, 48 x 10240, k 5120 390 and 382.
 static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
     const long long sms = ssb_sm_count(), chunks = (K + 15) / 16, turns = (K + 511) / 512;
     const auto waves = [&](int rows, int cols) {
@@ -784,6 +786,10 @@ static inline int gemm_f32_form(int n_batch, int M, int N, int K) {
     long long cost[6] = {32 * turns * (first + each * waves(rows, 16)), 3000 + 10 * chunks * (30 + 60 * waves(64, 64)),
                          3000 + 10 * chunks * (30 + 115 * waves(128, 64)), 3000 + 10 * chunks * 167 * waves(128, 128),
                          3000 + 10 * parts * 24 * waves(64, 16), 3000 + 10 * parts * 29 * waves(32, 32)};
+    if (rows == 16 && n_batch == 1 && K % 16 == 0) {
+        const long long steady = 4200 + 32 * turns * 93 * waves(16, 16);
+        if (steady < cost[0]) cost[0] = steady;
+    }
     if (walk) {
         const int width = gf_walk_width(N), turn = width == 1 ? 1300 : width == 2 ? 800 : M <= 1 ? 650 : M <= 2 ? 700 : 850;
         const long long held = sms * GF_WALK_WARPS, rounds = ((long long)((N + width - 1) / width) * n_batch + held - 1) / held;

@@ -58,6 +58,12 @@ def test_float32_products_by_chunks_are_the_general_kernels_bit_for_bit(m, n, k,
     test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, accumulate)
 
 
+# more than 16 rows whose groups of 16 stay for several waves: partial groups, a last tile that is not full
+@pytest.mark.parametrize("m,n,k", [(17, 3071, 2048), (32, 6144, 1024), (33, 5120, 8192), (80, 2558, 1024), (300, 512, 2544)])
+def test_float32_products_of_groups_that_stay_are_the_general_kernels_bit_for_bit(m, n, k):
+    test_float32_products_are_the_general_kernels_bit_for_bit(m, n, k, True)
+
+
 @pytest.mark.parametrize("T,H,K,N", [(1, 6, 64, 128), (133, 3, 128, 48), (70, 4, 24, 72), (8, 2, 16, 260), (1000, 2, 68, 5000)])
 def test_float32_head_products_are_the_general_kernels_bit_for_bit(T, H, K, N):
     x, w = rnd(T, H, K + 4, seed=T)[:, :, :K], rnd(H, N, K, seed=N)
